@@ -159,24 +159,34 @@ struct EnergyArgs {
   double* pair_tab;        // [3][np * np] per template bead pair (i, j): the Yukawa size factor,
                            // sbar^6, the attractive LJ shift at ecut (k_energy_tables)
   unsigned char* att_tab;  // [np * np] 1 = attractive by the directed LJ table
-  // cell grid of the pair pass (nc cells per axis, nc >= 3; nc = 0: every pair j > i is visited)
-  int nc;
-  int* cell_count;         // [nc^3] (zeroed before the count)
-  int* cell_start;         // [nc^3 + 1]
-  int* cell_fill;          // [nc^3] (zeroed before the scatter)
-  int* cell_beads;         // [n] system-local bead indices, ascending within each cell
-  int* bead_cell;          // [n]
+  const double* w;         // [np] DH weights q e^(kappa sigma/2) / (1 + kappa sigma/2) sqrt(lb)
+  double el_shift;         // e^(-kappa ecut_el) / ecut_el (with a DH cut-off)
+  double exp_scale;        // -kappa 64 / ln2
+  double inv_ecut3;        // 1 / ecut^3
+  int spc;                 // subunits per CTA of k_energy_sub
+  int4* sph;               // [subunits] centre bead (high words) and bounding radius (float bits)
+  int* rmax;               // largest bounding radius (float bits), zero between calls
+  double* partials;        // [kTotalCtas][7]
+  unsigned int* ticket;    // CTAs of k_energy_totals done, zero between calls
+  // the grid of subunit centres (large systems only)
+  const int* sub_cell_start = nullptr;
+  const int* cell_subs = nullptr;
   // encapsulation big beads of the system: fixed-point positions [3][total], the big-bead parts
-  // of ne and ce per subunit bead [n] and their sums ([2]: lj, electrostatic)
+  // of ne and ce per subunit bead [n]
   const long long* bb_fx = nullptr;
   int bb_total = 0;
   double* ne_bb = nullptr; double* ce_bb = nullptr;
-  double* bb_totals = nullptr;
 };
+constexpr int kTotalThreads = 256, kTotalCtas = 304;  // k_energy_totals: two CTAs per SM
+int energy_sub_per_cta(int np);
+size_t energy_sub_smem(const TplLayout& L, int spc);
+cudaError_t set_energy_smem(const TplLayout& L);
+bool energy_needs_cells(int n_sub);
 
 void launch_cells_count(const CellArgs& a, int grid, int block, cudaStream_t s);
 void launch_cells_scan(const CellArgs& a, cudaStream_t s);
 void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s);
+void launch_cells_sort(const CellArgs& a, cudaStream_t s);
 void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s);
 void launch_pairs(const PairArgs& a, int n_sub, size_t smem, cudaStream_t s);
 // k_pairs' chunk of candidates staged together, and its dynamic shared memory

@@ -97,6 +97,20 @@ __global__ void k_cells_scatter(CellArgs a) {
   a.cell_subs[a.cell_start[a.sub_cell[s]] + a.sub_rank[s]] = s;
 }
 
+// Each cell's subunits in ascending order (the scatter leaves them in the order of its atomics),
+// for callers that sum over them in cell order.  A few subunits per cell: insertion sort.
+__global__ void k_cells_sort(CellArgs a) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= a.total_cells) return;
+  int* b = a.cell_subs + a.cell_start[c];
+  const int m = a.cell_start[c + 1] - a.cell_start[c];
+  for (int i = 1; i < m; i++) {
+    const int v = b[i];
+    int k = i - 1;
+    for (; k >= 0 && b[k] > v; k--) b[k + 1] = b[k];
+    b[k + 1] = v;
+  }
+}
 
 // Margin (in length^2) within which the float test defers to the exact double test.
 __device__ __forceinline__ float pair_margin(float nl2) { return 1e-4f * (1.0f + nl2); }
@@ -531,6 +545,7 @@ void launch_cells_scan(const CellArgs& a, cudaStream_t s) { k_cells_scan<<<a.n_s
 void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s) {
   k_cells_scatter<<<grid, block, 0, s>>>(a);
 }
+void launch_cells_sort(const CellArgs& a, cudaStream_t s) { k_cells_sort<<<(a.total_cells + 127) / 128, 128, 0, s>>>(a); }
 void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s) {
   (void)grid;
   (void)block;

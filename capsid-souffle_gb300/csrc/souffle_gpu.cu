@@ -256,11 +256,16 @@ souffle_status upload(souffle_gpu_system* h) {
   // per-system DH weights w = q exp(kappa s/2) / (1 + kappa s/2) sqrt(lb): w_i w_j reproduces
   // q_i q_j lb exp(kappa shc) / ((1 + kappa s_i/2)(1 + kappa s_j/2)) of src/forces.cpp:98-103
   std::vector<float> w(h->n_sys * T.np);
+  std::vector<double> wd(h->n_sys * T.np);
   for (int s = 0; s < h->n_sys; s++) {
     const double k = h->prm[s].kappa, lb = h->prm[s].lb;
-    for (int i = 0; i < T.np; i++)
-      w[s * T.np + i] = (float)(T.q[i] * std::exp(k * T.sigma[i] / 2) / (1 + k * T.sigma[i] / 2) * std::sqrt(lb));
+    for (int i = 0; i < T.np; i++) {
+      wd[s * T.np + i] = T.q[i] * std::exp(k * T.sigma[i] / 2) / (1 + k * T.sigma[i] / 2) * std::sqrt(lb);
+      w[s * T.np + i] = (float)wd[s * T.np + i];
+    }
   }
+  CUDA_TRY(h->dh_wd.alloc(wd.size()));
+  CUDA_TRY(cudaMemcpy(h->dh_wd.p, wd.data(), wd.size() * sizeof(double), cudaMemcpyHostToDevice));
   CUDA_TRY(h->dh_w.alloc(w.size()));
   CUDA_TRY(cudaMemcpy(h->dh_w.p, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice));
 
@@ -319,7 +324,8 @@ CellArgs cell_args(souffle_gpu_system* h) {
   return a;
 }
 
-void launch_candidates_all(souffle_gpu_system* h) {
+// the grid of subunit centres at the current positions
+void launch_subunit_cells(souffle_gpu_system* h) {
   cudaStream_t st = h->stream;
   CellArgs c = cell_args(h);
   cudaMemsetAsync(h->cell_count.p, 0, sizeof(int) * h->total_cells, st);
@@ -327,6 +333,13 @@ void launch_candidates_all(souffle_gpu_system* h) {
   launch_cells_count(c, gb, tb, st);
   launch_cells_scan(c, st);
   launch_cells_scatter(c, gb, tb, st);
+}
+
+void launch_candidates_all(souffle_gpu_system* h) {
+  cudaStream_t st = h->stream;
+  CellArgs c = cell_args(h);
+  launch_subunit_cells(h);
+  const int tb = 128, gb = (h->S + tb - 1) / tb;
   CandArgs ca{};
   ca.c = c;
   ca.pos32 = h->pos32.p;
@@ -731,6 +744,13 @@ souffle_status souffle_gpu_create(const souffle_template* tpl, const souffle_par
     CUDA_TRY(cudaMemset(h->bd_fran.p, 0, sizeof(long long) * 3 * N));
   }
   CUDA_TRY(h->e_tot.alloc(8));
+  int max_sub = 0;
+  for (int k = 0; k < n_systems; k++) max_sub = std::max(max_sub, params[k].n_subunits);
+  CUDA_TRY(h->e_sph.alloc(max_sub));
+  CUDA_TRY(h->e_part.alloc(7 * kTotalCtas));
+  CUDA_TRY(h->e_scr.alloc(2));
+  CUDA_TRY(cudaMemset(h->e_scr.p, 0, 2 * sizeof(int)));
+  CUDA_TRY(set_energy_smem(L));
   CUDA_TRY(cudaMemset(h->intra_mask.p, 0, sizeof(unsigned int) * (size_t)h->S * np * L.words));
   CUDA_TRY(cudaMemset(h->inter_count.p, 0, sizeof(int) * N));
   CUDA_TRY(cudaMemset(h->force.p, 0, sizeof(long long) * 3 * N));
@@ -1115,7 +1135,6 @@ souffle_status souffle_gpu_energies(souffle_gpu_system* h, int32_t system, souff
     a.bb_total = (int)(h->bb_fx.n / 3);
     a.ne_bb = h->e_bead.p + 5 * (size_t)n;
     a.ce_bb = h->e_bead.p + 6 * (size_t)n;
-    a.bb_totals = h->e_tot.p + 5;
   }
   {
     const size_t np2 = (size_t)h->tpl.np * h->tpl.np;
@@ -1123,21 +1142,21 @@ souffle_status souffle_gpu_energies(souffle_gpu_system* h, int32_t system, souff
     if (h->e_att_tab.n != np2) CUDA_TRY(h->e_att_tab.alloc(np2));
     a.pair_tab = h->e_pair_tab.p;
     a.att_tab = h->e_att_tab.p;
-    // cell grid for the pair pass: cells at least the reach of every pair term wide (with a
-    // margin), at most 128 per axis; none without a DH cut-off (every pair then counts)
-    const double reach = std::max(std::max(p.ecut, p.ecut_el), 1.12246205 * a.sigma_max) * 1.01;
-    const int nc = p.ecut_el > 0 ? (int)std::min(128.0, std::floor(p.box / reach)) : 0;
-    a.nc = nc >= 3 ? nc : 0;
-    if (a.nc) {
-      const size_t ncell = (size_t)a.nc * a.nc * a.nc;
-      const size_t need = 3 * ncell + 1 + 2 * (size_t)n;
-      if (h->e_cells.n < need) CUDA_TRY(h->e_cells.alloc(need));
-      a.cell_count = h->e_cells.p;
-      a.cell_fill = h->e_cells.p + ncell;
-      a.cell_start = h->e_cells.p + 2 * ncell;
-      a.cell_beads = h->e_cells.p + 3 * ncell + 1;
-      a.bead_cell = a.cell_beads + n;
-    }
+  }
+  a.w = h->dh_wd.p + (size_t)system * h->tpl.np;
+  a.el_shift = p.ecut_el > 0 ? std::exp(-p.kappa * p.ecut_el) / p.ecut_el : 0.0;
+  a.exp_scale = -p.kappa * (64.0 / 0.69314718055994530942);
+  a.inv_ecut3 = 1.0 / (p.ecut * p.ecut * p.ecut);
+  a.spc = energy_sub_per_cta(h->tpl.np);
+  a.sph = h->e_sph.p;
+  a.rmax = h->e_scr.p;
+  a.ticket = reinterpret_cast<unsigned int*>(h->e_scr.p + 1);
+  a.partials = h->e_part.p;
+  if (p.ecut_el > 0 && energy_needs_cells(P.n_sub)) {
+    launch_subunit_cells(h);
+    launch_cells_sort(cell_args(h), h->stream);  // the sums do not depend on scheduling
+    a.sub_cell_start = h->cell_start.p;
+    a.cell_subs = h->cell_subs.p;
   }
   launch_energies(a, n, h->stream);
   CUDA_TRY(cudaGetLastError());

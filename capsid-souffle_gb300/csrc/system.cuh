@@ -81,7 +81,10 @@ struct souffle_gpu_system {
   DevBuf<int> type_d, lj_d;
   DevBuf<double> e_bead, e_tot, e_pair_tab;
   DevBuf<unsigned char> e_att_tab;
-  DevBuf<int> e_cells;  // the energy pass's cell grid: count, start, fill (3 nc^3 + 1), beads, bead cells (2 n)
+  DevBuf<double> dh_wd;   // [n_sys * np] the DH weights in double
+  DevBuf<int4> e_sph;     // energy pass: the subunits' bounding spheres
+  DevBuf<double> e_part;  // ... partial sums of the totals
+  DevBuf<int> e_scr;      // ... largest radius, finished CTAs (both zero between calls)
   DevBuf<unsigned int> err;
   unsigned int* err_host = nullptr;  // pinned landing word for the error flag's read-back
   // asynchronous snapshots (souffle_gpu_snapshot_enqueue / _wait): per slot a device copy of the
