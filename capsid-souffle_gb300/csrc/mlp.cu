@@ -29,7 +29,7 @@ bool mlp_fused_supported(int n_in, int width, int out_pad);
 cudaError_t mlp_forward_fused(const __nv_bfloat16* x, int ldx, int m_cap, const int* m_dyn, int n_in, int width,
                               const __nv_bfloat16* const w[4], const int ldw[4], int out_pad, const float* const bias[4],
                               float* y, int ldy, unsigned int* err, unsigned int err_bit, cudaStream_t st,
-                              __nv_bfloat16* yb = nullptr);
+                              __nv_bfloat16* yb = nullptr, const float* x32 = nullptr, int n_store = 0);
 }
 
 using namespace souffle;
@@ -516,12 +516,22 @@ souffle_status souffle_mlp_set_params(souffle_mlp* h, const float* host_in, int6
 souffle_status souffle_mlp_forward(souffle_mlp* h, const float* x_dev, int32_t m, float* y_dev) {
   if (!h || !x_dev || !y_dev || m < 1 || m > h->cap) return fail(SOUFFLE_ERR_BAD_INPUT, "bad argument");
   MLP_TRY(cudaSetDevice(h->device));
+  const int L = kLayers - 1;
+  if (mlp_fused_supported(h->n_in, h->width, h->out_pad[L]) && h->n_out % 4 == 0 &&
+      (reinterpret_cast<uintptr_t>(y_dev) & 15) == 0) {
+    // one kernel from the caller's FP32 rows to the caller's FP32 rows (its stores want 16-byte rows)
+    const __nv_bfloat16* w[4] = {h->wb[0].p, h->wb[1].p, h->wb[2].p, h->wb[3].p};
+    const int ldw[4] = {h->in[0], h->in[1], h->in[2], h->in[3]};
+    const float* b[4] = {h->b[0].p, h->b[1].p, h->b[2].p, h->b[3].p};
+    MLP_TRY(mlp_forward_fused(h->act[0].p, h->in_ld[0], m, nullptr, h->n_in, h->width, w, ldw, h->out_pad[L], b, y_dev,
+                              h->n_out, h->err.p, kErrSurrogateBit, h->stream, nullptr, x_dev, h->n_out));
+    return check_gemm_err(h);
+  }
   souffle_status s = pack_input(h, x_dev, m, false);
   if (s != SOUFFLE_OK) return s;
   const float* y = nullptr;
   int ldy = 0;
   MLP_TRY(souffle::mlp_forward_packed_async(h, m, nullptr, h->err.p, h->stream, &y, &ldy));
-  const int L = kLayers - 1;
   k_unpad<<<blocks((long long)m * h->n_out, 256), 256, 0, h->stream>>>(h->y.p, h->out_pad[L], m, h->n_out, y_dev);
   MLP_TRY(cudaGetLastError());
   return check_gemm_err(h);

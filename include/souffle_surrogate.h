@@ -49,7 +49,8 @@ souffle_status souffle_mlp_forward(souffle_mlp* h, const float* x_dev, int32_t m
 souffle_status souffle_mlp_forward_layered(souffle_mlp* h, const float* x_dev, int32_t m, float* y_dev);
 
 /* Benchmark utility: runs the forward pass over the m rows already in the network's input buffer
- * (the last souffle_mlp_forward call's input) iters times back to back on the network's stream,
+ * (whatever the last layered forward, training step or surrogate step left there; the time does
+ * not depend on the values) iters times back to back on the network's stream,
  * fused (1) or layer by layer (0), and reports the mean device time per pass in *us (CUDA
  * events around the launches; no input packing or output unpadding). */
 souffle_status souffle_mlp_profile_forward(souffle_mlp* h, int32_t m, int32_t iters, int32_t fused, double* us);
