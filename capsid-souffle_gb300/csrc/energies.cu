@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
     for (int k = 0; k < L.maxdeg; k++) {
       const int e = a.tpl_i[L.o_bead_edges + l * L.maxdeg + k];
       if (e < 0) break;
-      se += s_edge[s * ne + e];
+      se += s_edge[s * ne + (e & 0xffff)];
     }
     for (int k = 0; k < L.maxrole; k++) {
       const int r = a.tpl_i[L.o_bead_roles + l * L.maxrole + k];

@@ -1,0 +1,497 @@
+// The phases of one force evaluation over a CTA's run of subunits (a work item), shared by the
+// force kernel and the window kernel of forces.cu.
+//
+//   force_setup      template tables and per-item constants into shared memory
+//   force_rel        a bead's packed coordinates relative to its subunit's centre bead
+//   force_prefix     prefix sums of the inter-subunit list lengths
+//   force_terms      everything that depends on positions alone, in chunks of 32 lanes that the
+//                    warps take from a counter: intra-subunit Debye-Hueckel rows, bending quads,
+//                    inter-subunit pairs, edges (the costliest chunks first)
+//   force_gather     per bead: stretching and bending sums
+// Every contribution ends as an exact 2^-32 fixed-point sum in the bead's limbs in shared memory,
+// so the total does not depend on the CTA shape or on scheduling; the FP32 sums inside one
+// contribution have a fixed order (a bead's edges, its bending roles, its even and its odd
+// intra-subunit partners).
+//
+// What bounds them: instruction issue (a third of all instructions were the intra-subunit pairs),
+// and for systems of a wave of CTAs or less the latency of one phase after the other.  So the
+// intra-subunit row is walked densely, an even and an odd partner at a time in packed FP32 (f32x2)
+// registers -- about 15 instructions per directed pair against 33 for extracting partners from the
+// row's bitmask one by one; a pair off the list or beyond the cut-off is dropped by a select --
+// and the independent kinds of work share one phase instead of taking one each.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "kernels.cuh"
+
+namespace souffle {
+
+__device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
+__device__ __forceinline__ float3 operator+(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
+__device__ __forceinline__ float3 operator-(float3 a, float3 b) { return f3(a.x - b.x, a.y - b.y, a.z - b.z); }
+__device__ __forceinline__ float3 operator*(float3 a, float s) { return f3(a.x * s, a.y * s, a.z * s); }
+__device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ float3 cross3(float3 a, float3 b) {
+  return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
+__device__ __forceinline__ float3 dvec(int4 a, int4 b, float unit) {
+  return f3(hi_diff(a.x, b.x, unit), hi_diff(a.y, b.y, unit), hi_diff(a.z, b.z, unit));
+}
+
+// ---- packed FP32: two values per 64-bit register, each operation rounded like its scalar form ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// t / d by a multiplication: magic = ceil(2^32 / d) (0 for d = 1), exact for t < 2^32 / d
+__device__ __forceinline__ int fast_div(int t, unsigned int magic) { return magic ? (int)__umulhi((unsigned int)t, magic) : t; }
+
+// A bead's force component in 2^-32 fixed point kept as three 21-bit limbs in 32-bit words
+// (v = l2 2^42 + l1 2^21 + l0, l0 and l1 in [0, 2^21), l2 signed), so that pair forces can be
+// added with native 32-bit shared-memory atomics: the limb sums stay exact for up to 2^11 adds.
+__device__ __forceinline__ void limbs_add(unsigned int* L, long long v) {
+  atomicAdd(L, (unsigned int)(v & 0x1FFFFF));
+  atomicAdd(L + 1, (unsigned int)((v >> 21) & 0x1FFFFF));
+  atomicAdd(L + 2, (unsigned int)(int)(v >> 42));
+}
+__device__ __forceinline__ long long limbs_value(const unsigned int* L) {
+  const unsigned long long hi = (unsigned long long)(long long)(int)L[2] << 42;
+  return (long long)(hi + ((unsigned long long)L[1] << 21) + (unsigned long long)L[0]);
+}
+
+// true for a non-finite component or one beyond 1e9 in magnitude
+__device__ __forceinline__ bool force_bad(float x, float y, float z) {
+  const float s = fabsf(x) + fabsf(y) + fabsf(z);  // NaN or infinite when a component is
+  return !(s < 3.0e38f) || fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) > 1.0e9f;
+}
+
+// Shared memory of a work item, carved from the CTA's dynamic allocation (16-byte aligned pieces
+// first; force_smem_bytes is its size).
+struct ForceSmem {
+  float4* edge;        // [max_sub ne] length vector, stretching coefficient
+  float4* bend;        // [max_sub nb 4] bending contributions
+  int4* pos;           // [max_sub np] high words
+  float* rel;          // [max_sub npp 8] packed partners: (x0, x1, y0, y1, z0, z1, w0, w1) per two beads
+  long long* red;      // [4 warps]
+  unsigned int* F;     // force limbs, 9 per bead
+  int* pref;           // prefix sums of the inter-subunit list lengths
+  float* tpl_f;
+  int* tpl_i;
+  float* w;            // [np] DH weights
+};
+__device__ __forceinline__ ForceSmem force_smem(unsigned char* base, const ForceArgs& a, int warps) {
+  const TplLayout& L = a.L;
+  ForceSmem m;
+  const int npp = (L.np + 1) >> 1;
+  m.edge = reinterpret_cast<float4*>(base);
+  m.bend = m.edge + a.max_sub * L.ne;
+  m.pos = reinterpret_cast<int4*>(base + force_tile_bytes(a.max_sub, L.ne, L.nbend));
+  m.rel = reinterpret_cast<float*>(m.pos + a.max_sub * L.np);
+  m.red = reinterpret_cast<long long*>(m.rel + 8 * a.max_sub * npp);
+  m.F = reinterpret_cast<unsigned int*>(m.red + 4 * warps);
+  m.pref = reinterpret_cast<int*>(m.F + force_slot_len(a.max_sub * L.np));
+  m.tpl_f = reinterpret_cast<float*>(m.pref + force_pref_len(a.max_sub * L.np));  // [n_float], n_float % 4 == 0
+  m.tpl_i = reinterpret_cast<int*>(m.tpl_f + L.n_float);                          // [n_int], n_int % 4 == 0
+  m.w = reinterpret_cast<float*>(m.tpl_i + L.n_int);
+  return m;
+}
+
+// Template tables and the system's DH weights.
+__device__ __forceinline__ void force_setup(const ForceArgs& a, const WorkItem& w, const ForceSmem& m) {
+  const TplLayout& L = a.L;
+  const int4* gi = reinterpret_cast<const int4*>(a.tpl_i);
+  int4* si = reinterpret_cast<int4*>(m.tpl_i);
+  for (int t = threadIdx.x; t < (L.n_int >> 2); t += blockDim.x) si[t] = __ldg(gi + t);
+  const float4* gf = reinterpret_cast<const float4*>(a.tpl_f);
+  float4* sf = reinterpret_cast<float4*>(m.tpl_f);
+  for (int t = threadIdx.x; t < (L.n_float >> 2); t += blockDim.x) sf[t] = __ldg(gf + t);
+  for (int t = threadIdx.x; t < L.np; t += blockDim.x) m.w[t] = __ldg(&a.dh_w[w.sys * L.np + t]);
+}
+
+// The packed relative coordinates of bead t (subunit s, local index l) at high words p, centre
+// bead at c, DH weight wt; an odd subunit's last slot is filled with the bead itself (its partner
+// bit is never set).
+__device__ __forceinline__ void force_rel(const ForceSmem& m, int np, int s, int l, int4 p, int4 c, float wt, float unit) {
+  float* r = m.rel + 8 * (s * ((np + 1) >> 1) + (l >> 1)) + (l & 1);
+  const float x = hi_diff(p.x, c.x, unit), y = hi_diff(p.y, c.y, unit), z = hi_diff(p.z, c.z, unit);
+  r[0] = x;
+  r[2] = y;
+  r[4] = z;
+  r[6] = wt;
+  if (l == np - 1 && !(l & 1)) {
+    r[1] = x;
+    r[3] = y;
+    r[5] = z;
+    r[7] = 0.f;
+  }
+}
+
+// Exclusive prefix sums of the beads' inter-subunit list lengths (pref[nbead] = total): each thread
+// a run of `per` beads, a warp scan, then the warp totals (red is free until the end).  Contains
+// one barrier; the caller's next barrier makes pref visible.
+__device__ __forceinline__ void force_prefix(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int per = (nbead + blockDim.x - 1) / blockDim.x;
+  int my_cnt = 0;
+  for (int i = 0; i < per; i++) {
+    const int b = threadIdx.x * per + i;
+    if (b < nbead) my_cnt += __ldg(a.inter_count + bead0 + b);
+  }
+  int incl = my_cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int* s_wtot = reinterpret_cast<int*>(m.red);
+  if (lane == 31) s_wtot[wid] = incl;
+  __syncthreads();
+  int off = incl - my_cnt;
+  for (int q = 0; q < wid; q++) off += s_wtot[q];
+  for (int i = 0; i < per; i++) {
+    const int b = threadIdx.x * per + i;
+    if (b < nbead) {
+      m.pref[b] = off;
+      off += __ldg(a.inter_count + bead0 + b);
+    }
+  }
+  if (threadIdx.x == blockDim.x - 1) m.pref[nbead] = off;
+}
+
+// Edge t of the item: length vector and stretching coefficient (len0 - l) ks / l (BEAD::
+// update_stretching_force, src/bead.cpp:17-23, EDGE::update_length, src/edge.cpp:35-49).
+__device__ __forceinline__ void force_edge(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int t) {
+  const TplLayout& L = a.L;
+  const int s = fast_div(t, a.div_ne), e = t - s * L.ne;
+  const int pk = m.tpl_i[L.o_edge + e];
+  const int4* sp = m.pos + s * L.np;
+  const float3 lv = dvec(sp[pk & 0xffff], sp[pk >> 16], P.unit32);
+  const float l = sqrtf(dot3(lv, lv));
+  const float coef = (m.tpl_f[L.o_len0 + e] - l) * P.ks / l;
+  m.edge[t] = make_float4(lv.x, lv.y, lv.z, coef);
+}
+
+// Rest-angle option (no reference counterpart): E = kb (1 - cos(beta - beta0)) with beta the signed
+// bend angle of (across0, b0, b1, across1); -dE/dx = -kb sin(beta - beta0) dbeta/dx, dbeta/dx the
+// dihedral gradient (Blondel and Karplus 1996).  Out of line: it runs only for templates with a
+// rest shape.
+__device__ __noinline__ void force_quad_rest(const SysParams& P, int4 Q0, int4 Q1, int4 Q2, int4 Q3, float beta0, float4* o) {
+  const float unit = P.unit32;
+  const float3 v1 = dvec(Q0, Q2, unit), v2 = dvec(Q1, Q0, unit), v3 = dvec(Q3, Q1, unit);
+  const float3 m = cross3(v1, v2), n = cross3(v2, v3);
+  const float l2 = dot3(v2, v2), nv2 = sqrtf(l2);
+  const float beta = atan2f(-nv2 * dot3(v1, n), -dot3(m, n));
+  const float c = -P.kb * sinf(beta - beta0);
+  const float3 ga0 = m * (-nv2 / dot3(m, m)), ga1 = n * (nv2 / dot3(n, n));
+  const float p = dot3(v1, v2) / l2, q = dot3(v3, v2) / l2;
+  const float3 gb0 = ga0 * (-(1.0f + p)) + ga1 * q, gb1 = ga0 * p - ga1 * (1.0f + q);
+  o[0] = make_float4(gb0.x * c, gb0.y * c, gb0.z * c, 0.f);
+  o[1] = make_float4(gb1.x * c, gb1.y * c, gb1.z * c, 0.f);
+  o[2] = make_float4(ga0.x * c, ga0.y * c, ga0.z * c, 0.f);
+  o[3] = make_float4(ga1.x * c, ga1.y * c, ga1.z * c, 0.f);
+}
+
+// Bending quad t of the item: the four bead contributions of EDGE::update_bending_forces
+// (src/edge.cpp:69-188).  The in-place normal flip (src/edge.cpp:78-81) makes S = 4 |A0 . A1|
+// whatever the flip history.
+__device__ __forceinline__ void force_quad(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int t) {
+  const TplLayout& L = a.L;
+  const int s = fast_div(t, a.div_nb), k = t - s * L.nbend;
+  const int4* sp = m.pos + s * L.np;
+  const int4 bq = *reinterpret_cast<const int4*>(m.tpl_i + L.o_bend + 4 * k);
+  const int4 P0 = sp[bq.x], P1 = sp[bq.y], P2 = sp[bq.z], P3 = sp[bq.w];
+  float4* o = m.bend + (size_t)t * 4;
+  const float beta0 = m.tpl_f[L.o_beta0 + k];
+  if (beta0 != 0.f) {
+    force_quad_rest(P, P0, P1, P2, P3, beta0, o);
+    return;
+  }
+  const float unit = P.unit32;
+  // the edge's two faces: area vector 1/2 (b1 - b0) x (b2 - b1) and its magnitude
+  const int* f_b = m.tpl_i + L.o_face;
+  const int2 bf = *reinterpret_cast<const int2*>(m.tpl_i + L.o_bendf + 2 * k);
+  auto face = [&](int f) {
+    const int4 p0 = sp[f_b[3 * f]], p1 = sp[f_b[3 * f + 1]], p2 = sp[f_b[3 * f + 2]];
+    const float3 A = cross3(dvec(p1, p0, unit), dvec(p2, p1, unit)) * 0.5f;
+    return make_float4(A.x, A.y, A.z, sqrtf(dot3(A, A)));
+  };
+  const float4 F0 = face(bf.x), F1 = face(bf.y);
+  const float a0 = F0.w, a1 = F1.w;
+  const float S = 4.0f * fabsf(F0.x * F1.x + F0.y * F1.y + F0.z * F1.z);
+  const float3 d01 = dvec(P0, P1, unit), d02 = dvec(P0, P2, unit), d03 = dvec(P0, P3, unit);
+  const float3 d12 = dvec(P1, P2, unit), d13 = dvec(P1, P3, unit);
+  const float sa0 = S / a0, sa1 = S / a1, q0 = 0.25f / a0, q1 = 0.25f / a1;
+  const float kk = P.kb / (a0 * a1 * 4.0f);
+  {  // role itsB[0]
+    float3 d23 = d13, d32 = d13 * -1.0f, d20 = d01 * -1.0f, d21 = d12;
+    float3 c1 = cross3(d20, d21), c2 = cross3(d20, d32);
+    float3 gs = f3(d23.y * c1.z - d21.y * c2.z + d32.z * c1.y + d21.z * c2.y,
+                   d32.x * c1.z + d21.x * c2.z + d23.z * c1.x - d21.z * c2.x,
+                   d23.x * c1.y - d21.x * c2.y + d32.y * c1.x + d21.y * c2.x);
+    float3 g0 = cross3(d12, cross3(d02, d01)) * (-q0);
+    float3 g1 = cross3(d13, cross3(d03, d01)) * (-q1);
+    float3 r = (gs - (g0 * sa0 + g1 * sa1)) * kk;
+    o[0] = make_float4(r.x, r.y, r.z, 0.f);
+  }
+  {  // role itsB[1]
+    float3 d23 = d03, d32 = d03 * -1.0f, d20 = d01, d21 = d02;
+    float3 c1 = cross3(d20, d21), c2 = cross3(d20, d32);
+    float3 gs = f3(d23.y * c1.z - d21.y * c2.z + d32.z * c1.y + d21.z * c2.y,
+                   d32.x * c1.z + d21.x * c2.z + d23.z * c1.x - d21.z * c2.x,
+                   d23.x * c1.y - d21.x * c2.y + d32.y * c1.x + d21.y * c2.x);
+    float3 g0 = cross3(d02, cross3(d12, d01)) * q0;
+    float3 g1 = cross3(d03, cross3(d13, d01)) * q1;
+    float3 r = (gs - (g0 * sa0 + g1 * sa1)) * kk;
+    o[1] = make_float4(r.x, r.y, r.z, 0.f);
+  }
+  {  // role across face 0: r1x = -r13 (the bead of face 1 off the edge)
+    float3 gs = cross3(d01, cross3(d01, d13 * -1.0f));
+    float3 g0 = cross3(d01, cross3(d02, d01)) * (-q0);
+    float3 r = (gs - g0 * sa0) * kk;
+    o[2] = make_float4(r.x, r.y, r.z, 0.f);
+  }
+  {  // role across face 1: r1x = -r12
+    float3 gs = cross3(d01, cross3(d01, d12 * -1.0f));
+    float3 g1 = cross3(d01, cross3(d03, d01)) * (-q1);
+    float3 r = (gs - g1 * sa1) * kk;
+    o[3] = make_float4(r.x, r.y, r.z, 0.f);
+  }
+}
+
+// Intra-subunit Debye-Hueckel row of bead t (same subunit: no LJ, src/forces.cpp:79-80): all
+// partners in order, the even and the odd ones in the two lanes of packed FP32 sums; both sums go
+// to the bead's limbs.
+__device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w, int t) {
+  const TplLayout& L = a.L;
+  const int np = L.np, npp = (np + 1) >> 1, words = L.words;
+  const int s = fast_div(t, a.div_np), l = t - s * np;
+  const f32x2 nk2 = pack2(-P.kappa, -P.kappa), kap2 = pack2(P.kappa, P.kappa), le2 = pack2(1.44269504f, 1.44269504f);
+  const float cut2 = P.ecut_el2;
+  const float* rs = m.rel + 8 * s * npp;
+  const float* ri = rs + 8 * (l >> 1) + (l & 1);
+  const float nx = -ri[0], ny = -ri[2], nz = -ri[4], wi = ri[6];
+  const f32x2 nx2 = pack2(nx, nx), ny2 = pack2(ny, ny), nz2 = pack2(nz, nz), wi2 = pack2(wi, wi);
+  f32x2 fx = 0, fy = 0, fz = 0;
+  const unsigned int* mrow = a.intra_mask + ((size_t)(w.sub_begin + s) * np + l) * words;
+  const float4* q = reinterpret_cast<const float4*>(rs);
+  unsigned int next = __ldg(mrow);
+  for (int wd = 0; wd < words; wd++) {
+    unsigned int bits = next;
+    if (wd + 1 < words) next = __ldg(mrow + wd + 1);
+    const int b1 = min(npp, (wd + 1) << 4);
+#pragma unroll 2
+    for (int p = wd << 4; p < b1; p++, q += 2, bits >>= 2) {
+      const float4 xy = q[0], zw = q[1];
+      // partner - bead (the sums' sign is turned at the end; every operation is symmetric in it)
+      const f32x2 dx = add2(pack2(xy.x, xy.y), nx2), dy = add2(pack2(xy.z, xy.w), ny2), dz = add2(pack2(zw.x, zw.y), nz2);
+      const f32x2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+      float r2a, r2b;
+      unpack2(r2, r2a, r2b);
+      const f32x2 ir = pack2(rsqrt_ftz(r2a), rsqrt_ftz(r2b));
+      float ea, eb;  // e^(-kappa r) = 2^(-kappa r log2 e)
+      unpack2(mul2(mul2(nk2, mul2(r2, ir)), le2), ea, eb);
+      const f32x2 ex = pack2(ex2_ftz(ea), ex2_ftz(eb));
+      const f32x2 c = mul2(mul2(mul2(mul2(wi2, pack2(zw.z, zw.w)), ex), mul2(ir, ir)), add2(kap2, ir));
+      float ca, cb;
+      unpack2(c, ca, cb);
+      ca = (bits & 1u) && r2a < cut2 ? ca : 0.f;
+      cb = (bits & 2u) && r2b < cut2 ? cb : 0.f;
+      const f32x2 cc = pack2(ca, cb);
+      fx = fma2(dx, cc, fx);
+      fy = fma2(dy, cc, fy);
+      fz = fma2(dz, cc, fz);
+    }
+  }
+  float xe, xo, ye, yo, ze, zo;
+  unpack2(fx, xe, xo);
+  unpack2(fy, ye, yo);
+  unpack2(fz, ze, zo);
+  if (force_bad(xe, ye, ze) || force_bad(xo, yo, zo)) atomicOr(a.err, kErrNonFinite);
+  limbs_add(m.F + 9 * t, f32_to_fx32(-xe) + f32_to_fx32(-xo));
+  limbs_add(m.F + 9 * t + 3, f32_to_fx32(-ye) + f32_to_fx32(-yo));
+  limbs_add(m.F + 9 * t + 6, f32_to_fx32(-ze) + f32_to_fx32(-zo));
+}
+
+// Inter-subunit pairs p .. pend - 1 (DH + LJ/WCA, src/forces.cpp:81-138) of the flat sequence that
+// the beads' lists form (pref: exclusive prefix sums of their lengths), so a bead with a long list
+// holds nobody up: the pairs are walked bead by bead, the pair forces of each bead summed exactly
+// in 2^-32 fixed point in registers and added to the bead's limbs at its last pair
+// (order-independent).  kFresh: the partners' positions are rewritten by other CTAs while this
+// kernel runs (read past L1).
+template <bool kFresh>
+__device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
+                                            int p, int pend) {
+  const TplLayout& L = a.L;
+  const int* species = m.tpl_i + L.o_species;
+  const PairTable& pt = *a.pt;
+  const float unit = P.unit32, kappa = P.kappa, ecut_el2 = P.ecut_el2;
+  int lo = 0, hi = nbead;  // pref[lo] <= p < pref[hi]: the run starts in bead lo
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (m.pref[mid] <= p) lo = mid;
+    else hi = mid;
+  }
+  int b = lo, l = b - fast_div(b, a.div_np) * L.np, bend = m.pref[b + 1];
+  int4 pi = m.pos[b];
+  int si = species[l];
+  float wi = m.w[l];
+  // the row of bead b holds its pairs pref[b] .. pref[b + 1] - 1 of the flat sequence
+  long long row = (long long)(bead0 + b) * a.inter_cap - m.pref[b];
+  long long ax = 0, ay = 0, az = 0;
+  int j = __ldg(a.inter_ids + (row + p));
+  for (;;) {
+    const int4 pj = kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]);
+    const float3 d = dvec(pi, pj, unit);
+    const float r2 = dot3(d, d);
+    const int lj = pj.w, sj = species[lj];
+    const float wj = m.w[lj];
+    float c = 0.f;
+    if (wi * wj != 0.f && r2 < ecut_el2) {
+      const float ir = rsqrtf(r2);
+      const float r = r2 * ir;
+      c = wi * wj * __expf(-kappa * r) * (ir * ir) * (kappa + ir);
+    }
+    const int pidx = si * kMaxSpecies + sj;
+    if (r2 < pt.cut2[pidx]) {
+      const bool att = (L.lj_att_bits[si] >> sj) & 1;
+      const float eps = att ? (((L.type7_bits >> sj) & 1) ? 50.0f : P.elj_att) : 1.0f;
+      const float ir2 = 1.0f / r2;
+      const float s6 = pt.sig6[pidx] * ir2 * ir2 * ir2;
+      c += 48.0f * eps * s6 * (s6 - 0.5f) * ir2;
+    }
+    const float3 f = d * c;
+    if (force_bad(f.x, f.y, f.z)) {
+      atomicOr(a.err, kErrNonFinite);
+    } else {
+      ax += f32_to_fx32(f.x);
+      ay += f32_to_fx32(f.y);
+      az += f32_to_fx32(f.z);
+    }
+    p++;
+    if (p >= bend || p >= pend) {  // the bead's last pair here: add its sums to its limbs
+      limbs_add(m.F + 9 * b, ax);
+      limbs_add(m.F + 9 * b + 3, ay);
+      limbs_add(m.F + 9 * b + 6, az);
+      if (p >= pend) break;
+      ax = ay = az = 0;
+      do {
+        b++;
+        bend = m.pref[b + 1];
+      } while (p >= bend);
+      l = b - fast_div(b, a.div_np) * L.np;
+      pi = m.pos[b];
+      si = species[l];
+      wi = m.w[l];
+      row = (long long)(bead0 + b) * a.inter_cap - m.pref[b];
+    }
+    j = __ldg(a.inter_ids + (row + p));
+  }
+}
+
+// Everything that depends on positions alone, in chunks that the warps take from a counter (zero on
+// entry): the intra-subunit rows of 32 beads, 32 bending quads, 32 runs of kInterRun inter-subunit
+// pairs, 32 edges -- about 700, 450, 500 and 100 instructions.
+constexpr int kInterRun = 4;
+template <bool kFresh>
+__device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
+                                            int nbead, int bead0, int* counter) {
+  const TplLayout& L = a.L;
+  const int lane = threadIdx.x & 31;
+  const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne, n_inter = m.pref[nbead];
+  const int ci = (nbead + 31) >> 5, cq = ci + ((nq + 31) >> 5), cp = cq + (n_inter + 32 * kInterRun - 1) / (32 * kInterRun),
+            ce = cp + ((ne + 31) >> 5);
+  for (;;) {
+    int c = 0;
+    if (lane == 0) c = atomicAdd(counter, 1);
+    c = __shfl_sync(0xffffffffu, c, 0);
+    if (c >= ce) break;
+    if (c < ci) {
+      const int t = 32 * c + lane;
+      if (t < nbead) force_intra(a, P, m, w, t);
+    } else if (c < cq) {
+      const int t = 32 * (c - ci) + lane;
+      if (t < nq) force_quad(a, P, m, t);
+    } else if (c < cp) {
+      const int p = (32 * (c - cq) + lane) * kInterRun;
+      if (p < n_inter) force_inter<kFresh>(a, P, m, nbead, bead0, p, min(n_inter, p + kInterRun));
+    } else {
+      const int t = 32 * (c - cp) + lane;
+      if (t < ne) force_edge(a, P, m, t);
+    }
+    __syncwarp();
+  }
+}
+
+// Stretching and bending sums per bead, two threads per bead in different halves of the CTA, added
+// to the bead's limbs.
+__device__ __forceinline__ void force_gather(const ForceArgs& a, const ForceSmem& m, int nbead, int bead0) {
+  const TplLayout& L = a.L;
+  const int half = blockDim.x >> 1;
+  const int h = (int)threadIdx.x >= half ? 1 : 0;
+  const int* bead_edges = m.tpl_i + L.o_bead_edges;
+  const int* bead_roles = m.tpl_i + L.o_bead_roles;
+  for (int t = (int)threadIdx.x - h * half; t < nbead; t += half) {
+    const int s = fast_div(t, a.div_np), l = t - s * L.np, g = bead0 + t;
+    float3 f = f3(0.f, 0.f, 0.f);
+    if (h == 0) {  // stretching, in the bead's edge order
+      for (int k = 0; k < L.maxdeg; k++) {
+        const int e = bead_edges[l * L.maxdeg + k];
+        if (e < 0) break;
+        const float4 E = m.edge[s * L.ne + (e & 0xffff)];
+        const float c = __int_as_float(__float_as_int(E.w) ^ ((e >> 16) << 31));  // minus for the edge's second bead
+        f = f + f3(E.x, E.y, E.z) * c;
+      }
+      if (a.sfx) { a.sfx[g] = f.x; a.sfy[g] = f.y; a.sfz[g] = f.z; }
+    } else {  // bending, in template edge order
+      for (int k = 0; k < L.maxrole; k++) {
+        const int r = bead_roles[l * L.maxrole + k];
+        if (r < 0) break;
+        const float4 B = m.bend[s * L.nbend * 4 + r];
+        f = f + f3(B.x, B.y, B.z);
+      }
+      if (a.bfx) { a.bfx[g] = f.x; a.bfy[g] = f.y; a.bfz[g] = f.z; }
+    }
+    if (force_bad(f.x, f.y, f.z)) atomicOr(a.err, kErrNonFinite);
+    long long X = f32_to_fx32(f.x), Y = f32_to_fx32(f.y), Z = f32_to_fx32(f.z);
+    if (a.surr_f && h == 0) {  // far-field subunit pairs from the learned surrogate
+      const float4 sv = a.surr_f[g];
+      if (force_bad(sv.x, sv.y, sv.z)) atomicOr(a.err, kErrNonFinite);
+      X += f32_to_fx32(sv.x);
+      Y += f32_to_fx32(sv.y);
+      Z += f32_to_fx32(sv.z);
+    }
+    limbs_add(m.F + 9 * t, X);
+    limbs_add(m.F + 9 * t + 3, Y);
+    limbs_add(m.F + 9 * t + 6, Z);
+  }
+}
+
+}  // namespace souffle

@@ -85,6 +85,7 @@ struct ForceArgs {
   unsigned int* err;
   int n_beads_total;
   int max_sub;               // subunits per CTA (shared-memory sizing)
+  unsigned int div_np, div_ne, div_nb;  // fast_div multipliers of np, ne, nbend
   int mode;                  // 0: forces only, 1: MD step (kick + reductions), 2: begin (KE only)
 };
 

@@ -38,18 +38,18 @@ struct TplLayout {
   int o_face;         // [nf*3]
   int o_bend;         // [nbend*4] b0, b1, across0, across1
   int o_bendf;        // [nbend*2] face0, face1
-  int o_bead_edges;   // [np*maxdeg] edge index or -1
+  int o_bead_edges;   // [np*maxdeg] edge index (| 1 << 16 where the bead is the edge's second) or -1
   int o_bead_roles;   // [np*maxrole] bend*4+role or -1
   int o_type;         // [np]
   int o_species;      // [np]
-  int n_int;          // total ints
+  int n_int;          // ints that the force kernels stage (o_bend, o_bendf, o_face, o_edge, o_bead_*, o_species)
   // float buffer offsets
   int o_len0;         // [ne]
   int o_q;            // [np]
   int o_sigma;        // [np]
   int o_mass;         // [np]
   int o_beta0;        // [nbend] rest bend angle per bending edge (0 = no rest angle)
-  int n_float;
+  int n_float;        // floats that the force kernels stage (o_len0, o_mass, o_sigma, o_beta0)
   int nspecies;
   int lj_att_bits[kMaxSpecies];  // bit js of row is: (species is -> js) attractive
   int type7_bits;                // bit js: species js has type 7 (attractive epsilon 50)

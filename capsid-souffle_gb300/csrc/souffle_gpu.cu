@@ -88,6 +88,7 @@ souffle_status derive_template(const souffle_template* t, HostTemplate& h) {
   h.len0.assign(t->edge_len0, t->edge_len0 + h.ne);
   h.face.assign(t->face_beads, t->face_beads + 3 * h.nf);
   h.lj.assign(t->lj_types, t->lj_types + 2 * h.n_lj);
+  if (h.ne > 0xffff) return fail(SOUFFLE_ERR_BAD_INPUT, "more than 65535 edges");
   for (int v : h.edge)
     if (v < 0 || v >= h.np) return fail(SOUFFLE_ERR_BAD_INPUT, "edge bead index out of range");
   for (int v : h.face)
@@ -155,7 +156,8 @@ souffle_status derive_template(const souffle_template* t, HostTemplate& h) {
   h.bead_edges.assign(h.np * h.maxdeg, -1);
   h.bead_roles.assign(h.np * h.maxrole, -1);
   for (int i = 0; i < h.np; i++) {
-    for (size_t k = 0; k < be[i].size(); k++) h.bead_edges[i * h.maxdeg + k] = be[i][k];
+    for (size_t k = 0; k < be[i].size(); k++)  // the edge, and whether the bead is its second one
+      h.bead_edges[i * h.maxdeg + k] = be[i][k] | (h.edge[2 * be[i][k]] == i ? 0 : 1 << 16);
     for (size_t k = 0; k < br[i].size(); k++) h.bead_roles[i * h.maxrole + k] = br[i][k];
   }
   // species: distinct (type, sigma) pairs
@@ -192,28 +194,27 @@ souffle_status upload(souffle_gpu_system* h) {
   L.words = (T.np + 31) / 32;
   L.maxdeg = T.maxdeg;
   L.maxrole = T.maxrole;
-  L.o_edge = (int)ti.size();
-  for (int e = 0; e < T.ne; e++) ti.push_back(T.edge[2 * e] | (T.edge[2 * e + 1] << 16));
-  L.o_face = (int)ti.size();
-  ti.insert(ti.end(), T.face.begin(), T.face.end());
+  // the bending quads on a 16-byte boundary, their faces on an 8-byte one
   L.o_bend = (int)ti.size();
   ti.insert(ti.end(), T.bend.begin(), T.bend.end());
   L.o_bendf = (int)ti.size();
   ti.insert(ti.end(), T.bendf.begin(), T.bendf.end());
+  L.o_face = (int)ti.size();
+  ti.insert(ti.end(), T.face.begin(), T.face.end());
+  L.o_edge = (int)ti.size();
+  for (int e = 0; e < T.ne; e++) ti.push_back(T.edge[2 * e] | (T.edge[2 * e + 1] << 16));
   L.o_bead_edges = (int)ti.size();
   ti.insert(ti.end(), T.bead_edges.begin(), T.bead_edges.end());
   L.o_bead_roles = (int)ti.size();
   ti.insert(ti.end(), T.bead_roles.begin(), T.bead_roles.end());
-  L.o_type = (int)ti.size();
-  ti.insert(ti.end(), T.type.begin(), T.type.end());
   L.o_species = (int)ti.size();
   ti.insert(ti.end(), T.species.begin(), T.species.end());
   while (ti.size() % 4) ti.push_back(0);
   L.n_int = (int)ti.size();
+  L.o_type = (int)ti.size();
+  ti.insert(ti.end(), T.type.begin(), T.type.end());
   L.o_len0 = (int)tf.size();
   for (double v : T.len0) tf.push_back((float)v);
-  L.o_q = (int)tf.size();
-  for (double v : T.q) tf.push_back((float)v);
   L.o_sigma = (int)tf.size();
   for (double v : T.sigma) tf.push_back((float)v);
   L.o_mass = (int)tf.size();
@@ -222,6 +223,8 @@ souffle_status upload(souffle_gpu_system* h) {
   for (double v : T.beta0) tf.push_back((float)v);
   while (tf.size() % 4) tf.push_back(0.f);
   L.n_float = (int)tf.size();
+  L.o_q = (int)tf.size();
+  for (double v : T.q) tf.push_back((float)v);
   L.nspecies = T.nspecies;
   // directed attraction (src/forces.cpp:119-125) and the type-7 epsilon (src/forces.cpp:127)
   L.type7_bits = 0;
@@ -381,6 +384,9 @@ void launch_rebuild(souffle_gpu_system* h) {
   if (surrogate_enabled(h)) surrogate_compact(h);
 }
 
+// multiplier of fast_div: ceil(2^32 / d), 0 for d <= 1
+unsigned int div_magic(int d) { return d > 1 ? (unsigned int)((4294967296ull + d - 1) / d) : 0u; }
+
 ForceArgs force_args(souffle_gpu_system* h, int mode, bool want_parts) {
   ForceArgs a{};
   a.L = h->L;
@@ -422,6 +428,9 @@ ForceArgs force_args(souffle_gpu_system* h, int mode, bool want_parts) {
   a.bb_pos32 = h->bb_pos32.p;
   a.chain64 = h->opt.chain_fp64 ? h->chain64.p : nullptr;
   a.max_sub = h->subs_per_cta;
+  a.div_np = div_magic(h->tpl.np);
+  a.div_ne = div_magic(h->L.ne);
+  a.div_nb = div_magic(h->L.nbend);
   a.mode = mode;
   return a;
 }
@@ -483,7 +492,7 @@ void launch_step(souffle_gpu_system* h, bool rebuild, bool judge) {
 size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
   const TplLayout& L = h->L;
   const int np = h->tpl.np;
-  return force_tile_bytes(subs, L.ne, L.nbend) + (sizeof(int4) + sizeof(float4)) * subs * np +
+  return force_tile_bytes(subs, L.ne, L.nbend) + sizeof(int4) * subs * np + 8 * sizeof(float) * subs * ((np + 1) / 2) +
          sizeof(long long) * 4 * (threads / 32) + sizeof(unsigned int) * force_slot_len(subs * np) +
          sizeof(int) * force_pref_len(subs * np) + sizeof(float) * (np + L.n_float) + sizeof(int) * L.n_int;
 }
