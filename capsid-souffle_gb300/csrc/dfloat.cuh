@@ -25,6 +25,14 @@ namespace souffle {
 // Error-free transformations need each sum and product rounded on its own: on the device the
 // _rn intrinsics are never contracted into fused multiply-adds (host builds that compile this
 // header pass -ffp-contract=off).
+// The exponentials are kept out of line on the device: the thermostat runs each of them once per step
+// in one warp, so their instructions come from beyond the small instruction caches, and one copy
+// that several callers share is fetched once.
+#ifdef __CUDACC__
+#define DF_NOINLINE __noinline__
+#else
+#define DF_NOINLINE
+#endif
 #ifdef __CUDA_ARCH__
 #define DF_ADD(a, b) __fadd_rn(a, b)
 #define DF_SUB(a, b) __fsub_rn(a, b)
@@ -80,7 +88,7 @@ __host__ __device__ inline dfloat df_mul(dfloat a, dfloat b) {
 // tail T = 1/720 + x/5040 + ... is small enough (|x^5 T| < 5e-8) to be evaluated in FP32.
 // S = a + x^2 (b + x^2 c) with a = 1 + x/2, b = 1/6 + x/24, c = 1/120 + x T (Estrin's scheme:
 // a, b, c and x^2 are independent, so the dependent chain is half of Horner's).
-__host__ __device__ inline dfloat df_expm1_small(dfloat x) {
+DF_NOINLINE __host__ __device__ inline dfloat df_expm1_small(dfloat x) {
   const float xf = x.hi;
   const float t = fmaf(xf, fmaf(xf, fmaf(xf, fmaf(xf, 1.0f / 3628800.0f, 1.0f / 362880.0f), 1.0f / 40320.0f),
                                 1.0f / 5040.0f), 1.0f / 720.0f);
@@ -100,7 +108,7 @@ __host__ __device__ inline dfloat df_expm1_small(dfloat x) {
 // that brings |x|/2^s under 1/8 (each squaring doubles the relative error, so s <= 10 keeps it
 // near 2^-36 for |x| up to 128; larger |x| falls back to FP64 exp).  Results below ~1e-26
 // (x < -60) lose precision as the low word turns subnormal.
-__host__ __device__ inline dfloat df_exp(dfloat x) {
+DF_NOINLINE __host__ __device__ inline dfloat df_exp_big(dfloat x) {
   const float ax = fabsf(x.hi);
   if (!(ax <= 128.0f)) return df_from(exp(df_to(x)));
   int s = 0;
@@ -114,6 +122,10 @@ __host__ __device__ inline dfloat df_exp(dfloat x) {
   dfloat e = df_add(df_expm1_small(xs), dfloat{1.0f, 0.0f});
   for (int k = 0; k < s; k++) e = df_mul(e, e);
   return e;
+}
+__host__ __device__ inline dfloat df_exp(dfloat x) {
+  if (fabsf(x.hi) <= 0.125f) return df_add(df_expm1_small(x), dfloat{1.0f, 0.0f});  // the thermostat's range
+  return df_exp_big(x);
 }
 
 // e^x - 1 without cancellation: the series for |x| <= 1/8, beyond which |e^x - 1| > 0.11.

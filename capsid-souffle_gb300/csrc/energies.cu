@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(128) k_energy_inter(EnergyArgs a) {
                   gz = (cz + q % span + 2 * n) % n;
         const int cell = P.cell0 + (gx * n + gy) * n + gz;
         cur = a.sub_cell_start[cell];
-        end = a.sub_cell_start[cell + 1];
+        end = cur + a.sub_cell_count[cell];
       }
       while (__syncthreads_or(cur < end)) {
         const int j = cur < end ? a.cell_subs[cur] - P.sub0 : -1;

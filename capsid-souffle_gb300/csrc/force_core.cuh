@@ -351,27 +351,43 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
                                             int p, int pend) {
   const TplLayout& L = a.L;
   const int* species = m.tpl_i + L.o_species;
-  const PairTable& pt = *a.pt;
   const float unit = P.unit32, kappa = P.kappa, ecut_el2 = P.ecut_el2;
+  const int ns = L.nspecies;
   int lo = 0, hi = nbead;  // pref[lo] <= p < pref[hi]: the run starts in bead lo
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (m.pref[mid] <= p) lo = mid;
     else hi = mid;
   }
-  int b = lo, l = b - fast_div(b, a.div_np) * L.np, bend = m.pref[b + 1];
-  int4 pi = m.pos[b];
-  int si = species[l];
-  float wi = m.w[l];
-  // the row of bead b holds its pairs pref[b] .. pref[b + 1] - 1 of the flat sequence
-  long long row = (long long)(bead0 + b) * a.inter_cap - m.pref[b];
+  // the row of bead b holds its pairs pref[b] .. pref[b + 1] - 1 of the flat sequence; the next
+  // pair's bead, partner and partner position are fetched while the current one is evaluated
+  int nb = lo, nend = m.pref[nb + 1];
+  auto partner = [&](int q) { return __ldg(a.inter_ids + ((long long)(bead0 + nb) * a.inter_cap - m.pref[nb] + q)); };
+  auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
+  int4 next = position(partner(p));
+  int b = -1, si = 0;
+  int4 pi = make_int4(0, 0, 0, 0);
+  float wi = 0.f;
   long long ax = 0, ay = 0, az = 0;
-  int j = __ldg(a.inter_ids + (row + p));
-  for (;;) {
-    const int4 pj = kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]);
+  while (p < pend) {
+    const int4 pj = next;
+    if (nb != b) {  // first pair of a bead
+      b = nb;
+      pi = m.pos[b];
+      const int l = b - fast_div(b, a.div_np) * L.np;
+      si = species[l] * ns;
+      wi = m.w[l];
+    }
+    p++;
+    bool last = p >= pend;
+    if (!last) {
+      last = p >= nend;
+      while (p >= nend) nend = m.pref[++nb + 1];
+      next = position(partner(p));
+    }
     const float3 d = dvec(pi, pj, unit);
     const float r2 = dot3(d, d);
-    const int lj = pj.w, sj = species[lj];
+    const int lj = pj.w;
     const float wj = m.w[lj];
     float c = 0.f;
     if (wi * wj != 0.f && r2 < ecut_el2) {
@@ -379,12 +395,11 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
       const float r = r2 * ir;
       c = wi * wj * __expf(-kappa * r) * (ir * ir) * (kappa + ir);
     }
-    const int pidx = si * kMaxSpecies + sj;
-    if (r2 < pt.cut2[pidx]) {
-      const bool att = (L.lj_att_bits[si] >> sj) & 1;
-      const float eps = att ? (((L.type7_bits >> sj) & 1) ? 50.0f : P.elj_att) : 1.0f;
+    const float* pair = m.tpl_f + L.o_pair + 3 * (si + species[lj]);  // cut-off squared, sigma^6, epsilon
+    if (r2 < pair[0]) {
+      const float eps = pair[2] < 0.f ? P.elj_att : pair[2];
       const float ir2 = 1.0f / r2;
-      const float s6 = pt.sig6[pidx] * ir2 * ir2 * ir2;
+      const float s6 = pair[1] * ir2 * ir2 * ir2;
       c += 48.0f * eps * s6 * (s6 - 0.5f) * ir2;
     }
     const float3 f = d * c;
@@ -395,56 +410,57 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
       ay += f32_to_fx32(f.y);
       az += f32_to_fx32(f.z);
     }
-    p++;
-    if (p >= bend || p >= pend) {  // the bead's last pair here: add its sums to its limbs
+    if (last) {  // the bead's last pair here: add its sums to its limbs
       limbs_add(m.F + 9 * b, ax);
       limbs_add(m.F + 9 * b + 3, ay);
       limbs_add(m.F + 9 * b + 6, az);
-      if (p >= pend) break;
       ax = ay = az = 0;
-      do {
-        b++;
-        bend = m.pref[b + 1];
-      } while (p >= bend);
-      l = b - fast_div(b, a.div_np) * L.np;
-      pi = m.pos[b];
-      si = species[l];
-      wi = m.w[l];
-      row = (long long)(bead0 + b) * a.inter_cap - m.pref[b];
     }
-    j = __ldg(a.inter_ids + (row + p));
   }
 }
 
 // Everything that depends on positions alone, in chunks that the warps take from a counter (zero on
-// entry): the intra-subunit rows of 32 beads, 32 bending quads, 32 runs of kInterRun inter-subunit
-// pairs, 32 edges -- about 700, 450, 500 and 100 instructions.
-constexpr int kInterRun = 4;
-template <bool kFresh>
+// entry): the intra-subunit rows of 32 beads, 32 bending quads, 32 runs of inter-subunit pairs, 32
+// edges -- about 700, 450, 100 per pair of a run and 100 instructions.  The runs are as long as
+// gives every warp one chunk, at most eight pairs.  kFresh (the window kernel): the inter-subunit
+// pairs come last, and a warp's first one only after wait() -- by then the other CTAs have
+// published their new positions while this one worked on its own subunits.
+template <bool kFresh, class Wait>
 __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
-                                            int nbead, int bead0, int* counter) {
+                                            int nbead, int bead0, int* counter, Wait wait) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
   const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne, n_inter = m.pref[nbead];
-  const int ci = (nbead + 31) >> 5, cq = ci + ((nq + 31) >> 5), cp = cq + (n_inter + 32 * kInterRun - 1) / (32 * kInterRun),
-            ce = cp + ((ne + 31) >> 5);
+  const int run = min(8, (n_inter + (int)blockDim.x - 1) / (int)blockDim.x), per = 32 * run;
+  const int ki = (nbead + 31) >> 5, kq = (nq + 31) >> 5, ke = (ne + 31) >> 5,
+            kp = n_inter > 0 ? (n_inter + per - 1) / per : 0;
+  const int total = ki + kq + ke + kp;
+  bool waited = false;
   for (;;) {
-    int c = 0;
-    if (lane == 0) c = atomicAdd(counter, 1);
-    c = __shfl_sync(0xffffffffu, c, 0);
-    if (c >= ce) break;
-    if (c < ci) {
-      const int t = 32 * c + lane;
+    int k = 0;
+    if (lane == 0) k = atomicAdd(counter, 1);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= total) break;
+    if (k < ki) {
+      const int t = 32 * k + lane;
       if (t < nbead) force_intra(a, P, m, w, t);
-    } else if (c < cq) {
-      const int t = 32 * (c - ci) + lane;
+    } else if ((k -= ki) < kq) {
+      const int t = 32 * k + lane;
       if (t < nq) force_quad(a, P, m, t);
-    } else if (c < cp) {
-      const int p = (32 * (c - cq) + lane) * kInterRun;
-      if (p < n_inter) force_inter<kFresh>(a, P, m, nbead, bead0, p, min(n_inter, p + kInterRun));
     } else {
-      const int t = 32 * (c - cp) + lane;
-      if (t < ne) force_edge(a, P, m, t);
+      k -= kq;
+      const bool edge = kFresh ? k < ke : k >= kp;
+      if (edge) {
+        const int t = 32 * (kFresh ? k : k - kp) + lane;
+        if (t < ne) force_edge(a, P, m, t);
+      } else {
+        if (kFresh && !waited) {
+          wait();
+          waited = true;
+        }
+        const int p = (32 * (kFresh ? k - ke : k) + lane) * run;
+        if (p < n_inter) force_inter<kFresh>(a, P, m, nbead, bead0, p, min(n_inter, p + run));
+      }
     }
     __syncwarp();
   }

@@ -100,6 +100,58 @@ __device__ __noinline__ void bigbead_mask(const ForceArgs& a, const SysParams& P
   }
 }
 
+// The end of a step (mode 1) or of the initial forces (mode 2) for one system, from its kinetic
+// energy and momentum sums (2^-32 and 2^-40 units) into its state S in shared memory: warp 0 runs
+// the thermostat chain, warp 1 the centre-of-mass velocity.  The caller's barrier ends it.
+// chain_pre: warp 0's nhc_pre_warp of this step has run with this result, else ~0.
+template <bool kChain64>
+__device__ __forceinline__ void step_tail(const ForceArgs& a, const SysParams& P, int sys, SysState& S, const long long* sum,
+                                          dfloat* chain_scratch, unsigned int chain_pre = ~0u) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int vcom_warp = nw > 1 ? 1 : 0;
+  if (wid == 0) {
+    if (lane == 0) {
+      S.done = 0;
+      S.ke = df_from_fixed(sum[0], 2.3283064365386963e-10f);  // 2^-32
+      if (a.mode == 1) S.steps += 1;
+      if (P.brownian && a.mode == 1) {  // this step's draws are used: next step's generator state
+        S.fran_sum[0] = S.fran_sum[1] = S.fran_sum[2] = 0;
+        S.lcg = lcg_mul(S.lcg, P.lcg_step);
+      }
+    }
+    __syncwarp();
+    if constexpr (kChain64) {  // FP64 validation variant, one thread
+      if (lane == 0) {
+        Chain64& c = a.chain64[sys];
+        if (!chain64_tail(c, (double)sum[0] * 2.3283064365386963e-10, a.mode == 1, S))  // KE: 2^-32 units
+          atomicOr(a.err, kErrNonFinite);
+      }
+      __syncwarp();
+    } else {
+      const bool forward = a.mode == 1;
+      unsigned int active = chain_pre;
+      if (!forward) active = __ballot_sync(0xffffffffu, lane < S.m && nhc_active(S, lane));
+      else if (chain_pre == ~0u) active = nhc_pre_warp(S, lane, chain_scratch);
+      if (!nhc_post_warp(S, lane, chain_scratch, active, forward)) atomicOr(a.err, kErrNonFinite);
+    }
+  }
+  if (wid == vcom_warp && lane == 0) {
+    const long long x = sum[1], y = sum[2], z = sum[3];
+    if (a.mode == 1) {
+      // mean velocity, removed from every bead before the next kick (src/md.cpp:505-514)
+      const double vx = (double)x * S.inv_n, vy = (double)y * S.inv_n, vz = (double)z * S.inv_n;
+      S.vcom_fx[0] = __double2ll_rn(vx);
+      S.vcom_fx[1] = __double2ll_rn(vy);
+      S.vcom_fx[2] = __double2ll_rn(vz);
+      S.vsum[0] = x;  // (its magnitude is an output: formed on the host, an FP64 root takes 2 us here)
+      S.vsum[1] = y;
+      S.vsum[2] = z;
+    } else {
+      S.vcom_fx[0] = S.vcom_fx[1] = S.vcom_fx[2] = 0;
+    }
+  }
+}
+
 // 5 CTAs of 256 threads per SM (<= 51 registers) so 3-subunit work items fit one wave of
 // 152 x 5 CTAs at the 2000-subunit workload.
 // kChain64: the tail runs the FP64 validation chain (souffle_options.chain_fp64) instead of the
@@ -139,7 +191,7 @@ __global__ void __launch_bounds__(256, 5) k_forces(ForceArgs a) {
   if (threadIdx.x < 16 * kBBWords) s_bbm[threadIdx.x] = 0u;
   force_prefix(a, m, bead0, nbead);  // (its barrier makes the tile visible)
   __syncthreads();               // the prefix sums
-  force_terms<false>(a, P, m, w, nbead, bead0, &s_counter);
+  force_terms<false>(a, P, m, w, nbead, bead0, &s_counter, [] {});
   __syncthreads();
   const float* s_mass = tpl_f + L.o_mass;
   const SysState& st = a.state[w.sys];
@@ -253,43 +305,7 @@ __global__ void __launch_bounds__(256, 5) k_forces(ForceArgs a) {
   for (int q = threadIdx.x; q < kStateVecs; q += blockDim.x) st_dst[q] = __ldcg(st_src + q);
   if (threadIdx.x < 4) s_red[threadIdx.x] = sum;
   __syncthreads();
-  const int vcom_warp = nw > 1 ? 1 : 0;
-  if (wid == 0) {
-    if (lane == 0) {
-      S.done = 0;
-      S.ke = df_from_fixed(s_red[0], 2.3283064365386963e-10f);  // 2^-32
-      if (a.mode == 1) S.steps += 1;
-      if (P.brownian && a.mode == 1) {  // this step's draws are used: next step's generator state
-        S.fran_sum[0] = S.fran_sum[1] = S.fran_sum[2] = 0;
-        S.lcg = lcg_mul(S.lcg, P.lcg_step);
-      }
-    }
-    __syncwarp();
-    if constexpr (kChain64) {  // FP64 validation variant, one thread
-      if (lane == 0) {
-        Chain64& c = a.chain64[w.sys];
-        if (!chain64_tail(c, (double)s_red[0] * 2.3283064365386963e-10, a.mode == 1, S))  // KE: 2^-32 units
-          atomicOr(a.err, kErrNonFinite);
-      }
-      __syncwarp();
-    } else {
-      if (a.mode == 1) nhc_forward_warp(S, lane, chain_scratch);
-      if (!nhc_backward_warp(S, lane, chain_scratch + 2 * kMaxChain)) atomicOr(a.err, kErrNonFinite);
-    }
-  }
-  if (wid == vcom_warp && lane == 0) {
-    const long long x = s_red[1], y = s_red[2], z = s_red[3];
-    if (a.mode == 1) {
-      // mean velocity, removed from every bead before the next kick (src/md.cpp:505-514)
-      const double vx = (double)x * S.inv_n, vy = (double)y * S.inv_n, vz = (double)z * S.inv_n;
-      S.vcom_fx[0] = __double2ll_rn(vx);
-      S.vcom_fx[1] = __double2ll_rn(vy);
-      S.vcom_fx[2] = __double2ll_rn(vz);
-      S.vcom_mag = sqrt(vx * vx + vy * vy + vz * vz) * (1.0 / kVelScale);
-    } else {
-      S.vcom_fx[0] = S.vcom_fx[1] = S.vcom_fx[2] = 0;
-    }
-  }
+  step_tail<kChain64>(a, P, w.sys, S, s_red, chain_scratch);
   __syncthreads();
   for (int q = threadIdx.x; q < kStateVecs; q += blockDim.x) reinterpret_cast<int4*>(a.state + w.sys)[q] = st_dst[q];
   // per-bead kick coefficients c0 / m, one template bead per thread
@@ -324,6 +340,44 @@ __device__ __forceinline__ void drift_bead(int g, int l, long long c, long long 
   pos32[g] = make_int4(hi_word(X), hi_word(Y), hi_word(Z), l);
 }
 
+// Drag and random force of one bead for a Brownian step (src/md.cpp:415-421, 461-467), from its
+// velocity after the last centre-of-mass removal and the generator's state before the step: bead k
+// of the system takes draws 6k+1 .. 6k+6 (x, y, z: two draws each).  Both are stored for the force
+// kernel; r returns the random force.
+__device__ __forceinline__ void brownian_draws(const DriftArgs& a, const SysParams& P, unsigned int lcg, int sys, int g, int l,
+                                               long long vx, long long vy, long long vz, long long* r) {
+  const long long N = a.n_total;
+  const long long dc = a.bd_drag[(size_t)sys * a.np + l];
+  a.fdrag[g] = -mul_shr(vx, dc, 48);
+  a.fdrag[N + g] = -mul_shr(vy, dc, 48);
+  a.fdrag[2 * N + g] = -mul_shr(vz, dc, 48);
+  unsigned int x = lcg_mul(lcg, a.lcg_table[g - P.bead0]);
+  unsigned int d[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) d[k] = x = lcg_mul(x, 16807u);
+  const double sc = a.bd_noise[(size_t)sys * a.np + l];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    r[k] = __double2ll_rn(__dmul_rn(sc, lcg_uniform_half(d[2 * k], d[2 * k + 1])) * 4294967296.0);
+    a.fran[k * N + g] = r[k];
+  }
+}
+
+// A bead's three force components kept in the first six words of its limbs between steps.
+__device__ __forceinline__ void put_fx(unsigned int* F, long long x, long long y, long long z) {
+  F[0] = (unsigned int)x;
+  F[1] = (unsigned int)(x >> 32);
+  F[2] = (unsigned int)y;
+  F[3] = (unsigned int)(y >> 32);
+  F[4] = (unsigned int)z;
+  F[5] = (unsigned int)(z >> 32);
+}
+__device__ __forceinline__ void get_fx(const unsigned int* F, long long& x, long long& y, long long& z) {
+  x = (long long)((unsigned long long)F[1] << 32 | F[0]);
+  y = (long long)((unsigned long long)F[3] << 32 | F[2]);
+  z = (long long)((unsigned long long)F[5] << 32 | F[4]);
+}
+
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
@@ -347,31 +401,16 @@ __global__ void __launch_bounds__(256) k_drift(DriftArgs a) {
     // the last centre-of-mass removal, half-kick with the stored total force, drift; then this
     // step's random forces (src/md.cpp:461-467): bead k of the system takes draws 6k+1 .. 6k+6
     // of the generator after the previous steps' draws (x, y, z: two draws each)
-    const long long N = a.n_total;
     long long sx = 0, sy = 0, sz = 0;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
       const int g = bead0 + t, l = t % a.np;
-      const long long dc = a.bd_drag[(size_t)w.sys * a.np + l];
-      const long long vx = a.vx[g] - vcx, vy = a.vy[g] - vcy, vz = a.vz[g] - vcz;
-      a.fdrag[g] = -mul_shr(vx, dc, 48);
-      a.fdrag[N + g] = -mul_shr(vy, dc, 48);
-      a.fdrag[2 * N + g] = -mul_shr(vz, dc, 48);
+      long long r[3];
+      brownian_draws(a, P, S.lcg, w.sys, g, l, a.vx[g] - vcx, a.vy[g] - vcy, a.vz[g] - vcz, r);
       drift_bead(g, l, kick_c[l], 0, vcx, vcy, vcz, dx_fx, a.fx, a.fy, a.fz, a.vx, a.vy, a.vz, a.px, a.py, a.pz,
                  a.pos32);
-      unsigned int x = lcg_mul(S.lcg, a.lcg_table[g - P.bead0]);
-      unsigned int d[6];
-#pragma unroll
-      for (int k = 0; k < 6; k++) d[k] = x = lcg_mul(x, 16807u);
-      const double sc = a.bd_noise[(size_t)w.sys * a.np + l];
-      const long long rx = __double2ll_rn(__dmul_rn(sc, lcg_uniform_half(d[0], d[1])) * 4294967296.0);
-      const long long ry = __double2ll_rn(__dmul_rn(sc, lcg_uniform_half(d[2], d[3])) * 4294967296.0);
-      const long long rz = __double2ll_rn(__dmul_rn(sc, lcg_uniform_half(d[4], d[5])) * 4294967296.0);
-      a.fran[g] = rx;
-      a.fran[N + g] = ry;
-      a.fran[2 * N + g] = rz;
-      sx += rx;
-      sy += ry;
-      sz += rz;
+      sx += r[0];
+      sy += r[1];
+      sz += r[2];
     }
     sx = warp_sum_ll(sx);
     sy = warp_sum_ll(sy);
@@ -402,6 +441,310 @@ __global__ void __launch_bounds__(256) k_drift(DriftArgs a) {
     const int l = t % a.np;
     drift_bead(bead0 + t, l, kick_c[l], delta_fx, vcx, vcy, vcz, dx_fx, a.fx, a.fy, a.fz, a.vx, a.vy, a.vz, a.px, a.py,
                a.pz, a.pos32);
+  }
+}
+
+// ---- the window kernel ------------------------------------------------------------------------
+// A run of MD or Brownian steps between two pair-list rebuilds in one launch, for handles whose
+// work items all fit the GPU at once (one CTA per item, cooperative launch).  The CTA keeps its
+// beads' positions, velocities and forces, the template tables and the system's thermostat state
+// in shared memory; only the high words of the positions pass through global memory.  A step is
+//   drift      own beads; publish the new high words; arrive at the grid barrier
+//   terms      own subunits' rows, quads and edges, then (the barrier having long completed) the
+//              inter-subunit pairs
+//   finish     totals, second half kick, kinetic energy and momentum; arrive at the grid barrier
+//              with the sums; every CTA runs the thermostat chain itself, which costs the same
+//              3 us once per SM instead of in one CTA, and saves handing its result around
+// The same operations as k_drift and k_forces, so the results are the same bits.  What it removes
+// is latency, which is all a small system's step consists of: two launches per step, the reload of
+// tables, state and tile (about 3 us), and the serial hand-over to the last CTA.  Per step, rebuilds
+// included: 19.6 -> 11.9 us at 200 beads, 23.3 -> 14.7 at 2,688, 24.8 -> 16.8 at 13,986, 36.2 ->
+// 27.2 at 84,000.  What is left there: the chain (2.7 us), the two barriers (1.5 us) and the wait
+// for the CTA with the most pairs.
+// The two barriers of a step count their arrivals separately: a CTA without inter-subunit pairs
+// does not wait at the first one, and its early arrival at the second must not be taken for
+// another's at the first.
+struct GridBarrier {
+  unsigned int* count;    // arrivals, zero between launches
+  unsigned int* err;
+  unsigned int target;    // arrivals that complete the barrier in progress
+  // thread 0 of the CTA, after a CTA barrier behind the writes to publish
+  __device__ __forceinline__ void arrive() const {
+    __threadfence();
+    atomicAdd(count, 1u);
+  }
+  // any thread; false when the wait ran out (kWindowPolls tries, some seconds)
+  __device__ __forceinline__ bool wait(volatile int* abort_flag) const {
+    for (unsigned int i = 0; i < kWindowPolls; i++) {
+      unsigned int v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+      if ((int)(v - target) >= 0) return true;
+      if ((i & 255u) == 255u && *abort_flag) return false;
+    }
+    *abort_flag = 1;
+    atomicOr(err, kErrWindow);
+    return false;
+  }
+  static constexpr unsigned int kWindowPolls = 1u << 22;
+};
+
+__global__ void __launch_bounds__(256, 5) k_window(ForceArgs a, DriftArgs d, WindowArgs q) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const TplLayout& L = a.L;
+  const WorkItem w = a.work[blockIdx.x];
+  const SysParams& P = a.sys[w.sys];
+  const int np = L.np, nbead = w.nsub * np, bead0 = w.sub_begin * np;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const ForceSmem m = force_smem(smem, a, nw);
+  // behind the force kernel's shared memory: positions, velocities, kick coefficients, the state
+  const int nmax = a.max_sub * np;
+  long long* s_x = reinterpret_cast<long long*>(smem + q.force_bytes);  // [3][nmax]
+  long long* s_v = s_x + 3 * nmax;                                      // [3][nmax]
+  long long* s_kc = s_v + 3 * nmax;                                     // [np]
+  dfloat* s_im = reinterpret_cast<dfloat*>(s_kc + ((np + 1) & ~1));     // [np] 1 / m
+  SysState& S = *reinterpret_cast<SysState*>(s_im + ((np + 1) & ~1));
+  dfloat* chain_scratch = reinterpret_cast<dfloat*>(&S + 1);
+  __shared__ int s_counter, s_abort;
+  __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
+  GridBarrier moved{q.count, a.err, 0u}, summed{q.count + 1, a.err, 0u};  // positions published, sums complete
+  const float unit = P.unit32;
+  const bool bd = P.brownian;
+  if (threadIdx.x == 0) s_abort = 0;
+  force_setup(a, w, m);
+  {
+    const int4* src = reinterpret_cast<const int4*>(a.state + w.sys);
+    int4* dst = reinterpret_cast<int4*>(&S);
+    for (int t = threadIdx.x; t < (int)(sizeof(SysState) / 16); t += blockDim.x) dst[t] = __ldcg(src + t);
+    for (int l = threadIdx.x; l < np; l += blockDim.x) {
+      s_kc[l] = a.kick_c[(size_t)w.sys * np + l];
+      s_im[l] = a.inv_mass[l];
+    }
+  }
+  const bool own_c = nbead <= (int)blockDim.x;
+  long long my_c = 0;
+  dfloat inv_m = {0.f, 0.f};
+  if (own_c && (int)threadIdx.x < nbead) {
+    const int l = threadIdx.x - fast_div(threadIdx.x, a.div_np) * np;
+    my_c = a.kick_c[(size_t)w.sys * np + l];
+    inv_m = a.inv_mass[l];
+  }
+  for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+    const int g = bead0 + t;
+    s_x[t] = d.px[g];
+    s_x[nmax + t] = d.py[g];
+    s_x[2 * nmax + t] = d.pz[g];
+    s_v[t] = a.vx[g];
+    s_v[nmax + t] = a.vy[g];
+    s_v[2 * nmax + t] = a.vz[g];
+    unsigned int* F = m.F + 9 * t;
+    if (q.forces_first) {  // the first step's drift is done: its positions, no forces yet
+      m.pos[t] = a.pos32[g];
+#pragma unroll
+      for (int k = 0; k < 9; k++) F[k] = 0u;
+    } else {
+      put_fx(F, a.fx[g], a.fy[g], a.fz[g]);
+    }
+  }
+  force_prefix(a, m, bead0, nbead);  // (its barrier also shows the state and the beads)
+  __syncthreads();
+  const float* s_mass = m.tpl_f + L.o_mass;
+  for (int step = 0; step < q.steps; step++) {
+    long long* acc = q.acc + (size_t)(step % 3) * q.acc_stride;
+    const bool drift = step > 0 || !q.forces_first;
+    if (threadIdx.x == 0) s_counter = 0;
+    if (drift) {
+      long long rx = 0, ry = 0, rz = 0;
+      for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+        const int s = fast_div(t, a.div_np), l = t - s * np, g = bead0 + t;
+        const long long c = own_c ? my_c : s_kc[l], del = bd ? 0 : S.delta_fx;
+        unsigned int* F = m.F + 9 * t;
+        long long Fx, Fy, Fz;
+        get_fx(F, Fx, Fy, Fz);
+        long long vx = s_v[t] - S.vcom_fx[0], vy = s_v[nmax + t] - S.vcom_fx[1], vz = s_v[2 * nmax + t] - S.vcom_fx[2];
+        if (bd) {
+          long long r[3];
+          brownian_draws(d, P, S.lcg, w.sys, g, l, vx, vy, vz, r);
+          rx += r[0];
+          ry += r[1];
+          rz += r[2];
+        }
+        vx = vx - mul_shr(vx, del, 62) + mul_shr(Fx, c, 56);
+        vy = vy - mul_shr(vy, del, 62) + mul_shr(Fy, c, 56);
+        vz = vz - mul_shr(vz, del, 62) + mul_shr(Fz, c, 56);
+        s_v[t] = vx;
+        s_v[nmax + t] = vy;
+        s_v[2 * nmax + t] = vz;
+        const long long X = (long long)((unsigned long long)s_x[t] + (unsigned long long)mul_shr(vx, P.drift_fx, 40));
+        const long long Y = (long long)((unsigned long long)s_x[nmax + t] + (unsigned long long)mul_shr(vy, P.drift_fx, 40));
+        const long long Z = (long long)((unsigned long long)s_x[2 * nmax + t] + (unsigned long long)mul_shr(vz, P.drift_fx, 40));
+        s_x[t] = X;
+        s_x[nmax + t] = Y;
+        s_x[2 * nmax + t] = Z;
+        const int4 p = make_int4(hi_word(X), hi_word(Y), hi_word(Z), l);
+        m.pos[t] = p;
+        __stcg(&d.pos32[g], p);
+#pragma unroll
+        for (int k = 0; k < 9; k++) F[k] = 0u;
+      }
+      if (bd) {
+        rx = warp_sum_ll(rx);
+        ry = warp_sum_ll(ry);
+        rz = warp_sum_ll(rz);
+        if (lane == 0 && wid * 32 < nbead) {
+          unsigned long long* r = reinterpret_cast<unsigned long long*>(acc + 8 * w.sys + 4);
+          atomicAdd(r, (unsigned long long)rx);
+          atomicAdd(r + 1, (unsigned long long)ry);
+          atomicAdd(r + 2, (unsigned long long)rz);
+        }
+        __threadfence();
+      }
+      moved.target += gridDim.x;
+      __syncthreads();
+      if (threadIdx.x == 0) moved.arrive();
+    }
+    for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+      const int s = fast_div(t, a.div_np), l = t - s * np;
+      force_rel(m, np, s, l, m.pos[t], m.pos[s * np + P.center_local], m.w[l], unit);
+    }
+    __syncthreads();
+    force_terms<true>(a, P, m, w, nbead, bead0, &s_counter, [&] {
+      if (drift) {
+        if (lane == 0) moved.wait(&s_abort);
+        __syncwarp();
+      }
+    });
+    if (bd) {  // the step's random forces: their sum over the system
+      if (threadIdx.x < 3) {
+        if (drift) {
+          moved.wait(&s_abort);
+          s_sum[4 + threadIdx.x] = __ldcg(acc + 8 * w.sys + 4 + threadIdx.x);
+        } else {
+          s_sum[4 + threadIdx.x] = S.fran_sum[threadIdx.x];
+        }
+        s_sum[4 + threadIdx.x] = __double2ll_rn((double)s_sum[4 + threadIdx.x] * S.inv_n);  // mean
+      }
+    }
+    __syncthreads();
+    if (s_abort) return;  // uniform: nothing sets it between the barrier and here but a failed wait
+    force_gather(a, m, nbead, bead0);
+    __syncthreads();
+    long long ke_acc = 0, px_acc = 0, py_acc = 0, pz_acc = 0;
+    for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+      const int s = fast_div(t, a.div_np), l = t - s * np, g = bead0 + t;
+      unsigned int* F = m.F + 9 * t;
+      long long Fx = limbs_value(F), Fy = limbs_value(F + 3), Fz = limbs_value(F + 6);
+      if (bd) {
+        const long long N = a.n_beads_total;
+        Fx += a.fran[g] - s_sum[4] + a.fdrag[g];
+        Fy += a.fran[N + g] - s_sum[5] + a.fdrag[N + g];
+        Fz += a.fran[2 * N + g] - s_sum[6] + a.fdrag[2 * N + g];
+      }
+      put_fx(F, Fx, Fy, Fz);
+      const long long c = own_c ? my_c : s_kc[l], del = S.delta_fx;
+      long long vx = s_v[t], vy = s_v[nmax + t], vz = s_v[2 * nmax + t];
+      vx = vx - mul_shr(vx, del, 62) + mul_shr(Fx, c, 56);
+      vy = vy - mul_shr(vy, del, 62) + mul_shr(Fy, c, 56);
+      vz = vz - mul_shr(vz, del, 62) + mul_shr(Fz, c, 56);
+      s_v[t] = vx;
+      s_v[nmax + t] = vy;
+      s_v[2 * nmax + t] = vz;
+      px_acc += vx;
+      py_acc += vy;
+      pz_acc += vz;
+      const float ux = vel_to_f32(vx), uy = vel_to_f32(vy), uz = vel_to_f32(vz);
+      const float v2 = ux * ux + uy * uy + uz * uz;
+      if (!(v2 < 1.0e12f)) atomicOr(a.err, kErrNonFinite);  // |v| beyond 1e6: a blown-up run
+      ke_acc += f32_to_fx32(0.5f * s_mass[l] * v2);
+    }
+    // the CTA's sums by its working warps, then the system's
+    if (wid * 32 < nbead) {
+      ke_acc = warp_sum_ll(ke_acc);
+      px_acc = warp_sum_ll(px_acc);
+      py_acc = warp_sum_ll(py_acc);
+      pz_acc = warp_sum_ll(pz_acc);
+      if (lane == 0) {
+        m.red[wid * 4 + 0] = ke_acc;
+        m.red[wid * 4 + 1] = px_acc;
+        m.red[wid * 4 + 2] = py_acc;
+        m.red[wid * 4 + 3] = pz_acc;
+      }
+    }
+    __syncthreads();
+    summed.target += gridDim.x;
+    unsigned int chain_pre = 0;
+    if (wid == 0) {
+      // the next step's sums start from zero: their buffer was last read two steps ago, and every
+      // CTA has passed a barrier since
+      if (blockIdx.x == 0)
+        for (int k = lane; k < 8 * q.n_sys; k += 32) q.acc[(size_t)((step + 1) % 3) * q.acc_stride + k] = 0;
+      if (lane < 4) {
+        long long x = 0;
+        for (int k = 0; k < nw && k * 32 < nbead; k++) x += m.red[4 * k + lane];
+        atomicAdd(reinterpret_cast<unsigned long long*>(acc + 8 * w.sys + lane), (unsigned long long)x);
+      }
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) summed.arrive();
+      __syncwarp();
+      chain_pre = nhc_pre_warp(S, lane, chain_scratch);  // while the other CTAs arrive
+      if (lane < 4) {
+        summed.wait(&s_abort);
+        s_sum[lane] = __ldcg(acc + 8 * w.sys + lane);
+      }
+    }
+    __syncthreads();
+    if (s_abort) return;
+    step_tail<false>(a, P, w.sys, S, s_sum, chain_scratch, chain_pre);
+    __syncthreads();
+    // the next kicks' coefficients: a thread's only bead's stays in its register
+    if (own_c) {
+      if ((int)threadIdx.x < nbead && !nhc_kick_coefficient(S.kick_c0, inv_m, my_c)) atomicOr(a.err, kErrNonFinite);
+    } else {
+      for (int l = threadIdx.x; l < np; l += blockDim.x) {
+        long long c = 0;
+        if (!nhc_kick_coefficient(S.kick_c0, s_im[l], c)) atomicOr(a.err, kErrNonFinite);
+        s_kc[l] = c;
+      }
+      __syncthreads();
+    }
+  }
+  if (own_c) {
+    if ((int)threadIdx.x < np) s_kc[threadIdx.x] = my_c;  // (np <= nbead: the first subunit's beads)
+    __syncthreads();
+  }
+  // results back to global memory
+  for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+    const int g = bead0 + t;
+    d.px[g] = s_x[t];
+    d.py[g] = s_x[nmax + t];
+    d.pz[g] = s_x[2 * nmax + t];
+    a.vx[g] = s_v[t];
+    a.vy[g] = s_v[nmax + t];
+    a.vz[g] = s_v[2 * nmax + t];
+    long long Fx, Fy, Fz;
+    get_fx(m.F + 9 * t, Fx, Fy, Fz);
+    a.fx[g] = Fx;
+    a.fy[g] = Fy;
+    a.fz[g] = Fz;
+  }
+  if (w.sub_begin == P.sub0) {  // the CTA of the system's first subunit
+    int4* dst = reinterpret_cast<int4*>(a.state + w.sys);
+    const int4* src = reinterpret_cast<const int4*>(&S);
+    for (int t = threadIdx.x; t < (int)(sizeof(SysState) / 16); t += blockDim.x) dst[t] = src[t];
+    for (int l = threadIdx.x; l < np; l += blockDim.x) a.kick_c[(size_t)w.sys * np + l] = s_kc[l];
+  }
+  // the last CTA to leave clears the counters and sums for the next launch
+  __shared__ bool s_last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(q.count + 2, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (s_last) {
+    for (int k = threadIdx.x; k < (int)(3 * q.acc_stride); k += blockDim.x) q.acc[k] = 0;
+    if (threadIdx.x == 0) {
+      q.count[0] = q.count[1] = q.count[2] = 0u;
+    }
   }
 }
 
@@ -466,6 +809,28 @@ void launch_forces(const ForceArgs& a, int grid, int block, size_t smem, cudaStr
 }
 void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s) {
   k_drift<<<grid, block, 0, s>>>(a);
+}
+// shared memory of k_window: the force kernel's, then per-bead state, kick coefficients, system state
+size_t window_smem_bytes(size_t force_bytes, int subs, int np) {
+  return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (6 * (size_t)subs * np + 2 * (size_t)((np + 1) & ~1)) +
+         sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat);
+}
+cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
+                          cudaStream_t s) {
+  void* args[] = {const_cast<ForceArgs*>(&a), const_cast<DriftArgs*>(&d), const_cast<WindowArgs*>(&q)};
+  return cudaLaunchCooperativeKernel((const void*)k_window, dim3(grid), dim3(block), args, smem, s);
+}
+cudaError_t window_wave_ctas(int threads, size_t smem, int* ctas) {
+  *ctas = 0;
+  cudaError_t e = cudaFuncSetAttribute(k_window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_window, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess) return e;
+  int per_sm = 0, dev = 0, sms = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_window, threads, smem)) != cudaSuccess) return e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  *ctas = per_sm * sms;
+  return cudaSuccess;
 }
 void launch_state_in(const StateArgs& a, int grid, int block, cudaStream_t s) {
   k_state_in<<<grid, block, 0, s>>>(a);

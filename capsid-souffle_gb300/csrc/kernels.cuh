@@ -14,8 +14,8 @@ struct CellArgs {
   const SysParams* sys;
   const int* sub_sys;     // [S_total] system of each subunit
   int np, n_sub_total;
-  int* cell_count;        // [total cells]
-  int* cell_start;        // [total cells + 1]
+  int* cell_count;        // [total cells], then the number of subunits placed so far
+  int* cell_start;        // [total cells] first entry of the cell in cell_subs
   int* sub_rank;          // [S_total]
   int* sub_cell;          // [S_total]
   int* cell_subs;         // [S_total]
@@ -117,6 +117,17 @@ struct DriftArgs {
   long long n_total = 0;
 };
 
+// The window kernel: steps per launch, its grid barrier and sums.
+struct WindowArgs {
+  int steps;
+  int forces_first;        // the first step's drift has run (and the pair lists were rebuilt after it)
+  int n_sys;
+  unsigned int* count;     // [3] arrivals at the step's two barriers, CTAs that have left; zero between launches
+  long long* acc;          // [3][acc_stride]: per system 8 sums (kinetic energy, momentum, random forces)
+  size_t acc_stride;       // 8 n_sys
+  size_t force_bytes;      // the force kernel's part of the shared memory, 16-byte multiple
+};
+
 struct StateArgs {
   const SysParams* sys;
   SysState* state;
@@ -171,6 +182,7 @@ struct EnergyArgs {
   unsigned int* ticket;    // CTAs of k_energy_totals done, zero between calls
   // the grid of subunit centres (large systems only)
   const int* sub_cell_start = nullptr;
+  const int* sub_cell_count = nullptr;
   const int* cell_subs = nullptr;
   // encapsulation big beads of the system: fixed-point positions [3][total], the big-bead parts
   // of ne and ce per subunit bead [n]
@@ -185,17 +197,23 @@ cudaError_t set_energy_smem(const TplLayout& L);
 bool energy_needs_cells(int n_sub);
 
 void launch_cells_count(const CellArgs& a, int grid, int block, cudaStream_t s);
-void launch_cells_scan(const CellArgs& a, cudaStream_t s);
+void launch_cells_place(const CellArgs& a, cudaStream_t s);
 void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s);
 void launch_cells_sort(const CellArgs& a, cudaStream_t s);
 void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s);
-void launch_pairs(const PairArgs& a, int n_sub, size_t smem, cudaStream_t s);
+void launch_pairs(const PairArgs& a, int n_sub, bool search, cudaStream_t s);
+// k_pairs finds the candidates itself (no k_cells_* and k_candidates before it)
+bool pairs_search(int max_sub, int cand_cap);
 // k_pairs' chunk of candidates staged together, and its dynamic shared memory
 constexpr int kPairChunkMax = 32;
 int pair_chunk(int np, int words);
 size_t pair_smem_bytes(int np, int words, int chunk);
 void launch_forces(const ForceArgs& a, int grid, int block, size_t smem, cudaStream_t s);
 void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s);
+size_t window_smem_bytes(size_t force_bytes, int subs, int np);
+cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
+                          cudaStream_t s);
+cudaError_t window_wave_ctas(int threads, size_t smem, int* ctas);
 void launch_state_in(const StateArgs& a, int grid, int block, cudaStream_t s);
 void launch_state_out(const StateArgs& a, int grid, int block, cudaStream_t s);
 void launch_energies(const EnergyArgs& a, int n, cudaStream_t s);

@@ -37,58 +37,46 @@ __global__ void k_cells_count(CellArgs a) {
   a.sub_rank[s] = atomicAdd(&a.cell_count[cell], 1);
 }
 
-// Exclusive scan of cell counts, one CTA per system: a system's cells hold only its own
-// subunits, which are contiguous, so its scan starts at the system's first subunit and the
-// segments line up into one global cell_start array.  Each thread takes a run of kScanPer cells
-// (their loads in flight together) and the runs' sums are scanned across the CTA.
-constexpr int kScanPer = 8;
-__global__ void __launch_bounds__(1024) k_cells_scan(CellArgs a) {
-  __shared__ int warp_sums[32];
-  __shared__ int carry;
-  const SysParams& P = a.sys[blockIdx.x];
-  const int c0 = P.cell0, nc = P.ncell * P.ncell * P.ncell;
-  if (threadIdx.x == 0) carry = P.sub0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int base = 0; base < nc; base += blockDim.x * kScanPer) {
-    const int i0 = base + threadIdx.x * kScanPer;
-    int v[kScanPer];
-    int sum = 0;
+// A segment of cell_subs for every cell: each CTA scans its cells' counts and reserves room for all of
+// them with one atomic, so the segments' order depends on scheduling (the candidates are sorted
+// at the end, and k_cells_sort orders the cells' subunits, so nothing else does).  One CTA per
+// system scanning its cells in order took 57 us for the 79,507 cells of 20,000 subunits.
+constexpr int kPlacePer = 4;
+__global__ void __launch_bounds__(256) k_cells_place(CellArgs a) {
+  __shared__ int warp_sums[8];
+  __shared__ int s_base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int i0 = (blockIdx.x * 256 + threadIdx.x) * kPlacePer;
+  int v[kPlacePer], sum = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-      v[k] = (i0 + k < nc) ? a.cell_count[c0 + i0 + k] : 0;
-      sum += v[k];
-    }
-    int x = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      int w = (lane < nw) ? warp_sums[lane] : 0;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      warp_sums[lane] = w;  // inclusive
-    }
-    __syncthreads();
-    int excl = x - sum + (wid > 0 ? warp_sums[wid - 1] : 0) + carry;
-#pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-      if (i0 + k < nc) a.cell_start[c0 + i0 + k] = excl;
-      excl += v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl;  // the pass's end: carry + all its counts
-    __syncthreads();
+  for (int k = 0; k < kPlacePer; k++) {
+    v[k] = i0 + k < a.total_cells ? a.cell_count[i0 + k] : 0;
+    sum += v[k];
   }
-  // the end sentinel of the last system (other systems' ends are the next system's first start)
-  if (threadIdx.x == 0 && c0 + nc == a.total_cells) a.cell_start[a.total_cells] = carry;
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sums[wid] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int w = 0; w < 8; w++) {
+      const int t = warp_sums[w];
+      warp_sums[w] = total;
+      total += t;
+    }
+    s_base = total > 0 ? atomicAdd(a.cell_count + a.total_cells, total) : 0;
+  }
+  __syncthreads();
+  int off = s_base + warp_sums[wid] + x - sum;
+#pragma unroll
+  for (int k = 0; k < kPlacePer; k++) {
+    if (i0 + k < a.total_cells) a.cell_start[i0 + k] = off;
+    off += v[k];
+  }
 }
 
 __global__ void k_cells_scatter(CellArgs a) {
@@ -103,7 +91,7 @@ __global__ void k_cells_sort(CellArgs a) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.total_cells) return;
   int* b = a.cell_subs + a.cell_start[c];
-  const int m = a.cell_start[c + 1] - a.cell_start[c];
+  const int m = a.cell_count[c];
   for (int i = 1; i < m; i++) {
     const int v = b[i];
     int k = i - 1;
@@ -143,7 +131,7 @@ __global__ void __launch_bounds__(128) k_candidates(CandArgs a) {
     const int gz = (n < 3) ? dz : (cz + dz - 1 + n) % n;
     const int cell = p.cell0 + (gx * n + gy) * n + gz;
     s0 = a.c.cell_start[cell];
-    s1 = a.c.cell_start[cell + 1];
+    s1 = s0 + a.c.cell_count[cell];
   }
   const int4 pci = a.pos32[ci];
   const float pre2f = (float)p.pre2, marg = pair_margin(pre2f);
@@ -191,346 +179,287 @@ __global__ void __launch_bounds__(128) k_candidates(CandArgs a) {
 
 
 
-// One CTA per subunit i; thread t owns bead rows t, t + blockDim, ... (at most two: blockDim is
-// np rounded up to whole warps, at most 128, so that a one-wave grid holds every subunit).
-// Candidates are taken in ascending j, so each row's entries come out in ascending global id.
-// Runs of ordinary candidates are staged together (a chunk): their high words load in one round,
-// every (candidate, row) item computes its partner mask in parallel, and each row then appends
-// the chunk's partners in order -- a handful of barriers per chunk instead of per candidate.
-// Subunit i's own block (intra bits, each unordered pair once) and blocks with the stale-r2
-// semantics of the system's subunit 0 take the per-block path, one candidate at a time.
+// r2 < lim from the exact fixed-point differences of beads ga and gb (global indices); out of line:
+// only separations within the FP32 test's margin come here.
+__device__ __noinline__ bool pair_exact(const long long* px, const long long* py, const long long* pz, double fx, int ga,
+                                        int gb, double lim) {
+  const double x = fixed_diff(px[ga], px[gb], fx), y = fixed_diff(py[ga], py[gb], fx), z = fixed_diff(pz[ga], pz[gb], fx);
+  return x * x + y * y + z * z < lim;
+}
+
+// The pair lists of subunit i, one CTA of 128 threads (64 when the candidates are given and a block
+// has at most 96 items: many subunits, so throughput counts).  Candidates are taken in ascending j, so
+// each row's entries come out in ascending global id.
+//   search   (kSearch: systems of at most kSearchSubs subunits) the candidates by testing every
+//            subunit of the system, in order; otherwise they come from k_candidates
+//   stage    a chunk of candidates that stay in the pair list (far ones skipped by a warp ballot),
+//            their high words in shared memory, and each one's radius about its centre bead
+//   masks    every (candidate, row, 32 partners) item at once: FP32 test with a margin, exact FP64
+//            inside it; a row farther than R_j + r_list from a candidate's centre has no pair with
+//            it (triangle inequality, padded far beyond the rounding)
+//   stale    blocks with the system's subunit 0: the stale-distance entries of src/functions.cpp:97
+//            replaced (below)
+//   append   per row the offsets of the chunk's items, then every item writes its ids
+// Subunit i's own block gives the intra bits instead (electrostatic pairs only, :94-96).
+//
+// Bound by the latency of its rounds of loads and barriers, not by the tests: per-row appending by
+// one thread each, two threads' worth of rows per lane and a per-candidate FP64 path for every
+// block of subunit 0 took 48 us at 2,688 beads and 47 us at 84,000 in one launch behind four others;
+// now 14 us (its search included) and 23 us; a whole rebuild 43 -> 13 us, 64 -> 44 us, and 183 -> 135
+// us at 840,000.
+//
+// The stale-r2 reuse: the reference's test compares a local index with a global id, so a distance is
+// recomputed unless (i is subunit 0 and ii is its centre) or (j is subunit 0 and jj is its centre);
+// otherwise the r2 of the most recently computed pair (row-major over the visited pairs of the
+// block) is reused, starting from the centre-centre distance (or 0 when i == j).  So the centre
+// row of subunit 0 takes one value for all its entries -- the last computed pair of the rows
+// before it -- and every other row's entry in the centre column of subunit 0 takes the computed
+// pair before it in the row, or, when there is none, that of the rows before.
+constexpr int kSearchSubs = 1024;
+template <bool kSearch>
 __global__ void __launch_bounds__(128) k_pairs(PairArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  int4* s32 = reinterpret_cast<int4*>(smem_raw);                   // [np] 16-byte entries first
-  long long* sx = reinterpret_cast<long long*>(s32 + a.np);
-  long long* sy = sx + a.np;
-  long long* sz = sy + a.np;
-  double* row_last = reinterpret_cast<double*>(sz + a.np);         // [np] quirk pass
-  int* row_has = reinterpret_cast<int*>(row_last + a.np);          // [np]
-  float* sq = reinterpret_cast<float*>(row_has + a.np);           // [np]
-  unsigned int* s_imask = reinterpret_cast<unsigned int*>(sq + a.np);  // [np * words] intra bits
+  const int np = a.np, words = a.words, chunk = a.chunk;
+  int4* s_own = reinterpret_cast<int4*>(smem_raw);                                        // [np]
+  int4* c32 = s_own + np;                                                                 // [chunk np]
+  unsigned int* cmask = reinterpret_cast<unsigned int*>(c32 + (size_t)chunk * np);        // [chunk np words]
+  int* coff = reinterpret_cast<int*>(cmask + (size_t)chunk * np * words);                 // [chunk np]
+  int* s_n = coff + chunk * np;                                                           // [np] inter entries so far
+  int* s_cand = s_n + np;                                                                 // [cand_cap] (kSearch)
+  __shared__ unsigned int s_chg[kMaxNp / 32];  // charged beads
+  __shared__ int s_cj[kPairChunkMax], s_ctl[2], s_word[5];
+  __shared__ float s_cR[kPairChunkMax];
 
   const int i = blockIdx.x;
-  const int sysid = a.sub_sys[i];
-  const SysParams& p = a.sys[sysid];
-  const int np = a.np;
+  const SysParams& p = a.sys[a.sub_sys[i]];
   const int i_local = i - p.sub0;  // subunit index inside its system
-  const float unit = p.unit32;
-  const float nl2f = p.nl2_f;
-  const float margin = pair_margin(nl2f);
-  const int ncand = a.cand_count[i];
-  const int* cand = a.cand + (size_t)i * a.cand_cap;
-
-  for (int t = threadIdx.x; t < np; t += blockDim.x) sq[t] = a.q[t];
-
-  // per-row state held in registers for up to 2 rows per thread (np <= 256, blockDim 128)
-  int inter_n[2] = {0, 0};
-  unsigned int* mask_rows = a.intra_mask + (size_t)i * np * a.words;
-  for (int t = threadIdx.x; t < np * a.words; t += blockDim.x) mask_rows[t] = 0u;
-
-  const int ci_global = i * np + p.center_local;
-  const long long cxi = a.px[ci_global], cyi = a.py[ci_global], czi = a.pz[ci_global];
-
-  // Exact shortcut by the triangle inequality, from candidate j's radius about its centre bead
-  // (float on the high words, padded by eps far beyond their rounding): a row farther than
-  // R_j + r_list from j's centre has no pair with j.  Cases touched by the stale-r2 quirk skip it.
-  __shared__ float s_Rj;
+  const int cl = p.center_local;
+  const float unit = p.unit32, nl2f = p.nl2_f, margin = pair_margin(nl2f);
   const float r_list = sqrtf(nl2f), eps = 1e-3f * (1.0f + r_list);
-  for (int t = threadIdx.x; t < np * a.words; t += blockDim.x) s_imask[t] = 0u;
-
-  const bool skip_far = a.cand_far && *a.far_ok;
-  // chunk staging (after the per-block area, 16-byte aligned): the own rows' high words, the
-  // chunk's candidates' high words, and a mask of partners per (candidate, row)
-  const size_t blk_bytes = (size_t)np * (sizeof(int4) + 3 * sizeof(long long) + sizeof(double) + sizeof(int) +
-                                         sizeof(float)) + sizeof(unsigned int) * (size_t)np * a.words;
-  int4* s_own = reinterpret_cast<int4*>(smem_raw + ((blk_bytes + 15) & ~(size_t)15));
-  int4* c32 = s_own + np;
-  unsigned int* cmask = reinterpret_cast<unsigned int*>(c32 + (size_t)a.chunk * np);
-  __shared__ int s_cj[kPairChunkMax];
-  __shared__ float s_cR[kPairChunkMax];
-  for (int t = threadIdx.x; t < np; t += blockDim.x) s_own[t] = a.pos32[(size_t)i * np + t];
-  const bool cta_quirk = p.quirks && i_local == 0;  // every block of the system's subunit 0
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __shared__ int s_ctl[3];  // candidates consumed, chunk size, candidate for the per-block path (-1: none)
+  unsigned int* mask_rows = a.intra_mask + (size_t)i * np * words;
+  for (int t = threadIdx.x; t < np; t += blockDim.x) {
+    s_own[t] = a.pos32[(size_t)i * np + t];
+    s_n[t] = 0;
+  }
+  for (int t = threadIdx.x; t < np * words; t += blockDim.x) mask_rows[t] = 0u;
+  for (int w = wid; w < words; w += nw) {
+    const int l = 32 * w + lane;
+    const unsigned int m = __ballot_sync(0xffffffffu, l < np && a.q[l < np ? l : 0] != 0.0f);
+    if (lane == 0) s_chg[w] = m;
+  }
+  int ncand = 0;
+  if (kSearch) {
+    // centre distances to every subunit of the system (src/functions.cpp:80-91)
+    const int ci = i * np + cl;
+    const int4 pci = a.pos32[ci];
+    const float pre2f = (float)p.pre2, marg = pair_margin(pre2f);
+    for (int base = 0; base < p.n_sub; base += 128) {
+      const int j = p.sub0 + base + threadIdx.x;
+      bool take = false;
+      if (base + (int)threadIdx.x < p.n_sub) {
+        const int cj = j * np + cl;
+        const int4 pcj = a.pos32[cj];
+        const float fx = hi_diff(pci.x, pcj.x, unit), fy = hi_diff(pci.y, pcj.y, unit), fz = hi_diff(pci.z, pcj.z, unit);
+        const float r2f = fx * fx + fy * fy + fz * fz;
+        take = j == i || (fabsf(r2f - pre2f) > marg ? r2f < pre2f : pair_exact(a.px, a.py, a.pz, p.fx_to_len, ci, cj, p.pre2));
+      }
+      const unsigned int m = __ballot_sync(0xffffffffu, take);
+      if (lane == 0) s_word[wid] = __popc(m);
+      __syncthreads();
+      int off = ncand, total = 0;
+      for (int q = 0; q < 4; q++) {
+        if (q < wid) off += s_word[q];
+        total += s_word[q];
+      }
+      off += __popc(m & ((1u << lane) - 1u));
+      if (take && off < a.cand_cap) s_cand[off] = j;
+      ncand += total;
+      __syncthreads();
+    }
+    if (ncand > a.cand_cap) {
+      if (threadIdx.x == 0) atomicOr(a.err, kErrCandOverflow);
+      ncand = a.cand_cap;
+    }
+  } else {
+    ncand = a.cand_count[i];
+  }
+  const int* cand = kSearch ? s_cand : a.cand + (size_t)i * a.cand_cap;
+  const bool skip_far = !kSearch && a.cand_far && *a.far_ok;
+
+  // partners of row ii of this subunit among 32 beads w0 .. of the staged subunit at b32 (global
+  // subunit j): FP32 decisions, then the few within the margin exactly
+  auto test_word = [&](int ii, const int4* b32, int j, int w0) {
+    const int4 pi = s_own[ii];
+    const int n = min(32, np - w0);
+    unsigned int bits = 0, unsure = 0;
+#pragma unroll 4
+    for (int b = 0; b < n; b++) {
+      const int4 pj = b32[w0 + b];
+      const float dx = hi_diff(pi.x, pj.x, unit), dy = hi_diff(pi.y, pj.y, unit), dz = hi_diff(pi.z, pj.z, unit);
+      const float r2f = dx * dx + dy * dy + dz * dz;
+      bits |= (unsigned int)(r2f < nl2f) << b;
+      unsure |= (unsigned int)!(fabsf(r2f - nl2f) > margin) << b;
+    }
+    for (; unsure; unsure &= unsure - 1) {
+      const int b = __ffs(unsure) - 1;
+      const bool in = pair_exact(a.px, a.py, a.pz, p.fx_to_len, i * np + ii, j * np + w0 + b, p.nl2);
+      bits = (bits & ~(1u << b)) | (unsigned int)in << b;
+    }
+    return bits;
+  };
+  auto test_one = [&](int ii, const int4* b32, int j, int jj) {
+    const int4 pi = s_own[ii], pj = b32[jj];
+    const float dx = hi_diff(pi.x, pj.x, unit), dy = hi_diff(pi.y, pj.y, unit), dz = hi_diff(pi.z, pj.z, unit);
+    const float r2f = dx * dx + dy * dy + dz * dz;
+    if (fabsf(r2f - nl2f) > margin) return r2f < nl2f;
+    return pair_exact(a.px, a.py, a.pz, p.fx_to_len, i * np + ii, j * np + jj, p.nl2);
+  };
+
   int c = 0;
   while (c < ncand) {
-    __syncthreads();  // the previous chunk's readers are done
+    __syncthreads();  // the previous chunk's readers are done (and the search's list is complete)
     // Warp 0 looks at the next 32 candidates: far ones (left to the surrogate, or beyond every
-    // cut-off) are skipped; the chunk takes up to a.chunk ordinary candidates before the first
-    // one that needs the per-block path (subunit i itself, or a block with the stale-r2
-    // semantics); with no ordinary candidate before it, that one goes to the per-block path.
+    // cut-off) are skipped, up to `chunk` others are taken.
     if (wid == 0) {
       const int cc = c + lane;
       const bool valid = cc < ncand;
-      int j = -1;
-      bool far = false;
-      if (valid) {
-        j = cand[cc];
-        far = skip_far && a.cand_far[(size_t)i * a.cand_cap + cc];
-      }
-      const bool slow = valid && !far && (j == i || cta_quirk || (p.quirks && j == p.sub0));
-      const unsigned int sb = __ballot_sync(0xffffffffu, slow);
-      const unsigned int nb = __ballot_sync(0xffffffffu, valid && !far && !slow);
-      const int fs = sb ? __ffs(sb) - 1 : 32;  // first slow lane
-      const unsigned int take = fs < 32 ? nb & ((1u << fs) - 1u) : nb;
+      const int j = valid ? cand[cc] : -1;
+      const bool far = valid && skip_far && a.cand_far[(size_t)i * a.cand_cap + cc];
+      const unsigned int take = __ballot_sync(0xffffffffu, valid && !far);
       const int rank = __popc(take & ((1u << lane) - 1u));
-      const bool mine = ((take >> lane) & 1u) && rank < a.chunk;
+      const bool mine = ((take >> lane) & 1u) && rank < chunk;
       if (mine) s_cj[rank] = j;
-      const int nk = min(__popc(take), a.chunk);
-      int consumed, slow_j = -1;
-      if (__popc(take) > a.chunk) {  // full chunk: up to and including its last candidate
-        const unsigned int last = __ballot_sync(0xffffffffu, mine && rank == a.chunk - 1);
-        consumed = __ffs(last);
-      } else if (fs < 32) {
-        consumed = nk > 0 ? fs : fs + 1;
-        if (nk == 0) slow_j = __shfl_sync(0xffffffffu, j, fs);
-      } else {
-        consumed = min(32, ncand - c);
-      }
+      const unsigned int last = __ballot_sync(0xffffffffu, mine && rank == chunk - 1);
       if (lane == 0) {
-        s_ctl[0] = consumed;
-        s_ctl[1] = nk;
-        s_ctl[2] = slow_j;
+        s_ctl[0] = __popc(take) > chunk ? __ffs(last) : min(32, ncand - c);  // candidates consumed
+        s_ctl[1] = min(__popc(take), chunk);
       }
     }
     __syncthreads();
     const int nk = s_ctl[1];
-    const int slow_j = s_ctl[2];
     c += s_ctl[0];
-    if (nk > 0) {
-      for (int t = threadIdx.x; t < nk * np; t += blockDim.x) {
-        const int k = t / np;
-        c32[t] = a.pos32[(size_t)s_cj[k] * np + (t - k * np)];
-      }
-      __syncthreads();
-      // each candidate's radius about its centre bead, warp per candidate
-      for (int k = wid; k < nk; k += nw) {
-        const int4 pc = c32[k * np + p.center_local];
-        float m = 0.0f;
-        for (int t = lane; t < np; t += 32) {
-          const int4 pt = c32[k * np + t];
-          const float dx = hi_diff(pt.x, pc.x, unit), dy = hi_diff(pt.y, pc.y, unit), dz = hi_diff(pt.z, pc.z, unit);
-          m = fmaxf(m, sqrtf(dx * dx + dy * dy + dz * dz));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) s_cR[k] = m;
-      }
-      __syncthreads();
-      // partner masks of every (candidate, row) item: the same float test with its margin and
-      // exact fallback, and the same reach shortcut, as the per-block path
-      for (int t = threadIdx.x; t < nk * np; t += blockDim.x) {
-        const int k = t / np, ii = t - k * np;
-        unsigned int* mk = cmask + (size_t)t * a.words;
-        const int4* cj32 = c32 + k * np;
-        const int4 pi = s_own[ii];
-        const int4 pc = cj32[p.center_local];
-        const float reach = s_cR[k] + r_list + eps;
-        const float ex = hi_diff(pi.x, pc.x, unit), ey = hi_diff(pi.y, pc.y, unit), ez = hi_diff(pi.z, pc.z, unit);
-        const bool skip = ex * ex + ey * ey + ez * ez > reach * reach;
-        const int gi = i * np + ii, jbase = s_cj[k] * np;
-        for (int w0 = 0; w0 < np; w0 += 32) {
-          unsigned int bits = 0;
-          if (!skip) {
-            const int w1 = min(np, w0 + 32);
-            for (int jj = w0; jj < w1; jj++) {
-              const int4 pj = cj32[jj];
-              const float dx = hi_diff(pi.x, pj.x, unit), dy = hi_diff(pi.y, pj.y, unit), dz = hi_diff(pi.z, pj.z, unit);
-              const float r2f = dx * dx + dy * dy + dz * dz;
-              bool in;
-              if (fabsf(r2f - nl2f) > margin) {
-                in = r2f < nl2f;
-              } else {
-                const int gj = jbase + jj;
-                const double ex = fixed_diff(a.px[gi], a.px[gj], p.fx_to_len);
-                const double ey = fixed_diff(a.py[gi], a.py[gj], p.fx_to_len);
-                const double ez = fixed_diff(a.pz[gi], a.pz[gj], p.fx_to_len);
-                in = ex * ex + ey * ey + ez * ez < p.nl2;
-              }
-              if (in) bits |= 1u << (jj - w0);
-            }
-          }
-          mk[w0 >> 5] = bits;
-        }
-      }
-      __syncthreads();
-      // ids in ascending global order: candidates in order, partners in bead order
-      for (int r = 0, ii = threadIdx.x; ii < np; ii += blockDim.x, r++) {
-        const int gi = i * np + ii;
-        int n = inter_n[r];
-        for (int k = 0; k < nk; k++) {
-          const unsigned int* mk = cmask + (size_t)(k * np + ii) * a.words;
-          const int jbase = s_cj[k] * np;
-          for (int w = 0; w < a.words; w++) {
-            unsigned int bits = mk[w];
-            while (bits) {
-              const int b = __ffs(bits) - 1;
-              bits &= bits - 1;
-              if (n < a.inter_cap) a.inter_ids[(size_t)gi * a.inter_cap + n] = jbase + (w << 5) + b;
-              n++;
-            }
-          }
-        }
-        inter_n[r] = n;
-      }
-      continue;
-    }
-    if (slow_j < 0) continue;  // only far candidates in this window
-    // per-block path for candidate slow_j
-    const int j = slow_j;
-    __syncthreads();
-    if (threadIdx.x == 0) s_Rj = 0.0f;
-    for (int t = threadIdx.x; t < np; t += blockDim.x) {
-      int g = j * np + t;
-      sx[t] = a.px[g];
-      sy[t] = a.py[g];
-      sz[t] = a.pz[g];
-      s32[t] = a.pos32[g];
+    if (nk == 0) continue;  // only far candidates in this window
+    for (int t = threadIdx.x; t < nk * np; t += blockDim.x) {
+      const int k = t / np;
+      c32[t] = a.pos32[(size_t)s_cj[k] * np + (t - k * np)];
     }
     __syncthreads();
-    const int j_local = j - p.sub0;
-    const bool same = (j == i);
-    // exact squared distance between bead gi and staged bead jj of subunit j
-    auto d2_exact = [&](int gi, int jj) {
-      const double ex = fixed_diff(a.px[gi], sx[jj], p.fx_to_len);
-      const double ey = fixed_diff(a.py[gi], sy[jj], p.fx_to_len);
-      const double ez = fixed_diff(a.pz[gi], sz[jj], p.fx_to_len);
-      return ex * ex + ey * ey + ez * ez;
-    };
-    // r2 < r_list^2, decided in float unless within the margin of the cut-off
-    auto inside = [&](int gi, int4 pi, int jj) {
-      const int4 pj = s32[jj];
-      const float dx = hi_diff(pi.x, pj.x, unit), dy = hi_diff(pi.y, pj.y, unit), dz = hi_diff(pi.z, pj.z, unit);
-      const float r2f = dx * dx + dy * dy + dz * dz;
-      if (fabsf(r2f - nl2f) > margin) return r2f < nl2f;
-      return d2_exact(gi, jj) < p.nl2;
-    };
-    // The stale-r2 reuse of src/functions.cpp:97 can only trigger when subunit 0 of the system is
-    // involved.  The test there compares a local index with a global id, so a distance is
-    // recomputed unless (i is subunit 0 and ii is its centre) or (j is subunit 0 and jj is its
-    // centre); otherwise the r2 of the most recently computed pair (row-major over the block) is
-    // reused, starting from the centre-centre distance (or 0 when i == j).  Only two exact
-    // distances per row are ever needed for that: the row's last computed pair (carried into
-    // later rows) and the computed pair just before the stale column.
-    const bool quirk = p.quirks && (i_local == 0 || j_local == 0);
-    const int cl = p.center_local;
-    if (!same && !quirk) {  // radius of candidate j about its centre bead
-      const int4 pc = s32[cl];
-      for (int t = threadIdx.x; t < np; t += blockDim.x) {
-        const int4 pt = s32[t];
+    for (int k = wid; k < nk; k += nw) {  // each candidate's radius about its centre bead
+      const int4 pc = c32[k * np + cl];
+      float m = 0.0f;
+      for (int t = lane; t < np; t += 32) {
+        const int4 pt = c32[k * np + t];
         const float dx = hi_diff(pt.x, pc.x, unit), dy = hi_diff(pt.y, pc.y, unit), dz = hi_diff(pt.z, pc.z, unit);
-        atomicMax(reinterpret_cast<int*>(&s_Rj), __float_as_int(sqrtf(dx * dx + dy * dy + dz * dz)));
+        m = fmaxf(m, dx * dx + dy * dy + dz * dz);
       }
-      __syncthreads();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) s_cR[k] = sqrtf(m);
     }
-    const float reach_j = s_Rj + r_list + eps;
-    const bool i0 = quirk && (i_local == 0), j0 = quirk && (j_local == 0);
-    double init_r2 = 0.0;
-    if (quirk) {
-      if (!same) {
-        const int cj = j * np + cl;
-        const double ex = fixed_diff(cxi, a.px[cj], p.fx_to_len), ey = fixed_diff(cyi, a.py[cj], p.fx_to_len),
-                     ez = fixed_diff(czi, a.pz[cj], p.fx_to_len);
-        init_r2 = ex * ex + ey * ey + ez * ez;
+    __syncthreads();
+    const int items = nk * np * words;
+    const int rows = nk * np;  // items word by word: a warp's lanes have equally many partners to test
+    for (int t = threadIdx.x; t < items; t += blockDim.x) {
+      const int w = words == 1 ? 0 : t / rows, q = t - w * rows, k = q / np, ii = q - k * np;
+      const int j = s_cj[k];
+      const int4* b32 = c32 + k * np;
+      const int4 pi = s_own[ii], pc = b32[cl];
+      const float reach = s_cR[k] + r_list + eps;
+      const float ex = hi_diff(pi.x, pc.x, unit), ey = hi_diff(pi.y, pc.y, unit), ez = hi_diff(pi.z, pc.z, unit);
+      unsigned int bits = 0;
+      if (!(ex * ex + ey * ey + ez * ez > reach * reach)) bits = test_word(ii, b32, j, 32 * w);
+      if (j == i) {  // charged pairs of different beads
+        bits &= s_chg[w];
+        if ((ii >> 5) == w) bits &= ~(1u << (ii & 31));
+        if (!((s_chg[ii >> 5] >> (ii & 31)) & 1u)) bits = 0;
       }
-      for (int ii = threadIdx.x; ii < np; ii += blockDim.x) {  // pass 1
-        const int gi = i * np + ii;
-        const bool qi = sq[ii] != 0.0f;
-        double last = 0.0;
-        int has = 0;
-        if (!(i0 && ii == cl)) {
-          for (int jj = np - 1; jj >= 0; jj--) {
-            const bool cond = same ? (jj != ii && qi && sq[jj] != 0.0f) : true;
-            if (cond && !(j0 && jj == cl)) {
-              last = d2_exact(gi, jj);
-              has = 1;
-              break;
+      cmask[q * words + w] = bits;
+    }
+    __syncthreads();
+    if (p.quirks) {
+      for (int k = 0; k < nk; k++) {
+        const int j = s_cj[k];
+        const bool i0 = i_local == 0, j0 = j == p.sub0, same = j == i;
+        if (!i0 && !j0) continue;  // uniform
+        const int4* b32 = c32 + k * np;
+        auto visited = [&](int r, int w) {  // partners that the reference's loop looks at in row r
+          const unsigned int all = np - 32 * w >= 32 ? 0xffffffffu : (1u << (np - 32 * w)) - 1u;
+          if (!same) return all;
+          if (!((s_chg[r >> 5] >> (r & 31)) & 1u)) return 0u;
+          return s_chg[w] & ~((r >> 5) == w ? 1u << (r & 31) : 0u);
+        };
+        auto computed = [&](int r, int w) {  // ... and computes a distance for
+          if (i0 && r == cl) return 0u;
+          return visited(r, w) & ~(j0 && (cl >> 5) == w ? 1u << (cl & 31) : 0u);
+        };
+        for (int ii = threadIdx.x; ii < np; ii += blockDim.x) {
+          unsigned int* mk = cmask + (size_t)(k * np + ii) * words;
+          const bool row_stale = i0 && ii == cl;
+          if (!row_stale && !(j0 && ((visited(ii, cl >> 5) >> (cl & 31)) & 1u))) continue;
+          // the most recently computed pair (fr, fj): before the centre column in this row, else the
+          // last one of the rows before
+          int fr = -1, fj = -1;
+          if (!row_stale) {
+            for (int w = cl >> 5; w >= 0 && fj < 0; w--) {
+              const unsigned int m = computed(ii, w) & (w == (cl >> 5) ? (1u << (cl & 31)) - 1u : 0xffffffffu);
+              if (m) fj = 32 * w + 31 - __clz(m);
             }
+            if (fj >= 0) fr = ii;
           }
-        }
-        row_last[ii] = last;
-        row_has[ii] = has;
-      }
-      __syncthreads();
-    }
-    for (int r = 0, ii = threadIdx.x; ii < np; ii += blockDim.x, r++) {
-      const int gi = i * np + ii;
-      const int4 pi = a.pos32[gi];
-      const bool qi = sq[ii] != 0.0f;
-      double carried = init_r2;
-      if (quirk)
-        for (int k = ii - 1; k >= 0; k--)
-          if (row_has[k]) {
-            carried = row_last[k];
-            break;
-          }
-      if (same && !quirk) {
-        // each unordered pair once: row ii takes partners ii + d (mod np), d = 1 .. (np - 1) / 2,
-        // and d = np / 2 for ii < np / 2 when np is even (21 tests per row at np = 42).  The
-        // decision is symmetric in (ii, jj) in both the float and the exact test, so both rows
-        // get the bit the reference computes for each.
-        if (!qi) continue;
-        const int dmax = (np - 1) >> 1;
-        const int dlast = ((np & 1) == 0 && ii < (np >> 1)) ? (np >> 1) : dmax;
-        for (int dd = 1; dd <= dlast; dd++) {
-          int jj = ii + dd;
-          if (jj >= np) jj -= np;
-          if (sq[jj] == 0.0f || !inside(gi, pi, jj)) continue;
-          atomicOr(&s_imask[ii * a.words + (jj >> 5)], 1u << (jj & 31));
-          atomicOr(&s_imask[jj * a.words + (ii >> 5)], 1u << (ii & 31));
-        }
-        continue;
-      }
-      if (!same && !quirk) {  // a row out of reach of subunit j has no pair with it
-        const int4 pc = s32[cl];
-        const float dx = hi_diff(pi.x, pc.x, unit), dy = hi_diff(pi.y, pc.y, unit), dz = hi_diff(pi.z, pc.z, unit);
-        if (dx * dx + dy * dy + dz * dz > reach_j * reach_j) continue;
-      }
-      const bool row_stale = i0 && ii == cl;
-      int prev_jj = -1;  // last computed pair of this row
-      for (int w0 = 0; w0 < np; w0 += 32) {
-        unsigned int bits = 0;  // the row's intra-subunit mask word, stored once
-        const int w1 = min(np, w0 + 32);
-        for (int jj = w0; jj < w1; jj++) {
-          if (same && !(jj != ii && qi && sq[jj] != 0.0f)) continue;  // electrostatic only (:94-96)
-          bool in;
+          for (int r = ii - 1; r >= 0 && fj < 0; r--)
+            for (int w = words - 1; w >= 0 && fj < 0; w--) {
+              const unsigned int m = computed(r, w);
+              if (m) {
+                fj = 32 * w + 31 - __clz(m);
+                fr = r;
+              }
+            }
+          const bool in = fj >= 0 ? test_one(fr, b32, j, fj) : same || test_one(cl, b32, j, cl);
           if (row_stale) {
-            in = carried < p.nl2;
-          } else if (j0 && jj == cl) {
-            in = (prev_jj >= 0 ? d2_exact(gi, prev_jj) : carried) < p.nl2;
+            for (int w = 0; w < words; w++) mk[w] = in ? visited(ii, w) : 0u;
           } else {
-            in = inside(gi, pi, jj);
-            prev_jj = jj;
-          }
-          if (!in) continue;
-          if (same) {
-            bits |= 1u << (jj - w0);
-          } else {
-            int k = inter_n[r];
-            if (k < a.inter_cap) a.inter_ids[(size_t)gi * a.inter_cap + k] = j * np + jj;
-            inter_n[r] = k + 1;
+            const unsigned int b = 1u << (cl & 31);
+            mk[cl >> 5] = in ? mk[cl >> 5] | b : mk[cl >> 5] & ~b;
           }
         }
-        // the subunit's own block is the only one that sets intra bits (its candidate list holds
-        // it once), so the word is written whole
-        if (same) mask_rows[ii * a.words + (w0 >> 5)] = bits;
       }
-    }
-    if (same && !quirk) {  // the symmetric block's bits, complete once every row is done
       __syncthreads();
-      for (int t = threadIdx.x; t < np * a.words; t += blockDim.x) mask_rows[t] = s_imask[t];
+    }
+    // own block to the intra bits; the others' entries get their places in the rows
+    for (int ii = threadIdx.x; ii < np; ii += blockDim.x) {
+      int n = s_n[ii];
+      for (int k = 0; k < nk; k++) {
+        unsigned int* mk = cmask + (size_t)(k * np + ii) * words;
+        coff[k * np + ii] = n;
+        if (s_cj[k] == i) {
+          for (int w = 0; w < words; w++) mask_rows[ii * words + w] = mk[w];
+        } else {
+          for (int w = 0; w < words; w++) n += __popc(mk[w]);
+        }
+      }
+      s_n[ii] = n;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < items; t += blockDim.x) {
+      const int w = words == 1 ? 0 : t / rows, q = t - w * rows, k = q / np, ii = q - k * np;
+      unsigned int bits = cmask[q * words + w];
+      const int j = s_cj[k];
+      if (!bits || j == i) continue;
+      int n = coff[q];
+      for (int v = 0; v < w; v++) n += __popc(cmask[q * words + v]);
+      int* row = a.inter_ids + (size_t)(i * np + ii) * a.inter_cap;
+      const int base = j * np + 32 * w;
+      for (; bits && n < a.inter_cap; bits &= bits - 1) row[n++] = base + __ffs(bits) - 1;
     }
   }
   __syncthreads();
-  for (int r = 0, ii = threadIdx.x; ii < np; ii += blockDim.x, r++) {
-    const int gi = i * np + ii;
-    int n_inter = inter_n[r];
-    if (n_inter > a.inter_cap) {
-      atomicOr(a.err, kErrInterOverflow);
-    }
-    a.inter_count[gi] = n_inter < a.inter_cap ? n_inter : a.inter_cap;
+  for (int ii = threadIdx.x; ii < np; ii += blockDim.x) {
+    const int gi = i * np + ii, n_inter = s_n[ii];
+    if (n_inter > a.inter_cap) atomicOr(a.err, kErrInterOverflow);
+    a.inter_count[gi] = min(n_inter, a.inter_cap);
     int n_intra = 0;
-    for (int w = 0; w < a.words; w++) n_intra += __popc(mask_rows[ii * a.words + w]);
+    for (int w = 0; w < words; w++) n_intra += __popc(mask_rows[ii * words + w]);
     a.ref_len[gi] = n_intra + n_inter;
   }
 }
@@ -541,7 +470,9 @@ namespace souffle {
 void launch_cells_count(const CellArgs& a, int grid, int block, cudaStream_t s) {
   k_cells_count<<<grid, block, 0, s>>>(a);
 }
-void launch_cells_scan(const CellArgs& a, cudaStream_t s) { k_cells_scan<<<a.n_sys, 1024, 0, s>>>(a); }
+void launch_cells_place(const CellArgs& a, cudaStream_t s) {
+  k_cells_place<<<(a.total_cells + 256 * kPlacePer - 1) / (256 * kPlacePer), 256, 0, s>>>(a);
+}
 void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s) {
   k_cells_scatter<<<grid, block, 0, s>>>(a);
 }
@@ -553,23 +484,29 @@ void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s) {
   const int g = (a.c.n_sub_total + warps_per_block - 1) / warps_per_block;
   k_candidates<<<g, 32 * warps_per_block, sizeof(int) * warps_per_block * a.cap, s>>>(a);
 }
-// About 8 KB of staging per CTA (8 candidates of 42 beads), so that a one-wave grid of 64-thread
-// CTAs still fits the shared memory of an SM.
+// About 8 KB of staging per CTA (9 candidates of 42 beads), so that a one-wave grid of CTAs still
+// fits the shared memory of an SM.
 int pair_chunk(int np, int words) {
-  const int per = np * (int)(sizeof(int4) + sizeof(unsigned int) * words);
-  return std::max(1, std::min(kPairChunkMax, 8192 / per));
+  const int per = np * (int)(sizeof(int4) + sizeof(unsigned int) * words + sizeof(int));
+  return std::max(1, std::min(kPairChunkMax, 10240 / per));
 }
-size_t pair_smem_bytes(int np, int words, int chunk) {
-  const size_t blk = (size_t)np * (sizeof(int4) + 3 * sizeof(long long) + sizeof(double) + sizeof(int) + sizeof(float)) +
-                     sizeof(unsigned int) * (size_t)np * words;
-  return ((blk + 15) & ~(size_t)15) + sizeof(int4) * (size_t)np * (1 + chunk) +
-         sizeof(unsigned int) * (size_t)chunk * np * words;
+static size_t pair_smem_base(int np, int words, int chunk) {
+  return sizeof(int4) * (size_t)np * (1 + chunk) + sizeof(unsigned int) * (size_t)chunk * np * words +
+         sizeof(int) * (size_t)np * (chunk + 1);
 }
-void launch_pairs(const PairArgs& a, int n_sub, size_t smem, cudaStream_t s) {
-  const int block = std::min(128, 32 * ((a.np + 31) / 32));
-  k_pairs<<<n_sub, block, smem, s>>>(a);
+// Every subunit of a system is tested by every CTA up to kSearchSubs subunits per system (16 bytes
+// per test: 32 MB of L2 reads at 1024, less than 5 us), which replaces four launches (9 to 12 us);
+// beyond, and for the surrogate, which classifies the candidates first, they come from the cell grid.
+bool pairs_search(int max_sub, int cand_cap) { return max_sub <= kSearchSubs && cand_cap <= 4096; }
+size_t pair_smem_bytes(int np, int words, int chunk) { return pair_smem_base(np, words, chunk) + sizeof(int) * 4096; }
+void launch_pairs(const PairArgs& a, int n_sub, bool search, cudaStream_t s) {
+  const size_t smem = pair_smem_base(a.np, a.words, a.chunk);
+  if (search) k_pairs<true><<<n_sub, 128, smem + sizeof(int) * a.cand_cap, s>>>(a);
+  else k_pairs<false><<<n_sub, a.np * a.words <= 96 ? 64 : 128, smem, s>>>(a);
 }
 cudaError_t set_pairs_smem(size_t smem) {
-  return cudaFuncSetAttribute(k_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_pairs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_pairs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 }  // namespace souffle

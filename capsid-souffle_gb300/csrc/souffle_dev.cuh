@@ -49,7 +49,8 @@ struct TplLayout {
   int o_sigma;        // [np]
   int o_mass;         // [np]
   int o_beta0;        // [nbend] rest bend angle per bending edge (0 = no rest angle)
-  int n_float;        // floats that the force kernels stage (o_len0, o_mass, o_sigma, o_beta0)
+  int o_pair;         // [nspecies^2][3] LJ/WCA cut-off squared, sigma^6, epsilon (< 0: the system's attraction)
+  int n_float;        // floats that the force kernels stage (o_len0, o_sigma, o_mass, o_beta0, o_pair)
   int nspecies;
   int lj_att_bits[kMaxSpecies];  // bit js of row is: (species is -> js) attractive
   int type7_bits;                // bit js: species js has type 7 (attractive epsilon 50)
@@ -111,7 +112,7 @@ struct __align__(16) SysState {
   dfloat kick_c0;        // dt sqrt(expfac) / 2 of the next step (per-bead kick c = c0 / m)
   long long delta_fx;    // (1 - expfac) * 2^62 for the integer kicks, expfac = exp(-dt xi0 / 2)
   long long vcom_fx[3];  // mean velocity (2^-40 units) still to subtract from vel (0 once applied)
-  double vcom_mag;       // |mean velocity| removed at the last step (src/md.cpp:623)
+  long long vsum[3];     // velocity sum of the last step (2^-40 units): |vsum| / n is the mean velocity removed (src/md.cpp:623)
   unsigned int done;     // arrival counter for the last-block reduction
   unsigned int steps;    // MD steps completed since md_begin
   long long fran_sum[3]; // Brownian: sum of this step's random forces (2^-32 units)
@@ -161,6 +162,7 @@ enum : unsigned int {
   kErrInterOverflow = 1u,
   kErrCandOverflow = 2u,
   kErrNonFinite = 4u,
+  kErrWindow = 16u,    // a bounded wait of the window kernel's grid barrier ran out
   kErrSurrogate = 8u,  // a bounded wait of the surrogate network's tensor-core kernels ran out
 };
 

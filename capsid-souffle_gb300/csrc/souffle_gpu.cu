@@ -213,18 +213,6 @@ souffle_status upload(souffle_gpu_system* h) {
   L.n_int = (int)ti.size();
   L.o_type = (int)ti.size();
   ti.insert(ti.end(), T.type.begin(), T.type.end());
-  L.o_len0 = (int)tf.size();
-  for (double v : T.len0) tf.push_back((float)v);
-  L.o_sigma = (int)tf.size();
-  for (double v : T.sigma) tf.push_back((float)v);
-  L.o_mass = (int)tf.size();
-  for (double v : T.mass) tf.push_back((float)v);
-  L.o_beta0 = (int)tf.size();
-  for (double v : T.beta0) tf.push_back((float)v);
-  while (tf.size() % 4) tf.push_back(0.f);
-  L.n_float = (int)tf.size();
-  L.o_q = (int)tf.size();
-  for (double v : T.q) tf.push_back((float)v);
   L.nspecies = T.nspecies;
   // directed attraction (src/forces.cpp:119-125) and the type-7 epsilon (src/forces.cpp:127)
   L.type7_bits = 0;
@@ -235,11 +223,6 @@ souffle_status upload(souffle_gpu_system* h) {
       for (int k = 0; k < T.n_lj; k++)
         if (T.sp_type[a] == T.lj[2 * k] && T.sp_type[b] == T.lj[2 * k + 1]) L.lj_att_bits[a] |= 1 << b;
   }
-  CUDA_TRY(h->tpl_i.alloc(ti.size()));
-  CUDA_TRY(h->tpl_f.alloc(tf.size()));
-  CUDA_TRY(cudaMemcpy(h->tpl_i.p, ti.data(), ti.size() * sizeof(int), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(h->tpl_f.p, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
-
   // pair-species tables (ecut is common to all systems: it depends only on sigma in nm)
   PairTable pt{};
   const double replj2 = 1.12246205 * 1.12246205;
@@ -253,6 +236,31 @@ souffle_status upload(souffle_gpu_system* h) {
       pt.cut2[idx] = (float)(att ? ecut * ecut : replj2 * shc * shc);
       pt.skip2[idx] = (float)std::max(ecut * ecut, replj2 * shc * shc);
     }
+  L.o_len0 = (int)tf.size();
+  for (double v : T.len0) tf.push_back((float)v);
+  L.o_sigma = (int)tf.size();
+  for (double v : T.sigma) tf.push_back((float)v);
+  L.o_mass = (int)tf.size();
+  for (double v : T.mass) tf.push_back((float)v);
+  L.o_beta0 = (int)tf.size();
+  for (double v : T.beta0) tf.push_back((float)v);
+  L.o_pair = (int)tf.size();
+  for (int a = 0; a < T.nspecies; a++)
+    for (int b = 0; b < T.nspecies; b++) {
+      const bool att = (L.lj_att_bits[a] >> b) & 1;
+      tf.push_back(pt.cut2[a * kMaxSpecies + b]);
+      tf.push_back(pt.sig6[a * kMaxSpecies + b]);
+      tf.push_back(!att ? 1.0f : (L.type7_bits >> b) & 1 ? 50.0f : -1.0f);  // src/forces.cpp:119-130
+    }
+  while (tf.size() % 4) tf.push_back(0.f);
+  L.n_float = (int)tf.size();
+  L.o_q = (int)tf.size();
+  for (double v : T.q) tf.push_back((float)v);
+  CUDA_TRY(h->tpl_i.alloc(ti.size()));
+  CUDA_TRY(h->tpl_f.alloc(tf.size()));
+  CUDA_TRY(cudaMemcpy(h->tpl_i.p, ti.data(), ti.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(h->tpl_f.p, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
+
   CUDA_TRY(h->pt.alloc(1));
   CUDA_TRY(cudaMemcpy(h->pt.p, &pt, sizeof(pt), cudaMemcpyHostToDevice));
 
@@ -297,6 +305,11 @@ souffle_status check_err(souffle_gpu_system* h) {
   const unsigned int e = *h->err_host;
   if (e) {
     CUDA_TRY(cudaMemsetAsync(h->err.p, 0, sizeof(unsigned int), h->stream));
+    if (e & kErrWindow) {  // the counters stand where the launch gave up
+      CUDA_TRY(cudaMemsetAsync(h->win_count.p, 0, sizeof(unsigned int) * h->win_count.n, h->stream));
+      CUDA_TRY(cudaMemsetAsync(h->win_acc.p, 0, sizeof(long long) * h->win_acc.n, h->stream));
+      return fail(SOUFFLE_ERR_CUDA, "window kernel: a bounded wait ran out");
+    }
     if (e & kErrNonFinite) return fail(SOUFFLE_ERR_NONFINITE, "non-finite force or kinetic energy");
     if (e & kErrInterOverflow)
       return fail(SOUFFLE_ERR_NL_OVERFLOW, "inter-subunit pair list exceeded inter_capacity");
@@ -305,6 +318,12 @@ souffle_status check_err(souffle_gpu_system* h) {
     if (e & kErrSurrogate) return fail(SOUFFLE_ERR_CUDA, "surrogate network: a bounded wait ran out");
   }
   return SOUFFLE_OK;
+}
+
+// |mean velocity| removed at the last step (src/md.cpp:505-514, 623)
+double vcom_magnitude(const SysState& S) {
+  const double x = (double)S.vsum[0] * S.inv_n, y = (double)S.vsum[1] * S.inv_n, z = (double)S.vsum[2] * S.inv_n;
+  return std::sqrt(std::fma(z, z, std::fma(x, x, y * y))) * (1.0 / kVelScale);
 }
 
 CellArgs cell_args(souffle_gpu_system* h) {
@@ -331,10 +350,10 @@ CellArgs cell_args(souffle_gpu_system* h) {
 void launch_subunit_cells(souffle_gpu_system* h) {
   cudaStream_t st = h->stream;
   CellArgs c = cell_args(h);
-  cudaMemsetAsync(h->cell_count.p, 0, sizeof(int) * h->total_cells, st);
+  cudaMemsetAsync(h->cell_count.p, 0, sizeof(int) * (h->total_cells + 1), st);
   const int tb = 128, gb = (h->S + tb - 1) / tb;
   launch_cells_count(c, gb, tb, st);
-  launch_cells_scan(c, st);
+  launch_cells_place(c, st);
   launch_cells_scatter(c, gb, tb, st);
 }
 
@@ -356,7 +375,8 @@ void launch_candidates_all(souffle_gpu_system* h) {
 void launch_rebuild(souffle_gpu_system* h) {
   cudaStream_t st = h->stream;
   CellArgs c = cell_args(h);
-  launch_candidates_all(h);
+  const bool search = !surrogate_enabled(h) && pairs_search(h->max_sub, h->cand_cap);
+  if (!search) launch_candidates_all(h);
   PairArgs pa{};
   pa.px = c.px;
   pa.py = c.py;
@@ -380,7 +400,7 @@ void launch_rebuild(souffle_gpu_system* h) {
   pa.chunk = h->pair_chunk;
   pa.err = h->err.p;
   if (surrogate_enabled(h)) surrogate_classify(h, pa);
-  launch_pairs(pa, h->S, h->pair_smem, st);
+  launch_pairs(pa, h->S, search, st);
   if (surrogate_enabled(h)) surrogate_compact(h);
 }
 
@@ -489,6 +509,28 @@ void launch_step(souffle_gpu_system* h, bool rebuild, bool judge) {
 }
 
 
+// Steps through the window kernel: MD or Brownian steps with the double-float chain whose forces
+// come from the pair lists alone (no network, no big beads), every work item resident at once.
+bool window_usable(const souffle_gpu_system* h) {
+  if (!h->window_ok || h->opt.chain_fp64 || surrogate_enabled(h)) return false;
+  for (const SysParams& P : h->sp)
+    if (P.nbb > 0) return false;
+  return true;
+}
+
+// `len` steps in one launch; forces_first: the drift of the first one has been launched already
+cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_first) {
+  WindowArgs q{};
+  q.steps = len;
+  q.forces_first = forces_first ? 1 : 0;
+  q.n_sys = h->n_sys;
+  q.count = h->win_count.p;
+  q.acc = h->win_acc.p;
+  q.acc_stride = 8 * (size_t)h->n_sys;
+  q.force_bytes = (h->force_smem + 15) & ~(size_t)15;
+  return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->threads, h->window_smem, h->stream);
+}
+
 size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
   const TplLayout& L = h->L;
   const int np = h->tpl.np;
@@ -512,8 +554,10 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   if (smem > 200 * 1024) return fail(SOUFFLE_ERR_BAD_INPUT, "template too large for shared memory");
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   CUDA_TRY(set_kernel_smem(smem, threads, h->pair_smem));
-  int wave = 0;
+  int wave = 0, win_wave = 0;
   CUDA_TRY(force_wave_ctas(threads, smem, &wave));
+  const size_t win_smem = window_smem_bytes(smem, subs, h->tpl.np);
+  if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(threads, win_smem, &win_wave));
   std::vector<WorkItem> work;
   std::vector<int2> slots;
   int sub0 = 0;
@@ -563,6 +607,14 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   h->subs_per_cta = subs;
   h->threads = threads;
   h->force_smem = smem;
+  h->window_smem = win_smem;
+  h->window_ok = (int)h->work.size() <= win_wave;
+  if (h->window_ok && h->win_count.n == 0) {
+    CUDA_TRY(h->win_count.alloc(3));
+    CUDA_TRY(h->win_acc.alloc(24 * (size_t)h->n_sys));
+    CUDA_TRY(cudaMemset(h->win_count.p, 0, 3 * sizeof(unsigned int)));
+    CUDA_TRY(cudaMemset(h->win_acc.p, 0, sizeof(long long) * h->win_acc.n));
+  }
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.second);
   h->graphs.clear();
   return SOUFFLE_OK;
@@ -708,8 +760,8 @@ souffle_status souffle_gpu_create(const souffle_template* tpl, const souffle_par
   CUDA_TRY(h->ref_len.alloc(N));
   CUDA_TRY(h->cand.alloc((size_t)h->cand_cap * h->S));
   CUDA_TRY(h->cand_count.alloc(h->S));
-  CUDA_TRY(h->cell_count.alloc(h->total_cells));
-  CUDA_TRY(h->cell_start.alloc(h->total_cells + 1));
+  CUDA_TRY(h->cell_count.alloc(h->total_cells + 1));
+  CUDA_TRY(h->cell_start.alloc(h->total_cells));
   CUDA_TRY(h->sub_rank.alloc(h->S));
   CUDA_TRY(h->sub_cell.alloc(h->S));
   CUDA_TRY(h->cell_subs.alloc(h->S));
@@ -753,9 +805,8 @@ souffle_status souffle_gpu_create(const souffle_template* tpl, const souffle_par
     CUDA_TRY(cudaMemset(h->bd_fran.p, 0, sizeof(long long) * 3 * N));
   }
   CUDA_TRY(h->e_tot.alloc(8));
-  int max_sub = 0;
-  for (int k = 0; k < n_systems; k++) max_sub = std::max(max_sub, params[k].n_subunits);
-  CUDA_TRY(h->e_sph.alloc(max_sub));
+  for (int k = 0; k < n_systems; k++) h->max_sub = std::max(h->max_sub, params[k].n_subunits);
+  CUDA_TRY(h->e_sph.alloc(h->max_sub));
   CUDA_TRY(h->e_part.alloc(7 * kTotalCtas));
   CUDA_TRY(h->e_scr.alloc(2));
   CUDA_TRY(cudaMemset(h->e_scr.p, 0, 2 * sizeof(int)));
@@ -1165,6 +1216,7 @@ souffle_status souffle_gpu_energies(souffle_gpu_system* h, int32_t system, souff
     launch_subunit_cells(h);
     launch_cells_sort(cell_args(h), h->stream);  // the sums do not depend on scheduling
     a.sub_cell_start = h->cell_start.p;
+    a.sub_cell_count = h->cell_count.p;
     a.cell_subs = h->cell_subs.p;
   }
   launch_energies(a, n, h->stream);
@@ -1198,7 +1250,7 @@ souffle_status souffle_gpu_energies(souffle_gpu_system* h, int32_t system, souff
     out->thermo_pe = tpe;
     out->thermo_ke = tke;
     out->temperature = tot[0] * 2 / (3.0 * n);
-    out->vcom_magnitude = S.vcom_mag;
+    out->vcom_magnitude = vcom_magnitude(S);
     out->bigbead_lj = tot[5];
     out->bigbead_electrostatic = tot[6];
   }
@@ -1307,8 +1359,18 @@ souffle_status souffle_gpu_md_enqueue(souffle_gpu_system* h, int64_t first_step,
     if (it == h->graphs.end()) {
       cudaGraph_t g;
       CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < len; k++) launch_step(h, k == 0 && rebuild_first, (judge_mask >> k) & 1ull);
+      cudaError_t launched = cudaSuccess;
+      if (len > 1 && window_usable(h)) {
+        if (rebuild_first) {
+          launch_drift(drift_args(h), (int)h->work.size(), h->threads, h->stream);
+          launch_rebuild(h);
+        }
+        launched = launch_window_steps(h, len, rebuild_first);
+      } else {
+        for (int k = 0; k < len; k++) launch_step(h, k == 0 && rebuild_first, (judge_mask >> k) & 1ull);
+      }
       CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
+      CUDA_TRY(launched);
       cudaGraphExec_t ge;
       CUDA_TRY(cudaGraphInstantiate(&ge, g, 0));
       cudaGraphDestroy(g);
@@ -1384,7 +1446,7 @@ souffle_status souffle_gpu_md_scalars(souffle_gpu_system* h, int32_t system, dou
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   if (ke) *ke = df_to(S.ke);
   if (xi0) *xi0 = df_to(S.xi[0]);
-  if (vcom) *vcom = S.vcom_mag;
+  if (vcom) *vcom = vcom_magnitude(S);
   return SOUFFLE_OK;
 }
 

@@ -46,11 +46,17 @@ struct souffle_gpu_system {
   int n_sys = 0;
   int64_t N = 0;
   int S = 0;
+  int max_sub = 0;  // subunits of the largest system
   int subs_per_cta = 1;
   int threads = 128;
   int total_cells = 0;
   std::vector<WorkItem> work;
   std::vector<int2> slots;
+  // window kernel: usable with this plan (every work item resident at once), its shared memory
+  bool window_ok = false;
+  size_t window_smem = 0;
+  DevBuf<unsigned int> win_count;
+  DevBuf<long long> win_acc;
   int inter_cap = 96, cand_cap = 128;
   size_t force_smem = 0, pair_smem = 0;
   int pair_chunk = 1;

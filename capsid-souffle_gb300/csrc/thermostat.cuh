@@ -159,49 +159,80 @@ static __device__ __noinline__ bool chain64_tail(Chain64& c, double ke, bool for
 
 static_assert(kMaxChain <= 32, "one lane per chain link");
 
-// Forward half on one warp: lane j evaluates link j's exponential, A_j, B_j and eta_j at once;
-// then every lane runs the link recurrence itself from those shared operands (no lane-to-lane
-// hand-off in the dependent chain) and lane j stores xi_j.  scratch: 2 kMaxChain dfloats of
-// shared memory.
-__device__ inline void nhc_forward_warp(SysState& s, int lane, dfloat* scratch) {
-  const int m = s.m;
-  dfloat* As = scratch;
-  dfloat* Bs = scratch + kMaxChain;
-  if (lane < m) {
-    const bool on = nhc_active(s, lane);
+// Both halves on one warp, in two parts.  The first needs no kinetic energy, so it can run while the
+// step's sums are still on their way: lane j evaluates link j's exponential, A_j, B_j and eta_j of the
+// forward half (for link 0 e4 and xi_0 e4).  The second runs the forward recurrence, the G_j of the
+// backward half (lane j from its own x_{j-1}) and the backward recurrence; every lane runs the
+// recurrences itself from operands in shared memory (no lane-to-lane hand-off in the dependent
+// chain) and lane j stores link j's results.  The operations are those of nhc_forward and
+// nhc_backward, so the results are the same bits.  scratch: 3 kMaxChain dfloats of shared memory.
+// About 2,600 dependent cycles with 5 links, of which the exponentials are half; with the
+// first part inside and operands fetched between the links both took 7,000.
+__device__ inline unsigned int nhc_pre_warp(SysState& s, int lane, dfloat* scratch) {
+  const bool on = lane < s.m && nhc_active(s, lane);
+  if (lane < s.m) {
+    dfloat A = s.xi_b[lane], B = dfloat{0.0f, 0.0f};  // an inactive link keeps its xi
+    if (on) {  // nhc_forward_terms without a branch on the link
+      const dfloat e4 = nhc_e4(s, s.xi_b[lane + 1]);
+      const dfloat p = df_mul(A, e4);
+      const dfloat Aj = df_mul(e4, df_add(p, df_neg(df_mul(s.c_hdt_inv_q[lane], s.c_dof_t[lane]))));
+      const dfloat Bj = df_mul(df_mul(e4, s.c_hdt_inv_q[lane]), s.c_q[lane > 0 ? lane - 1 : 0]);
+      A = lane == 0 ? p : Aj;
+      B = lane == 0 ? e4 : Bj;
+    }
     s.eta[lane] = on ? nhc_eta(s, s.eta_b[lane], s.xi_b[lane]) : s.eta_b[lane];
-    if (on) nhc_forward_terms(s, lane, As[lane], Bs[lane]);
+    scratch[lane] = A;
+    scratch[kMaxChain + lane] = B;
   }
+  const unsigned int active = __ballot_sync(0xffffffffu, on);
   __syncwarp();
-  dfloat prev = {0.0f, 0.0f};
-  for (int j = 0; j < m; j++) {
-    dfloat x = s.xi_b[j];
-    if (nhc_active(s, j)) x = nhc_forward_link(j, As[j], Bs[j], prev);
-    if (lane == j) s.xi[j] = x;
-    prev = x;
-  }
-  __syncwarp();
+  return active;
 }
 
-// Backward half on one warp: lane j evaluates c_j G_j (reads xi_{j-1} before it changes); then
-// every lane runs the recurrence j = M-1 .. 0 and lane j stores xi_j; lane 0 sets the kick
-// factors (its return value is the one that counts).  scratch: kMaxChain dfloats.
-__device__ inline bool nhc_backward_warp(SysState& s, int lane, dfloat* scratch) {
-  __syncwarp();  // xi / eta written by other lanes (the forward half) are visible from here on
+// The backward half from the chain (xi, eta): forward = false runs it alone (the initial forces).
+// Returns false (lane 0's value counts) when the kick factors leave their range.
+__device__ inline bool nhc_post_warp(SysState& s, int lane, dfloat* scratch, unsigned int active, bool forward) {
   const int m = s.m;
-  dfloat* cgs = scratch;
-  if (lane < m && nhc_active(s, lane))
-    cgs[lane] = df_mul(s.c_hdt_inv_q[lane], nhc_g(s, lane > 0 ? s.xi[lane - 1] : dfloat{0.0f, 0.0f}, lane));
-  __syncwarp();
-  dfloat next = {0.0f, 0.0f};
-  for (int j = m - 1; j > -1; j--) {
-    dfloat x = s.xi[j];
-    if (nhc_active(s, j)) x = nhc_link(x, nhc_e4(s, next), cgs[j]);
-    if (lane == j) s.xi_b[j] = x;
-    next = x;
+  dfloat* cgs = scratch + 2 * kMaxChain;
+  dfloat before = {0.0f, 0.0f};  // x_{lane - 1} after the forward half
+  const dfloat cg0 = df_mul(s.c_hdt_inv_q[0], nhc_g(s, dfloat{0.0f, 0.0f}, 0));
+  if (forward) {
+    dfloat prev = scratch[0], mine = prev;
+    if (active & 1u) prev = mine = df_mul(scratch[kMaxChain], df_add(scratch[0], cg0));
+    dfloat A = scratch[1], B = scratch[kMaxChain + 1];
+    for (int j = 1; j < m; j++) {
+      const dfloat nA = scratch[j + 1], nB = scratch[kMaxChain + j + 1];  // (scratch has a third row behind)
+      const dfloat x = (active >> j) & 1u ? nhc_forward_link(j, A, B, prev) : A;
+      if (lane == j) {
+        mine = x;
+        before = prev;
+      }
+      prev = x;
+      A = nA;
+      B = nB;
+    }
+    if (lane < m) s.xi[lane] = mine;
+    __syncwarp();
+  } else if (lane > 0 && lane < m) {
+    before = s.xi[lane - 1];
   }
+  if ((active >> lane) & 1u) cgs[lane] = lane == 0 ? cg0 : df_mul(s.c_hdt_inv_q[lane], nhc_g(s, before, lane));
   __syncwarp();
-  if (lane < m) s.eta_b[lane] = nhc_active(s, lane) ? nhc_eta(s, s.eta[lane], s.xi_b[lane]) : s.eta[lane];
+  dfloat next = {0.0f, 0.0f}, mine = {0.0f, 0.0f};
+  dfloat x = s.xi[m - 1 > 0 ? m - 1 : 0], cg = cgs[m - 1 > 0 ? m - 1 : 0];
+  for (int j = m - 1; j > -1; j--) {
+    const int jn = j > 0 ? j - 1 : 0;
+    const dfloat nx = s.xi[jn], ncg = cgs[jn];
+    if ((active >> j) & 1u) x = nhc_link(x, nhc_e4(s, next), cg);
+    if (lane == j) mine = x;
+    next = x;
+    x = nx;
+    cg = ncg;
+  }
+  if (lane < m) {
+    s.xi_b[lane] = mine;
+    s.eta_b[lane] = (active >> lane) & 1u ? nhc_eta(s, s.eta[lane], mine) : s.eta[lane];
+  }
   return lane == 0 ? nhc_kick_factors(s, next) : true;
 }
 #endif
