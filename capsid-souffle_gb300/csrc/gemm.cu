@@ -3,7 +3,7 @@
 //   warp 0, lane 0  TMA producer: 128 x 64 A and BN x 64 B tiles (128-byte swizzle) into a
 //                   4-stage shared-memory ring that runs across tile boundaries, one mbarrier per
 //                   stage ("full"), freed by the MMA issuer ("empty")
-//   warp 1, lane 0  MMA issuer: four K = 16 tcgen05.mma per stage into one of two FP32
+//   warp 1          MMA issuer (an elected lane): four K = 16 tcgen05.mma per stage into one of two FP32
 //                   accumulators in tensor memory (tile i uses accumulator i % 2);
 //                   tcgen05.commit frees the stage and, after a tile's last stage, signals the
 //                   epilogue ("tmem full")
@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <utility>
 
 #include "gemm.cuh"
 #include "umma.cuh"
@@ -69,8 +70,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tfull0 = bars + 16 * G::kStages, tempty0 = tfull0 + 16, drain = tempty0 + 16;
   const uint32_t tmem_slot = bars + G::kBars * 8;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_rows = e.m_dyn ? min(e.M, *e.m_dyn) : e.M;
+  const int warp = (int)__reduce_max_sync(0xffffffffu, threadIdx.x >> 5), lane = threadIdx.x & 31;  // (known uniform)
+  if (e.m_dyn) pdl_wait();  // the count comes from an earlier kernel
+  const int m_rows = (int)__reduce_max_sync(0xffffffffu, (unsigned)(e.m_dyn ? max(0, min(e.M, *e.m_dyn)) : e.M));
   const int m_tiles = (m_rows + kBM - 1) / kBM;
   const int n_tiles = (e.N + BN - 1) / BN;
   const int tiles = m_tiles * n_tiles;
@@ -97,6 +99,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tma_prefetch_map(&ta);
     tma_prefetch_map(&tb);
   }
+  pdl_launch();
+  pdl_wait();
   if (e.bias)
     for (int t = threadIdx.x; t < e.N; t += blockDim.x) s_bias[t] = e.bias[t];
   tc_fence_before();
@@ -128,40 +132,41 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int q = (g > G::kStages ? g - G::kStages : 0); q < g; q++)
       if (!mbar_wait(full0 + 8 * (q % G::kStages), (uint32_t)(q / G::kStages) & 1u)) ok = false;
     if (!ok) atomicOr(e.err, e.err_bit);
-  } else if (warp == 1 && lane == 0) {
-    // ---- MMA issuer
+  } else if (warp == 1) {
+    // ---- MMA issuer: the whole warp walks the k-steps, one elected lane issues.  No branch depends
+    // on a wait's outcome, so the walk stays uniform; after a failed wait it runs out on data that
+    // nobody uses.
     constexpr uint32_t idesc = umma_idesc_bf16(kBM, BN);
     int g = 0, it = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, it++) {
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, it++) {
       const int b = it & 1;
       const uint32_t u = (uint32_t)(it >> 1);
-      if (u > 0 && !mbar_wait(tempty0 + 8 * b, (u - 1) & 1u)) {  // the epilogue has drained it
-        ok = false;
-        break;
-      }
+      if (u > 0 && ok) ok = mbar_wait(tempty0 + 8 * b, (u - 1) & 1u);  // the epilogue has drained it
       tc_fence_after();
       const uint32_t acc = tmem + (uint32_t)(b * BN);
       for (int kt = 0; kt < nk; kt++, g++) {
         const int s = g % G::kStages;
-        if (!mbar_wait(full0 + 8 * s, (uint32_t)(g / G::kStages) & 1u)) {
-          ok = false;
-          break;
-        }
+        if (ok) ok = mbar_wait(full0 + 8 * s, (uint32_t)(g / G::kStages) & 1u);
         tc_fence_after();
         const uint32_t a_s = base + s * G::kStage;
         const uint64_t ad = sw128_kmajor_desc(a_s), bd = sw128_kmajor_desc(a_s + G::kA);
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < kBK / 16; j++) umma_bf16(acc, ad + 2 * j, bd + 2 * j, idesc, (kt | j) != 0 ? 1u : 0u);
-        umma_commit(empty0 + 8 * s);
+          for (int j = 0; j < kBK / 16; j++) umma_bf16(acc, ad + 2 * j, bd + 2 * j, idesc, (kt | j) != 0 ? 1u : 0u);
+          umma_commit(empty0 + 8 * s);
+          if (kt == nk - 1) umma_commit(tfull0 + 8 * b);  // after every MMA issued above has completed
+        }
+        __syncwarp();
       }
-      umma_commit(tfull0 + 8 * b);  // after every MMA issued above has completed
     }
     if (!ok) {
-      atomicOr(e.err, e.err_bit);
       // MMAs issued before the timeout may still be writing tensor memory: wait (bounded) for
       // them before the CTA releases it
-      umma_commit(drain);
+      if (elect_one()) {
+        atomicOr(e.err, e.err_bit);
+        umma_commit(drain);
+      }
       mbar_wait(drain, 0);
     }
   } else if (warp >= 4) {
@@ -314,6 +319,23 @@ bool make_map(CUtensorMap* m, const void* p, int rows, int cols, int ld, int box
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A launch whose set-up (tensor memory, barriers, descriptors) may overlap the end of the kernel
+// before it; every kernel launched so calls pdl_wait before it touches global memory.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
 template <int BN, int ACT>
 cudaError_t launch(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const GemmEpi& e, cudaStream_t st) {
   using G = GemmTile<BN>;
@@ -335,9 +357,7 @@ cudaError_t launch(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int 
   });
   const long long tiles = (long long)((e.M + kBM - 1) / kBM) * ((e.N + BN - 1) / BN);
   const int gx = (int)std::min<long long>(tiles, sms > 0 ? sms : 148);
-  dim3 grid(gx);
-  k_gemm_bf16<BN, ACT><<<grid, kThreads, G::kSmem, st>>>(ta, tb, e);
-  return cudaGetLastError();
+  return launch_pdl(k_gemm_bf16<BN, ACT>, gx, kThreads, G::kSmem, st, ta, tb, e);
 }
 
 template <int BN>
@@ -351,6 +371,221 @@ cudaError_t launch_act(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, 
 }
 
 }  // namespace
+
+// ---- weight gradients ------------------------------------------------------------------------
+// One CTA per (tile, split): 128 x 128 of one layer's gradient over `steps` 64-wide K steps of the
+// batch.  A layer is one to four tiles with K the whole batch (4096 rows), so one GEMM per layer
+// kept one to six SMs busy for 20 us, and the bias sums took another 7 us launch each; split over
+// the batch all layers together fill the chip: 7 us (and 9 us cold for adding the splits and the bias
+// sums) where the layers' launches took 129 us at 4096 rows, width 128.
+//   warp 0, lane 0  TMA producer, warp 1 MMA issuer as above; warps 4-11 epilogue: the FP32 sums to
+//   the workspace as [column / 4][row][4], so that a warp's stores are whole lines
+using GD = GemmTile<128>;
+__global__ void __launch_bounds__(kThreads, 1)
+    k_gemm_dw(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensorMap b0,
+              const __grid_constant__ CUtensorMap a1, const __grid_constant__ CUtensorMap b1,
+              const __grid_constant__ CUtensorMap a2, const __grid_constant__ CUtensorMap b2,
+              const __grid_constant__ CUtensorMap a3, const __grid_constant__ CUtensorMap b3, DwArgs d) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  const uint32_t bars = base + GD::kStages * GD::kStage;
+  const uint32_t full0 = bars, empty0 = bars + 8 * GD::kStages, done = bars + 16 * GD::kStages;
+  const uint32_t tmem_slot = bars + GD::kBars * 8;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
+  const int warp = (int)__reduce_max_sync(0xffffffffu, threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / d.splits, split = blockIdx.x - tile * d.splits;
+  int l = 0;
+  while (l + 1 < d.layers && tile >= d.layer[l + 1].tile0) l++;
+  const int q = tile - d.layer[l].tile0, m0 = q / d.layer[l].tiles_n * 128, n0 = q % d.layer[l].tiles_n * 128;
+  const int nk = (d.K + kBK - 1) / kBK, k0 = split * d.steps, k1 = min(nk, k0 + d.steps);  // k0 < k1 for every split
+  const CUtensorMap* ta = l == 0 ? &a0 : l == 1 ? &a1 : l == 2 ? &a2 : &a3;
+  const CUtensorMap* tb = l == 0 ? &b0 : l == 1 ? &b1 : l == 2 ? &b2 : &b3;
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, 128);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < GD::kStages; s++) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    mbar_init(done, 1);
+    mbar_fence_init();
+  }
+  pdl_launch();
+  pdl_wait();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot_ptr;
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      int g = 0;
+      for (int k = k0; k < k1; k++, g++) {
+        const int s = g % GD::kStages;
+        if (g >= GD::kStages && !mbar_wait(empty0 + 8 * s, (uint32_t)(g / GD::kStages - 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        const uint32_t a_s = base + s * GD::kStage;
+        mbar_expect_tx(full0 + 8 * s, GD::kStage);
+        tma_load_2d(a_s, ta, k * kBK, m0, full0 + 8 * s);
+        tma_load_2d(a_s + GD::kA, tb, k * kBK, n0, full0 + 8 * s);
+      }
+      // every copy started here has landed before the CTA can leave
+      for (int p = (g > GD::kStages ? g - GD::kStages : 0); p < g; p++)
+        if (!mbar_wait(full0 + 8 * (p % GD::kStages), (uint32_t)(p / GD::kStages) & 1u)) ok = false;
+      if (!ok) atomicOr(d.err, 1u);
+    }
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = umma_idesc_bf16(kBM, 128);
+    bool ok = true;
+    int g = 0;
+    for (int k = k0; k < k1; k++, g++) {
+      const int s = g % GD::kStages;
+      if (ok) ok = mbar_wait(full0 + 8 * s, (uint32_t)(g / GD::kStages) & 1u);
+      tc_fence_after();
+      const uint32_t a_s = base + s * GD::kStage;
+      const uint64_t ad = sw128_kmajor_desc(a_s), bd = sw128_kmajor_desc(a_s + GD::kA);
+      if (elect_one()) {
+#pragma unroll
+        for (int j = 0; j < kBK / 16; j++) umma_bf16(tmem, ad + 2 * j, bd + 2 * j, idesc, (g | j) != 0 ? 1u : 0u);
+        umma_commit(empty0 + 8 * s);
+        if (k == k1 - 1) umma_commit(done);
+      }
+      __syncwarp();
+    }
+    if (!ok) {
+      if (lane == 0) atomicOr(d.err, 1u);
+      mbar_wait(done, 0);  // (bounded) MMAs issued so far may still be writing tensor memory
+    }
+  } else if (warp >= 4) {
+    const int quarter = warp & 3, half = (warp - 4) >> 2;
+    if (mbar_wait(done, 0)) {
+      tc_fence_after();
+      const int row = quarter * 32 + lane;
+      float4* out = reinterpret_cast<float4*>(d.ws + (size_t)blockIdx.x * kDwTile);
+#pragma unroll 1
+      for (int c = 64 * half; c < 64 * half + 64; c += 32) {
+        float v[32];
+        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          out[(c / 4 + k) * 128 + row] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      }
+    } else {
+      atomicOr(d.err, 1u);
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 128);
+  }
+}
+
+// Adds the splits of every tile in order (thread per four columns of a row), sums the layers' A rows
+// over the batch for the bias gradients (warp per row), and the loss partials (last CTA).
+__global__ void __launch_bounds__(256) k_dw_reduce(DwArgs d, int w_blocks, int b_blocks) {
+  const int lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < w_blocks) {
+    const int i = blockIdx.x * 256 + threadIdx.x;  // tile, column / 4, row
+    const int tile = i / (32 * 128), r = i - tile * (32 * 128), c4 = r >> 7, row = r & 127;
+    if (tile >= d.tiles) return;
+    int l = 0;
+    while (l + 1 < d.layers && tile >= d.layer[l + 1].tile0) l++;
+    const DwLayer& y = d.layer[l];
+    const int q = tile - y.tile0, gr = q / y.tiles_n * 128 + row, gc = q % y.tiles_n * 128 + 4 * c4;
+    if (gr >= y.rows || gc >= y.cols) return;
+    const float4* p = reinterpret_cast<const float4*>(d.ws + (size_t)tile * d.splits * kDwTile) + r;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < d.splits; k++) {
+      const float4 v = __ldcg(p + (size_t)k * (kDwTile / 4));
+      s.x += v.x;
+      s.y += v.y;
+      s.z += v.z;
+      s.w += v.w;
+    }
+    *reinterpret_cast<float4*>(y.out + (size_t)gr * y.cols + gc) = s;  // cols a multiple of 8, 16-byte aligned
+    return;
+  }
+  if ((int)blockIdx.x < w_blocks + b_blocks) {
+    int row = (blockIdx.x - w_blocks) * 8 + (threadIdx.x >> 5), l = 0;
+    while (l < d.layers && row >= d.layer[l].rows) row -= d.layer[l++].rows;
+    if (l == d.layers) return;
+    const __nv_bfloat16* g = d.layer[l].A + (size_t)row * d.ld;
+    float s = 0.f;
+    const int n8 = d.K >> 3;
+#pragma unroll 4
+    for (int c = lane; c < n8; c += 32) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(g) + c);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
+        s += f.x + f.y;
+      }
+    }
+    for (int c = 8 * n8 + lane; c < d.K; c += 32) s += __bfloat162float(g[c]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) d.layer[l].bias_out[row] = s;
+    return;
+  }
+  __shared__ float red[256];
+  float s = 0.0f;
+  for (int i = threadIdx.x; i < d.n_partial; i += 256) s += d.loss_partial[i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int k = 128; k > 0; k >>= 1) {
+    if ((int)threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *d.loss = red[0];
+}
+
+// Tiles, and as many splits of the batch as give every SM an item (152, at least two K steps each).
+void dw_plan(DwArgs& a) {
+  a.tiles = 0;
+  for (int l = 0; l < a.layers; l++) {
+    DwLayer& y = a.layer[l];
+    y.tile0 = a.tiles;
+    y.tiles_n = (y.cols + 127) / 128;
+    a.tiles += (y.rows + 127) / 128 * y.tiles_n;
+  }
+  const int nk = (a.K + kBK - 1) / kBK;
+  const int want = std::max(1, std::min((nk + 1) / 2, 152 / a.tiles));
+  a.steps = (nk + want - 1) / want;
+  a.splits = (nk + a.steps - 1) / a.steps;
+}
+
+cudaError_t dw_gemm(const DwArgs& a, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] { attr = cudaFuncSetAttribute(k_gemm_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, GD::kSmem); });
+  if (attr != cudaSuccess) return attr;
+  if (a.layers < 1 || a.layers > 4 || a.K < 1 || a.ld < a.K || a.ld % 8 || a.tiles * a.splits > kDwItems || !a.ws || !a.err)
+    return cudaErrorInvalidValue;
+  CUtensorMap m[8];
+  for (int l = 0; l < 4; l++) {
+    const DwLayer& y = a.layer[l < a.layers ? l : 0];
+    if (!make_map(&m[2 * l], y.A, y.rows, a.K, a.ld, kBM) || !make_map(&m[2 * l + 1], y.B, y.cols, a.K, a.ld, 128))
+      return cudaErrorInvalidValue;
+  }
+  return launch_pdl(k_gemm_dw, a.tiles * a.splits, kThreads, GD::kSmem, st, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
+}
+
+cudaError_t dw_reduce(const DwArgs& a, cudaStream_t st) {
+  int rows = 0;
+  for (int l = 0; l < a.layers; l++) rows += a.layer[l].rows;
+  const int w_blocks = a.tiles * 16, b_blocks = (rows + 7) / 8;
+  k_dw_reduce<<<w_blocks + b_blocks + 1, 256, 0, st>>>(a, w_blocks, b_blocks);
+  return cudaGetLastError();
+}
 
 cudaError_t gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const GemmEpi& e,
                       cudaStream_t stream) {

@@ -51,70 +51,93 @@ souffle_status fail(souffle_status s, const std::string& msg) {
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
-// x [m][n_in] FP32 -> a0 [m][ld] BF16 row-major and a0T [n_in][ldt] BF16
+// x [m][n_in] FP32 -> a0 [m][ld] BF16 row-major
 // (rows >= *m_dyn skipped when m_dyn is given; grid-stride over the rest)
-__global__ void k_pack_input(const float* x, int m, int n_in, __nv_bfloat16* a0, int ld, __nv_bfloat16* a0t, int ldt,
-                             const int* m_dyn = nullptr) {
+__global__ void k_pack_input(const float* x, int m, int n_in, __nv_bfloat16* a0, int ld, const int* m_dyn = nullptr) {
   const int rows = m_dyn ? min(m, *m_dyn) : m;
   const long long n = (long long)rows * n_in;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(i / n_in), c = (int)(i - (long long)r * n_in);
     const __nv_bfloat16 v = __float2bfloat16_rn(x[i]);
     a0[(size_t)r * ld + c] = v;
-    if (a0t) a0t[(size_t)c * ldt + r] = v;
   }
 }
 
-// dY = 2 (y - t) / (m n_out) as BF16 (row-major and transposed, zero beyond n_out), and per-block
-// partial sums of (y - t)^2 in a fixed order.
-__global__ void k_loss(const float* y, int ldy, const float* t, int m, int n_out, int n_pad, __nv_bfloat16* dy,
-                       __nv_bfloat16* dyt, int ldt, float* partial) {
-  __shared__ float red[256];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float sq = 0.0f;
-  if (i < m * n_pad) {
-    const int r = i / n_pad, c = i - r * n_pad;
-    float g = 0.0f;
-    if (c < n_out) {
-      const float d = y[(size_t)r * ldy + c] - t[(size_t)r * n_out + c];
-      sq = d * d;
-      g = 2.0f * d / ((float)m * (float)n_out);
+// The same with the transpose for training: 32 rows x 64 columns through shared memory, so that both
+// outputs are written in whole sectors.
+constexpr int kPackRows = 32;
+__global__ void __launch_bounds__(256) k_pack_input_t(const float* x, int m, int n_in, __nv_bfloat16* a0, int ld,
+                                                      __nv_bfloat16* a0t, int ldt) {
+  __shared__ __nv_bfloat16 s[kPackRows][66];
+  const int r0 = blockIdx.x * kPackRows, c0 = blockIdx.y * 64;
+  const int c = threadIdx.x & 63, q0 = threadIdx.x >> 6;
+  float v[kPackRows / 4];
+#pragma unroll
+  for (int k = 0; k < kPackRows / 4; k++) {
+    const int r = r0 + q0 + 4 * k;
+    v[k] = r < m && c0 + c < n_in ? x[(size_t)r * n_in + c0 + c] : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < kPackRows / 4; k++) {
+    const int q = q0 + 4 * k;
+    const __nv_bfloat16 b = __float2bfloat16_rn(v[k]);
+    if (r0 + q < m && c0 + c < n_in) a0[(size_t)(r0 + q) * ld + c0 + c] = b;
+    s[q][c] = b;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 64 * kPackRows / 256; k++) {
+    const int t = threadIdx.x + 256 * k, cc = t / kPackRows, q = t % kPackRows;
+    if (r0 + q < m && c0 + cc < n_in) a0t[(size_t)(c0 + cc) * ldt + r0 + q] = s[q][cc];
+  }
+}
+
+// dY = 2 (y - t) / (m n_out) as BF16 (row-major and transposed, zero beyond n_out), and the CTA's
+// sum of (y - t)^2 with a fixed tree.  16 rows per CTA, two per warp with all loads in flight; the
+// transpose goes through shared memory in whole sectors.
+constexpr int kLossRows = 16, kLossMaxPad = 256;
+__global__ void __launch_bounds__(256) k_loss(const float* y, int ldy, const float* t, int m, int n_out, int n_pad,
+                                              __nv_bfloat16* dy, __nv_bfloat16* dyt, int ldt, float* partial) {
+  __shared__ float red[8];
+  __shared__ __nv_bfloat16 s[kLossRows][kLossMaxPad + 2];
+  const int r0 = blockIdx.x * kLossRows, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const float den = (float)m * (float)n_out;
+  float d[2][kLossMaxPad / 32];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int r = r0 + wid + 8 * k;
+#pragma unroll
+    for (int j = 0; j < kLossMaxPad / 32; j++) {
+      const int c = lane + 32 * j;
+      d[k][j] = r < m && c < n_out ? y[(size_t)r * ldy + c] - t[(size_t)r * n_out + c] : 0.f;
     }
-    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    dy[(size_t)r * n_pad + c] = gb;
-    dyt[(size_t)c * ldt + r] = gb;
   }
-  red[threadIdx.x] = sq;
+  float sq = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int q = wid + 8 * k, r = r0 + q;
+#pragma unroll
+    for (int j = 0; j < kLossMaxPad / 32; j++) {
+      const int c = lane + 32 * j;
+      if (c >= n_pad) break;
+      sq += d[k][j] * d[k][j];
+      const __nv_bfloat16 gb = __float2bfloat16_rn(2.0f * d[k][j] / den);
+      if (r < m) dy[(size_t)r * n_pad + c] = gb;
+      s[q][c] = gb;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  if (lane == 0) red[wid] = sq;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  for (int i = threadIdx.x; i < kLossRows * n_pad; i += 256) {
+    const int c = i / kLossRows, q = i % kLossRows;
+    if (r0 + q < m) dyt[(size_t)c * ldt + r0 + q] = s[q][c];
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
-}
-
-// row sums of a transposed BF16 gradient [n][ldt] over its first m columns: the bias gradient.
-// One warp per row, fixed order.
-__global__ void k_row_sums(const __nv_bfloat16* g, int n, int m, int ldt, float* out) {
-  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-  if (row >= n) return;
-  float s = 0.0f;
-  for (int c = lane; c < m; c += 32) s += __bfloat162float(g[(size_t)row * ldt + c]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[row] = s;
-}
-
-__global__ void k_sum(const float* p, int n, float* out) {
-  __shared__ float red[256];
-  float s = 0.0f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += p[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    float p = 0.f;
+    for (int w = 0; w < 8; w++) p += red[w];
+    partial[blockIdx.x] = p;
   }
-  if (threadIdx.x == 0) *out = red[0];
 }
 
 // Adam on one weight matrix [rows][cols] (rows >= valid_rows stay zero) and refresh of its BF16
@@ -168,12 +191,17 @@ struct souffle_mlp {
   int in_ld[kLayers];                               // row stride of the layer input (mult. of 8)
   cudaStream_t stream = nullptr;
   DevBuf<float> w[kLayers], b[kLayers], mw[kLayers], vw[kLayers], mb[kLayers], vb[kLayers];
-  DevBuf<float> gw[kLayers], gb[kLayers];
+  DevBuf<float> grads;                 // flat, the parameters' layout, then the loss
+  float* gw[kLayers] = {};             // inside grads
+  float* gb[kLayers] = {};
+  DevBuf<float> dw_ws;                 // partial weight gradients (allocated by the first training call)
   DevBuf<__nv_bfloat16> wb[kLayers], wbt[kLayers];
   DevBuf<__nv_bfloat16> act[kLayers], act_t[kLayers];  // a_0 .. a_3 and transposes
   DevBuf<float> z[kLayers];                            // z_1 .. z_3 (index l for layer l output)
   DevBuf<__nv_bfloat16> dz[kLayers + 1], dz_t[kLayers + 1];  // dZ_l for l = 1..4 (4 = dY)
-  DevBuf<float> y, partial, loss;
+  DevBuf<float> y, partial;
+  float* loss = nullptr;               // inside grads
+  float* host = nullptr;               // pinned: loss and error word of the last training call
   DevBuf<__nv_bfloat16> yb;  // BF16 copy of the output rows (fused forward for the surrogate)
   DevBuf<unsigned int> err;
   long long steps = 0;
@@ -239,27 +267,15 @@ souffle_status forward(souffle_mlp* h, int m, bool keep) {
 souffle_status backward(souffle_mlp* h, const float* t, int m) {
   const int L = kLayers - 1;
   const int np_out = h->out_pad[L];
-  const int nb = blocks((long long)m * np_out, 256);
+  const int nb = blocks(m, kLossRows);
   MLP_TRY(h->partial.n < (size_t)nb ? cudaErrorInvalidValue : cudaSuccess);
+  if (h->dw_ws.n == 0) MLP_TRY(h->dw_ws.alloc(kDwItems * kDwTile));
   k_loss<<<nb, 256, 0, h->stream>>>(h->y.p, np_out, t, m, h->n_out, np_out, h->dz[L + 1].p, h->dz_t[L + 1].p, h->cap,
                                     h->partial.p);
   MLP_TRY(cudaGetLastError());
-  k_sum<<<1, 256, 0, h->stream>>>(h->partial.p, nb, h->loss.p);
-  for (int l = L; l >= 0; l--) {
-    // dW_l [out_pad][in] = dZ_l^T a_{l-1}: A = dZ_l^T [out_pad][m], B = a_{l-1}^T [in][m], K = m
+  // dZ_l (input side of layer l) = (dZ_{l+1} W_l) * SiLU'(z_l): A = dZ [m][rows], B = W_l^T [in][rows]
+  for (int l = L; l > 0; l--) {
     const int rows = (l == L) ? np_out : h->out[l];
-    GemmEpi e;
-    e.M = rows;
-    e.N = h->in[l];
-    e.K = m;
-    e.err = h->err.p;
-    e.out_f32 = h->gw[l].p;
-    e.ldo = h->in[l];
-    MLP_TRY(gemm_bf16(h->dz_t[l + 1].p, h->cap, h->act_t[l].p, h->cap, e, h->stream));
-    k_row_sums<<<blocks(rows, 8), 256, 0, h->stream>>>(h->dz_t[l + 1].p, rows, m, h->cap, h->gb[l].p);
-    MLP_TRY(cudaGetLastError());
-    if (l == 0) break;
-    // dZ_{l} (input side of layer l) = (dZ_{l+1} W_l) * SiLU'(z_l): A = dZ [m][rows], B = W_l^T [in][rows]
     GemmEpi d;
     d.M = m;
     d.N = h->in[l];
@@ -274,13 +290,53 @@ souffle_status backward(souffle_mlp* h, const float* t, int m) {
     d.ldt = h->cap;
     MLP_TRY(gemm_bf16(h->dz[l + 1].p, rows, h->wbt[l].p, rows, d, h->stream));
   }
+  // every layer's dW_l [out][in] = dZ_{l+1}^T a_l (contraction over the batch) and db_l = row sums of
+  // dZ_{l+1}^T
+  DwArgs w;
+  w.layers = kLayers;
+  w.K = m;
+  w.ld = h->cap;
+  w.ws = h->dw_ws.p;
+  w.err = h->err.p;
+  w.loss_partial = h->partial.p;
+  w.n_partial = nb;
+  w.loss = h->loss;
+  for (int l = 0; l < kLayers; l++) {
+    w.layer[l].A = h->dz_t[l + 1].p;
+    w.layer[l].B = h->act_t[l].p;
+    w.layer[l].rows = h->out[l];
+    w.layer[l].cols = h->in[l];
+    w.layer[l].out = h->gw[l];
+    w.layer[l].bias_out = h->gb[l];
+  }
+  dw_plan(w);
+  MLP_TRY(dw_gemm(w, h->stream));
+  MLP_TRY(dw_reduce(w, h->stream));
   return SOUFFLE_OK;
 }
 
 souffle_status pack_input(souffle_mlp* h, const float* x, int m, bool keep) {
-  k_pack_input<<<blocks((long long)m * h->n_in, 256), 256, 0, h->stream>>>(
-      x, m, h->n_in, h->act[0].p, h->in_ld[0], keep ? h->act_t[0].p : nullptr, h->cap);
+  if (keep)
+    k_pack_input_t<<<dim3(blocks(m, kPackRows), blocks(h->n_in, 64)), 256, 0, h->stream>>>(x, m, h->n_in, h->act[0].p, h->in_ld[0],
+                                                                                    h->act_t[0].p, h->cap);
+  else
+    k_pack_input<<<blocks((long long)m * h->n_in, 256), 256, 0, h->stream>>>(x, m, h->n_in, h->act[0].p, h->in_ld[0]);
   MLP_TRY(cudaGetLastError());
+  return SOUFFLE_OK;
+}
+
+// Waits for a training call's work; its loss, and its error word as a status.
+souffle_status training_result(souffle_mlp* h, int m, float* loss) {
+  MLP_TRY(cudaMemcpyAsync(h->host, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+  MLP_TRY(cudaMemcpyAsync(h->host + 1, h->err.p, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
+  MLP_TRY(cudaStreamSynchronize(h->stream));
+  unsigned int e;
+  std::memcpy(&e, h->host + 1, sizeof(e));
+  if (e) {
+    cudaMemsetAsync(h->err.p, 0, sizeof(unsigned int), h->stream);
+    return fail(SOUFFLE_ERR_CUDA, "tensor-core GEMM: a bounded wait ran out");
+  }
+  if (loss) *loss = h->host[0] / ((float)m * (float)h->n_out);
   return SOUFFLE_OK;
 }
 
@@ -291,10 +347,10 @@ souffle_status refresh_bf16(souffle_mlp* h, float lr) {
   for (int l = 0; l < kLayers; l++) {
     const int rows = h->out_pad[l], cols = h->in[l];
     k_adam_w<<<blocks((long long)rows * cols, 256), 256, 0, h->stream>>>(
-        h->w[l].p, h->mw[l].p, h->vw[l].p, h->gw[l].p, rows, h->out[l], cols, lr, c1, c2, h->wb[l].p, h->wbt[l].p);
+        h->w[l].p, h->mw[l].p, h->vw[l].p, h->gw[l], rows, h->out[l], cols, lr, c1, c2, h->wb[l].p, h->wbt[l].p);
     MLP_TRY(cudaGetLastError());
     if (lr > 0.0f) {
-      k_adam_b<<<blocks(h->out[l], 256), 256, 0, h->stream>>>(h->b[l].p, h->mb[l].p, h->vb[l].p, h->gb[l].p, h->out[l],
+      k_adam_b<<<blocks(h->out[l], 256), 256, 0, h->stream>>>(h->b[l].p, h->mb[l].p, h->vb[l].p, h->gb[l], h->out[l],
                                                               lr, c1, c2);
       MLP_TRY(cudaGetLastError());
     }
@@ -318,7 +374,7 @@ cudaError_t mlp_forward_async(souffle_mlp* h, const float* x, int m_cap, const i
                               cudaStream_t st, const float** y, int* ldy) {
   if (m_cap < 1 || m_cap > h->cap) return cudaErrorInvalidValue;
   k_pack_input<<<std::min(blocks((long long)m_cap * h->n_in, 256), 152 * 8), 256, 0, st>>>(
-      x, m_cap, h->n_in, h->act[0].p, h->in_ld[0], nullptr, h->cap, m_dyn);
+      x, m_cap, h->n_in, h->act[0].p, h->in_ld[0], m_dyn);
   cudaError_t r = cudaGetLastError();
   if (r != cudaSuccess) return r;
   return mlp_forward_packed_async(h, m_cap, m_dyn, err, st, y, ldy);
@@ -407,6 +463,7 @@ souffle_status souffle_mlp_create(int32_t n_in, int32_t width, int32_t n_out, in
     h->in_ld[l] = round_up(dims[l], 8);
   }
   auto cleanup = [&](souffle_status s) {
+    if (h->host) cudaFreeHost(h->host);
     delete h;
     return s;
   };
@@ -424,12 +481,12 @@ souffle_status souffle_mlp_create(int32_t n_in, int32_t width, int32_t n_out, in
     std::uniform_real_distribution<float> u(-lim, lim);
     for (int r = 0; r < h->out[l]; r++)
       for (int c = 0; c < h->in[l]; c++) w[(size_t)r * h->in[l] + c] = u(rng);
-    for (auto* buf : {&h->w[l], &h->mw[l], &h->vw[l], &h->gw[l]}) {
+    for (auto* buf : {&h->w[l], &h->mw[l], &h->vw[l]}) {
       MLP_TRY_C(buf->alloc(nw));
       MLP_TRY_C(cudaMemset(buf->p, 0, nw * sizeof(float)));
     }
     MLP_TRY_C(cudaMemcpy(h->w[l].p, w.data(), nw * sizeof(float), cudaMemcpyHostToDevice));
-    for (auto* buf : {&h->b[l], &h->mb[l], &h->vb[l], &h->gb[l]}) {
+    for (auto* buf : {&h->b[l], &h->mb[l], &h->vb[l]}) {
       MLP_TRY_C(buf->alloc(h->out_pad[l]));
       MLP_TRY_C(cudaMemset(buf->p, 0, h->out_pad[l] * sizeof(float)));
     }
@@ -451,8 +508,21 @@ souffle_status souffle_mlp_create(int32_t n_in, int32_t width, int32_t n_out, in
   MLP_TRY_C(h->yb.alloc((size_t)h->cap * h->out_pad[kLayers - 1]));
   for (auto* b : {&h->x_mean, &h->x_istd}) MLP_TRY_C(b->alloc(n_in));
   for (auto* b : {&h->t_mean, &h->t_std, &h->t_istd}) MLP_TRY_C(b->alloc(n_out));
-  MLP_TRY_C(h->partial.alloc(blocks((long long)h->cap * h->out_pad[kLayers - 1], 256)));
-  MLP_TRY_C(h->loss.alloc(1));
+  MLP_TRY_C(h->partial.alloc(blocks(h->cap, kLossRows)));
+  {  // gradients in the parameters' flat layout; every matrix starts on a 16-byte boundary there
+    size_t n = 0;
+    for (int l = 0; l < kLayers; l++) n += (size_t)h->out[l] * h->in[l] + h->out[l];
+    MLP_TRY_C(h->grads.alloc(n + 1));
+    MLP_TRY_C(cudaMemset(h->grads.p, 0, (n + 1) * sizeof(float)));
+    float* p = h->grads.p;
+    for (int l = 0; l < kLayers; l++) {
+      h->gw[l] = p;
+      h->gb[l] = p + (size_t)h->out[l] * h->in[l];
+      p = h->gb[l] + h->out[l];
+    }
+    h->loss = p;
+  }
+  MLP_TRY_C(cudaMallocHost(&h->host, 2 * sizeof(float)));
   MLP_TRY_C(h->err.alloc(1));
   MLP_TRY_C(cudaMemset(h->err.p, 0, sizeof(unsigned int)));
 #undef MLP_TRY_C
@@ -470,6 +540,7 @@ souffle_status souffle_mlp_destroy(souffle_mlp* h) {
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->stream);
   cudaStream_t s = h->stream;
+  if (h->host) cudaFreeHost(h->host);
   delete h;
   if (s) cudaStreamDestroy(s);
   return SOUFFLE_OK;
@@ -588,21 +659,9 @@ souffle_status souffle_mlp_gradients(souffle_mlp* h, const float* x_dev, const f
   if (s == SOUFFLE_OK) s = forward(h, m, true);
   if (s == SOUFFLE_OK) s = backward(h, t_dev, m);
   if (s != SOUFFLE_OK) return s;
-  s = check_gemm_err(h);
-  if (s != SOUFFLE_OK) return s;
-  float* p = grad_host;
-  for (int l = 0; l < kLayers; l++) {
-    MLP_TRY(cudaMemcpy(p, h->gw[l].p, sizeof(float) * h->out[l] * h->in[l], cudaMemcpyDeviceToHost));
-    p += (size_t)h->out[l] * h->in[l];
-    MLP_TRY(cudaMemcpy(p, h->gb[l].p, sizeof(float) * h->out[l], cudaMemcpyDeviceToHost));
-    p += h->out[l];
-  }
-  if (loss) {
-    float sq = 0;
-    MLP_TRY(cudaMemcpy(&sq, h->loss.p, sizeof(float), cudaMemcpyDeviceToHost));
-    *loss = sq / ((float)m * (float)h->n_out);
-  }
-  return SOUFFLE_OK;
+  MLP_TRY(cudaMemcpyAsync(grad_host, h->grads.p, sizeof(float) * (size_t)souffle_mlp_param_count(h), cudaMemcpyDeviceToHost,
+                          h->stream));
+  return training_result(h, m, loss);
 }
 
 souffle_status souffle_mlp_train_step(souffle_mlp* h, const float* x_dev, const float* t_dev, int32_t m, float lr,
@@ -614,14 +673,7 @@ souffle_status souffle_mlp_train_step(souffle_mlp* h, const float* x_dev, const 
   if (s == SOUFFLE_OK) s = backward(h, t_dev, m);
   if (s == SOUFFLE_OK) s = refresh_bf16(h, lr);
   if (s != SOUFFLE_OK) return s;
-  s = check_gemm_err(h);
-  if (s != SOUFFLE_OK) return s;
-  if (loss) {
-    float sq = 0;
-    MLP_TRY(cudaMemcpy(&sq, h->loss.p, sizeof(float), cudaMemcpyDeviceToHost));
-    *loss = sq / ((float)m * (float)h->n_out);
-  }
-  return SOUFFLE_OK;
+  return training_result(h, m, loss);
 }
 
 souffle_status souffle_gemm_bf16(const float* a_dev, const float* b_dev, int32_t m, int32_t n, int32_t k, float* c_dev,
@@ -637,8 +689,8 @@ souffle_status souffle_gemm_bf16(const float* a_dev, const float* b_dev, int32_t
   MLP_TRY(b.alloc((size_t)n * ldk));
   MLP_TRY(err.alloc(1));
   MLP_TRY(cudaMemset(err.p, 0, sizeof(unsigned int)));
-  k_pack_input<<<blocks((long long)m * k, 256), 256>>>(a_dev, m, k, a.p, ldk, nullptr, 0);
-  k_pack_input<<<blocks((long long)n * k, 256), 256>>>(b_dev, n, k, b.p, ldk, nullptr, 0);
+  k_pack_input<<<blocks((long long)m * k, 256), 256>>>(a_dev, m, k, a.p, ldk);
+  k_pack_input<<<blocks((long long)n * k, 256), 256>>>(b_dev, n, k, b.p, ldk);
   MLP_TRY(cudaGetLastError());
   GemmEpi e;
   e.M = m;

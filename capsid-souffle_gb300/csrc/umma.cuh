@@ -30,6 +30,12 @@ __device__ __forceinline__ bool elect_one() {
   return ok != 0;
 }
 
+// Programmatic dependent launch: pdl_wait blocks until the kernels that this one depends on have
+// completed (at once without the launch attribute); pdl_launch lets the next one start its own
+// set-up.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
