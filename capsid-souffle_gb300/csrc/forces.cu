@@ -796,6 +796,15 @@ __global__ void k_state_out(StateArgs a) {
     a.force_out[3 * g + 1] = (double)a.fy_in[g] * inv;
     a.force_out[3 * g + 2] = (double)a.fz_in[g] * inv;
   }
+  const long long N = a.n;
+  for (int k = 0; k < 2; k++) {  // the parts, when asked for
+    double* out = k == 0 ? a.sforce_out : a.bforce_out;
+    if (!out) continue;
+    const float* in = a.sb_in + 3 * k * N + g;
+    out[3 * g] = (double)in[0];
+    out[3 * g + 1] = (double)in[N];
+    out[3 * g + 2] = (double)in[2 * N];
+  }
 }
 
 }  // namespace souffle

@@ -142,6 +142,9 @@ struct StateArgs {
   double* vel_out;
   double* force_out;     // [N*3] optional
   const long long* fx_in; const long long* fy_in; const long long* fz_in;
+  double* sforce_out;    // [N*3] optional: stretching and bending force from sb_in
+  double* bforce_out;
+  const float* sb_in;    // [6][N]
 };
 
 struct EnergyArgs {

@@ -1020,22 +1020,9 @@ void souffle_gpu_host_free(void* p) {
   if (p) cudaFreeHost(p);
 }
 
-static souffle_status copy_force_out(souffle_gpu_system* h, const float* dev3, double* host) {
-  // device float SoA [3][N] -> host double xyz interleaved
-  const int64_t N = h->N;
-  std::vector<float> tmp(3 * N);
-  CUDA_TRY(cudaMemcpyAsync(tmp.data(), dev3, sizeof(float) * 3 * N, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
-  for (int64_t i = 0; i < N; i++) {
-    host[3 * i] = tmp[i];
-    host[3 * i + 1] = tmp[N + i];
-    host[3 * i + 2] = tmp[2 * N + i];
-  }
-  return SOUFFLE_OK;
-}
-
-// Total force (int64, 2^-32 units) to host doubles, xyz interleaved.
-static souffle_status copy_total_force_out(souffle_gpu_system* h, double* host) {
+// Total (int64, 2^-32 units), stretching and bending forces (FP32) as doubles, xyz interleaved, in the
+// staging buffer: stretching at 0, bending at 3 N, total at 6 N.
+static void launch_force_out(souffle_gpu_system* h, bool total, bool stretch, bool bend) {
   const int64_t N = h->N;
   StateArgs a{};
   a.sys = h->d_sys.p;
@@ -1043,15 +1030,14 @@ static souffle_status copy_total_force_out(souffle_gpu_system* h, double* host) 
   a.bead_sys = h->d_bead_sys.p;
   a.np = h->tpl.np;
   a.n = (int)N;
-  a.force_out = h->staging.p + 6 * N;
+  if (total) a.force_out = h->staging.p + 6 * N;
   a.fx_in = h->force.p;
   a.fy_in = h->force.p + N;
   a.fz_in = h->force.p + 2 * N;
+  if (stretch) a.sforce_out = h->staging.p;
+  if (bend) a.bforce_out = h->staging.p + 3 * N;
+  a.sb_in = h->sbforce.p;
   launch_state_out(a, (int)((N + 255) / 256), 256, h->stream);
-  CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaMemcpyAsync(host, a.force_out, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
-  return SOUFFLE_OK;
 }
 
 souffle_status souffle_gpu_forces(souffle_gpu_system* h, int32_t rebuild, double* tforce, double* sforce,
@@ -1064,6 +1050,7 @@ souffle_status souffle_gpu_forces(souffle_gpu_system* h, int32_t rebuild, double
   for (int attempt = 0; attempt < 4; attempt++) {
     if (rebuild) launch_rebuild(h);
     launch_forces_all(h, 0, parts);
+    launch_force_out(h, tforce != nullptr, sforce != nullptr, bforce != nullptr);
     CUDA_TRY(cudaGetLastError());
     s = check_err(h);
     // a forces-only call changes no state, so an overflowing list is rebuilt with twice the room
@@ -1080,9 +1067,12 @@ souffle_status souffle_gpu_forces(souffle_gpu_system* h, int32_t rebuild, double
     h->graphs.clear();
   }
   if (s != SOUFFLE_OK) return s;
-  if (tforce && (s = copy_total_force_out(h, tforce)) != SOUFFLE_OK) return s;
-  if (sforce && (s = copy_force_out(h, h->sbforce.p, sforce)) != SOUFFLE_OK) return s;
-  if (bforce && (s = copy_force_out(h, h->sbforce.p + 3 * h->N, bforce)) != SOUFFLE_OK) return s;
+  const int64_t N = h->N;
+  double* const out[3] = {sforce, bforce, tforce};
+  for (int k = 0; k < 3; k++)
+    if (out[k])
+      CUDA_TRY(cudaMemcpyAsync(out[k], h->staging.p + 3 * k * N, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
   return SOUFFLE_OK;
 }
 
