@@ -247,3 +247,50 @@ def test_driver_analysis_writes_the_reference_files(tmp_path, name):
     for fn in FILES:
         assert (out / fn).read_text() == str(g["out_" + fn.replace(".", "_")]), fn
     assert r.stdout == str(g["ref_stdout"])
+
+
+@pytest.mark.parametrize("F, crowded", [(1, ()), (8, (7,)), (9, (0,)), (19, (3, 8, 18))])
+def test_many_frames_equal_one_frame_calls(F, crowded):
+    """Frames are taken through two input slots, eight to a chunk: chunk edges, frames in the middle
+    and at the end of a chunk whose candidate pairs do not fit and are run again, types that differ
+    from frame to frame, and the last frame's types kept for a call without any."""
+    S, np_, L = 150, 43, 60.0
+    rng = np.random.default_rng(F)
+    frames = [_synthetic(60 + k, S, np_, L, so_per=4 + k % 3, pcf_per=3 + k % 2) for k in range(F)]
+    types = np.stack([f[0] for f in frames])
+    pos = np.stack([f[1] for f in frames])
+    for k in crowded:
+        pos[k] = np.concatenate([c + rng.uniform(-1.5, 1.5, (np_, 3)) for c in rng.uniform(-1.5, 1.5, (S, 3))])
+    many = _analysis(S * np_, np_, L, ao.IMAGE_REFERENCE)
+    one = _analysis(S * np_, np_, L, ao.IMAGE_REFERENCE)
+    r = many.frames(pos, types)
+    last = many.last_counts()
+    for k in range(F):
+        ref = one.frames(pos[k:k + 1], types[k])
+        for key in r:
+            np.testing.assert_array_equal(r[key][k], ref[key][0], err_msg=f"{key} of frame {k}")
+    assert last[0] == one.last_counts()[0]
+    again = many.frames(pos, None)
+    for k in range(F):
+        ref = one.frames(pos[k:k + 1], None)
+        for key in r:
+            np.testing.assert_array_equal(again[key][k], ref[key][0], err_msg=f"{key} of frame {k}, kept types")
+
+
+def test_types_after_a_bad_frame_are_that_frames():
+    """A call without types after an error in the middle of a chunk takes the failed frame's."""
+    from souffle_gb300.gpu import SouffleError
+    S, np_, L = 60, 43, 40.0
+    frames = [_synthetic(90 + k, S, np_, L, so_per=4 + k % 3) for k in range(12)]
+    types = np.stack([f[0] for f in frames]).astype(np.int32)
+    pos = np.stack([f[1] for f in frames])
+    a = _analysis(S * np_, np_, L, ao.IMAGE_REFERENCE)
+    ref = a.frames(pos, types)
+    kept = a.frames(pos[:1], types[10])
+    bad = pos.copy()
+    bad[10] += 40.0
+    with pytest.raises(SouffleError):
+        a.frames(bad, types)
+    again = a.frames(pos[:1], None)
+    for key in ref:
+        np.testing.assert_array_equal(again[key], kept[key], err_msg=key)
