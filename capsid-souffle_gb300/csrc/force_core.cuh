@@ -3,7 +3,7 @@
 //
 //   force_setup      template tables and per-item constants into shared memory
 //   force_rel        a bead's packed coordinates relative to its subunit's centre bead
-//   force_prefix     prefix sums of the inter-subunit list lengths
+//   force_rows       the beads that have inter-subunit pairs, those with long lists apart
 //   force_terms      everything that depends on positions alone, in chunks of 32 lanes that the
 //                    warps take from a counter: intra-subunit Debye-Hueckel rows, bending quads,
 //                    inter-subunit pairs, edges (the costliest chunks first)
@@ -102,7 +102,7 @@ struct ForceSmem {
   float* rel;          // [max_sub npp 8] packed partners: (x0, x1, y0, y1, z0, z1, w0, w1) per two beads
   long long* red;      // [4 warps]
   unsigned int* F;     // force limbs, 9 per bead
-  int* pref;           // prefix sums of the inter-subunit list lengths
+  int* rows;           // beads with inter-subunit pairs: bead | list length << 16, long lists from the front, others from the back
   float* tpl_f;
   int* tpl_i;
   float* w;            // [np] DH weights
@@ -117,8 +117,8 @@ __device__ __forceinline__ ForceSmem force_smem(unsigned char* base, const Force
   m.rel = reinterpret_cast<float*>(m.pos + a.max_sub * L.np);
   m.red = reinterpret_cast<long long*>(m.rel + 8 * a.max_sub * npp);
   m.F = reinterpret_cast<unsigned int*>(m.red + 4 * warps);
-  m.pref = reinterpret_cast<int*>(m.F + force_slot_len(a.max_sub * L.np));
-  m.tpl_f = reinterpret_cast<float*>(m.pref + force_pref_len(a.max_sub * L.np));  // [n_float], n_float % 4 == 0
+  m.rows = reinterpret_cast<int*>(m.F + force_slot_len(a.max_sub * L.np));
+  m.tpl_f = reinterpret_cast<float*>(m.rows + force_rows_len(a.max_sub * L.np));  // [n_float], n_float % 4 == 0
   m.tpl_i = reinterpret_cast<int*>(m.tpl_f + L.n_float);                          // [n_int], n_int % 4 == 0
   m.w = reinterpret_cast<float*>(m.tpl_i + L.n_int);
   return m;
@@ -154,36 +154,32 @@ __device__ __forceinline__ void force_rel(const ForceSmem& m, int np, int s, int
   }
 }
 
-// Exclusive prefix sums of the beads' inter-subunit list lengths (pref[nbead] = total): each thread
-// a run of `per` beads, a warp scan, then the warp totals (red is free until the end).  Contains
-// one barrier; the caller's next barrier makes pref visible.
-__device__ __forceinline__ void force_prefix(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int per = (nbead + blockDim.x - 1) / blockDim.x;
-  int my_cnt = 0;
-  for (int i = 0; i < per; i++) {
-    const int b = threadIdx.x * per + i;
-    if (b < nbead) my_cnt += __ldg(a.inter_count + bead0 + b);
-  }
-  int incl = my_cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  int* s_wtot = reinterpret_cast<int*>(m.red);
-  if (lane == 31) s_wtot[wid] = incl;
-  __syncthreads();
-  int off = incl - my_cnt;
-  for (int q = 0; q < wid; q++) off += s_wtot[q];
-  for (int i = 0; i < per; i++) {
-    const int b = threadIdx.x * per + i;
-    if (b < nbead) {
-      m.pref[b] = off;
-      off += __ldg(a.inter_count + bead0 + b);
+// What the warps of a CTA share: the position of the chunk queue and the numbers of long and short
+// inter-subunit rows.  Zero before force_rows.
+struct ForceQueue {
+  int next, n_long, n_short;
+};
+constexpr int kLongRow = 48;  // rows above this length take a whole warp (see force_inter)
+
+// The beads with inter-subunit pairs into m.rows (their order does not matter: every sum is exact).
+// The caller's next barrier makes them visible.
+__device__ __forceinline__ void force_rows(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead, ForceQueue* q) {
+  const int lane = threadIdx.x & 31;
+  for (int base = (int)threadIdx.x - lane; base < nbead; base += blockDim.x) {
+    const int t = base + lane;
+    const int n = t < nbead ? __ldg(a.inter_count + bead0 + t) : 0;
+    const unsigned int lg = __ballot_sync(0xffffffffu, n > kLongRow), sh = __ballot_sync(0xffffffffu, n > 0) & ~lg;
+    int l0 = 0, s0 = 0;
+    if (lane == 0) {
+      if (lg) l0 = atomicAdd(&q->n_long, __popc(lg));
+      if (sh) s0 = atomicAdd(&q->n_short, __popc(sh));
     }
+    l0 = __shfl_sync(0xffffffffu, l0, 0);
+    s0 = __shfl_sync(0xffffffffu, s0, 0);
+    const unsigned int below = (1u << lane) - 1u;
+    if (n > kLongRow) m.rows[l0 + __popc(lg & below)] = t | n << 16;
+    else if (n > 0) m.rows[nbead - 1 - (s0 + __popc(sh & below))] = t | n << 16;
   }
-  if (threadIdx.x == blockDim.x - 1) m.pref[nbead] = off;
 }
 
 // Edge t of the item: length vector and stretching coefficient (len0 - l) ks / l (BEAD::
@@ -340,127 +336,188 @@ __device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams&
   limbs_add(m.F + 9 * t + 6, f32_to_fx32(-ze) + f32_to_fx32(-zo));
 }
 
-// Inter-subunit pairs p .. pend - 1 (DH + LJ/WCA, src/forces.cpp:81-138) of the flat sequence that
-// the beads' lists form (pref: exclusive prefix sums of their lengths), so a bead with a long list
-// holds nobody up: the pairs are walked bead by bead, the pair forces of each bead summed exactly
-// in 2^-32 fixed point in registers and added to the bead's limbs at its last pair
-// (order-independent).  kFresh: the partners' positions are rewritten by other CTAs while this
-// kernel runs (read past L1).
-template <bool kFresh>
-__device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
-                                            int p, int pend) {
-  const TplLayout& L = a.L;
-  const int* species = m.tpl_i + L.o_species;
-  const float unit = P.unit32, kappa = P.kappa, ecut_el2 = P.ecut_el2;
-  const int ns = L.nspecies;
-  int lo = 0, hi = nbead;  // pref[lo] <= p < pref[hi]: the run starts in bead lo
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (m.pref[mid] <= p) lo = mid;
-    else hi = mid;
+// The sums of eight lanes' (or, whole, the warp's) force vectors added to a bead's limbs: the nine
+// limbs are halved among the lanes while they are summed, ten exchanges and two atomics of distinct
+// addresses; nine atomics of eight lanes on one address each cost 72 shared-memory cycles.
+__device__ __forceinline__ void limbs_add_lanes(unsigned int* F, long long x, long long y, long long z, bool valid, bool whole) {
+  const int lane = threadIdx.x & 31;
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+  const unsigned int v[9] = {(unsigned int)(x & 0x1FFFFF), (unsigned int)((x >> 21) & 0x1FFFFF), (unsigned int)(int)(x >> 42),
+                             (unsigned int)(y & 0x1FFFFF), (unsigned int)((y >> 21) & 0x1FFFFF), (unsigned int)(int)(y >> 42),
+                             (unsigned int)(z & 0x1FFFFF), (unsigned int)((z >> 21) & 0x1FFFFF), (unsigned int)(int)(z >> 42)};
+  unsigned int w[5], u[3], t[2];
+#pragma unroll
+  for (int k = 0; k < 5; k++) {  // limbs 0-4 to the even lanes, 5-8 to the odd
+    const unsigned int lo = v[k], hi = k < 4 ? v[5 + k] : 0u;
+    w[k] = (b0 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b0 ? lo : hi, 1);
   }
-  // the row of bead b holds its pairs pref[b] .. pref[b + 1] - 1 of the flat sequence; the next
-  // pair's bead, partner and partner position are fetched while the current one is evaluated
-  int nb = lo, nend = m.pref[nb + 1];
-  auto partner = [&](int q) { return __ldg(a.inter_ids + ((long long)(bead0 + nb) * a.inter_cap - m.pref[nb] + q)); };
-  auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
-  int4 next = position(partner(p));
-  int b = -1, si = 0;
-  int4 pi = make_int4(0, 0, 0, 0);
-  float wi = 0.f;
-  long long ax = 0, ay = 0, az = 0;
-  while (p < pend) {
-    const int4 pj = next;
-    if (nb != b) {  // first pair of a bead
-      b = nb;
-      pi = m.pos[b];
-      const int l = b - fast_div(b, a.div_np) * L.np;
-      si = species[l] * ns;
-      wi = m.w[l];
-    }
-    p++;
-    bool last = p >= pend;
-    if (!last) {
-      last = p >= nend;
-      while (p >= nend) nend = m.pref[++nb + 1];
-      next = position(partner(p));
-    }
-    const float3 d = dvec(pi, pj, unit);
-    const float r2 = dot3(d, d);
-    const int lj = pj.w;
-    const float wj = m.w[lj];
-    float c = 0.f;
-    if (wi * wj != 0.f && r2 < ecut_el2) {
-      const float ir = rsqrtf(r2);
-      const float r = r2 * ir;
-      c = wi * wj * __expf(-kappa * r) * (ir * ir) * (kappa + ir);
-    }
-    const float* pair = m.tpl_f + L.o_pair + 3 * (si + species[lj]);  // cut-off squared, sigma^6, epsilon
-    if (r2 < pair[0]) {
-      const float eps = pair[2] < 0.f ? P.elj_att : pair[2];
-      const float ir2 = 1.0f / r2;
-      const float s6 = pair[1] * ir2 * ir2 * ir2;
-      c += 48.0f * eps * s6 * (s6 - 0.5f) * ir2;
-    }
-    const float3 f = d * c;
-    if (force_bad(f.x, f.y, f.z)) {
-      atomicOr(a.err, kErrNonFinite);
-    } else {
-      ax += f32_to_fx32(f.x);
-      ay += f32_to_fx32(f.y);
-      az += f32_to_fx32(f.z);
-    }
-    if (last) {  // the bead's last pair here: add its sums to its limbs
-      limbs_add(m.F + 9 * b, ax);
-      limbs_add(m.F + 9 * b + 3, ay);
-      limbs_add(m.F + 9 * b + 6, az);
-      ax = ay = az = 0;
-    }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const unsigned int lo = w[k], hi = k < 2 ? w[3 + k] : 0u;
+    u[k] = (b1 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 2);
   }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const unsigned int lo = u[k], hi = k < 1 ? u[2] : 0u;
+    t[k] = (b2 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 4);
+  }
+  if (whole) {
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+      t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+      t[1] += __shfl_xor_sync(0xffffffffu, t[1], o);
+    }
+    valid = valid && lane < 8;
+  }
+  // a lane's limbs and how many of its two values are one
+  const int first = (b0 ? 5 : 0) + (b1 ? 3 : 0) + (b2 ? 2 : 0);
+  const int n = b1 ? (b2 ? 0 : b0 ? 1 : 2) : (b2 ? 1 : 2);
+  if (valid && n > 0) atomicAdd(F + first, t[0]);
+  if (valid && n > 1) atomicAdd(F + first + 1, t[1]);
 }
 
-// Everything that depends on positions alone, in chunks that the warps take from a counter (zero on
-// entry): the intra-subunit rows of 32 beads, 32 bending quads, 32 runs of inter-subunit pairs, 32
-// edges -- about 700, 450, 100 per pair of a run and 100 instructions.  The runs are as long as
-// gives every warp one chunk, at most eight pairs.  kFresh (the window kernel): the inter-subunit
-// pairs come last, and a warp's first one only after wait() -- by then the other CTAs have
-// published their new positions while this one worked on its own subunits.
-template <bool kFresh, class Wait>
-__device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
-                                            int nbead, int bead0, int* counter, Wait wait) {
+// LJ or WCA term of a pair (src/forces.cpp:81-138) added to its force coefficient.
+__device__ __forceinline__ float lj_add(float c, float r2, const float* pair, float elj_att) {
+  const float eps = pair[2] < 0.f ? elj_att : pair[2];
+  const float ir2 = 1.0f / r2;
+  const float s6 = pair[1] * ir2 * ir2 * ir2;
+  c += 48.0f * eps * s6 * (s6 - 0.5f) * ir2;
+  return c;
+}
+
+// Inter-subunit pairs (DH + LJ/WCA, src/forces.cpp:81-138) of a chunk of rows: four beads by eight
+// lanes each, or one bead with a long list (more than kLongRow pairs) by the whole warp -- at 48
+// pairs both take the same number of rounds per bead.  A lane evaluates two of the row's pairs at a
+// time in packed FP32, adds its pair forces exactly in 2^-32 fixed point in registers, and the
+// lanes' sums go to the bead's limbs at the end (order-independent).  What bounds it is the chain
+// of loads and arithmetic from one pair to the next, and in systems with a few crowded subunits
+// their CTA, which everyone else waits for.  So a row is spread over lanes: neighbouring lanes read
+// neighbouring partners, no lane searches for its bead, and lanes finish a row together.
+// Against runs of eight consecutive pairs of the flat pair sequence per thread: 2,000 subunits, a
+// tenth of them in contact, 3,900 -> 3,430 us per 100 steps; 64: 1,870 -> 1,765; 64 dense replicas 1.5 %.
+// kFresh: the partners' positions are rewritten by other CTAs while this kernel runs (read past L1).
+// kAhead: also the next two pairs' positions are fetched ahead, not their indices alone; worth the
+// registers where few warps share an SM (64 subunits: 1765 against 1846 us per 100 steps), not
+// where five CTAs do (2,000 subunits: 3543 against 3431).
+template <bool kFresh, bool kAhead>
+__device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
+                                            const ForceQueue& q, int chunk) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
-  const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne, n_inter = m.pref[nbead];
-  const int run = min(8, (n_inter + (int)blockDim.x - 1) / (int)blockDim.x), per = 32 * run;
-  const int ki = (nbead + 31) >> 5, kq = (nq + 31) >> 5, ke = (ne + 31) >> 5,
-            kp = n_inter > 0 ? (n_inter + per - 1) / per : 0;
-  const int total = ki + kq + ke + kp;
+  const int* species = m.tpl_i + L.o_species;
+  const float unit = P.unit32, ecut_el2 = P.ecut_el2;
+  const bool whole = chunk < q.n_long;
+  const int lanes = whole ? 32 : 8;
+  const int row = whole ? chunk : 4 * (chunk - q.n_long) + (lane >> 3);
+  const int rec = whole || row < q.n_short ? m.rows[whole ? row : nbead - 1 - row] : 0;
+  const int b = rec & 0xffff, n = rec >> 16;
+  const int* ids = a.inter_ids + (long long)(bead0 + b) * a.inter_cap;
+  const int4 pi = m.pos[b];
+  const int l = b - fast_div(b, a.div_np) * L.np;
+  const int si = species[l] * L.nspecies;
+  const float wi = m.w[l];
+  const f32x2 nk2 = pack2(-P.kappa, -P.kappa), kap2 = pack2(P.kappa, P.kappa), le2 = pack2(1.44269504f, 1.44269504f),
+              wi2 = pack2(wi, wi);
+  // (past the row's end: the bead itself, dropped below)
+  auto partner = [&](int i) { return i < n ? __ldg(ids + i) : bead0 + b; };
+  auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
+  int i = lane & (lanes - 1);
+  int j0 = partner(i), j1 = partner(i + lanes);
+  int4 n0, n1;
+  if (kAhead) n0 = position(j0), n1 = position(j1);
+  long long ax = 0, ay = 0, az = 0;
+  while (i < n) {
+    const int4 p0 = kAhead ? n0 : position(j0), p1 = kAhead ? n1 : position(j1);
+    const bool two = i + lanes < n;
+    i += 2 * lanes;
+    j0 = partner(i);  // the next two pairs, while these are evaluated
+    j1 = partner(i + lanes);
+    if (kAhead) n0 = position(j0), n1 = position(j1);
+    const f32x2 u2 = pack2(unit, unit);
+    const f32x2 dx = mul2(pack2((float)(int)((unsigned)pi.x - (unsigned)p0.x), (float)(int)((unsigned)pi.x - (unsigned)p1.x)), u2);
+    const f32x2 dy = mul2(pack2((float)(int)((unsigned)pi.y - (unsigned)p0.y), (float)(int)((unsigned)pi.y - (unsigned)p1.y)), u2);
+    const f32x2 dz = mul2(pack2((float)(int)((unsigned)pi.z - (unsigned)p0.z), (float)(int)((unsigned)pi.z - (unsigned)p1.z)), u2);
+    const f32x2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+    float ra, rb;
+    unpack2(r2, ra, rb);
+    const f32x2 ww = mul2(wi2, pack2(m.w[p0.w], m.w[p1.w]));
+    const f32x2 ir = pack2(rsqrt_ftz(ra), rsqrt_ftz(rb));
+    float ea, eb;
+    unpack2(mul2(mul2(nk2, mul2(r2, ir)), le2), ea, eb);
+    const f32x2 c = mul2(mul2(mul2(ww, pack2(ex2_ftz(ea), ex2_ftz(eb))), mul2(ir, ir)), add2(kap2, ir));
+    float wa, wb, ca, cb;
+    unpack2(ww, wa, wb);
+    unpack2(c, ca, cb);
+    ca = wa != 0.f && ra < ecut_el2 ? ca : 0.f;
+    cb = two && wb != 0.f && rb < ecut_el2 ? cb : 0.f;
+    const float* qa = m.tpl_f + L.o_pair + 3 * (si + species[p0.w]);  // cut-off squared, sigma^6, epsilon
+    const float* qb = m.tpl_f + L.o_pair + 3 * (si + species[p1.w]);
+    const bool la = ra < qa[0], lb = two && rb < qb[0];
+    if (la || lb) {
+      const float ta = lj_add(ca, ra, qa, P.elj_att), tb = lj_add(cb, rb, qb, P.elj_att);
+      ca = la ? ta : ca;
+      cb = lb ? tb : cb;
+    }
+    const f32x2 c2 = pack2(ca, cb);
+    float xa, xb, ya, yb, za, zb;
+    unpack2(mul2(dx, c2), xa, xb);
+    unpack2(mul2(dy, c2), ya, yb);
+    unpack2(mul2(dz, c2), za, zb);
+    // (a sum below the bound of one component: every component is good)
+    if (!(fabsf(xa) + fabsf(ya) + fabsf(za) + fabsf(xb) + fabsf(yb) + fabsf(zb) < 1.0e9f)) {
+      const bool bad_a = force_bad(xa, ya, za), bad_b = force_bad(xb, yb, zb);
+      if (bad_a || bad_b) atomicOr(a.err, kErrNonFinite);
+      if (bad_a) xa = ya = za = 0.f;
+      if (bad_b) xb = yb = zb = 0.f;
+    }
+    ax += f32_to_fx32(xa) + f32_to_fx32(xb);
+    ay += f32_to_fx32(ya) + f32_to_fx32(yb);
+    az += f32_to_fx32(za) + f32_to_fx32(zb);
+  }
+  __syncwarp();
+  limbs_add_lanes(m.F + 9 * b, ax, ay, az, n > 0, whole);
+}
+
+// Everything that depends on positions alone, in chunks that the warps take from the queue: long
+// inter-subunit rows, the intra-subunit rows of 32 beads (700 instructions), 32 bending quads (450),
+// four short inter-subunit rows, 32 edges (100).  kFresh (the window kernel): the inter-subunit
+// pairs come last, and a warp's first one only after wait() -- by then the other CTAs have
+// published their new positions while this one worked on its own subunits.
+template <bool kFresh, bool kAhead, class Wait>
+__device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
+                                            int nbead, int bead0, ForceQueue* q, Wait wait) {
+  const TplLayout& L = a.L;
+  const int lane = threadIdx.x & 31;
+  const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne;
+  const int ki = (nbead + 31) >> 5, kq = (nq + 31) >> 5, ke = (ne + 31) >> 5;
+  const ForceQueue rows{0, q->n_long, q->n_short};
+  const int kl = rows.n_long, ks = (rows.n_short + 3) >> 2;
+  // the order of the kinds of chunk
+  const int first_intra = kFresh ? 0 : kl, first_quad = first_intra + ki;
+  const int first_edge = first_quad + kq + (kFresh ? 0 : ks);
+  const int total = kl + ki + kq + ks + ke;
   bool waited = false;
   for (;;) {
     int k = 0;
-    if (lane == 0) k = atomicAdd(counter, 1);
+    if (lane == 0) k = atomicAdd(&q->next, 1);
     k = __shfl_sync(0xffffffffu, k, 0);
     if (k >= total) break;
-    if (k < ki) {
-      const int t = 32 * k + lane;
+    if (k >= first_intra && k < first_quad) {
+      const int t = 32 * (k - first_intra) + lane;
       if (t < nbead) force_intra(a, P, m, w, t);
-    } else if ((k -= ki) < kq) {
-      const int t = 32 * k + lane;
+    } else if (k >= first_quad && k < first_quad + kq) {
+      const int t = 32 * (k - first_quad) + lane;
       if (t < nq) force_quad(a, P, m, t);
+    } else if (k >= first_edge && k < first_edge + ke) {
+      const int t = 32 * (k - first_edge) + lane;
+      if (t < ne) force_edge(a, P, m, t);
     } else {
-      k -= kq;
-      const bool edge = kFresh ? k < ke : k >= kp;
-      if (edge) {
-        const int t = 32 * (kFresh ? k : k - kp) + lane;
-        if (t < ne) force_edge(a, P, m, t);
-      } else {
-        if (kFresh && !waited) {
-          wait();
-          waited = true;
-        }
-        const int p = (32 * (kFresh ? k - ke : k) + lane) * run;
-        if (p < n_inter) force_inter<kFresh>(a, P, m, nbead, bead0, p, min(n_inter, p + run));
+      if (kFresh && !waited) {
+        wait();
+        waited = true;
       }
+      // the long rows are the first kl of these chunks
+      force_inter<kFresh, kAhead>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq);
     }
     __syncwarp();
   }

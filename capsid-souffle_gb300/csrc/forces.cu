@@ -174,8 +174,10 @@ __global__ void __launch_bounds__(256, 5) k_forces(ForceArgs a) {
   const float* tpl_f = m.tpl_f;
   const float* s_w = m.w;
   const float unit = P.unit32;
-  __shared__ int s_counter;
-  if (threadIdx.x == 0) s_counter = 0;
+  __shared__ ForceQueue s_queue;
+  if (threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0};
+  __syncthreads();
+  force_rows(a, m, bead0, nbead, &s_queue);
   force_setup(a, w, m);
   for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
     const int4 p = a.pos32[bead0 + t];
@@ -189,9 +191,8 @@ __global__ void __launch_bounds__(256, 5) k_forces(ForceArgs a) {
   __shared__ unsigned int s_bbm[16 * kBBWords];
   const bool bb_filter = P.nbb > 0 && P.nbb <= 32 * kBBWords && w.nsub <= 16;
   if (threadIdx.x < 16 * kBBWords) s_bbm[threadIdx.x] = 0u;
-  force_prefix(a, m, bead0, nbead);  // (its barrier makes the tile visible)
-  __syncthreads();               // the prefix sums
-  force_terms<false>(a, P, m, w, nbead, bead0, &s_counter, [] {});
+  __syncthreads();
+  force_terms<false, false>(a, P, m, w, nbead, bead0, &s_queue, [] {});
   __syncthreads();
   const float* s_mass = tpl_f + L.o_mass;
   const SysState& st = a.state[w.sys];
@@ -488,7 +489,9 @@ struct GridBarrier {
   static constexpr unsigned int kWindowPolls = 1u << 22;
 };
 
-__global__ void __launch_bounds__(256, 5) k_window(ForceArgs a, DriftArgs d, WindowArgs q) {
+// kWide: 512 threads and 64 registers (two CTAs per SM) instead of 256 and 48, for grids that fit.
+template <bool kWide>
+__global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(ForceArgs a, DriftArgs d, WindowArgs q) {
   extern __shared__ __align__(16) unsigned char smem[];
   const TplLayout& L = a.L;
   const WorkItem w = a.work[blockIdx.x];
@@ -504,12 +507,18 @@ __global__ void __launch_bounds__(256, 5) k_window(ForceArgs a, DriftArgs d, Win
   dfloat* s_im = reinterpret_cast<dfloat*>(s_kc + ((np + 1) & ~1));     // [np] 1 / m
   SysState& S = *reinterpret_cast<SysState*>(s_im + ((np + 1) & ~1));
   dfloat* chain_scratch = reinterpret_cast<dfloat*>(&S + 1);
-  __shared__ int s_counter, s_abort;
+  __shared__ ForceQueue s_queue;
+  __shared__ int s_abort;
   __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
   GridBarrier moved{q.count, a.err, 0u}, summed{q.count + 1, a.err, 0u};  // positions published, sums complete
   const float unit = P.unit32;
   const bool bd = P.brownian;
-  if (threadIdx.x == 0) s_abort = 0;
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    s_queue = ForceQueue{0, 0, 0};
+  }
+  __syncthreads();
+  force_rows(a, m, bead0, nbead, &s_queue);
   force_setup(a, w, m);
   {
     const int4* src = reinterpret_cast<const int4*>(a.state + w.sys);
@@ -545,13 +554,12 @@ __global__ void __launch_bounds__(256, 5) k_window(ForceArgs a, DriftArgs d, Win
       put_fx(F, a.fx[g], a.fy[g], a.fz[g]);
     }
   }
-  force_prefix(a, m, bead0, nbead);  // (its barrier also shows the state and the beads)
   __syncthreads();
   const float* s_mass = m.tpl_f + L.o_mass;
   for (int step = 0; step < q.steps; step++) {
     long long* acc = q.acc + (size_t)(step % 3) * q.acc_stride;
     const bool drift = step > 0 || !q.forces_first;
-    if (threadIdx.x == 0) s_counter = 0;
+    if (threadIdx.x == 0) s_queue.next = 0;
     if (drift) {
       long long rx = 0, ry = 0, rz = 0;
       for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
@@ -607,7 +615,7 @@ __global__ void __launch_bounds__(256, 5) k_window(ForceArgs a, DriftArgs d, Win
       force_rel(m, np, s, l, m.pos[t], m.pos[s * np + P.center_local], m.w[l], unit);
     }
     __syncthreads();
-    force_terms<true>(a, P, m, w, nbead, bead0, &s_counter, [&] {
+    force_terms<true, kWide>(a, P, m, w, nbead, bead0, &s_queue, [&] {
       if (drift) {
         if (lane == 0) moved.wait(&s_abort);
         __syncwarp();
@@ -827,15 +835,17 @@ size_t window_smem_bytes(size_t force_bytes, int subs, int np) {
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
                           cudaStream_t s) {
   void* args[] = {const_cast<ForceArgs*>(&a), const_cast<DriftArgs*>(&d), const_cast<WindowArgs*>(&q)};
-  return cudaLaunchCooperativeKernel((const void*)k_window, dim3(grid), dim3(block), args, smem, s);
+  return cudaLaunchCooperativeKernel(q.wide ? (const void*)k_window<true> : (const void*)k_window<false>, dim3(grid), dim3(block),
+                                     args, smem, s);
 }
-cudaError_t window_wave_ctas(int threads, size_t smem, int* ctas) {
+cudaError_t window_wave_ctas(bool wide, int threads, size_t smem, int* ctas) {
   *ctas = 0;
-  cudaError_t e = cudaFuncSetAttribute(k_window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const void* fn = wide ? (const void*)k_window<true> : (const void*)k_window<false>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(k_window, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess) return e;
   int per_sm = 0, dev = 0, sms = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_window, threads, smem)) != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem)) != cudaSuccess) return e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   *ctas = per_sm * sms;

@@ -119,6 +119,7 @@ struct DriftArgs {
 
 // The window kernel: steps per launch, its grid barrier and sums.
 struct WindowArgs {
+  int wide;              // the 512-thread form (as window_wave_ctas was asked about)
   int steps;
   int forces_first;        // the first step's drift has run (and the pair lists were rebuilt after it)
   int n_sys;
@@ -216,7 +217,7 @@ void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s);
 size_t window_smem_bytes(size_t force_bytes, int subs, int np);
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
                           cudaStream_t s);
-cudaError_t window_wave_ctas(int threads, size_t smem, int* ctas);
+cudaError_t window_wave_ctas(bool wide, int threads, size_t smem, int* ctas);
 void launch_state_in(const StateArgs& a, int grid, int block, cudaStream_t s);
 void launch_state_out(const StateArgs& a, int grid, int block, cudaStream_t s);
 void launch_energies(const EnergyArgs& a, int n, cudaStream_t s);

@@ -518,25 +518,26 @@ bool window_usable(const souffle_gpu_system* h) {
   return true;
 }
 
-// `len` steps in one launch; forces_first: the drift of the first one has been launched already
-cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_first) {
-  WindowArgs q{};
-  q.steps = len;
-  q.forces_first = forces_first ? 1 : 0;
-  q.n_sys = h->n_sys;
-  q.count = h->win_count.p;
-  q.acc = h->win_acc.p;
-  q.acc_stride = 8 * (size_t)h->n_sys;
-  q.force_bytes = (h->force_smem + 15) & ~(size_t)15;
-  return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->threads, h->window_smem, h->stream);
-}
-
 size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
   const TplLayout& L = h->L;
   const int np = h->tpl.np;
   return force_tile_bytes(subs, L.ne, L.nbend) + sizeof(int4) * subs * np + 8 * sizeof(float) * subs * ((np + 1) / 2) +
          sizeof(long long) * 4 * (threads / 32) + sizeof(unsigned int) * force_slot_len(subs * np) +
-         sizeof(int) * force_pref_len(subs * np) + sizeof(float) * (np + L.n_float) + sizeof(int) * L.n_int;
+         sizeof(int) * force_rows_len(subs * np) + sizeof(float) * (np + L.n_float) + sizeof(int) * L.n_int;
+}
+
+// `len` steps in one launch; forces_first: the drift of the first one has been launched already
+cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_first) {
+  WindowArgs q{};
+  q.steps = len;
+  q.wide = h->window_wide ? 1 : 0;
+  q.forces_first = forces_first ? 1 : 0;
+  q.n_sys = h->n_sys;
+  q.count = h->win_count.p;
+  q.acc = h->win_acc.p;
+  q.acc_stride = 8 * (size_t)h->n_sys;
+  q.force_bytes = (force_smem_for(h, h->subs_per_cta, h->window_threads) + 15) & ~(size_t)15;
+  return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->window_threads, h->window_smem, h->stream);
 }
 
 // Work items of up to `subs` subunits of one system each (one force-kernel CTA per item, in
@@ -556,8 +557,8 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   CUDA_TRY(set_kernel_smem(smem, threads, h->pair_smem));
   int wave = 0, win_wave = 0;
   CUDA_TRY(force_wave_ctas(threads, smem, &wave));
-  const size_t win_smem = window_smem_bytes(smem, subs, h->tpl.np);
-  if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(threads, win_smem, &win_wave));
+  size_t win_smem = window_smem_bytes(smem, subs, h->tpl.np);
+  if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(false, threads, win_smem, &win_wave));
   std::vector<WorkItem> work;
   std::vector<int2> slots;
   int sub0 = 0;
@@ -607,8 +608,29 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   h->subs_per_cta = subs;
   h->threads = threads;
   h->force_smem = smem;
-  h->window_smem = win_smem;
   h->window_ok = (int)h->work.size() <= win_wave;
+  h->window_wide = false;
+  h->window_threads = threads;
+  // Few enough items for two CTAs of 512 threads per SM (and no CTA shape asked for): the window
+  // kernel takes a warp per chunk of a subunit's work (rows, quads, edges and four beads' lists
+  // each), so that a crowded subunit, which all others wait for, is done sooner:
+  // 64 subunits 1,765 -> 1,645 us per 100 steps, 20 small ones 1,310 -> 1,240 (no spilled registers).
+  if (h->window_ok && !h->opt.threads_per_cta) {
+    const int np = h->tpl.np;
+    int ns = 1;
+    for (const WorkItem& w : h->work) ns = std::max(ns, w.nsub);
+    const int chunks = (ns * np + 31) / 32 + (ns * h->L.nbend + 31) / 32 + (ns * h->L.ne + 31) / 32 + (ns * np + 3) / 4;
+    const int wide = std::min(512, std::max(128, 32 * chunks));
+    const size_t bytes = window_smem_bytes(force_smem_for(h, subs, wide), subs, np);
+    int wide_wave = 0;
+    if (bytes <= 227 * 1024) CUDA_TRY(window_wave_ctas(true, wide, bytes, &wide_wave));
+    if ((int)h->work.size() <= wide_wave) {
+      h->window_wide = true;
+      h->window_threads = wide;
+      win_smem = bytes;
+    }
+  }
+  h->window_smem = win_smem;
   if (h->window_ok && h->win_count.n == 0) {
     CUDA_TRY(h->win_count.alloc(3));
     CUDA_TRY(h->win_acc.alloc(24 * (size_t)h->n_sys));

@@ -54,6 +54,8 @@ struct souffle_gpu_system {
   std::vector<int2> slots;
   // window kernel: usable with this plan (every work item resident at once), its shared memory
   bool window_ok = false;
+  bool window_wide = false;
+  int window_threads = 256;
   size_t window_smem = 0;
   DevBuf<unsigned int> win_count;
   DevBuf<long long> win_acc;
