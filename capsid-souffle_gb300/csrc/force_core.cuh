@@ -3,7 +3,7 @@
 //
 //   force_setup      template tables and per-item constants into shared memory
 //   force_rel        a bead's packed coordinates relative to its subunit's centre bead
-//   force_rows       the beads that have inter-subunit pairs, those with long lists apart
+//   force_rows       the inter-subunit lists cut into pieces of like length
 //   force_terms      everything that depends on positions alone, in chunks of 32 lanes that the
 //                    warps take from a counter: intra-subunit Debye-Hueckel rows, bending quads,
 //                    inter-subunit pairs, edges (the costliest chunks first)
@@ -87,6 +87,25 @@ __device__ __forceinline__ long long limbs_value(const unsigned int* L) {
   return (long long)(hi + ((unsigned long long)L[1] << 21) + (unsigned long long)L[0]);
 }
 
+// f32_to_fx32 of two values at once, |v| < 2^22, for sums: the floor by an addition that rounds down at
+// 2^23 + 2^22, whose bits are that constant's plus the floor.  Those bits are added as they are: sum -=
+// fx_bias(n) after n values.
+__device__ __forceinline__ void fx_add2(unsigned long long& sum, f32x2 v) {
+  f32x2 t;
+  const f32x2 magic = pack2(12582912.0f, 12582912.0f);
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(t) : "l"(v), "l"(magic));
+  const f32x2 hi = add2(t, pack2(-12582912.0f, -12582912.0f));
+  float ha, hb;
+  unpack2(hi, ha, hb);
+  const f32x2 frac = mul2(add2(v, pack2(-ha, -hb)), pack2(4294967296.0f, 4294967296.0f));
+  float fa, fb, ta, tb;
+  unpack2(frac, fa, fb);
+  unpack2(t, ta, tb);
+  sum += (unsigned long long)__float_as_uint(ta) << 32 | __float2uint_rn(fa);
+  sum += (unsigned long long)__float_as_uint(tb) << 32 | __float2uint_rn(fb);
+}
+__device__ __forceinline__ unsigned long long fx_bias(int n) { return (unsigned long long)(0x4B400000u * (unsigned int)n) << 32; }
+
 // true for a non-finite component or one beyond 1e9 in magnitude
 __device__ __forceinline__ bool force_bad(float x, float y, float z) {
   const float s = fabsf(x) + fabsf(y) + fabsf(z);  // NaN or infinite when a component is
@@ -102,7 +121,7 @@ struct ForceSmem {
   float* rel;          // [max_sub npp 8] packed partners: (x0, x1, y0, y1, z0, z1, w0, w1) per two beads
   long long* red;      // [4 warps]
   unsigned int* F;     // force limbs, 9 per bead
-  int* rows;           // beads with inter-subunit pairs: bead | list length << 16, long lists from the front, others from the back
+  int* rows;           // pieces of the beads' inter-subunit lists (force_rows)
   float* tpl_f;
   int* tpl_i;
   float* w;            // [np] DH weights
@@ -124,8 +143,8 @@ __device__ __forceinline__ ForceSmem force_smem(unsigned char* base, const Force
   return m;
 }
 
-// Template tables and the system's DH weights.
-__device__ __forceinline__ void force_setup(const ForceArgs& a, const WorkItem& w, const ForceSmem& m) {
+// Template tables.
+__device__ __forceinline__ void force_setup(const ForceArgs& a, const ForceSmem& m) {
   const TplLayout& L = a.L;
   const int4* gi = reinterpret_cast<const int4*>(a.tpl_i);
   int4* si = reinterpret_cast<int4*>(m.tpl_i);
@@ -133,7 +152,6 @@ __device__ __forceinline__ void force_setup(const ForceArgs& a, const WorkItem& 
   const float4* gf = reinterpret_cast<const float4*>(a.tpl_f);
   float4* sf = reinterpret_cast<float4*>(m.tpl_f);
   for (int t = threadIdx.x; t < (L.n_float >> 2); t += blockDim.x) sf[t] = __ldg(gf + t);
-  for (int t = threadIdx.x; t < L.np; t += blockDim.x) m.w[t] = __ldg(&a.dh_w[w.sys * L.np + t]);
 }
 
 // The packed relative coordinates of bead t (subunit s, local index l) at high words p, centre
@@ -154,31 +172,42 @@ __device__ __forceinline__ void force_rel(const ForceSmem& m, int np, int s, int
   }
 }
 
-// What the warps of a CTA share: the position of the chunk queue and the numbers of long and short
-// inter-subunit rows.  Zero before force_rows.
+// What the warps of a CTA share: the position of the chunk queue and the numbers of pieces of the
+// inter-subunit lists.  Zero before force_rows.
 struct ForceQueue {
-  int next, n_long, n_short;
+  int next, n_long, n_full, n_short;
 };
-constexpr int kLongRow = 48;  // rows above this length take a whole warp (see force_inter)
+constexpr int kPiece = 16;    // pairs of a piece
+constexpr int kLongRow = 48;  // lists above this length are one piece, for a whole warp
 
-// The beads with inter-subunit pairs into m.rows (their order does not matter: every sum is exact).
-// The caller's next barrier makes them visible.
-__device__ __forceinline__ void force_rows(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead, ForceQueue* q) {
+// The beads' inter-subunit lists in pieces into m.rows: whole lists above kLongRow pairs (at 0 ..),
+// pieces of 9 to 16 pairs (at nbead ..) and of at most 8 (from 4 nbead down), each as
+// bead | first pair / kPiece << 16 | pairs << 18.  Lists differ in length from bead to bead, and lanes
+// that share a chunk wait for its longest piece.  (Order does not matter: every sum is exact.)  The
+// caller's next barrier makes them visible.  thread: this thread's place among the CTA's.
+__device__ __forceinline__ void force_rows(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead, int thread, ForceQueue* q) {
   const int lane = threadIdx.x & 31;
-  for (int base = (int)threadIdx.x - lane; base < nbead; base += blockDim.x) {
+  const unsigned int below = (1u << lane) - 1u;
+  for (int base = thread - lane; base < nbead; base += blockDim.x) {
     const int t = base + lane;
     const int n = t < nbead ? __ldg(a.inter_count + bead0 + t) : 0;
-    const unsigned int lg = __ballot_sync(0xffffffffu, n > kLongRow), sh = __ballot_sync(0xffffffffu, n > 0) & ~lg;
-    int l0 = 0, s0 = 0;
-    if (lane == 0) {
-      if (lg) l0 = atomicAdd(&q->n_long, __popc(lg));
-      if (sh) s0 = atomicAdd(&q->n_short, __popc(sh));
-    }
-    l0 = __shfl_sync(0xffffffffu, l0, 0);
-    s0 = __shfl_sync(0xffffffffu, s0, 0);
-    const unsigned int below = (1u << lane) - 1u;
-    if (n > kLongRow) m.rows[l0 + __popc(lg & below)] = t | n << 16;
-    else if (n > 0) m.rows[nbead - 1 - (s0 + __popc(sh & below))] = t | n << 16;
+    if (!__any_sync(0xffffffffu, n > 0)) continue;
+    const int cut = n <= kLongRow ? n : 0, rest = cut & (kPiece - 1);
+    const int full = (cut + 7) / kPiece;  // pieces of 9 to 16 pairs
+    const bool sh = rest > 0 && rest <= 8;
+    const unsigned int lg = __ballot_sync(0xffffffffu, n > kLongRow), sb = __ballot_sync(0xffffffffu, sh);
+    const unsigned int f1 = __ballot_sync(0xffffffffu, full > 0), f2 = __ballot_sync(0xffffffffu, full > 1),
+                       f3 = __ballot_sync(0xffffffffu, full > 2);
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&q->n_long, __popc(lg));
+    if (lane == 1) at = atomicAdd(&q->n_full, __popc(f1) + __popc(f2) + __popc(f3));
+    if (lane == 2) at = atomicAdd(&q->n_short, __popc(sb));
+    const int l0 = __shfl_sync(0xffffffffu, at, 0) + __popc(lg & below);
+    const int s0 = __shfl_sync(0xffffffffu, at, 2) + __popc(sb & below);
+    const int f0 = __shfl_sync(0xffffffffu, at, 1) + __popc(f1 & below) + __popc(f2 & below) + __popc(f3 & below);
+    if (n > kLongRow) m.rows[l0] = t | n << 18;
+    for (int k = 0; k < full; k++) m.rows[nbead + f0 + k] = t | k << 16 | min(kPiece, cut - k * kPiece) << 18;
+    if (sh) m.rows[4 * nbead - 1 - s0] = t | full << 16 | rest << 18;
   }
 }
 
@@ -336,16 +365,18 @@ __device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams&
   limbs_add(m.F + 9 * t + 6, f32_to_fx32(-ze) + f32_to_fx32(-zo));
 }
 
-// The sums of eight lanes' (or, whole, the warp's) force vectors added to a bead's limbs: the nine
-// limbs are halved among the lanes while they are summed, ten exchanges and two atomics of distinct
-// addresses; nine atomics of eight lanes on one address each cost 72 shared-memory cycles.
+// The sums of kLanes (4 or 8) lanes' force vectors, or (whole) the warp's, added to a bead's limbs: the
+// nine limbs are halved among the lanes while they are summed, ten exchanges (8 lanes) and two
+// atomics of distinct addresses; nine atomics of eight lanes on one address each cost 72
+// shared-memory cycles.
+template <int kLanes>
 __device__ __forceinline__ void limbs_add_lanes(unsigned int* F, long long x, long long y, long long z, bool valid, bool whole) {
   const int lane = threadIdx.x & 31;
   const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
   const unsigned int v[9] = {(unsigned int)(x & 0x1FFFFF), (unsigned int)((x >> 21) & 0x1FFFFF), (unsigned int)(int)(x >> 42),
                              (unsigned int)(y & 0x1FFFFF), (unsigned int)((y >> 21) & 0x1FFFFF), (unsigned int)(int)(y >> 42),
                              (unsigned int)(z & 0x1FFFFF), (unsigned int)((z >> 21) & 0x1FFFFF), (unsigned int)(int)(z >> 42)};
-  unsigned int w[5], u[3], t[2];
+  unsigned int w[5], u[3];
 #pragma unroll
   for (int k = 0; k < 5; k++) {  // limbs 0-4 to the even lanes, 5-8 to the odd
     const unsigned int lo = v[k], hi = k < 4 ? v[5 + k] : 0u;
@@ -356,24 +387,27 @@ __device__ __forceinline__ void limbs_add_lanes(unsigned int* F, long long x, lo
     const unsigned int lo = w[k], hi = k < 2 ? w[3 + k] : 0u;
     u[k] = (b1 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 2);
   }
+  F += (b0 ? 5 : 0) + (b1 ? 3 : 0);
+  int n = b1 ? (b0 ? 1 : 2) : 3;  // how many of the values are limbs
+  if (kLanes == 8) {
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const unsigned int lo = u[k], hi = k < 1 ? u[2] : 0u;
-    t[k] = (b2 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 4);
+    for (int k = 0; k < 2; k++) {
+      const unsigned int lo = u[k], hi = k < 1 ? u[2] : 0u;
+      u[k] = (b2 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 4);
+    }
+    F += b2 ? 2 : 0;
+    n = b2 ? max(0, n - 2) : min(n, 2);
   }
   if (whole) {
 #pragma unroll
-    for (int o = 8; o <= 16; o <<= 1) {
-      t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
-      t[1] += __shfl_xor_sync(0xffffffffu, t[1], o);
-    }
-    valid = valid && lane < 8;
+    for (int o = kLanes; o <= 16; o <<= 1)
+#pragma unroll
+      for (int k = 0; k < (kLanes == 8 ? 2 : 3); k++) u[k] += __shfl_xor_sync(0xffffffffu, u[k], o);
+    valid = valid && lane < kLanes;
   }
-  // a lane's limbs and how many of its two values are one
-  const int first = (b0 ? 5 : 0) + (b1 ? 3 : 0) + (b2 ? 2 : 0);
-  const int n = b1 ? (b2 ? 0 : b0 ? 1 : 2) : (b2 ? 1 : 2);
-  if (valid && n > 0) atomicAdd(F + first, t[0]);
-  if (valid && n > 1) atomicAdd(F + first + 1, t[1]);
+#pragma unroll
+  for (int k = 0; k < (kLanes == 8 ? 2 : 3); k++)
+    if (valid && n > k) atomicAdd(F + k, u[k]);
 }
 
 // LJ or WCA term of a pair (src/forces.cpp:81-138) added to its force coefficient.
@@ -385,33 +419,46 @@ __device__ __forceinline__ float lj_add(float c, float r2, const float* pair, fl
   return c;
 }
 
-// Inter-subunit pairs (DH + LJ/WCA, src/forces.cpp:81-138) of a chunk of rows: four beads by eight
-// lanes each, or one bead with a long list (more than kLongRow pairs) by the whole warp -- at 48
-// pairs both take the same number of rounds per bead.  A lane evaluates two of the row's pairs at a
-// time in packed FP32, adds its pair forces exactly in 2^-32 fixed point in registers, and the
-// lanes' sums go to the bead's limbs at the end (order-independent).  What bounds it is the chain
-// of loads and arithmetic from one pair to the next, and in systems with a few crowded subunits
-// their CTA, which everyone else waits for.  So a row is spread over lanes: neighbouring lanes read
-// neighbouring partners, no lane searches for its bead, and lanes finish a row together.
+// Inter-subunit pairs (DH + LJ/WCA, src/forces.cpp:81-138) of a chunk: 32 / kLanes pieces by kLanes
+// lanes each, or one long list by the whole warp.  A lane evaluates two of its piece's pairs at a time
+// in packed FP32, adds its pair forces exactly in 2^-32 fixed point in registers, and the lanes' sums
+// go to the bead's limbs at the end (order-independent).  In small systems what bounds it is the chain
+// of loads and arithmetic from one pair to the next, and of a few crowded subunits' CTAs, which
+// everyone else waits for; in large ones the instructions.  So a list is spread over lanes:
+// neighbouring lanes read neighbouring partners, no lane searches for its bead, and lanes finish
+// together.  Eight lanes take a piece in one round (the chain); four in two, with half the work of
+// adding up (the instructions): the run form of the force kernel.
 // Against runs of eight consecutive pairs of the flat pair sequence per thread: 2,000 subunits, a
-// tenth of them in contact, 3,900 -> 3,430 us per 100 steps; 64: 1,870 -> 1,765; 64 dense replicas 1.5 %.
+// tenth of them in contact, 3,900 -> 3,450 us per 100 steps; 64: 1,870 -> 1,490; a force evaluation of
+// 64 dense replicas (17,286 subunits) 222 -> 203 us.
 // kFresh: the partners' positions are rewritten by other CTAs while this kernel runs (read past L1).
-// kAhead: also the next two pairs' positions are fetched ahead, not their indices alone; worth the
-// registers where few warps share an SM (64 subunits: 1765 against 1846 us per 100 steps), not
-// where five CTAs do (2,000 subunits: 3543 against 3431).
-template <bool kFresh, bool kAhead>
+template <bool kFresh, int kLanes>
 __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
                                             const ForceQueue& q, int chunk) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
   const int* species = m.tpl_i + L.o_species;
   const float unit = P.unit32, ecut_el2 = P.ecut_el2;
+  constexpr int kRows = 32 / kLanes;
   const bool whole = chunk < q.n_long;
-  const int lanes = whole ? 32 : 8;
-  const int row = whole ? chunk : 4 * (chunk - q.n_long) + (lane >> 3);
-  const int rec = whole || row < q.n_short ? m.rows[whole ? row : nbead - 1 - row] : 0;
-  const int b = rec & 0xffff, n = rec >> 16;
-  const int* ids = a.inter_ids + (long long)(bead0 + b) * a.inter_cap;
+  const int lanes = whole ? 32 : kLanes;
+  int at = chunk;  // the piece's place in m.rows
+  bool valid = true;
+  if (!whole) {
+    const int kf = (q.n_full + kRows - 1) / kRows, c = chunk - q.n_long;
+    if (c < kf) {
+      const int k = kRows * c + lane / kLanes;
+      valid = k < q.n_full;
+      at = nbead + k;
+    } else {
+      const int k = kRows * (c - kf) + lane / kLanes;
+      valid = k < q.n_short;
+      at = 4 * nbead - 1 - k;
+    }
+  }
+  const int rec = valid ? m.rows[at] : 0;
+  const int b = rec & 0xffff, n = rec >> 18;
+  const int* ids = a.inter_ids + (long long)(bead0 + b) * a.inter_cap + ((rec >> 16) & 3) * kPiece;
   const int4 pi = m.pos[b];
   const int l = b - fast_div(b, a.div_np) * L.np;
   const int si = species[l] * L.nspecies;
@@ -423,16 +470,14 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
   auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
   int i = lane & (lanes - 1);
   int j0 = partner(i), j1 = partner(i + lanes);
-  int4 n0, n1;
-  if (kAhead) n0 = position(j0), n1 = position(j1);
-  long long ax = 0, ay = 0, az = 0;
+  unsigned long long ax = 0, ay = 0, az = 0;
+  int added = 0;  // values added by fx_add2
   while (i < n) {
-    const int4 p0 = kAhead ? n0 : position(j0), p1 = kAhead ? n1 : position(j1);
+    const int4 p0 = position(j0), p1 = position(j1);
     const bool two = i + lanes < n;
     i += 2 * lanes;
-    j0 = partner(i);  // the next two pairs, while these are evaluated
+    j0 = partner(i);  // the next two pairs' partners, while these are evaluated
     j1 = partner(i + lanes);
-    if (kAhead) n0 = position(j0), n1 = position(j1);
     const f32x2 u2 = pack2(unit, unit);
     const f32x2 dx = mul2(pack2((float)(int)((unsigned)pi.x - (unsigned)p0.x), (float)(int)((unsigned)pi.x - (unsigned)p1.x)), u2);
     const f32x2 dy = mul2(pack2((float)(int)((unsigned)pi.y - (unsigned)p0.y), (float)(int)((unsigned)pi.y - (unsigned)p1.y)), u2);
@@ -459,39 +504,50 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
       cb = lb ? tb : cb;
     }
     const f32x2 c2 = pack2(ca, cb);
+    const f32x2 fx = mul2(dx, c2), fy = mul2(dy, c2), fz = mul2(dz, c2);
     float xa, xb, ya, yb, za, zb;
-    unpack2(mul2(dx, c2), xa, xb);
-    unpack2(mul2(dy, c2), ya, yb);
-    unpack2(mul2(dz, c2), za, zb);
-    // (a sum below the bound of one component: every component is good)
-    if (!(fabsf(xa) + fabsf(ya) + fabsf(za) + fabsf(xb) + fabsf(yb) + fabsf(zb) < 1.0e9f)) {
+    unpack2(fx, xa, xb);
+    unpack2(fy, ya, yb);
+    unpack2(fz, za, zb);
+    // (a sum below a bound of one component: every component is)
+    if (fabsf(xa) + fabsf(ya) + fabsf(za) + fabsf(xb) + fabsf(yb) + fabsf(zb) < 4.0e6f) {
+      fx_add2(ax, fx);
+      fx_add2(ay, fy);
+      fx_add2(az, fz);
+      added += 2;
+    } else {  // large or not finite
       const bool bad_a = force_bad(xa, ya, za), bad_b = force_bad(xb, yb, zb);
       if (bad_a || bad_b) atomicOr(a.err, kErrNonFinite);
       if (bad_a) xa = ya = za = 0.f;
       if (bad_b) xb = yb = zb = 0.f;
+      ax += (unsigned long long)(f32_to_fx32(xa) + f32_to_fx32(xb));
+      ay += (unsigned long long)(f32_to_fx32(ya) + f32_to_fx32(yb));
+      az += (unsigned long long)(f32_to_fx32(za) + f32_to_fx32(zb));
     }
-    ax += f32_to_fx32(xa) + f32_to_fx32(xb);
-    ay += f32_to_fx32(ya) + f32_to_fx32(yb);
-    az += f32_to_fx32(za) + f32_to_fx32(zb);
   }
+  const unsigned long long bias = fx_bias(added);
+  ax -= bias;
+  ay -= bias;
+  az -= bias;
   __syncwarp();
-  limbs_add_lanes(m.F + 9 * b, ax, ay, az, n > 0, whole);
+  limbs_add_lanes<kLanes>(m.F + 9 * b, (long long)ax, (long long)ay, (long long)az, n > 0, whole);
 }
 
 // Everything that depends on positions alone, in chunks that the warps take from the queue: long
-// inter-subunit rows, the intra-subunit rows of 32 beads (700 instructions), 32 bending quads (450),
-// four short inter-subunit rows, 32 edges (100).  kFresh (the window kernel): the inter-subunit
+// inter-subunit lists, the intra-subunit rows of 32 beads (900 instructions), 32 bending quads (400),
+// pieces of inter-subunit lists, 64 edges (100).  kFresh (the window kernel): the inter-subunit
 // pairs come last, and a warp's first one only after wait() -- by then the other CTAs have
 // published their new positions while this one worked on its own subunits.
-template <bool kFresh, bool kAhead, class Wait>
+template <bool kFresh, int kLanes, class Wait>
 __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
                                             int nbead, int bead0, ForceQueue* q, Wait wait) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
   const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne;
-  const int ki = (nbead + 31) >> 5, kq = (nq + 31) >> 5, ke = (ne + 31) >> 5;
-  const ForceQueue rows{0, q->n_long, q->n_short};
-  const int kl = rows.n_long, ks = (rows.n_short + 3) >> 2;
+  const int ki = (nbead + 31) >> 5, kq = (nq + 31) >> 5, ke = (ne + 63) >> 6;
+  const ForceQueue rows{0, q->n_long, q->n_full, q->n_short};
+  constexpr int kRows = 32 / kLanes;
+  const int kl = rows.n_long, ks = (rows.n_full + kRows - 1) / kRows + (rows.n_short + kRows - 1) / kRows;
   // the order of the kinds of chunk
   const int first_intra = kFresh ? 0 : kl, first_quad = first_intra + ki;
   const int first_edge = first_quad + kq + (kFresh ? 0 : ks);
@@ -509,15 +565,16 @@ __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams&
       const int t = 32 * (k - first_quad) + lane;
       if (t < nq) force_quad(a, P, m, t);
     } else if (k >= first_edge && k < first_edge + ke) {
-      const int t = 32 * (k - first_edge) + lane;
+      const int t = 64 * (k - first_edge) + lane;
       if (t < ne) force_edge(a, P, m, t);
+      if (t + 32 < ne) force_edge(a, P, m, t + 32);
     } else {
       if (kFresh && !waited) {
         wait();
         waited = true;
       }
-      // the long rows are the first kl of these chunks
-      force_inter<kFresh, kAhead>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq);
+      // the long lists are the first kl of these chunks
+      force_inter<kFresh, kLanes>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq);
     }
     __syncwarp();
   }

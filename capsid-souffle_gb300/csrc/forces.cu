@@ -100,6 +100,20 @@ __device__ __noinline__ void bigbead_mask(const ForceArgs& a, const SysParams& P
   }
 }
 
+// Four int64 sums over the warp: halved among the lanes while they are added (12 exchanges instead
+// of 40).  Lane l < 4 returns the total of value warp_sum4_index(l).
+__device__ __forceinline__ int warp_sum4_index(int lane) { return 2 * (lane & 1) + ((lane >> 1) & 1); }
+__device__ __forceinline__ long long warp_sum4_ll(long long v0, long long v1, long long v2, long long v3) {
+  const int lane = threadIdx.x & 31;
+  const bool b0 = lane & 1, b1 = lane & 2;
+  const long long k0 = (b0 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, b0 ? v0 : v2, 1);
+  const long long k1 = (b0 ? v3 : v1) + __shfl_xor_sync(0xffffffffu, b0 ? v1 : v3, 1);
+  long long x = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
 // The end of a step (mode 1) or of the initial forces (mode 2) for one system, from its kinetic
 // energy and momentum sums (2^-32 and 2^-40 units) into its state S in shared memory: warp 0 runs
 // the thermostat chain, warp 1 the centre-of-mass velocity.  The caller's barrier ends it.
@@ -152,170 +166,206 @@ __device__ __forceinline__ void step_tail(const ForceArgs& a, const SysParams& P
   }
 }
 
-// 5 CTAs of 256 threads per SM (<= 51 registers) so 3-subunit work items fit one wave of
-// 152 x 5 CTAs at the 2000-subunit workload.
-// kChain64: the tail runs the FP64 validation chain (souffle_options.chain_fp64) instead of the
-// double-float one; a separate instantiation, so that the default kernel's code is untouched.
+// The end of a step of one system by a whole CTA: the system's sums (cleared for the next launch)
+// and state come into shared memory in one round of loads, step_tail, the state goes back, and the
+// per-bead kick coefficients c0 / m follow, one template bead per thread.  smem: the state and the
+// chain's scratch.
 template <bool kChain64>
-__global__ void __launch_bounds__(256, 5) k_forces(ForceArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const TplLayout& L = a.L;
-  const WorkItem w = a.work[blockIdx.x];
-  const SysParams& P = a.sys[w.sys];
-  const int np = L.np;
-  const int nbead = w.nsub * np;
-  const int bead0 = w.sub_begin * np;  // global index of the first bead
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // (the tail of the system's last CTA reuses the first region for the system state)
-  const ForceSmem m = force_smem(smem, a, nw);
-  int4* s_pos = m.pos;
-  long long* s_red = m.red;
-  unsigned int* s_F = m.F;
-  const float* tpl_f = m.tpl_f;
-  const float* s_w = m.w;
-  const float unit = P.unit32;
-  __shared__ ForceQueue s_queue;
-  if (threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0};
-  __syncthreads();
-  force_rows(a, m, bead0, nbead, &s_queue);
-  force_setup(a, w, m);
-  for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-    const int4 p = a.pos32[bead0 + t];
-    const int s = fast_div(t, a.div_np), l = t - s * np;
-    const int4 c = __ldg(&a.pos32[bead0 + s * np + P.center_local]);
-    s_pos[t] = p;
-    force_rel(m, np, s, l, p, c, __ldg(&a.dh_w[w.sys * np + l]), unit);
-  }
-  for (int t = threadIdx.x; t < 9 * nbead; t += blockDim.x) s_F[t] = 0u;  // the beads' force limbs
-  // big beads within reach of each of the CTA's subunits (s_bbm), flagged before phase 3
-  __shared__ unsigned int s_bbm[16 * kBBWords];
-  const bool bb_filter = P.nbb > 0 && P.nbb <= 32 * kBBWords && w.nsub <= 16;
-  if (threadIdx.x < 16 * kBBWords) s_bbm[threadIdx.x] = 0u;
-  __syncthreads();
-  force_terms<false, false>(a, P, m, w, nbead, bead0, &s_queue, [] {});
-  __syncthreads();
-  const float* s_mass = tpl_f + L.o_mass;
-  const SysState& st = a.state[w.sys];
-  const long long delta_fx = st.delta_fx;
-  const long long* kick_c = a.kick_c + (size_t)w.sys * np;
-  long long ke_acc = 0, px_acc = 0, py_acc = 0, pz_acc = 0;
-  const bool bd = P.brownian && a.mode == 1;  // Brownian MD step
-  force_gather(a, m, nbead, bead0);
-  if (bb_filter) bigbead_mask(a, P, s_pos, m.rel, w.nsub, np, unit, s_bbm);
-  __syncthreads();
-
-  // Phase 3: the bead's total force, the second half kick and the kinetic-energy and momentum
-  // sums, one thread per bead
-  for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-    const int sub = fast_div(t, a.div_np), l = t - sub * np, g = bead0 + t;
-    long long Fx = limbs_value(s_F + 9 * t), Fy = limbs_value(s_F + 9 * t + 3), Fz = limbs_value(s_F + 9 * t + 6);
-    if (P.nbb) {
-      const float3 fb = bigbead_force(a, P, s_pos[t], s_w[l], tpl_f[L.o_sigma + l], unit,
-                                      bb_filter ? s_bbm + sub * kBBWords : nullptr);
-      if (!(isfinite(fb.x) && isfinite(fb.y) && isfinite(fb.z)) ||
-          fmaxf(fmaxf(fabsf(fb.x), fabsf(fb.y)), fabsf(fb.z)) > 1.0e9f)
-        atomicOr(a.err, kErrNonFinite);
-      Fx += f32_to_fx32(fb.x);
-      Fy += f32_to_fx32(fb.y);
-      Fz += f32_to_fx32(fb.z);
-    }
-    if (bd) {
-      // Brownian: tforce + (fran - mean fran over the system) + fdrag (src/md.cpp:468-494,
-      // src/bead.h:147-149)
-      const long long N = a.n_beads_total;
-      Fx += a.fran[g] - __double2ll_rn((double)st.fran_sum[0] * st.inv_n) + a.fdrag[g];
-      Fy += a.fran[N + g] - __double2ll_rn((double)st.fran_sum[1] * st.inv_n) + a.fdrag[N + g];
-      Fz += a.fran[2 * N + g] - __double2ll_rn((double)st.fran_sum[2] * st.inv_n) + a.fdrag[2 * N + g];
-    }
-    a.fx[g] = Fx;
-    a.fy[g] = Fy;
-    a.fz[g] = Fz;
-    if (a.mode == 1 || a.mode == 2) {
-      long long vx = a.vx[g], vy = a.vy[g], vz = a.vz[g];
-      if (a.mode == 1) {  // v <- v exp(-dt xi/2) + F dt sqrt(expfac)/(2m)  (src/bead.h:113-117)
-        const long long c = kick_c[l];
-        vx = vx - mul_shr(vx, delta_fx, 62) + mul_shr(Fx, c, 56);
-        vy = vy - mul_shr(vy, delta_fx, 62) + mul_shr(Fy, c, 56);
-        vz = vz - mul_shr(vz, delta_fx, 62) + mul_shr(Fz, c, 56);
-        a.vx[g] = vx;
-        a.vy[g] = vy;
-        a.vz[g] = vz;
-        px_acc += vx;
-        py_acc += vy;
-        pz_acc += vz;
-      }
-      const float ux = vel_to_f32(vx), uy = vel_to_f32(vy), uz = vel_to_f32(vz);
-      const float v2 = ux * ux + uy * uy + uz * uz;
-      if (!(v2 < 1.0e12f)) atomicOr(a.err, kErrNonFinite);  // |v| beyond 1e6: a blown-up run
-      ke_acc += f32_to_fx32(0.5f * s_mass[l] * v2);
-    }
-  }
-  if (a.mode == 0) return;
-
-  // exact CTA reduction in int64
-  ke_acc = warp_sum_ll(ke_acc);
-  px_acc = warp_sum_ll(px_acc);
-  py_acc = warp_sum_ll(py_acc);
-  pz_acc = warp_sum_ll(pz_acc);
-  if (lane == 0) {
-    s_red[wid * 4 + 0] = ke_acc;
-    s_red[wid * 4 + 1] = px_acc;
-    s_red[wid * 4 + 2] = py_acc;
-    s_red[wid * 4 + 3] = pz_acc;
-  }
-  __syncthreads();
-  __shared__ bool last;
-  // the system's running sums (kinetic energy, momentum) for this launch: exact int64 adds,
-  // order-independent; the last CTA reads them and clears them for the next launch
-  unsigned long long* acc = reinterpret_cast<unsigned long long*>(a.partial) + 4 * (size_t)w.sys;
-  if (threadIdx.x == 0) {
-    long long k = 0, x = 0, y = 0, z = 0;
-    for (int q = 0; q < nw; q++) {
-      k += s_red[q * 4];
-      x += s_red[q * 4 + 1];
-      y += s_red[q * 4 + 2];
-      z += s_red[q * 4 + 3];
-    }
-    atomicAdd(acc + 0, (unsigned long long)k);
-    atomicAdd(acc + 1, (unsigned long long)x);
-    atomicAdd(acc + 2, (unsigned long long)y);
-    atomicAdd(acc + 3, (unsigned long long)z);
-    __threadfence();
-    const int2 sl = a.sys_slots[w.sys];
-    unsigned int prev = atomicAdd(&a.state[w.sys].done, 1u);
-    last = (prev == (unsigned int)sl.y - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-
-  // Last CTA of this system: the running sums and the system's state come into shared memory
-  // (the tile area, free by now) in one round of loads; then warp 0 runs the thermostat chain
-  // and warp 1 the centre-of-mass velocity.
-  __threadfence();
+__device__ __forceinline__ void step_end(const ForceArgs& a, int sys, unsigned char* smem, long long* s_sum) {
+  const int np = a.L.np;
+  unsigned long long* acc = reinterpret_cast<unsigned long long*>(a.partial) + 4 * (size_t)sys;
   static_assert(sizeof(SysState) % 16 == 0, "SysState is copied as int4");
   constexpr int kStateVecs = (int)(sizeof(SysState) / 16);
   SysState& S = *reinterpret_cast<SysState*>(smem);
   dfloat* chain_scratch = reinterpret_cast<dfloat*>(smem + sizeof(SysState));  // 3 kMaxChain
-  const int4* st_src = reinterpret_cast<const int4*>(a.state + w.sys);
+  const int4* st_src = reinterpret_cast<const int4*>(a.state + sys);
   int4* st_dst = reinterpret_cast<int4*>(&S);
-  long long sum = 0;
   if (threadIdx.x < 4) {
-    sum = (long long)__ldcg(acc + threadIdx.x);  // L2 (coherent), not L1
+    s_sum[threadIdx.x] = (long long)__ldcg(acc + threadIdx.x);  // L2 (coherent), not L1
     acc[threadIdx.x] = 0;
   }
   for (int q = threadIdx.x; q < kStateVecs; q += blockDim.x) st_dst[q] = __ldcg(st_src + q);
-  if (threadIdx.x < 4) s_red[threadIdx.x] = sum;
   __syncthreads();
-  step_tail<kChain64>(a, P, w.sys, S, s_red, chain_scratch);
+  step_tail<kChain64>(a, a.sys[sys], sys, S, s_sum, chain_scratch);
   __syncthreads();
-  for (int q = threadIdx.x; q < kStateVecs; q += blockDim.x) reinterpret_cast<int4*>(a.state + w.sys)[q] = st_dst[q];
-  // per-bead kick coefficients c0 / m, one template bead per thread
-  long long* kc = a.kick_c + (size_t)w.sys * np;
+  for (int q = threadIdx.x; q < kStateVecs; q += blockDim.x) reinterpret_cast<int4*>(a.state + sys)[q] = st_dst[q];
+  long long* kc = a.kick_c + (size_t)sys * np;
   for (int l = threadIdx.x; l < np; l += blockDim.x) {
     long long c = 0;
     if (!nhc_kick_coefficient(S.kick_c0, a.inv_mass[l], c)) atomicOr(a.err, kErrNonFinite);
     kc[l] = c;
   }
+}
+
+// One system per CTA, after a force kernel whose CTAs took several work items.
+template <bool kChain64>
+__global__ void __launch_bounds__(64) k_step_end(ForceArgs a) {
+  __shared__ __align__(16) unsigned char smem[sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat)];
+  __shared__ long long s_sum[4];
+  step_end<kChain64>(a, blockIdx.x, smem, s_sum);
+}
+
+// One item per CTA (kRun false), 5 CTAs of 256 threads per SM (<= 51 registers) so that 3-subunit
+// work items fit one wave of 152 x 5 CTAs at the 2000-subunit workload.  Items beyond one wave
+// (kRun): a wave of CTAs that draw items from a counter, 4 per SM with 64 registers.  The tables are
+// then loaded once, the upper warps fetch the next item while the lower ones finish the beads of
+// one, an item has three barriers instead of six, and the sums leave the CTA once per run of items of
+// one system, not with each item and a fence and a ticket behind them; k_step_end ends the step.
+// Those serial stretches were a third of the time: 840,000 beads 160 -> 141 us.
+// kChain64: the tail runs the FP64 validation chain (souffle_options.chain_fp64) instead of the
+// double-float one; a separate instantiation, so that the default kernel's code is untouched.
+template <bool kChain64, bool kRun>
+__global__ void __launch_bounds__(256, kRun ? 4 : 5) k_forces(ForceArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const TplLayout& L = a.L;
+  const int np = L.np;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // a thread's place when an item's beads are fetched: with kRun the upper half of the warps first
+  const int fetch = kRun ? 32 * (wid >= (nw >> 1) ? wid - (nw >> 1) : wid + nw - (nw >> 1)) + lane : threadIdx.x;
+  // (the tail of a system's last CTA reuses the first region for the system state)
+  const ForceSmem m = force_smem(smem, a, nw);
+  const float* s_mass = m.tpl_f + L.o_mass;
+  __shared__ ForceQueue s_queue;
+  __shared__ WorkItem s_work;                       // the item in work, then the next one
+  __shared__ int s_next;
+  __shared__ long long s_sum[4];                    // kinetic energy and momentum of this CTA's beads
+  __shared__ unsigned int s_bbm[16 * kBBWords];     // big beads within reach of each of the item's subunits
+  if (threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0, 0};
+  if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
+  force_setup(a, m);
+  for (int t = threadIdx.x; t < 9 * a.max_sub * np; t += blockDim.x) m.F[t] = 0u;  // the beads' force limbs
+  int sys = -1;
+  auto flush = [&]() {  // this CTA's sums of system `sys`: exact int64 adds, order-independent
+    unsigned long long* acc = reinterpret_cast<unsigned long long*>(a.partial) + 4 * (size_t)sys;
+    if (threadIdx.x < 4) {
+      atomicAdd(acc + threadIdx.x, (unsigned long long)s_sum[threadIdx.x]);
+      s_sum[threadIdx.x] = 0;
+    }
+  };
+  if (threadIdx.x == 0) s_work = a.work[blockIdx.x];
+  __syncthreads();
+  for (;;) {
+    const WorkItem w = s_work;
+    const SysParams& P = a.sys[w.sys];
+    const int nbead = w.nsub * np;
+    const int bead0 = w.sub_begin * np;  // global index of the first bead
+    const float unit = P.unit32;
+    force_rows(a, m, bead0, nbead, fetch, &s_queue);
+    for (int t = fetch; t < nbead; t += blockDim.x) {
+      const int4 p = a.pos32[bead0 + t];
+      const int s = fast_div(t, a.div_np), l = t - s * np;
+      const int4 c = __ldg(&a.pos32[bead0 + s * np + P.center_local]);
+      m.pos[t] = p;
+      force_rel(m, np, s, l, p, c, __ldg(&a.dh_w[w.sys * np + l]), unit);
+    }
+    if (w.sys != sys)
+      for (int l = fetch; l < np; l += blockDim.x) m.w[l] = __ldg(&a.dh_w[w.sys * np + l]);
+    const bool bb_filter = P.nbb > 0 && P.nbb <= 32 * kBBWords && w.nsub <= 16;
+    if (bb_filter && threadIdx.x < 16 * kBBWords) s_bbm[threadIdx.x] = 0u;
+    __syncthreads();
+    if (w.sys != sys) {
+      if (kRun && sys >= 0 && a.mode != 0) flush();
+      sys = w.sys;
+    }
+    if (kRun && wid == nw - 1 && lane == 0) {  // the next item, while the others begin
+      // (items are drawn in order, every CTA's last draw past the end: the last of all clears the counter)
+      const unsigned int v = atomicAdd(a.ticket, 1u);
+      if (v == (unsigned int)a.n_items - 1) *a.ticket = 0;
+      s_next = (int)(gridDim.x + v);
+      if (s_next < a.n_items) s_work = a.work[s_next];
+    }
+    force_terms<false, kRun ? 4 : 8>(a, P, m, w, nbead, bead0, &s_queue, [] {});
+    __syncthreads();
+    if (kRun && threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0, 0};
+    force_gather(a, m, nbead, bead0);
+    if (bb_filter) bigbead_mask(a, P, m.pos, m.rel, w.nsub, np, unit, s_bbm);
+    __syncthreads();
+
+    // The bead's total force, the second half kick and the kinetic-energy and momentum sums, one
+    // thread per bead; nothing here reads what the next item's fetch writes
+    const SysState& st = a.state[w.sys];
+    const long long delta_fx = st.delta_fx;
+    const long long* kick_c = a.kick_c + (size_t)w.sys * np;
+    long long ke_acc = 0, px_acc = 0, py_acc = 0, pz_acc = 0;
+    const bool bd = P.brownian && a.mode == 1;  // Brownian MD step
+    for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
+      const int sub = fast_div(t, a.div_np), l = t - sub * np, g = bead0 + t;
+      unsigned int* F = m.F + 9 * t;
+      long long Fx = limbs_value(F), Fy = limbs_value(F + 3), Fz = limbs_value(F + 6);
+      if (kRun)
+#pragma unroll
+        for (int k = 0; k < 9; k++) F[k] = 0u;
+      if (P.nbb) {
+        const float3 fb = bigbead_force(a, P, m.pos[t], m.w[l], m.tpl_f[L.o_sigma + l], unit,
+                                        bb_filter ? s_bbm + sub * kBBWords : nullptr);
+        if (!(isfinite(fb.x) && isfinite(fb.y) && isfinite(fb.z)) ||
+            fmaxf(fmaxf(fabsf(fb.x), fabsf(fb.y)), fabsf(fb.z)) > 1.0e9f)
+          atomicOr(a.err, kErrNonFinite);
+        Fx += f32_to_fx32(fb.x);
+        Fy += f32_to_fx32(fb.y);
+        Fz += f32_to_fx32(fb.z);
+      }
+      if (bd) {
+        // Brownian: tforce + (fran - mean fran over the system) + fdrag (src/md.cpp:468-494,
+        // src/bead.h:147-149)
+        const long long N = a.n_beads_total;
+        Fx += a.fran[g] - __double2ll_rn((double)st.fran_sum[0] * st.inv_n) + a.fdrag[g];
+        Fy += a.fran[N + g] - __double2ll_rn((double)st.fran_sum[1] * st.inv_n) + a.fdrag[N + g];
+        Fz += a.fran[2 * N + g] - __double2ll_rn((double)st.fran_sum[2] * st.inv_n) + a.fdrag[2 * N + g];
+      }
+      a.fx[g] = Fx;
+      a.fy[g] = Fy;
+      a.fz[g] = Fz;
+      if (a.mode == 1 || a.mode == 2) {
+        long long vx = a.vx[g], vy = a.vy[g], vz = a.vz[g];
+        if (a.mode == 1) {  // v <- v exp(-dt xi/2) + F dt sqrt(expfac)/(2m)  (src/bead.h:113-117)
+          const long long c = kick_c[l];
+          vx = vx - mul_shr(vx, delta_fx, 62) + mul_shr(Fx, c, 56);
+          vy = vy - mul_shr(vy, delta_fx, 62) + mul_shr(Fy, c, 56);
+          vz = vz - mul_shr(vz, delta_fx, 62) + mul_shr(Fz, c, 56);
+          a.vx[g] = vx;
+          a.vy[g] = vy;
+          a.vz[g] = vz;
+          px_acc += vx;
+          py_acc += vy;
+          pz_acc += vz;
+        }
+        const float ux = vel_to_f32(vx), uy = vel_to_f32(vy), uz = vel_to_f32(vz);
+        const float v2 = ux * ux + uy * uy + uz * uz;
+        if (!(v2 < 1.0e12f)) atomicOr(a.err, kErrNonFinite);  // |v| beyond 1e6: a blown-up run
+        ke_acc += f32_to_fx32(0.5f * s_mass[l] * v2);
+      }
+    }
+    if (a.mode != 0 && wid * 32 < nbead) {
+      const long long x = warp_sum4_ll(ke_acc, px_acc, py_acc, pz_acc);
+      if (lane < 4) atomicAdd(reinterpret_cast<unsigned long long*>(s_sum + warp_sum4_index(lane)), (unsigned long long)x);
+    }
+    if (!kRun) break;
+    if (P.nbb) __syncthreads();  // (the big beads' pass reads the item's positions and weights)
+    if (s_next >= a.n_items) break;
+  }
+  if (a.mode == 0) return;
+  __syncthreads();
+  if (kRun) {  // k_step_end follows
+    flush();
+    return;
+  }
+
+  // one item per CTA: the last CTA of a system ends its step
+  __shared__ bool last;
+  if (wid == 0) {
+    flush();
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) {
+      const unsigned int prev = atomicAdd(&a.state[sys].done, 1u);
+      last = (prev == (unsigned int)a.sys_slots[sys].y - 1);
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  step_end<kChain64>(a, sys, smem, s_sum);
 }
 
 // Half-kick and drift of one bead (src/md.cpp:409-414, src/bead.h:72-81,113-117), with the
@@ -499,14 +549,19 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   const int np = L.np, nbead = w.nsub * np, bead0 = w.sub_begin * np;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const ForceSmem m = force_smem(smem, a, nw);
-  // behind the force kernel's shared memory: positions, velocities, kick coefficients, the state
+  // behind the force kernel's shared memory: velocities, kick coefficients, the state, the low words of
+  // the positions (the high words are the tile's)
   const int nmax = a.max_sub * np;
-  long long* s_x = reinterpret_cast<long long*>(smem + q.force_bytes);  // [3][nmax]
-  long long* s_v = s_x + 3 * nmax;                                      // [3][nmax]
+  long long* s_v = reinterpret_cast<long long*>(smem + q.force_bytes);  // [3][nmax]
   long long* s_kc = s_v + 3 * nmax;                                     // [np]
   dfloat* s_im = reinterpret_cast<dfloat*>(s_kc + ((np + 1) & ~1));     // [np] 1 / m
   SysState& S = *reinterpret_cast<SysState*>(s_im + ((np + 1) & ~1));
   dfloat* chain_scratch = reinterpret_cast<dfloat*>(&S + 1);
+  unsigned int* s_lo = reinterpret_cast<unsigned int*>(chain_scratch + 3 * kMaxChain);  // [3][nmax]
+  // (high words are rounded, so the low ones are signed offsets from them)
+  auto whole = [](int hi, unsigned int lo) {
+    return (long long)(((unsigned long long)(unsigned int)hi << 32) + (unsigned long long)(long long)(int)lo);
+  };
   __shared__ ForceQueue s_queue;
   __shared__ int s_abort;
   __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
@@ -515,11 +570,12 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   const bool bd = P.brownian;
   if (threadIdx.x == 0) {
     s_abort = 0;
-    s_queue = ForceQueue{0, 0, 0};
+    s_queue = ForceQueue{0, 0, 0, 0};
   }
   __syncthreads();
-  force_rows(a, m, bead0, nbead, &s_queue);
-  force_setup(a, w, m);
+  force_rows(a, m, bead0, nbead, threadIdx.x, &s_queue);
+  force_setup(a, m);
+  for (int t = threadIdx.x; t < np; t += blockDim.x) m.w[t] = __ldg(&a.dh_w[w.sys * np + t]);
   {
     const int4* src = reinterpret_cast<const int4*>(a.state + w.sys);
     int4* dst = reinterpret_cast<int4*>(&S);
@@ -539,15 +595,16 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   }
   for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
     const int g = bead0 + t;
-    s_x[t] = d.px[g];
-    s_x[nmax + t] = d.py[g];
-    s_x[2 * nmax + t] = d.pz[g];
+    const long long X = d.px[g], Y = d.py[g], Z = d.pz[g];
+    s_lo[t] = (unsigned int)X;
+    s_lo[nmax + t] = (unsigned int)Y;
+    s_lo[2 * nmax + t] = (unsigned int)Z;
+    m.pos[t] = make_int4(hi_word(X), hi_word(Y), hi_word(Z), t - fast_div(t, a.div_np) * np);
     s_v[t] = a.vx[g];
     s_v[nmax + t] = a.vy[g];
     s_v[2 * nmax + t] = a.vz[g];
     unsigned int* F = m.F + 9 * t;
-    if (q.forces_first) {  // the first step's drift is done: its positions, no forces yet
-      m.pos[t] = a.pos32[g];
+    if (q.forces_first) {  // the first step's drift is done: no forces yet
 #pragma unroll
       for (int k = 0; k < 9; k++) F[k] = 0u;
     } else {
@@ -582,12 +639,13 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
         s_v[t] = vx;
         s_v[nmax + t] = vy;
         s_v[2 * nmax + t] = vz;
-        const long long X = (long long)((unsigned long long)s_x[t] + (unsigned long long)mul_shr(vx, P.drift_fx, 40));
-        const long long Y = (long long)((unsigned long long)s_x[nmax + t] + (unsigned long long)mul_shr(vy, P.drift_fx, 40));
-        const long long Z = (long long)((unsigned long long)s_x[2 * nmax + t] + (unsigned long long)mul_shr(vz, P.drift_fx, 40));
-        s_x[t] = X;
-        s_x[nmax + t] = Y;
-        s_x[2 * nmax + t] = Z;
+        const int4 old = m.pos[t];
+        const long long X = (long long)((unsigned long long)whole(old.x, s_lo[t]) + (unsigned long long)mul_shr(vx, P.drift_fx, 40));
+        const long long Y = (long long)((unsigned long long)whole(old.y, s_lo[nmax + t]) + (unsigned long long)mul_shr(vy, P.drift_fx, 40));
+        const long long Z = (long long)((unsigned long long)whole(old.z, s_lo[2 * nmax + t]) + (unsigned long long)mul_shr(vz, P.drift_fx, 40));
+        s_lo[t] = (unsigned int)X;
+        s_lo[nmax + t] = (unsigned int)Y;
+        s_lo[2 * nmax + t] = (unsigned int)Z;
         const int4 p = make_int4(hi_word(X), hi_word(Y), hi_word(Z), l);
         m.pos[t] = p;
         __stcg(&d.pos32[g], p);
@@ -615,7 +673,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       force_rel(m, np, s, l, m.pos[t], m.pos[s * np + P.center_local], m.w[l], unit);
     }
     __syncthreads();
-    force_terms<true, kWide>(a, P, m, w, nbead, bead0, &s_queue, [&] {
+    force_terms<true, 8>(a, P, m, w, nbead, bead0, &s_queue, [&] {
       if (drift) {
         if (lane == 0) moved.wait(&s_abort);
         __syncwarp();
@@ -666,16 +724,8 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     }
     // the CTA's sums by its working warps, then the system's
     if (wid * 32 < nbead) {
-      ke_acc = warp_sum_ll(ke_acc);
-      px_acc = warp_sum_ll(px_acc);
-      py_acc = warp_sum_ll(py_acc);
-      pz_acc = warp_sum_ll(pz_acc);
-      if (lane == 0) {
-        m.red[wid * 4 + 0] = ke_acc;
-        m.red[wid * 4 + 1] = px_acc;
-        m.red[wid * 4 + 2] = py_acc;
-        m.red[wid * 4 + 3] = pz_acc;
-      }
+      const long long x = warp_sum4_ll(ke_acc, px_acc, py_acc, pz_acc);
+      if (lane < 4) m.red[wid * 4 + warp_sum4_index(lane)] = x;
     }
     __syncthreads();
     summed.target += gridDim.x;
@@ -723,9 +773,10 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   // results back to global memory
   for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
     const int g = bead0 + t;
-    d.px[g] = s_x[t];
-    d.py[g] = s_x[nmax + t];
-    d.pz[g] = s_x[2 * nmax + t];
+    const int4 p = m.pos[t];
+    d.px[g] = whole(p.x, s_lo[t]);
+    d.py[g] = whole(p.y, s_lo[nmax + t]);
+    d.pz[g] = whole(p.z, s_lo[2 * nmax + t]);
     a.vx[g] = s_v[t];
     a.vy[g] = s_v[nmax + t];
     a.vz[g] = s_v[2 * nmax + t];
@@ -818,19 +869,31 @@ __global__ void k_state_out(StateArgs a) {
 }  // namespace souffle
 
 namespace souffle {
-void launch_forces(const ForceArgs& a, int grid, int block, size_t smem, cudaStream_t s) {
+void launch_forces(const ForceArgs& a, int n_sys, int grid, int block, size_t smem, cudaStream_t s) {
+  if (grid == a.n_items) {
+    if (a.chain64)
+      k_forces<true, false><<<grid, block, smem, s>>>(a);
+    else
+      k_forces<false, false><<<grid, block, smem, s>>>(a);
+    return;
+  }
   if (a.chain64)
-    k_forces<true><<<grid, block, smem, s>>>(a);
+    k_forces<true, true><<<grid, block, smem, s>>>(a);
   else
-    k_forces<false><<<grid, block, smem, s>>>(a);
+    k_forces<false, true><<<grid, block, smem, s>>>(a);
+  if (a.mode == 0) return;
+  if (a.chain64)
+    k_step_end<true><<<n_sys, 64, 0, s>>>(a);
+  else
+    k_step_end<false><<<n_sys, 64, 0, s>>>(a);
 }
 void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s) {
   k_drift<<<grid, block, 0, s>>>(a);
 }
 // shared memory of k_window: the force kernel's, then per-bead state, kick coefficients, system state
 size_t window_smem_bytes(size_t force_bytes, int subs, int np) {
-  return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (6 * (size_t)subs * np + 2 * (size_t)((np + 1) & ~1)) +
-         sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat);
+  return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (3 * (size_t)subs * np + 2 * (size_t)((np + 1) & ~1)) +
+         sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat) + 3 * sizeof(unsigned int) * (size_t)subs * np;
 }
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
                           cudaStream_t s) {
@@ -857,32 +920,42 @@ void launch_state_in(const StateArgs& a, int grid, int block, cudaStream_t s) {
 void launch_state_out(const StateArgs& a, int grid, int block, cudaStream_t s) {
   k_state_out<<<grid, block, 0, s>>>(a);
 }
-cudaError_t set_kernel_smem(size_t force_smem, int force_threads, size_t pair_smem) {
-  cudaError_t e = cudaFuncSetAttribute(k_forces<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem);
+namespace {
+// Ask for a shared-memory carveout that holds as many force CTAs as the registers allow (the
+// default may be smaller, which splits a one-wave grid into two waves).
+template <class Kernel>
+cudaError_t set_force_smem(Kernel* fn, size_t smem, int threads, int regs_sm, int smem_sm) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_forces<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem);
-  if (e != cudaSuccess) return e;
-  // Ask for a shared-memory carveout that holds as many force CTAs as the registers allow (the
-  // default may be smaller, which splits a one-wave grid into two waves).
   cudaFuncAttributes fa{};
-  if ((e = cudaFuncGetAttributes(&fa, k_forces<false>)) != cudaSuccess) return e;
+  if ((e = cudaFuncGetAttributes(&fa, fn)) != cudaSuccess) return e;
+  const int warp_regs = ((fa.numRegs * 32 + 255) / 256) * 256;
+  const int ctas = regs_sm / (warp_regs * ((threads + 31) / 32));
+  const size_t need = (size_t)ctas * (smem + fa.sharedSizeBytes + 1024);
+  const int percent = (int)std::min<size_t>(100, (need * 100 + smem_sm - 1) / (size_t)smem_sm);
+  return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+}
+}  // namespace
+
+cudaError_t set_kernel_smem(size_t force_smem, int force_threads, size_t pair_smem) {
+  cudaError_t e;
   int dev = 0, regs_sm = 0, smem_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
-  const int warp_regs = ((fa.numRegs * 32 + 255) / 256) * 256;
-  const int ctas = regs_sm / (warp_regs * ((force_threads + 31) / 32));
-  const size_t need = (size_t)ctas * (force_smem + fa.sharedSizeBytes + 1024);
-  const int percent = (int)std::min<size_t>(100, (need * 100 + smem_sm - 1) / (size_t)smem_sm);
-  if ((e = cudaFuncSetAttribute(k_forces<false>, cudaFuncAttributePreferredSharedMemoryCarveout, percent)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_forces<true>, cudaFuncAttributePreferredSharedMemoryCarveout, percent)) != cudaSuccess)
+  if ((e = set_force_smem(k_forces<false, false>, force_smem, force_threads, regs_sm, smem_sm)) != cudaSuccess ||
+      (e = set_force_smem(k_forces<false, true>, force_smem, force_threads, regs_sm, smem_sm)) != cudaSuccess ||
+      (e = set_force_smem(k_forces<true, false>, force_smem, force_threads, regs_sm, smem_sm)) != cudaSuccess ||
+      (e = set_force_smem(k_forces<true, true>, force_smem, force_threads, regs_sm, smem_sm)) != cudaSuccess)
     return e;
   return set_pairs_smem(pair_smem);
 }
 
-cudaError_t force_wave_ctas(int threads, size_t smem, int* ctas) {
+// CTAs of the force kernel resident at once: one item each, or (run) drawing items
+cudaError_t force_wave_ctas(bool run, int threads, size_t smem, int* ctas) {
   int per_sm = 0, dev = 0, sms = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_forces<false>, threads, smem);
+  cudaError_t e = run ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_forces<false, true>, threads, smem)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_forces<false, false>, threads, smem);
   if (e != cudaSuccess) return e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;

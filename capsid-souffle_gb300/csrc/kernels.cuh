@@ -62,6 +62,8 @@ struct ForceArgs {
   const SysParams* sys;
   SysState* state;
   const WorkItem* work;
+  int n_items;
+  unsigned int* ticket;      // items drawn by the CTAs of a launch, zero between launches
   const int2* sys_slots;     // per system: first work item in system order, work-item (CTA) count
   const int4* pos32;
   const unsigned int* intra_mask;
@@ -212,7 +214,8 @@ bool pairs_search(int max_sub, int cand_cap);
 constexpr int kPairChunkMax = 32;
 int pair_chunk(int np, int words);
 size_t pair_smem_bytes(int np, int words, int chunk);
-void launch_forces(const ForceArgs& a, int grid, int block, size_t smem, cudaStream_t s);
+// grid: at most a wave of CTAs; with fewer than a.n_items a second kernel ends the step of n_sys systems
+void launch_forces(const ForceArgs& a, int n_sys, int grid, int block, size_t smem, cudaStream_t s);
 void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s);
 size_t window_smem_bytes(size_t force_bytes, int subs, int np);
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
@@ -223,7 +226,7 @@ void launch_state_out(const StateArgs& a, int grid, int block, cudaStream_t s);
 void launch_energies(const EnergyArgs& a, int n, cudaStream_t s);
 cudaError_t set_kernel_smem(size_t force_smem, int force_threads, size_t pair_smem);
 // force-kernel CTAs of the given shape resident on the device at once (one wave)
-cudaError_t force_wave_ctas(int threads, size_t smem, int* ctas);
+cudaError_t force_wave_ctas(bool run, int threads, size_t smem, int* ctas);
 cudaError_t set_pairs_smem(size_t smem);
 
 }  // namespace souffle

@@ -131,10 +131,10 @@ struct Chain64 {
 };
 
 // Lengths of the force kernel's per-bead fixed-point force limbs (3 components x 3 32-bit limbs
-// per bead, padded to keep 16-byte alignment) and of its list of beads with inter-subunit pairs
-// (padded to a multiple of 4).
+// per bead, padded to keep 16-byte alignment) and of its list of pieces of the
+// inter-subunit lists (at most four places per bead: a long list's, three pieces').
 __host__ __device__ inline int force_slot_len(int nbead_max) { return 9 * ((nbead_max + 3) & ~3); }
-__host__ __device__ inline int force_rows_len(int nbead_max) { return (nbead_max + 3) & ~3; }
+__host__ __device__ inline int force_rows_len(int nbead_max) { return 4 * nbead_max; }
 
 // Bytes of the force kernel's first shared-memory region: the bonded tile (edge and bending
 // terms of max_sub subunits), and at least the system state plus the thermostat scratch

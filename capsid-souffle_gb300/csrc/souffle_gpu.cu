@@ -448,6 +448,8 @@ ForceArgs force_args(souffle_gpu_system* h, int mode, bool want_parts) {
   a.bb_pos32 = h->bb_pos32.p;
   a.chain64 = h->opt.chain_fp64 ? h->chain64.p : nullptr;
   a.max_sub = h->subs_per_cta;
+  a.n_items = (int)h->work.size();
+  a.ticket = h->force_ticket.p;
   a.div_np = div_magic(h->tpl.np);
   a.div_ne = div_magic(h->L.ne);
   a.div_nb = div_magic(h->L.nbend);
@@ -492,6 +494,13 @@ DriftArgs drift_args(souffle_gpu_system* h) {
   return a;
 }
 
+// k_drift: a thread per bead; twice as many where the upper half prefetches
+void launch_drift_all(souffle_gpu_system* h) {
+  const DriftArgs a = drift_args(h);
+  const int threads = a.inter_ids ? h->threads : std::min(h->threads, (h->subs_per_cta * h->tpl.np + 31) / 32 * 32);
+  launch_drift(a, (int)h->work.size(), threads, h->stream);
+}
+
 // k_forces, preceded by the surrogate's far-field forces when it is on
 void launch_forces_all(souffle_gpu_system* h, int mode, bool want_parts, bool judge = false) {
   ForceArgs fa = force_args(h, mode, want_parts);
@@ -499,11 +508,11 @@ void launch_forces_all(souffle_gpu_system* h, int mode, bool want_parts, bool ju
     surrogate_forces(h, fa);
     if (judge) surrogate_judge(h);
   }
-  launch_forces(fa, (int)h->work.size(), h->threads, h->force_smem, h->stream);
+  launch_forces(fa, h->n_sys, h->force_grid, h->threads, h->force_smem, h->stream);
 }
 
 void launch_step(souffle_gpu_system* h, bool rebuild, bool judge) {
-  launch_drift(drift_args(h), (int)h->work.size(), h->threads, h->stream);
+  launch_drift_all(h);
   if (rebuild) launch_rebuild(h);
   launch_forces_all(h, 1, false, judge);
 }
@@ -555,8 +564,9 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   if (smem > 200 * 1024) return fail(SOUFFLE_ERR_BAD_INPUT, "template too large for shared memory");
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   CUDA_TRY(set_kernel_smem(smem, threads, h->pair_smem));
-  int wave = 0, win_wave = 0;
-  CUDA_TRY(force_wave_ctas(threads, smem, &wave));
+  int wave = 0, run_wave = 0, win_wave = 0;
+  CUDA_TRY(force_wave_ctas(false, threads, smem, &wave));
+  CUDA_TRY(force_wave_ctas(true, threads, smem, &run_wave));
   size_t win_smem = window_smem_bytes(smem, subs, h->tpl.np);
   if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(false, threads, win_smem, &win_wave));
   std::vector<WorkItem> work;
@@ -603,11 +613,17 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   CUDA_TRY(cudaMemcpy(h->d_slots.p, slots.data(), sizeof(int2) * slots.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(h->partial.alloc(4 * work.size()));  // the force kernel's per-system running sums
   CUDA_TRY(cudaMemset(h->partial.p, 0, sizeof(long long) * h->partial.n));
+  if (h->force_ticket.n == 0) {
+    CUDA_TRY(h->force_ticket.alloc(1));
+    CUDA_TRY(cudaMemset(h->force_ticket.p, 0, sizeof(unsigned int)));
+  }
   h->work.swap(work);
   h->slots.swap(slots);
   h->subs_per_cta = subs;
   h->threads = threads;
   h->force_smem = smem;
+  // more items than one wave of CTAs: the form whose CTAs draw items
+  h->force_grid = (int)h->work.size() <= std::max(wave, run_wave) ? (int)h->work.size() : run_wave;
   h->window_ok = (int)h->work.size() <= win_wave;
   h->window_wide = false;
   h->window_threads = threads;
@@ -1374,7 +1390,7 @@ souffle_status souffle_gpu_md_enqueue(souffle_gpu_system* h, int64_t first_step,
       cudaError_t launched = cudaSuccess;
       if (len > 1 && window_usable(h)) {
         if (rebuild_first) {
-          launch_drift(drift_args(h), (int)h->work.size(), h->threads, h->stream);
+          launch_drift_all(h);
           launch_rebuild(h);
         }
         launched = launch_window_steps(h, len, rebuild_first);
@@ -1421,7 +1437,7 @@ souffle_status souffle_gpu_md_profile(souffle_gpu_system* h, int64_t first_step,
   for (int64_t a = first_step; a < first_step + n_steps && st == SOUFFLE_OK; a++) {
     const bool rb = (a % B == 0);
     cudaEventRecord(ev[0], h->stream);
-    launch_drift(drift_args(h), (int)h->work.size(), h->threads, h->stream);
+    launch_drift_all(h);
     cudaEventRecord(ev[1], h->stream);
     if (rb) launch_rebuild(h);
     cudaEventRecord(ev[2], h->stream);

@@ -1,6 +1,6 @@
-"""Inter-subunit forces over lists of every length class: none, a part of eight lanes, one and several
-rounds of eight lanes by two, and rows long enough for a whole warp, by the force kernel and by both
-forms of the window kernel.  Reference: FP64 numpy sums over the pairs of the kernel's own lists (the
+"""Inter-subunit forces over lists of every length class: none, short and full pieces, several pieces, and
+lists long enough for a whole warp, by both forms of the force kernel (one item per CTA, CTAs that draw
+items) and of the window kernel.  Reference: FP64 numpy sums over the pairs of the kernel's own lists (the
 formulas of src/forces.cpp:67-145).
 
 Tolerance, derived: a pair's separation carries 6e-8 of relative rounding, which the steepest term (the
@@ -58,11 +58,12 @@ def direct(t, d, elj, pos, i, j):
     (33, 12, 7.4, 2.5, {}), (33, 12, 7.4, 6.4, {}), (33, 12, 7.4, 6.4, {"threads_per_cta": 96, "subunits_per_cta": 5}),
     (42, 30, 7.8, 9.0, {}),                         # several rounds of a whole warp
     (42, 400, 7.8, 2.4, {}),                        # the narrow window kernel
+    (20, 900, 6.6, 4.0, {"subunits_per_cta": 1}),   # more items than CTAs
 ])
 def test_forces_over_all_row_lengths(n, S, per_sub, e_cut, kw):
     t, o, d, pos, s = system(n, S, per_sub, e_cut, **kw)
     f = s.forces(rebuild=True)
-    counts, ids = s.pairlist(1600)
+    counts, ids = s.pairlist(1600 if S < 900 else 256)
     i = np.repeat(np.arange(len(pos)), counts)
     j = ids[np.arange(ids.shape[1])[None] < counts[:, None]]
     want, mag, k = direct(t, d, 2.1, s.get_state()[0], i, j)
@@ -76,3 +77,40 @@ def test_forces_over_all_row_lengths(n, S, per_sub, e_cut, kw):
         one.md_steps(a, 1)
     for x, y in zip((*s.get_state(), s.forces(rebuild=False)), (*one.get_state(), one.forces(rebuild=False))):
         assert np.array_equal(x, y)
+
+
+BIG = dict(sigma=6.0, charge=-78.0, shc=3.5)
+
+
+@pytest.mark.parametrize("over,kw,big", [({}, {}, False), ({"D": "b", "d": 100.0}, {}, False),
+                                         ({}, {"chain_fp64": True}, False), ({}, {}, True)])
+def test_drawn_items_equal_separate_systems(over, kw, big):
+    """A batch of more work items than a wave of CTAs (CTAs draw items of several systems, a second
+    kernel ends the step) against each system in a handle of its own: bitwise the same."""
+    from souffle_gb300 import geometry, workloads
+    t = geometry.template_by_name("bilayer_n5")
+    ws = [workloads.make(t, S, seed=5 + S, **over) for S in (1501, 700, 302)]
+    par = [gpu.system_params(w.opt, w.derived, int(w.opt.S), w.center_local) for w in ws]
+    places = workloads.place_big_beads(ws[1], 3, radius=BIG["sigma"] / 2, seed=8)
+    batch = gpu.GpuSystem(t, par, **kw)
+    batch.set_state(np.concatenate([w.state.pos for w in ws]), np.concatenate([w.state.vel for w in ws]))
+    if big:
+        batch.set_big_beads(places, system=1, **BIG)
+    batch.md_begin()
+    batch.md_steps(0, 13)
+    pb, vb = batch.get_state()
+    fb = batch.forces(rebuild=False)
+    off = 0
+    for k, (w, p) in enumerate(zip(ws, par)):
+        one = gpu.GpuSystem(t, [p], **kw)
+        one.set_state(w.state.pos, w.state.vel)
+        if big and k == 1:
+            one.set_big_beads(places, **BIG)
+        one.md_begin()
+        one.md_steps(0, 13)
+        po, vo = one.get_state()
+        n = len(po)
+        assert np.array_equal(pb[off:off + n], po) and np.array_equal(vb[off:off + n], vo)
+        assert np.array_equal(fb[off:off + n], one.forces(rebuild=False))
+        assert np.array_equal(batch.md_scalars(k), one.md_scalars(0))
+        off += n
