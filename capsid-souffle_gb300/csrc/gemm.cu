@@ -373,15 +373,40 @@ cudaError_t launch_act(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, 
 }  // namespace
 
 // ---- weight gradients ------------------------------------------------------------------------
-// One CTA per (tile, split): 128 x 128 of one layer's gradient over `steps` 64-wide K steps of the
-// batch.  A layer is one to four tiles with K the whole batch (4096 rows), so one GEMM per layer
-// kept one to six SMs busy for 20 us, and the bias sums took another 7 us launch each; split over
-// the batch all layers together fill the chip: 7 us (and 9 us cold for adding the splits and the bias
-// sums) where the layers' launches took 129 us at 4096 rows, width 128.
-//   warp 0, lane 0  TMA producer, warp 1 MMA issuer as above; warps 4-11 epilogue: the FP32 sums to
-//   the workspace as [column / 4][row][4], so that a warp's stores are whole lines
-using GD = GemmTile<128>;
-__global__ void __launch_bounds__(kThreads, 1)
+// All layers' weight gradients, the bias sums and the loss in one launch.  A layer is one to four
+// 128 x 128 tiles with K the whole batch (4096 rows), so one GEMM per layer kept one to six SMs busy for
+// 20 us, and the bias sums took another 7 us launch each.  Here a tile is 128 x 32, so that all layers
+// together are up to 58 CTAs, and the bias rows are CTAs beside them.  A narrower tile costs re-reads of
+// A from L2 and idle tensor columns, but what bounds a CTA is its K steps one after the other; splitting
+// the batch over CTAs as well was 3 us faster, but changes the order of the sums, and with it every
+// trained network.  A gradient call of 4096 rows: 307 us with a launch per layer and sum, 104 us now.
+//   warp 0, lane 0  TMA producer, warp 1 MMA issuer as above; warps 4-7 epilogue.
+// CTAs past the tiles: a warp per two rows of A for the bias gradients (lane l adds columns l, l + 32, ..., a
+// fixed tree adds the lanes); the last CTA adds the loss partials.
+constexpr int kDwBN = 32, kDwStages = 8, kDwStage = (kBM + kDwBN) * kBK * 2, kDwBars = 2 * kDwStages + 1;
+constexpr int kDwSmem = 1024 + kDwStages * kDwStage + kDwBars * 8 + 16;
+constexpr int kDwThreads = 256, kDwRows = 2 * kDwThreads / 32;
+__device__ __forceinline__ void dw_bias_row(const DwArgs& d, int row) {
+  const int lane = threadIdx.x & 31;
+  int l = 0;
+  while (l < d.layers && row >= d.layer[l].rows) row -= d.layer[l++].rows;
+  if (l == d.layers) return;
+  const __nv_bfloat16* g = d.layer[l].A + (size_t)row * d.ld;
+  float s = 0.f;
+  int c = lane;
+  for (; c + 31 * 32 < d.K; c += 32 * 32) {  // 32 loads in flight, added in order
+    __nv_bfloat16 v[32];
+#pragma unroll
+    for (int k = 0; k < 32; k++) v[k] = g[c + 32 * k];
+#pragma unroll
+    for (int k = 0; k < 32; k++) s += __bfloat162float(v[k]);
+  }
+  for (; c < d.K; c += 32) s += __bfloat162float(g[c]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) d.layer[l].bias_out[row] = s;
+}
+
+__global__ void __launch_bounds__(kDwThreads, 1)
     k_gemm_dw(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensorMap b0,
               const __grid_constant__ CUtensorMap a1, const __grid_constant__ CUtensorMap b1,
               const __grid_constant__ CUtensorMap a2, const __grid_constant__ CUtensorMap b2,
@@ -389,24 +414,43 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t bars = base + GD::kStages * GD::kStage;
-  const uint32_t full0 = bars, empty0 = bars + 8 * GD::kStages, done = bars + 16 * GD::kStages;
-  const uint32_t tmem_slot = bars + GD::kBars * 8;
+  const uint32_t bars = base + kDwStages * kDwStage;
+  const uint32_t full0 = bars, empty0 = bars + 8 * kDwStages, done = bars + 16 * kDwStages;
+  const uint32_t tmem_slot = bars + kDwBars * 8;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
   const int warp = (int)__reduce_max_sync(0xffffffffu, threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int tile = blockIdx.x / d.splits, split = blockIdx.x - tile * d.splits;
+  const int tile = blockIdx.x;
+  if (tile >= d.tiles) {
+    pdl_launch();
+    pdl_wait();
+    if (blockIdx.x < gridDim.x - 1) {
+      for (int r = warp; r < kDwRows; r += kDwThreads / 32) dw_bias_row(d, (tile - d.tiles) * kDwRows + r);
+      return;
+    }
+    __shared__ float red[kDwThreads];
+    float s = 0.0f;
+    for (int i = threadIdx.x; i < d.n_partial; i += kDwThreads) s += d.loss_partial[i];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int k = kDwThreads / 2; k > 0; k >>= 1) {
+      if ((int)threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *d.loss = red[0];
+    return;
+  }
   int l = 0;
   while (l + 1 < d.layers && tile >= d.layer[l + 1].tile0) l++;
-  const int q = tile - d.layer[l].tile0, m0 = q / d.layer[l].tiles_n * 128, n0 = q % d.layer[l].tiles_n * 128;
-  const int nk = (d.K + kBK - 1) / kBK, k0 = split * d.steps, k1 = min(nk, k0 + d.steps);  // k0 < k1 for every split
+  const int q = tile - d.layer[l].tile0, m0 = q / d.layer[l].tiles_n * kBM, n0 = q % d.layer[l].tiles_n * kDwBN;
+  const int nk = (d.K + kBK - 1) / kBK;
   const CUtensorMap* ta = l == 0 ? &a0 : l == 1 ? &a1 : l == 2 ? &a2 : &a3;
   const CUtensorMap* tb = l == 0 ? &b0 : l == 1 ? &b1 : l == 2 ? &b2 : &b3;
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 128);
+    tmem_alloc(tmem_slot, kDwBN);
     tmem_relinquish();
   }
   if (threadIdx.x == 32) {
-    for (int s = 0; s < GD::kStages; s++) {
+    for (int s = 0; s < kDwStages; s++) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
@@ -422,38 +466,37 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) {
     if (lane == 0) {
       bool ok = true;
-      int g = 0;
-      for (int k = k0; k < k1; k++, g++) {
-        const int s = g % GD::kStages;
-        if (g >= GD::kStages && !mbar_wait(empty0 + 8 * s, (uint32_t)(g / GD::kStages - 1) & 1u)) {
+      int k = 0;
+      for (; k < nk; k++) {
+        const int s = k % kDwStages;
+        if (k >= kDwStages && !mbar_wait(empty0 + 8 * s, (uint32_t)(k / kDwStages - 1) & 1u)) {
           ok = false;
           break;
         }
-        const uint32_t a_s = base + s * GD::kStage;
-        mbar_expect_tx(full0 + 8 * s, GD::kStage);
+        const uint32_t a_s = base + s * kDwStage;
+        mbar_expect_tx(full0 + 8 * s, kDwStage);
         tma_load_2d(a_s, ta, k * kBK, m0, full0 + 8 * s);
-        tma_load_2d(a_s + GD::kA, tb, k * kBK, n0, full0 + 8 * s);
+        tma_load_2d(a_s + kBM * kBK * 2, tb, k * kBK, n0, full0 + 8 * s);
       }
       // every copy started here has landed before the CTA can leave
-      for (int p = (g > GD::kStages ? g - GD::kStages : 0); p < g; p++)
-        if (!mbar_wait(full0 + 8 * (p % GD::kStages), (uint32_t)(p / GD::kStages) & 1u)) ok = false;
+      for (int p = (k > kDwStages ? k - kDwStages : 0); p < k; p++)
+        if (!mbar_wait(full0 + 8 * (p % kDwStages), (uint32_t)(p / kDwStages) & 1u)) ok = false;
       if (!ok) atomicOr(d.err, 1u);
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc = umma_idesc_bf16(kBM, 128);
+    constexpr uint32_t idesc = umma_idesc_bf16(kBM, kDwBN);
     bool ok = true;
-    int g = 0;
-    for (int k = k0; k < k1; k++, g++) {
-      const int s = g % GD::kStages;
-      if (ok) ok = mbar_wait(full0 + 8 * s, (uint32_t)(g / GD::kStages) & 1u);
+    for (int k = 0; k < nk; k++) {
+      const int s = k % kDwStages;
+      if (ok) ok = mbar_wait(full0 + 8 * s, (uint32_t)(k / kDwStages) & 1u);
       tc_fence_after();
-      const uint32_t a_s = base + s * GD::kStage;
-      const uint64_t ad = sw128_kmajor_desc(a_s), bd = sw128_kmajor_desc(a_s + GD::kA);
+      const uint32_t a_s = base + s * kDwStage;
+      const uint64_t ad = sw128_kmajor_desc(a_s), bd = sw128_kmajor_desc(a_s + kBM * kBK * 2);
       if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < kBK / 16; j++) umma_bf16(tmem, ad + 2 * j, bd + 2 * j, idesc, (g | j) != 0 ? 1u : 0u);
+        for (int j = 0; j < kBK / 16; j++) umma_bf16(tmem, ad + 2 * j, bd + 2 * j, idesc, (k | j) != 0 ? 1u : 0u);
         umma_commit(empty0 + 8 * s);
-        if (k == k1 - 1) umma_commit(done);
+        if (k == nk - 1) umma_commit(done);
       }
       __syncwarp();
     }
@@ -462,19 +505,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_wait(done, 0);  // (bounded) MMAs issued so far may still be writing tensor memory
     }
   } else if (warp >= 4) {
-    const int quarter = warp & 3, half = (warp - 4) >> 2;
+    const int quarter = warp & 3;
     if (mbar_wait(done, 0)) {
       tc_fence_after();
-      const int row = quarter * 32 + lane;
-      float4* out = reinterpret_cast<float4*>(d.ws + (size_t)blockIdx.x * kDwTile);
-#pragma unroll 1
-      for (int c = 64 * half; c < 64 * half + 64; c += 32) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
+      const DwLayer& y = d.layer[l];
+      const int row = m0 + quarter * 32 + lane;
+      float v[32];
+      tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16), v);
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-          out[(c / 4 + k) * 128 + row] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-      }
+      for (int k = 0; k < 8; k++)  // cols a multiple of 8, rows 16-byte aligned
+        if (row < y.rows && n0 + 4 * k < y.cols)
+          *reinterpret_cast<float4*>(y.out + (size_t)row * y.cols + n0 + 4 * k) =
+              make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     } else {
       atomicOr(d.err, 1u);
     }
@@ -484,107 +526,32 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, 128);
+    tmem_dealloc(tmem, kDwBN);
   }
 }
 
-// Adds the splits of every tile in order (thread per four columns of a row), sums the layers' A rows
-// over the batch for the bias gradients (warp per row), and the loss partials (last CTA).
-__global__ void __launch_bounds__(256) k_dw_reduce(DwArgs d, int w_blocks, int b_blocks) {
-  const int lane = threadIdx.x & 31;
-  if ((int)blockIdx.x < w_blocks) {
-    const int i = blockIdx.x * 256 + threadIdx.x;  // tile, column / 4, row
-    const int tile = i / (32 * 128), r = i - tile * (32 * 128), c4 = r >> 7, row = r & 127;
-    if (tile >= d.tiles) return;
-    int l = 0;
-    while (l + 1 < d.layers && tile >= d.layer[l + 1].tile0) l++;
-    const DwLayer& y = d.layer[l];
-    const int q = tile - y.tile0, gr = q / y.tiles_n * 128 + row, gc = q % y.tiles_n * 128 + 4 * c4;
-    if (gr >= y.rows || gc >= y.cols) return;
-    const float4* p = reinterpret_cast<const float4*>(d.ws + (size_t)tile * d.splits * kDwTile) + r;
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int k = 0; k < d.splits; k++) {
-      const float4 v = __ldcg(p + (size_t)k * (kDwTile / 4));
-      s.x += v.x;
-      s.y += v.y;
-      s.z += v.z;
-      s.w += v.w;
-    }
-    *reinterpret_cast<float4*>(y.out + (size_t)gr * y.cols + gc) = s;  // cols a multiple of 8, 16-byte aligned
-    return;
-  }
-  if ((int)blockIdx.x < w_blocks + b_blocks) {
-    int row = (blockIdx.x - w_blocks) * 8 + (threadIdx.x >> 5), l = 0;
-    while (l < d.layers && row >= d.layer[l].rows) row -= d.layer[l++].rows;
-    if (l == d.layers) return;
-    const __nv_bfloat16* g = d.layer[l].A + (size_t)row * d.ld;
-    float s = 0.f;
-    const int n8 = d.K >> 3;
-#pragma unroll 4
-    for (int c = lane; c < n8; c += 32) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(g) + c);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-        s += f.x + f.y;
-      }
-    }
-    for (int c = 8 * n8 + lane; c < d.K; c += 32) s += __bfloat162float(g[c]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) d.layer[l].bias_out[row] = s;
-    return;
-  }
-  __shared__ float red[256];
-  float s = 0.0f;
-  for (int i = threadIdx.x; i < d.n_partial; i += 256) s += d.loss_partial[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = 128; k > 0; k >>= 1) {
-    if ((int)threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *d.loss = red[0];
-}
-
-// Tiles, and as many splits of the batch as give every SM an item (152, at least two K steps each).
-void dw_plan(DwArgs& a) {
-  a.tiles = 0;
-  for (int l = 0; l < a.layers; l++) {
-    DwLayer& y = a.layer[l];
-    y.tile0 = a.tiles;
-    y.tiles_n = (y.cols + 127) / 128;
-    a.tiles += (y.rows + 127) / 128 * y.tiles_n;
-  }
-  const int nk = (a.K + kBK - 1) / kBK;
-  const int want = std::max(1, std::min((nk + 1) / 2, 152 / a.tiles));
-  a.steps = (nk + want - 1) / want;
-  a.splits = (nk + a.steps - 1) / a.steps;
-}
-
-cudaError_t dw_gemm(const DwArgs& a, cudaStream_t st) {
+cudaError_t weight_gradients(DwArgs a, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] { attr = cudaFuncSetAttribute(k_gemm_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, GD::kSmem); });
+  std::call_once(once, [] { attr = cudaFuncSetAttribute(k_gemm_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmem); });
   if (attr != cudaSuccess) return attr;
-  if (a.layers < 1 || a.layers > 4 || a.K < 1 || a.ld < a.K || a.ld % 8 || a.tiles * a.splits > kDwItems || !a.ws || !a.err)
-    return cudaErrorInvalidValue;
+  if (a.layers < 1 || a.layers > 4 || a.K < 1 || a.ld < a.K || a.ld % 8 || !a.err) return cudaErrorInvalidValue;
   CUtensorMap m[8];
+  int rows = 0;
+  a.tiles = 0;
   for (int l = 0; l < 4; l++) {
-    const DwLayer& y = a.layer[l < a.layers ? l : 0];
-    if (!make_map(&m[2 * l], y.A, y.rows, a.K, a.ld, kBM) || !make_map(&m[2 * l + 1], y.B, y.cols, a.K, a.ld, 128))
+    DwLayer& y = a.layer[l < a.layers ? l : 0];
+    if (l < a.layers) {
+      y.tile0 = a.tiles;
+      y.tiles_n = (y.cols + kDwBN - 1) / kDwBN;
+      a.tiles += (y.rows + kBM - 1) / kBM * y.tiles_n;
+      rows += y.rows;
+    }
+    if (!make_map(&m[2 * l], y.A, y.rows, a.K, a.ld, kBM) || !make_map(&m[2 * l + 1], y.B, y.cols, a.K, a.ld, kDwBN))
       return cudaErrorInvalidValue;
   }
-  return launch_pdl(k_gemm_dw, a.tiles * a.splits, kThreads, GD::kSmem, st, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
-}
-
-cudaError_t dw_reduce(const DwArgs& a, cudaStream_t st) {
-  int rows = 0;
-  for (int l = 0; l < a.layers; l++) rows += a.layer[l].rows;
-  const int w_blocks = a.tiles * 16, b_blocks = (rows + 7) / 8;
-  k_dw_reduce<<<w_blocks + b_blocks + 1, 256, 0, st>>>(a, w_blocks, b_blocks);
-  return cudaGetLastError();
+  return launch_pdl(k_gemm_dw, a.tiles + (rows + kDwRows - 1) / kDwRows + 1, kDwThreads, kDwSmem, st, m[0], m[1], m[2], m[3],
+                    m[4], m[5], m[6], m[7], a);
 }
 
 cudaError_t gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const GemmEpi& e,

@@ -38,32 +38,26 @@ struct MlpNorm {
 };
 
 // Weight gradients of up to four layers in one launch: for layer l, G_l [rows][cols] = A_l B_l^T with A_l
-// [rows][K] and B_l [cols][K] BF16 (K contiguous, row strides ld), K the batch.  The contraction is
-// split over CTAs; split s of tile t leaves FP32 sums in ws + (first + t splits + s) kDwTile, and
-// dw_reduce adds a tile's splits in order.
+// [rows][K] and B_l [cols][K] BF16 (K contiguous, row strides ld), K the batch; the sums of A's rows; and
+// the sum of the loss partials.
 struct DwLayer {
   const __nv_bfloat16* A = nullptr;
   const __nv_bfloat16* B = nullptr;
   int rows = 0, cols = 0;
   float* out = nullptr;            // [rows][cols]
   float* bias_out = nullptr;       // [rows] sums of A's rows over the batch
-  int tile0 = 0, tiles_n = 0;      // filled by dw_plan: first tile, tiles per row of tiles
+  int tile0 = 0, tiles_n = 0;      // filled by weight_gradients: first tile, tiles per row of tiles
 };
 struct DwArgs {
   DwLayer layer[4];
   int layers = 0, K = 0, ld = 0;
-  int tiles = 0, splits = 0, steps = 0;  // filled by dw_plan: 64-wide K steps per split
-  float* ws = nullptr;
+  int tiles = 0;                         // filled by weight_gradients
   unsigned int* err = nullptr;
-  const float* loss_partial = nullptr;   // summed into *loss by dw_reduce
+  const float* loss_partial = nullptr;   // summed into *loss
   int n_partial = 0;
   float* loss = nullptr;
 };
-constexpr size_t kDwTile = 128 * 128;    // floats of one tile's partial sums
-constexpr int kDwItems = 192;            // most (tile, split) items of a launch: the workspace holds so many
-void dw_plan(DwArgs& a);
-cudaError_t dw_gemm(const DwArgs& a, cudaStream_t st);
-cudaError_t dw_reduce(const DwArgs& a, cudaStream_t st);
+cudaError_t weight_gradients(DwArgs a, cudaStream_t st);
 
 // Launches on the stream; A/B base addresses 16-byte aligned, lda/ldb multiples of 8 elements.
 cudaError_t gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const GemmEpi& e,

@@ -194,7 +194,6 @@ struct souffle_mlp {
   DevBuf<float> grads;                 // flat, the parameters' layout, then the loss
   float* gw[kLayers] = {};             // inside grads
   float* gb[kLayers] = {};
-  DevBuf<float> dw_ws;                 // partial weight gradients (allocated by the first training call)
   DevBuf<__nv_bfloat16> wb[kLayers], wbt[kLayers];
   DevBuf<__nv_bfloat16> act[kLayers], act_t[kLayers];  // a_0 .. a_3 and transposes
   DevBuf<float> z[kLayers];                            // z_1 .. z_3 (index l for layer l output)
@@ -269,7 +268,6 @@ souffle_status backward(souffle_mlp* h, const float* t, int m) {
   const int np_out = h->out_pad[L];
   const int nb = blocks(m, kLossRows);
   MLP_TRY(h->partial.n < (size_t)nb ? cudaErrorInvalidValue : cudaSuccess);
-  if (h->dw_ws.n == 0) MLP_TRY(h->dw_ws.alloc(kDwItems * kDwTile));
   k_loss<<<nb, 256, 0, h->stream>>>(h->y.p, np_out, t, m, h->n_out, np_out, h->dz[L + 1].p, h->dz_t[L + 1].p, h->cap,
                                     h->partial.p);
   MLP_TRY(cudaGetLastError());
@@ -296,7 +294,6 @@ souffle_status backward(souffle_mlp* h, const float* t, int m) {
   w.layers = kLayers;
   w.K = m;
   w.ld = h->cap;
-  w.ws = h->dw_ws.p;
   w.err = h->err.p;
   w.loss_partial = h->partial.p;
   w.n_partial = nb;
@@ -309,9 +306,7 @@ souffle_status backward(souffle_mlp* h, const float* t, int m) {
     w.layer[l].out = h->gw[l];
     w.layer[l].bias_out = h->gb[l];
   }
-  dw_plan(w);
-  MLP_TRY(dw_gemm(w, h->stream));
-  MLP_TRY(dw_reduce(w, h->stream));
+  MLP_TRY(weight_gradients(w, h->stream));
   return SOUFFLE_OK;
 }
 

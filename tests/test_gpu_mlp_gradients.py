@@ -1,5 +1,5 @@
-"""Weight gradients split over the batch, at the edges of the split: batches below one K step, of odd
-length, and large enough for every split, outputs off the tile size, both widths.  Against the CPU
+"""Weight gradients of all layers in one launch, at the edges of its tiles: batches below one K step, of
+odd length, and of many steps, outputs off the tile size, both widths.  Against the CPU
 restatement, with the tolerances of test_gpu_mlp.py (BF16 activations: 1e-2 of each tensor's norm)."""
 import os
 import sys
