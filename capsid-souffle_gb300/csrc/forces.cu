@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   // the positions (the high words are the tile's)
   const int nmax = a.max_sub * np;
   long long* s_v = reinterpret_cast<long long*>(smem + q.force_bytes);  // [3][nmax]
-  long long* s_kc = s_v + 3 * nmax;                                     // [np]
+  long long* s_kc = s_v + ((3 * nmax + 1) & ~1);                        // [np] (16-byte aligned, as the state)
   dfloat* s_im = reinterpret_cast<dfloat*>(s_kc + ((np + 1) & ~1));     // [np] 1 / m
   SysState& S = *reinterpret_cast<SysState*>(s_im + ((np + 1) & ~1));
   dfloat* chain_scratch = reinterpret_cast<dfloat*>(&S + 1);
@@ -892,7 +892,8 @@ void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s) {
 }
 // shared memory of k_window: the force kernel's, then per-bead state, kick coefficients, system state
 size_t window_smem_bytes(size_t force_bytes, int subs, int np) {
-  return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (3 * (size_t)subs * np + 2 * (size_t)((np + 1) & ~1)) +
+  const size_t vel = (3 * (size_t)subs * np + 1) & ~(size_t)1;
+  return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (vel + 2 * (size_t)((np + 1) & ~1)) +
          sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat) + 3 * sizeof(unsigned int) * (size_t)subs * np;
 }
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
