@@ -512,9 +512,14 @@ __global__ void __launch_bounds__(256) k_drift(DriftArgs a) {
 // included: 19.6 -> 11.9 us at 200 beads, 23.3 -> 14.7 at 2,688, 24.8 -> 16.8 at 13,986, 36.2 ->
 // 27.2 at 84,000.  What is left there: the chain (2.7 us), the two barriers (1.5 us) and the wait
 // for the CTA with the most pairs.
-// The two barriers of a step count their arrivals separately: a CTA without inter-subunit pairs
-// does not wait at the first one, and its early arrival at the second must not be taken for
-// another's at the first.
+// A step has two waits, both among the CTAs of one system.  The first (positions published) counts
+// arrivals behind a fence.  The second needs none: the sums themselves count.  A sum's 64 bits are
+// added as two words of 32 with 1 << kSumCount on top, so whoever reads as many counts as the system
+// has CTAs reads complete sums, one trip through L2 after they were sent (with a fence and a counter
+// behind them, two: 20 subunits 1,256 -> 1,196 us per 100 steps, 333 Brownian ones 1,242 -> 1,172 per 50).  A CTA without inter-subunit pairs does not wait at the first; it cannot
+// get further than the second, so arrivals of two steps never mix.
+constexpr int kSumCount = 50;     // up to 2^14 CTAs, sums of up to 2^18 32-bit words
+constexpr int kWinWords = 16;     // a system's words per step: 8 of sums, 3 of random forces
 struct GridBarrier {
   unsigned int* count;    // arrivals, zero between launches
   unsigned int* err;
@@ -565,7 +570,9 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   __shared__ ForceQueue s_queue;
   __shared__ int s_abort;
   __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
-  GridBarrier moved{q.count, a.err, 0u}, summed{q.count + 1, a.err, 0u};  // positions published, sums complete
+  GridBarrier moved{q.count + 1 + w.sys, a.err, 0u};  // positions published
+  const int n_cta = a.sys_slots[w.sys].y;             // CTAs of the system
+  const bool first_cta = w.sub_begin == P.sub0;       // of them, the one with the first subunit
   const float unit = P.unit32;
   const bool bd = P.brownian;
   if (threadIdx.x == 0) {
@@ -614,8 +621,14 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   __syncthreads();
   const float* s_mass = m.tpl_f + L.o_mass;
   for (int step = 0; step < q.steps; step++) {
-    long long* acc = q.acc + (size_t)(step % 3) * q.acc_stride;
+    unsigned long long* acc = q.acc + (size_t)(step % 3) * q.acc_stride + (size_t)kWinWords * w.sys;
     const bool drift = step > 0 || !q.forces_first;
+    // The next step's sums start from zero: their words were last read two steps ago, and every CTA of
+    // the system has sent the last step's sums since.  (Seen before this step's sums complete.)
+    if (first_cta && threadIdx.x < kWinWords) {
+      q.acc[(size_t)((step + 1) % 3) * q.acc_stride + (size_t)kWinWords * w.sys + threadIdx.x] = 0;
+      __threadfence();
+    }
     if (threadIdx.x == 0) s_queue.next = 0;
     if (drift) {
       long long rx = 0, ry = 0, rz = 0;
@@ -657,14 +670,13 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
         ry = warp_sum_ll(ry);
         rz = warp_sum_ll(rz);
         if (lane == 0 && wid * 32 < nbead) {
-          unsigned long long* r = reinterpret_cast<unsigned long long*>(acc + 8 * w.sys + 4);
-          atomicAdd(r, (unsigned long long)rx);
-          atomicAdd(r + 1, (unsigned long long)ry);
-          atomicAdd(r + 2, (unsigned long long)rz);
+          atomicAdd(acc + 8, (unsigned long long)rx);
+          atomicAdd(acc + 9, (unsigned long long)ry);
+          atomicAdd(acc + 10, (unsigned long long)rz);
         }
         __threadfence();
       }
-      moved.target += gridDim.x;
+      moved.target += n_cta;
       __syncthreads();
       if (threadIdx.x == 0) moved.arrive();
     }
@@ -683,7 +695,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       if (threadIdx.x < 3) {
         if (drift) {
           moved.wait(&s_abort);
-          s_sum[4 + threadIdx.x] = __ldcg(acc + 8 * w.sys + 4 + threadIdx.x);
+          s_sum[4 + threadIdx.x] = (long long)__ldcg(acc + 8 + threadIdx.x);
         } else {
           s_sum[4 + threadIdx.x] = S.fran_sum[threadIdx.x];
         }
@@ -728,27 +740,30 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       if (lane < 4) m.red[wid * 4 + warp_sum4_index(lane)] = x;
     }
     __syncthreads();
-    summed.target += gridDim.x;
     unsigned int chain_pre = 0;
     if (wid == 0) {
-      // the next step's sums start from zero: their buffer was last read two steps ago, and every
-      // CTA has passed a barrier since
-      if (blockIdx.x == 0)
-        for (int k = lane; k < 8 * q.n_sys; k += 32) q.acc[(size_t)((step + 1) % 3) * q.acc_stride + k] = 0;
-      if (lane < 4) {
+      if (lane < 8) {
         long long x = 0;
-        for (int k = 0; k < nw && k * 32 < nbead; k++) x += m.red[4 * k + lane];
-        atomicAdd(reinterpret_cast<unsigned long long*>(acc + 8 * w.sys + lane), (unsigned long long)x);
+        for (int k = 0; k < nw && k * 32 < nbead; k++) x += m.red[4 * k + (lane >> 1)];
+        const unsigned long long part = lane & 1 ? (unsigned long long)((x >> 32) + 2147483648ll) : (unsigned long long)(unsigned int)x;
+        atomicAdd(acc + lane, (1ull << kSumCount) + part);
       }
-      __threadfence();
       __syncwarp();
-      if (lane == 0) summed.arrive();
-      __syncwarp();
-      chain_pre = nhc_pre_warp(S, lane, chain_scratch);  // while the other CTAs arrive
-      if (lane < 4) {
-        summed.wait(&s_abort);
-        s_sum[lane] = __ldcg(acc + 8 * w.sys + lane);
+      chain_pre = nhc_pre_warp(S, lane, chain_scratch);  // while the other CTAs' sums arrive
+      unsigned long long v = 0;
+      bool done = false;
+      for (unsigned int i = 0; i < GridBarrier::kWindowPolls; i++) {
+        if (lane < 8) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(acc + lane) : "memory");
+        done = __all_sync(0xffffffffu, lane >= 8 || (v >> kSumCount) == (unsigned long long)n_cta);
+        if (done || ((i & 255u) == 255u && *(volatile int*)&s_abort)) break;
       }
+      if (!done && lane == 0) {
+        s_abort = 1;
+        atomicOr(a.err, kErrWindow);
+      }
+      v &= (1ull << kSumCount) - 1;
+      const unsigned long long hi = __shfl_down_sync(0xffffffffu, v, 1) - ((unsigned long long)n_cta << 31);
+      if (lane < 8 && !(lane & 1)) s_sum[lane >> 1] = (long long)(v + (hi << 32));
     }
     __syncthreads();
     if (s_abort) return;
@@ -786,7 +801,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     a.fy[g] = Fy;
     a.fz[g] = Fz;
   }
-  if (w.sub_begin == P.sub0) {  // the CTA of the system's first subunit
+  if (first_cta) {
     int4* dst = reinterpret_cast<int4*>(a.state + w.sys);
     const int4* src = reinterpret_cast<const int4*>(&S);
     for (int t = threadIdx.x; t < (int)(sizeof(SysState) / 16); t += blockDim.x) dst[t] = src[t];
@@ -796,13 +811,14 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   __shared__ bool s_last;
   if (threadIdx.x == 0) {
     __threadfence();
-    s_last = atomicAdd(q.count + 2, 1u) == gridDim.x - 1;
+    s_last = atomicAdd(q.count, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (s_last) {
     for (int k = threadIdx.x; k < (int)(3 * q.acc_stride); k += blockDim.x) q.acc[k] = 0;
+    for (int k = threadIdx.x; k < q.n_sys; k += blockDim.x) q.count[1 + k] = 0u;
     if (threadIdx.x == 0) {
-      q.count[0] = q.count[1] = q.count[2] = 0u;
+      q.count[0] = 0u;
     }
   }
 }

@@ -125,9 +125,9 @@ struct WindowArgs {
   int steps;
   int forces_first;        // the first step's drift has run (and the pair lists were rebuilt after it)
   int n_sys;
-  unsigned int* count;     // [3] arrivals at the step's two barriers, CTAs that have left; zero between launches
-  long long* acc;          // [3][acc_stride]: per system 8 sums (kinetic energy, momentum, random forces)
-  size_t acc_stride;       // 8 n_sys
+  unsigned int* count;     // [1 + n_sys] CTAs that have left, then per system arrivals with new positions; zero between launches
+  unsigned long long* acc; // [3][acc_stride]: per system 16 words (sums of kinetic energy, momentum, random forces), likewise
+  size_t acc_stride;       // 16 n_sys
   size_t force_bytes;      // the force kernel's part of the shared memory, 16-byte multiple
 };
 

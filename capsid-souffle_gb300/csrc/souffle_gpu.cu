@@ -307,7 +307,7 @@ souffle_status check_err(souffle_gpu_system* h) {
     CUDA_TRY(cudaMemsetAsync(h->err.p, 0, sizeof(unsigned int), h->stream));
     if (e & kErrWindow) {  // the counters stand where the launch gave up
       CUDA_TRY(cudaMemsetAsync(h->win_count.p, 0, sizeof(unsigned int) * h->win_count.n, h->stream));
-      CUDA_TRY(cudaMemsetAsync(h->win_acc.p, 0, sizeof(long long) * h->win_acc.n, h->stream));
+      CUDA_TRY(cudaMemsetAsync(h->win_acc.p, 0, sizeof(unsigned long long) * h->win_acc.n, h->stream));
       return fail(SOUFFLE_ERR_CUDA, "window kernel: a bounded wait ran out");
     }
     if (e & kErrNonFinite) return fail(SOUFFLE_ERR_NONFINITE, "non-finite force or kinetic energy");
@@ -544,7 +544,7 @@ cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_firs
   q.n_sys = h->n_sys;
   q.count = h->win_count.p;
   q.acc = h->win_acc.p;
-  q.acc_stride = 8 * (size_t)h->n_sys;
+  q.acc_stride = 16 * (size_t)h->n_sys;
   q.force_bytes = (force_smem_for(h, h->subs_per_cta, h->window_threads) + 15) & ~(size_t)15;
   return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->window_threads, h->window_smem, h->stream);
 }
@@ -648,10 +648,10 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   }
   h->window_smem = win_smem;
   if (h->window_ok && h->win_count.n == 0) {
-    CUDA_TRY(h->win_count.alloc(3));
-    CUDA_TRY(h->win_acc.alloc(24 * (size_t)h->n_sys));
-    CUDA_TRY(cudaMemset(h->win_count.p, 0, 3 * sizeof(unsigned int)));
-    CUDA_TRY(cudaMemset(h->win_acc.p, 0, sizeof(long long) * h->win_acc.n));
+    CUDA_TRY(h->win_count.alloc(1 + (size_t)h->n_sys));
+    CUDA_TRY(h->win_acc.alloc(48 * (size_t)h->n_sys));
+    CUDA_TRY(cudaMemset(h->win_count.p, 0, sizeof(unsigned int) * h->win_count.n));
+    CUDA_TRY(cudaMemset(h->win_acc.p, 0, sizeof(unsigned long long) * h->win_acc.n));
   }
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.second);
   h->graphs.clear();

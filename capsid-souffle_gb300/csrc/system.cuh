@@ -59,7 +59,7 @@ struct souffle_gpu_system {
   size_t window_smem = 0;
   DevBuf<unsigned int> win_count;
   DevBuf<unsigned int> force_ticket;  // force kernel: work items drawn
-  DevBuf<long long> win_acc;
+  DevBuf<unsigned long long> win_acc;
   int inter_cap = 96, cand_cap = 128;
   int force_grid = 1;  // CTAs of the force kernel: one wave at most
   size_t force_smem = 0, pair_smem = 0;
