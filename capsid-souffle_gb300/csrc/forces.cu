@@ -516,8 +516,9 @@ __global__ void __launch_bounds__(256) k_drift(DriftArgs a) {
 // arrivals behind a fence.  The second needs none: the sums themselves count.  A sum's 64 bits are
 // added as two words of 32 with 1 << kSumCount on top, so whoever reads as many counts as the system
 // has CTAs reads complete sums, one trip through L2 after they were sent (with a fence and a counter
-// behind them, two: 20 subunits 1,256 -> 1,196 us per 100 steps, 333 Brownian ones 1,242 -> 1,172 per 50).  A CTA without inter-subunit pairs does not wait at the first; it cannot
-// get further than the second, so arrivals of two steps never mix.
+// behind them, two: 20 subunits 1,256 -> 1,196 us per 100 steps, 333 Brownian ones 1,242 -> 1,172 per
+// 50).  A CTA without inter-subunit pairs does not wait at the first; it cannot get further than the
+// second, so arrivals of two steps never mix.
 constexpr int kSumCount = 50;     // up to 2^14 CTAs, sums of up to 2^18 32-bit words
 constexpr int kWinWords = 16;     // a system's words per step: 8 of sums, 3 of random forces
 struct GridBarrier {
