@@ -432,9 +432,10 @@ __device__ __forceinline__ float lj_add(float c, float r2, const float* pair, fl
 // tenth of them in contact, 3,900 -> 3,450 us per 100 steps; 64: 1,870 -> 1,490; a force evaluation of
 // 64 dense replicas (17,286 subunits) 222 -> 203 us.
 // kFresh: the partners' positions are rewritten by other CTAs while this kernel runs (read past L1).
-template <bool kFresh, int kLanes>
+// wait: called once the first partners are known, before their positions are read.
+template <bool kFresh, int kLanes, class Wait>
 __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
-                                            const ForceQueue& q, int chunk) {
+                                            const ForceQueue& q, int chunk, Wait wait) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
   const int* species = m.tpl_i + L.o_species;
@@ -470,6 +471,10 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
   auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
   int i = lane & (lanes - 1);
   int j0 = partner(i), j1 = partner(i + lanes);
+  if (kFresh) {
+    asm volatile("" ::"r"(j0), "r"(j1));  // (loaded before the wait)
+    wait();
+  }
   unsigned long long ax = 0, ay = 0, az = 0;
   int added = 0;  // values added by fx_add2
   while (i < n) {
@@ -569,12 +574,11 @@ __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams&
       if (t < ne) force_edge(a, P, m, t);
       if (t + 32 < ne) force_edge(a, P, m, t + 32);
     } else {
-      if (kFresh && !waited) {
-        wait();
-        waited = true;
-      }
       // the long lists are the first kl of these chunks
-      force_inter<kFresh, kLanes>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq);
+      force_inter<kFresh, kLanes>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq, [&] {
+        if (!waited) wait();
+        waited = true;
+      });
     }
     __syncwarp();
   }

@@ -395,13 +395,27 @@ __device__ __forceinline__ void drift_bead(int g, int l, long long c, long long 
 // velocity after the last centre-of-mass removal and the generator's state before the step: bead k
 // of the system takes draws 6k+1 .. 6k+6 (x, y, z: two draws each).  Both are stored for the force
 // kernel; r returns the random force.
-__device__ __forceinline__ void brownian_draws(const DriftArgs& a, const SysParams& P, unsigned int lcg, int sys, int g, int l,
-                                               long long vx, long long vy, long long vz, long long* r) {
+__device__ __forceinline__ void brownian_drag(const DriftArgs& a, int sys, int g, int l, long long vx, long long vy, long long vz) {
   const long long N = a.n_total;
   const long long dc = a.bd_drag[(size_t)sys * a.np + l];
   a.fdrag[g] = -mul_shr(vx, dc, 48);
   a.fdrag[N + g] = -mul_shr(vy, dc, 48);
   a.fdrag[2 * N + g] = -mul_shr(vz, dc, 48);
+}
+// component k of bead g's random force alone
+__device__ __forceinline__ long long brownian_draw(const DriftArgs& a, const SysParams& P, unsigned int lcg, int sys, int g, int l,
+                                                   int k) {
+  unsigned int x = lcg_mul(lcg_mul(lcg, a.lcg_table[g - P.bead0]), 16807u);
+  for (int i = 0; i < 2 * k; i++) x = lcg_mul(x, 16807u);
+  const double sc = a.bd_noise[(size_t)sys * a.np + l];
+  const long long r = __double2ll_rn(__dmul_rn(sc, lcg_uniform_half(x, lcg_mul(x, 16807u))) * 4294967296.0);
+  a.fran[k * (long long)a.n_total + g] = r;
+  return r;
+}
+__device__ __forceinline__ void brownian_draws(const DriftArgs& a, const SysParams& P, unsigned int lcg, int sys, int g, int l,
+                                               long long vx, long long vy, long long vz, long long* r) {
+  const long long N = a.n_total;
+  brownian_drag(a, sys, g, l, vx, vy, vz);
   unsigned int x = lcg_mul(lcg, a.lcg_table[g - P.bead0]);
   unsigned int d[6];
 #pragma unroll
@@ -569,6 +583,8 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     return (long long)(((unsigned long long)(unsigned int)hi << 32) + (unsigned long long)(long long)(int)lo);
   };
   __shared__ ForceQueue s_queue;
+  __shared__ unsigned int s_active;     // the chain's active links
+  __shared__ long long s_draw[3];       // sums of the random forces drawn ahead
   __shared__ int s_abort;
   __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
   GridBarrier moved{q.count + 1 + w.sys, a.err, 0u};  // positions published
@@ -621,6 +637,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   }
   __syncthreads();
   const float* s_mass = m.tpl_f + L.o_mass;
+  bool drawn = false;  // the step's random forces have been drawn in the one before
   for (int step = 0; step < q.steps; step++) {
     unsigned long long* acc = q.acc + (size_t)(step % 3) * q.acc_stride + (size_t)kWinWords * w.sys;
     const bool drift = step > 0 || !q.forces_first;
@@ -631,6 +648,12 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       __threadfence();
     }
     if (threadIdx.x == 0) s_queue.next = 0;
+    // the part of the chain that needs no sums, by a warp that has no beads (in small systems)
+    if (wid == nw - 1) {
+      const unsigned int active = nhc_pre_warp(S, lane, chain_scratch);
+      if (lane == 0) s_active = active;
+    }
+    const unsigned int lcg = S.lcg;
     if (drift) {
       long long rx = 0, ry = 0, rz = 0;
       for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
@@ -640,9 +663,11 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
         long long Fx, Fy, Fz;
         get_fx(F, Fx, Fy, Fz);
         long long vx = s_v[t] - S.vcom_fx[0], vy = s_v[nmax + t] - S.vcom_fx[1], vz = s_v[2 * nmax + t] - S.vcom_fx[2];
-        if (bd) {
+        if (bd && drawn) {
+          brownian_drag(d, w.sys, g, l, vx, vy, vz);
+        } else if (bd) {
           long long r[3];
-          brownian_draws(d, P, S.lcg, w.sys, g, l, vx, vy, vz, r);
+          brownian_draws(d, P, lcg, w.sys, g, l, vx, vy, vz, r);
           rx += r[0];
           ry += r[1];
           rz += r[2];
@@ -666,7 +691,10 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
 #pragma unroll
         for (int k = 0; k < 9; k++) F[k] = 0u;
       }
-      if (bd) {
+      if (bd && drawn) {
+        if (threadIdx.x < 3) atomicAdd(acc + 8 + threadIdx.x, (unsigned long long)s_draw[threadIdx.x]);
+        __threadfence();
+      } else if (bd) {
         rx = warp_sum_ll(rx);
         ry = warp_sum_ll(ry);
         rz = warp_sum_ll(rz);
@@ -694,6 +722,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     });
     if (bd) {  // the step's random forces: their sum over the system
       if (threadIdx.x < 3) {
+        s_draw[threadIdx.x] = 0;  // (sent before this step's first wait)
         if (drift) {
           moved.wait(&s_abort);
           s_sum[4 + threadIdx.x] = (long long)__ldcg(acc + 8 + threadIdx.x);
@@ -749,8 +778,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
         const unsigned long long part = lane & 1 ? (unsigned long long)((x >> 32) + 2147483648ll) : (unsigned long long)(unsigned int)x;
         atomicAdd(acc + lane, (1ull << kSumCount) + part);
       }
-      __syncwarp();
-      chain_pre = nhc_pre_warp(S, lane, chain_scratch);  // while the other CTAs' sums arrive
+      chain_pre = s_active;
       unsigned long long v = 0;
       bool done = false;
       for (unsigned int i = 0; i < GridBarrier::kWindowPolls; i++) {
@@ -765,9 +793,26 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       v &= (1ull << kSumCount) - 1;
       const unsigned long long hi = __shfl_down_sync(0xffffffffu, v, 1) - ((unsigned long long)n_cta << 31);
       if (lane < 8 && !(lane & 1)) s_sum[lane >> 1] = (long long)(v + (hi << 32));
+    } else if (bd && step + 1 < q.steps) {
+      // Meanwhile the other warps draw the next step's random forces (this step's are used up), a
+      // component per thread: their FP64 operations took 8,000 cycles before each drift.
+      const unsigned int next = lcg_mul(lcg, P.lcg_step);
+      long long r[3] = {0, 0, 0};
+      for (int u = threadIdx.x - 32; u < 3 * nbead; u += blockDim.x - 32) {
+        const int k = u >= 2 * nbead ? 2 : u >= nbead ? 1 : 0, t = u - k * nbead;
+        const int l = t - fast_div(t, a.div_np) * np;
+        const long long f = brownian_draw(d, P, next, w.sys, bead0 + t, l, k);
+        if (k == 0) r[0] += f;
+        else if (k == 1) r[1] += f;
+        else r[2] += f;
+      }
+      const long long x = warp_sum4_ll(r[0], r[1], r[2], 0);
+      if (lane < 4 && warp_sum4_index(lane) < 3)
+        atomicAdd(reinterpret_cast<unsigned long long*>(s_draw + warp_sum4_index(lane)), (unsigned long long)x);
     }
     __syncthreads();
     if (s_abort) return;
+    drawn = bd && nw > 1 && step + 1 < q.steps;
     step_tail<false>(a, P, w.sys, S, s_sum, chain_scratch, chain_pre);
     __syncthreads();
     // the next kicks' coefficients: a thread's only bead's stays in its register
