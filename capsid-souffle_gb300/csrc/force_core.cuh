@@ -172,6 +172,17 @@ __device__ __forceinline__ void force_rel(const ForceSmem& m, int np, int s, int
   }
 }
 
+// Global index of an item's bead t, of its subunit s: a run of subunits, or subunits dealt to the CTAs
+// (first[s]: the subunit's first bead less s np).
+struct RunBeads {
+  int bead0;
+  __device__ __forceinline__ int operator()(int, int t) const { return bead0 + t; }
+};
+struct DealtBeads {
+  const int* first;
+  __device__ __forceinline__ int operator()(int s, int t) const { return first[s] + t; }
+};
+
 // What the warps of a CTA share: the position of the chunk queue and the numbers of pieces of the
 // inter-subunit lists.  Zero before force_rows.
 struct ForceQueue {
@@ -185,12 +196,14 @@ constexpr int kLongRow = 48;  // lists above this length are one piece, for a wh
 // bead | first pair / kPiece << 16 | pairs << 18.  Lists differ in length from bead to bead, and lanes
 // that share a chunk wait for its longest piece.  (Order does not matter: every sum is exact.)  The
 // caller's next barrier makes them visible.  thread: this thread's place among the CTA's.
-__device__ __forceinline__ void force_rows(const ForceArgs& a, const ForceSmem& m, int bead0, int nbead, int thread, ForceQueue* q) {
+template <class Beads>
+__device__ __forceinline__ void force_rows(const ForceArgs& a, const ForceSmem& m, const Beads& bead, int nbead, int thread,
+                                           ForceQueue* q) {
   const int lane = threadIdx.x & 31;
   const unsigned int below = (1u << lane) - 1u;
   for (int base = thread - lane; base < nbead; base += blockDim.x) {
     const int t = base + lane;
-    const int n = t < nbead ? __ldg(a.inter_count + bead0 + t) : 0;
+    const int n = t < nbead ? __ldg(a.inter_count + bead(fast_div(t, a.div_np), t)) : 0;
     if (!__any_sync(0xffffffffu, n > 0)) continue;
     const int cut = n <= kLongRow ? n : 0, rest = cut & (kPiece - 1);
     const int full = (cut + 7) / kPiece;  // pieces of 9 to 16 pairs
@@ -314,7 +327,8 @@ __device__ __forceinline__ void force_quad(const ForceArgs& a, const SysParams& 
 // Intra-subunit Debye-Hueckel row of bead t (same subunit: no LJ, src/forces.cpp:79-80): all
 // partners in order, the even and the odd ones in the two lanes of packed FP32 sums; both sums go
 // to the bead's limbs.
-__device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w, int t) {
+template <class Beads>
+__device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const Beads& bead, int t) {
   const TplLayout& L = a.L;
   const int np = L.np, npp = (np + 1) >> 1, words = L.words;
   const int s = fast_div(t, a.div_np), l = t - s * np;
@@ -325,7 +339,7 @@ __device__ __forceinline__ void force_intra(const ForceArgs& a, const SysParams&
   const float nx = -ri[0], ny = -ri[2], nz = -ri[4], wi = ri[6];
   const f32x2 nx2 = pack2(nx, nx), ny2 = pack2(ny, ny), nz2 = pack2(nz, nz), wi2 = pack2(wi, wi);
   f32x2 fx = 0, fy = 0, fz = 0;
-  const unsigned int* mrow = a.intra_mask + ((size_t)(w.sub_begin + s) * np + l) * words;
+  const unsigned int* mrow = a.intra_mask + (size_t)bead(s, t) * words;
   const float4* q = reinterpret_cast<const float4*>(rs);
   unsigned int next = __ldg(mrow);
   for (int wd = 0; wd < words; wd++) {
@@ -433,8 +447,8 @@ __device__ __forceinline__ float lj_add(float c, float r2, const float* pair, fl
 // 64 dense replicas (17,286 subunits) 222 -> 203 us.
 // kFresh: the partners' positions are rewritten by other CTAs while this kernel runs (read past L1).
 // wait: called once the first partners are known, before their positions are read.
-template <bool kFresh, int kLanes, class Wait>
-__device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, int bead0,
+template <bool kFresh, int kLanes, class Beads, class Wait>
+__device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams& P, const ForceSmem& m, int nbead, const Beads& bead,
                                             const ForceQueue& q, int chunk, Wait wait) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
@@ -459,15 +473,16 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
   }
   const int rec = valid ? m.rows[at] : 0;
   const int b = rec & 0xffff, n = rec >> 18;
-  const int* ids = a.inter_ids + (long long)(bead0 + b) * a.inter_cap + ((rec >> 16) & 3) * kPiece;
+  const int sub = fast_div(b, a.div_np), g = bead(sub, b);
+  const int* ids = a.inter_ids + (long long)g * a.inter_cap + ((rec >> 16) & 3) * kPiece;
   const int4 pi = m.pos[b];
-  const int l = b - fast_div(b, a.div_np) * L.np;
+  const int l = b - sub * L.np;
   const int si = species[l] * L.nspecies;
   const float wi = m.w[l];
   const f32x2 nk2 = pack2(-P.kappa, -P.kappa), kap2 = pack2(P.kappa, P.kappa), le2 = pack2(1.44269504f, 1.44269504f),
               wi2 = pack2(wi, wi);
   // (past the row's end: the bead itself, dropped below)
-  auto partner = [&](int i) { return i < n ? __ldg(ids + i) : bead0 + b; };
+  auto partner = [&](int i) { return i < n ? __ldg(ids + i) : g; };
   auto position = [&](int j) { return kFresh ? __ldcg(&a.pos32[j]) : __ldg(&a.pos32[j]); };
   int i = lane & (lanes - 1);
   int j0 = partner(i), j1 = partner(i + lanes);
@@ -543,9 +558,9 @@ __device__ __forceinline__ void force_inter(const ForceArgs& a, const SysParams&
 // pieces of inter-subunit lists, 64 edges (100).  kFresh (the window kernel): the inter-subunit
 // pairs come last, and a warp's first one only after wait() -- by then the other CTAs have
 // published their new positions while this one worked on its own subunits.
-template <bool kFresh, int kLanes, class Wait>
+template <bool kFresh, int kLanes, class Beads, class Wait>
 __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams& P, const ForceSmem& m, const WorkItem& w,
-                                            int nbead, int bead0, ForceQueue* q, Wait wait) {
+                                            int nbead, const Beads& bead, ForceQueue* q, Wait wait) {
   const TplLayout& L = a.L;
   const int lane = threadIdx.x & 31;
   const int nq = w.nsub * L.nbend, ne = w.nsub * L.ne;
@@ -565,7 +580,7 @@ __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams&
     if (k >= total) break;
     if (k >= first_intra && k < first_quad) {
       const int t = 32 * (k - first_intra) + lane;
-      if (t < nbead) force_intra(a, P, m, w, t);
+      if (t < nbead) force_intra(a, P, m, bead, t);
     } else if (k >= first_quad && k < first_quad + kq) {
       const int t = 32 * (k - first_quad) + lane;
       if (t < nq) force_quad(a, P, m, t);
@@ -575,7 +590,7 @@ __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams&
       if (t + 32 < ne) force_edge(a, P, m, t + 32);
     } else {
       // the long lists are the first kl of these chunks
-      force_inter<kFresh, kLanes>(a, P, m, nbead, bead0, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq, [&] {
+      force_inter<kFresh, kLanes>(a, P, m, nbead, bead, rows, kFresh ? k - first_edge - ke : k < kl ? k : k - ki - kq, [&] {
         if (!waited) wait();
         waited = true;
       });
@@ -586,14 +601,15 @@ __device__ __forceinline__ void force_terms(const ForceArgs& a, const SysParams&
 
 // Stretching and bending sums per bead, two threads per bead in different halves of the CTA, added
 // to the bead's limbs.
-__device__ __forceinline__ void force_gather(const ForceArgs& a, const ForceSmem& m, int nbead, int bead0) {
+template <class Beads>
+__device__ __forceinline__ void force_gather(const ForceArgs& a, const ForceSmem& m, int nbead, const Beads& bead) {
   const TplLayout& L = a.L;
   const int half = blockDim.x >> 1;
   const int h = (int)threadIdx.x >= half ? 1 : 0;
   const int* bead_edges = m.tpl_i + L.o_bead_edges;
   const int* bead_roles = m.tpl_i + L.o_bead_roles;
   for (int t = (int)threadIdx.x - h * half; t < nbead; t += half) {
-    const int s = fast_div(t, a.div_np), l = t - s * L.np, g = bead0 + t;
+    const int s = fast_div(t, a.div_np), l = t - s * L.np, g = bead(s, t);
     float3 f = f3(0.f, 0.f, 0.f);
     if (h == 0) {  // stretching, in the bead's edge order
       for (int k = 0; k < L.maxdeg; k++) {

@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(256, kRun ? 4 : 5) k_forces(ForceArgs a) {
     const int nbead = w.nsub * np;
     const int bead0 = w.sub_begin * np;  // global index of the first bead
     const float unit = P.unit32;
-    force_rows(a, m, bead0, nbead, fetch, &s_queue);
+    const RunBeads bead{bead0};
+    force_rows(a, m, bead, nbead, fetch, &s_queue);
     for (int t = fetch; t < nbead; t += blockDim.x) {
       const int4 p = a.pos32[bead0 + t];
       const int s = fast_div(t, a.div_np), l = t - s * np;
@@ -274,10 +275,10 @@ __global__ void __launch_bounds__(256, kRun ? 4 : 5) k_forces(ForceArgs a) {
       s_next = (int)(gridDim.x + v);
       if (s_next < a.n_items) s_work = a.work[s_next];
     }
-    force_terms<false, kRun ? 4 : 8>(a, P, m, w, nbead, bead0, &s_queue, [] {});
+    force_terms<false, kRun ? 4 : 8>(a, P, m, w, nbead, bead, &s_queue, [] {});
     __syncthreads();
     if (kRun && threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0, 0};
-    force_gather(a, m, nbead, bead0);
+    force_gather(a, m, nbead, bead);
     if (bb_filter) bigbead_mask(a, P, m.pos, m.rel, w.nsub, np, unit, s_bbm);
     __syncthreads();
 
@@ -509,6 +510,61 @@ __global__ void __launch_bounds__(256) k_drift(DriftArgs a) {
   }
 }
 
+// Deals a system's subunits to the window kernel's CTAs after a rebuild, so that crowded ones do not
+// meet: every CTA of a step waits for the one with the most inter-subunit pairs, and subunits differ
+// (2,000 of them, a tenth in contact: 94 pairs on average, 1,600 at most; runs of three: 3,150).  A
+// warp per subunit sums its list lengths; the last CTA sorts the subunits by them (counting sort, most
+// first) and deals them out in rounds, back and forth, the first round starting at the items with the
+// fewest places.  Any order gives the same bits.  100 steps 3,526 -> 3,192 us.
+__global__ void __launch_bounds__(1024) k_deal(DealArgs a) {
+  __shared__ int s_bin[kDealBins], s_warp[kDealBins / 32];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int sub = blockIdx.x * 32 + wid;
+  if (sub < a.n_sub) {
+    int n = 0;
+    for (int l = lane; l < a.np; l += 32) n += __ldg(a.inter_count + (size_t)sub * a.np + l);
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) a.key[sub] = kDealBins - 1 - min(n / kDealPairs, kDealBins - 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    if (s_last) *a.ticket = 0u;
+  }
+  if (threadIdx.x < kDealBins) s_bin[threadIdx.x] = 0;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int s = threadIdx.x; s < a.n_sub; s += blockDim.x) atomicAdd(&s_bin[__ldcg(a.key + s)], 1);
+  __syncthreads();
+  int mine = 0, incl = 0;
+  if (threadIdx.x < kDealBins) {
+    incl = mine = s_bin[threadIdx.x];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[wid] = incl;
+  }
+  __syncthreads();
+  if (threadIdx.x < kDealBins) {
+    int off = incl - mine;
+    for (int k = 0; k < wid; k++) off += s_warp[k];
+    s_bin[threadIdx.x] = off;
+  }
+  __syncthreads();
+  const int per = a.n_sub / a.items, more = a.n_sub - per * a.items;  // items of per + 1 subunits first
+  for (int s = threadIdx.x; s < a.n_sub; s += blockDim.x) {
+    const int rank = atomicAdd(&s_bin[__ldcg(a.key + s)], 1);
+    const int round = rank / a.items, k = rank - round * a.items;
+    const int item = round < per && !(round & 1) ? a.items - 1 - k : k;
+    a.deal[item * per + min(item, more) + round] = s;
+  }
+}
+
 // ---- the window kernel ------------------------------------------------------------------------
 // A run of MD or Brownian steps between two pair-list rebuilds in one launch, for handles whose
 // work items all fit the GPU at once (one CTA per item, cooperative launch).  The CTA keeps its
@@ -566,7 +622,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   const TplLayout& L = a.L;
   const WorkItem w = a.work[blockIdx.x];
   const SysParams& P = a.sys[w.sys];
-  const int np = L.np, nbead = w.nsub * np, bead0 = w.sub_begin * np;
+  const int np = L.np, nbead = w.nsub * np;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const ForceSmem m = force_smem(smem, a, nw);
   // behind the force kernel's shared memory: velocities, kick coefficients, the state, the low words of
@@ -578,6 +634,11 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   SysState& S = *reinterpret_cast<SysState*>(s_im + ((np + 1) & ~1));
   dfloat* chain_scratch = reinterpret_cast<dfloat*>(&S + 1);
   unsigned int* s_lo = reinterpret_cast<unsigned int*>(chain_scratch + 3 * kMaxChain);  // [3][nmax]
+  int* s_first = reinterpret_cast<int*>(s_lo + 3 * nmax);                               // [max_sub]
+  const auto bead = [&] {  // (wide grids are one subunit per item, or asked for: nothing to deal)
+    if constexpr (kWide) return RunBeads{w.sub_begin * np};
+    else return DealtBeads{s_first};
+  }();
   // (high words are rounded, so the low ones are signed offsets from them)
   auto whole = [](int hi, unsigned int lo) {
     return (long long)(((unsigned long long)(unsigned int)hi << 32) + (unsigned long long)(long long)(int)lo);
@@ -596,8 +657,10 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     s_abort = 0;
     s_queue = ForceQueue{0, 0, 0, 0};
   }
+  for (int s = threadIdx.x; !kWide && s < w.nsub; s += blockDim.x)
+    s_first[s] = ((q.deal ? q.deal[w.sub_begin + s] : w.sub_begin + s) - s) * np;
   __syncthreads();
-  force_rows(a, m, bead0, nbead, threadIdx.x, &s_queue);
+  force_rows(a, m, bead, nbead, threadIdx.x, &s_queue);
   force_setup(a, m);
   for (int t = threadIdx.x; t < np; t += blockDim.x) m.w[t] = __ldg(&a.dh_w[w.sys * np + t]);
   {
@@ -618,7 +681,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     inv_m = a.inv_mass[l];
   }
   for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-    const int g = bead0 + t;
+    const int g = bead(fast_div(t, a.div_np), t);
     const long long X = d.px[g], Y = d.py[g], Z = d.pz[g];
     s_lo[t] = (unsigned int)X;
     s_lo[nmax + t] = (unsigned int)Y;
@@ -657,7 +720,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     if (drift) {
       long long rx = 0, ry = 0, rz = 0;
       for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-        const int s = fast_div(t, a.div_np), l = t - s * np, g = bead0 + t;
+        const int s = fast_div(t, a.div_np), l = t - s * np, g = bead(s, t);
         const long long c = own_c ? my_c : s_kc[l], del = bd ? 0 : S.delta_fx;
         unsigned int* F = m.F + 9 * t;
         long long Fx, Fy, Fz;
@@ -714,7 +777,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       force_rel(m, np, s, l, m.pos[t], m.pos[s * np + P.center_local], m.w[l], unit);
     }
     __syncthreads();
-    force_terms<true, 8>(a, P, m, w, nbead, bead0, &s_queue, [&] {
+    force_terms<true, 8>(a, P, m, w, nbead, bead, &s_queue, [&] {
       if (drift) {
         if (lane == 0) moved.wait(&s_abort);
         __syncwarp();
@@ -734,11 +797,11 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     }
     __syncthreads();
     if (s_abort) return;  // uniform: nothing sets it between the barrier and here but a failed wait
-    force_gather(a, m, nbead, bead0);
+    force_gather(a, m, nbead, bead);
     __syncthreads();
     long long ke_acc = 0, px_acc = 0, py_acc = 0, pz_acc = 0;
     for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-      const int s = fast_div(t, a.div_np), l = t - s * np, g = bead0 + t;
+      const int s = fast_div(t, a.div_np), l = t - s * np, g = bead(s, t);
       unsigned int* F = m.F + 9 * t;
       long long Fx = limbs_value(F), Fy = limbs_value(F + 3), Fz = limbs_value(F + 6);
       if (bd) {
@@ -800,8 +863,8 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       long long r[3] = {0, 0, 0};
       for (int u = threadIdx.x - 32; u < 3 * nbead; u += blockDim.x - 32) {
         const int k = u >= 2 * nbead ? 2 : u >= nbead ? 1 : 0, t = u - k * nbead;
-        const int l = t - fast_div(t, a.div_np) * np;
-        const long long f = brownian_draw(d, P, next, w.sys, bead0 + t, l, k);
+        const int s = fast_div(t, a.div_np), l = t - s * np;
+        const long long f = brownian_draw(d, P, next, w.sys, bead(s, t), l, k);
         if (k == 0) r[0] += f;
         else if (k == 1) r[1] += f;
         else r[2] += f;
@@ -833,7 +896,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   }
   // results back to global memory
   for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
-    const int g = bead0 + t;
+    const int g = bead(fast_div(t, a.div_np), t);
     const int4 p = m.pos[t];
     d.px[g] = whole(p.x, s_lo[t]);
     d.py[g] = whole(p.y, s_lo[nmax + t]);
@@ -956,7 +1019,7 @@ void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s) {
 size_t window_smem_bytes(size_t force_bytes, int subs, int np) {
   const size_t vel = (3 * (size_t)subs * np + 1) & ~(size_t)1;
   return ((force_bytes + 15) & ~(size_t)15) + sizeof(long long) * (vel + 2 * (size_t)((np + 1) & ~1)) +
-         sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat) + 3 * sizeof(unsigned int) * (size_t)subs * np;
+         sizeof(SysState) + 3 * kMaxChain * sizeof(dfloat) + sizeof(unsigned int) * (3 * (size_t)subs * np + subs);
 }
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
                           cudaStream_t s) {
@@ -977,6 +1040,7 @@ cudaError_t window_wave_ctas(bool wide, int threads, size_t smem, int* ctas) {
   *ctas = per_sm * sms;
   return cudaSuccess;
 }
+void launch_deal(const DealArgs& a, cudaStream_t s) { k_deal<<<(a.n_sub + 31) / 32, 1024, 0, s>>>(a); }
 void launch_state_in(const StateArgs& a, int grid, int block, cudaStream_t s) {
   k_state_in<<<grid, block, 0, s>>>(a);
 }

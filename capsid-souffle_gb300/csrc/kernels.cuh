@@ -119,6 +119,17 @@ struct DriftArgs {
   long long n_total = 0;
 };
 
+// Subunits of one system dealt to work items by their inter-subunit pairs (k_deal).
+constexpr int kDealBins = 512, kDealPairs = 16;  // sorted by pairs / kDealPairs, up to 8,192
+struct DealArgs {
+  const int* inter_count;  // [n_sub np]
+  int n_sub, np, items;    // items of n_sub / items subunits, or one more in the first n_sub % items
+  int* key;                // [n_sub] scratch
+  unsigned int* ticket;    // zero between launches
+  int* deal;               // [n_sub] out: the subunit at each place of the items' run
+};
+void launch_deal(const DealArgs& a, cudaStream_t s);
+
 // The window kernel: steps per launch, its grid barrier and sums.
 struct WindowArgs {
   int wide;              // the 512-thread form (as window_wave_ctas was asked about)
@@ -128,6 +139,7 @@ struct WindowArgs {
   unsigned int* count;     // [1 + n_sys] CTAs that have left, then per system arrivals with new positions; zero between launches
   unsigned long long* acc; // [3][acc_stride]: per system 16 words (sums of kinetic energy, momentum, random forces), likewise
   size_t acc_stride;       // 16 n_sys
+  const int* deal;         // [S] the subunit at each place of the items (k_deal), or null: in order
   size_t force_bytes;      // the force kernel's part of the shared memory, 16-byte multiple
 };
 

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <numeric>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -535,6 +536,10 @@ size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
          sizeof(int) * force_rows_len(subs * np) + sizeof(float) * (np + L.n_float) + sizeof(int) * L.n_int;
 }
 
+DealArgs deal_args(souffle_gpu_system* h) {
+  return DealArgs{h->inter_count.p, h->S, h->tpl.np, (int)h->work.size(), h->deal_key.p, h->deal_ticket.p, h->deal.p};
+}
+
 // `len` steps in one launch; forces_first: the drift of the first one has been launched already
 cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_first) {
   WindowArgs q{};
@@ -545,6 +550,7 @@ cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_firs
   q.count = h->win_count.p;
   q.acc = h->win_acc.p;
   q.acc_stride = 16 * (size_t)h->n_sys;
+  q.deal = h->deal_ok ? h->deal.p : nullptr;
   q.force_bytes = (force_smem_for(h, h->subs_per_cta, h->window_threads) + 15) & ~(size_t)15;
   return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->window_threads, h->window_smem, h->stream);
 }
@@ -571,12 +577,14 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(false, threads, win_smem, &win_wave));
   std::vector<WorkItem> work;
   std::vector<int2> slots;
+  bool even_items = false;  // of floor or ceil(S / items) subunits, the longer ones first
   int sub0 = 0;
   for (int k = 0; k < h->n_sys; k++) {
     const int n = h->prm[k].n_subunits;
     const int first = (int)work.size();
     const int w0 = (n + subs - 1) / subs;
     if (h->n_sys == 1 && wave > w0) {
+      even_items = true;
       const int items = std::min(wave, n), q = n / items, r = n % items;
       for (int i = 0, b = 0; i < items; i++) {
         const int len = q + (i < r ? 1 : 0);
@@ -627,20 +635,22 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   h->window_ok = (int)h->work.size() <= win_wave;
   h->window_wide = false;
   h->window_threads = threads;
-  // Few enough items for two CTAs of 512 threads per SM (and no CTA shape asked for): the window
-  // kernel takes a warp per chunk of a subunit's work (rows, quads, edges and four beads' lists
-  // each), so that a crowded subunit, which all others wait for, is done sooner:
-  // 64 subunits 1,765 -> 1,645 us per 100 steps, 20 small ones 1,310 -> 1,240 (no spilled registers).
+  // Few enough items for CTAs of 64 registers (and no CTA shape asked for): the window kernel takes a warp
+  // per chunk of a subunit's work (rows, quads, edges and four beads' lists each), up to 512 threads and
+  // down to 256 as the items fit the GPU, so that a crowded subunit, which all others wait for, is done
+  // sooner: 64 subunits 1,765 -> 1,645 us per 100 steps, 20 small ones 1,310 -> 1,240 (no spilled
+  // registers), 333 Brownian ones 1,053 -> 970 per 50.
   if (h->window_ok && !h->opt.threads_per_cta) {
     const int np = h->tpl.np;
     int ns = 1;
     for (const WorkItem& w : h->work) ns = std::max(ns, w.nsub);
     const int chunks = (ns * np + 31) / 32 + (ns * h->L.nbend + 31) / 32 + (ns * h->L.ne + 31) / 32 + (ns * np + 3) / 4;
-    const int wide = std::min(512, std::max(128, 32 * chunks));
-    const size_t bytes = window_smem_bytes(force_smem_for(h, subs, wide), subs, np);
-    int wide_wave = 0;
-    if (bytes <= 227 * 1024) CUDA_TRY(window_wave_ctas(true, wide, bytes, &wide_wave));
-    if ((int)h->work.size() <= wide_wave) {
+    const int most = std::min(512, std::max(128, 32 * chunks));
+    for (int wide = most; wide >= std::min(most, 256) && !h->window_wide; wide -= 32) {
+      const size_t bytes = window_smem_bytes(force_smem_for(h, subs, wide), subs, np);
+      int wide_wave = 0;
+      if (bytes <= 227 * 1024) CUDA_TRY(window_wave_ctas(true, wide, bytes, &wide_wave));
+      if ((int)h->work.size() > wide_wave) continue;
       h->window_wide = true;
       h->window_threads = wide;
       win_smem = bytes;
@@ -652,6 +662,20 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
     CUDA_TRY(h->win_acc.alloc(48 * (size_t)h->n_sys));
     CUDA_TRY(cudaMemset(h->win_count.p, 0, sizeof(unsigned int) * h->win_count.n));
     CUDA_TRY(cudaMemset(h->win_acc.p, 0, sizeof(unsigned long long) * h->win_acc.n));
+  }
+  // one system cut into items of like length, some of them of several subunits: the window kernel takes
+  // the subunits in an order by cost (in order until the first rebuild)
+  h->deal_ok = h->window_ok && !h->window_wide && even_items && h->S > (int)h->work.size();
+  if (h->deal_ok) {
+    std::vector<int> order(h->S);
+    std::iota(order.begin(), order.end(), 0);
+    if (h->deal.n == 0) {
+      CUDA_TRY(h->deal.alloc(h->S));
+      CUDA_TRY(h->deal_key.alloc(h->S));
+      CUDA_TRY(h->deal_ticket.alloc(1));
+      CUDA_TRY(cudaMemset(h->deal_ticket.p, 0, sizeof(unsigned int)));
+    }
+    CUDA_TRY(cudaMemcpy(h->deal.p, order.data(), sizeof(int) * h->S, cudaMemcpyHostToDevice));
   }
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.second);
   h->graphs.clear();
@@ -1392,6 +1416,7 @@ souffle_status souffle_gpu_md_enqueue(souffle_gpu_system* h, int64_t first_step,
         if (rebuild_first) {
           launch_drift_all(h);
           launch_rebuild(h);
+          if (h->deal_ok) launch_deal(deal_args(h), h->stream);
         }
         launched = launch_window_steps(h, len, rebuild_first);
       } else {

@@ -60,6 +60,9 @@ struct souffle_gpu_system {
   DevBuf<unsigned int> win_count;
   DevBuf<unsigned int> force_ticket;  // force kernel: work items drawn
   DevBuf<unsigned long long> win_acc;
+  bool deal_ok = false;              // subunits are dealt to the window kernel's CTAs by their pairs
+  DevBuf<int> deal, deal_key;        // [S]
+  DevBuf<unsigned int> deal_ticket;
   int inter_cap = 96, cand_cap = 128;
   int force_grid = 1;  // CTAs of the force kernel: one wave at most
   size_t force_smem = 0, pair_smem = 0;

@@ -28,7 +28,8 @@ def result(s, n_sys):
     ("bilayer_n5", [3], {}, {"subunits_per_cta": 2, "threads_per_cta": 96}),   # an item of one, a partial warp half
     ("bilayer_n5", [64], {}, {}),
     ("bilayer_n5", [64], {}, {"subunits_per_cta": 8, "threads_per_cta": 256}),  # more beads than threads
-    ("bilayer_n5", [800], {}, {}),                                              # mixed items of one and two subunits
+    ("bilayer_n5", [400], {"D": "b", "d": 100.0}, {}), ("bilayer_n5", [600], {}, {}),   # 512, 320, 256 threads
+    ("bilayer_n5", [800], {}, {}), ("bilayer_n5", [1700], {}, {}),              # dealt subunits: items of one and two, two and three
     ("bilayer_n5", [5, 17, 2], {}, {}),                                         # systems of a batch, one grid barrier
     ("bilayer_n5", [33], {"D": "b", "d": 100.0}, {}),
     ("bilayer_n5", [9, 30], {"D": "b", "d": 100.0}, {}),
