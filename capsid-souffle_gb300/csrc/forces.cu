@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256, kRun ? 4 : 5) k_forces(ForceArgs a) {
     force_terms<false, kRun ? 4 : 8>(a, P, m, w, nbead, bead, &s_queue, [] {});
     __syncthreads();
     if (kRun && threadIdx.x == 0) s_queue = ForceQueue{0, 0, 0, 0};
-    force_gather(a, m, nbead, bead);
+    force_gather<1>(a, m, nbead, bead);
     if (bb_filter) bigbead_mask(a, P, m.pos, m.rel, w.nsub, np, unit, s_bbm);
     __syncthreads();
 
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
     }
     __syncthreads();
     if (s_abort) return;  // uniform: nothing sets it between the barrier and here but a failed wait
-    force_gather(a, m, nbead, bead);
+    force_gather<kWide ? 4 : 1>(a, m, nbead, bead);
     __syncthreads();
     long long ke_acc = 0, px_acc = 0, py_acc = 0, pz_acc = 0;
     for (int t = threadIdx.x; t < nbead; t += blockDim.x) {
