@@ -29,6 +29,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
+#include <memory>
 #include <string>
 
 #include "devbuf.cuh"
@@ -549,32 +551,47 @@ int g_sm_count(int dev) {
 
 }  // namespace
 
-// souffle_analysis_frames works on up to kFrameChunk frames between host waits: a frame's input is
-// copied into one of two slots on a stream of its own while the frame before it is analysed, and
-// the chunk's outputs come back in one copy per array.  Waiting for every frame, with five copies
-// each, took 206 us per frame of 86,000 beads; now 107 us, of which the kernels are 78 (105 with the
-// pair correlation in line with the contacts instead of beside them).
+// souffle_analysis_frames works on up to kFrameChunk frames between host waits, alternately in two lanes: a
+// lane has an input slot, workspaces and streams of its own, so a frame's input is copied and its small
+// kernels run beside those of the frame before, and the chunk's outputs come back in one copy per array.
+// Waiting for every frame, with five copies each, took 206 us per frame of 86,000 beads (105 us of it
+// kernels); one lane 130; two 125, of which the host copies of pageable input are most.
 constexpr int kFrameChunk = 8;
+constexpr size_t kChunkBytes = size_t(64) << 20;  // most output memory for more than one frame of a chunk
+
+struct AnLane {
+  cudaStream_t st = nullptr, pcf_st = nullptr;
+  cudaEvent_t copied = nullptr, prepared = nullptr, pcf_done = nullptr, done = nullptr;
+  DevBuf<double> pos;
+  DevBuf<int> types;
+  DevBuf<float4> posf, sph;
+  DevBuf<int> pcf_idx, parent_sub, parent_bead, size_sub, size_bead;
+  DevBuf<int2> cand;
+  DevBuf<unsigned int> cnt;
+  ~AnLane() {
+    if (st) cudaStreamSynchronize(st);
+    if (pcf_st) cudaStreamSynchronize(pcf_st);
+    for (cudaEvent_t v : {copied, prepared, pcf_done, done})
+      if (v) cudaEventDestroy(v);
+    if (pcf_st) cudaStreamDestroy(pcf_st);
+    if (st) cudaStreamDestroy(st);
+  }
+};
 
 struct souffle_analysis {
   int dev = 0;
   int sms = 1;
-  cudaStream_t st = nullptr, copy_st = nullptr, pcf_st = nullptr;
-  cudaEvent_t prepared = nullptr, pcf_done = nullptr;
-  cudaEvent_t copied[2] = {nullptr, nullptr}, done[2] = {nullptr, nullptr};
+  cudaStream_t copy_st = nullptr;
   AnParams P{};
-  DevBuf<double> pos[2];
-  DevBuf<int> types[2];
-  int types_slot = 0;                // slot of the last types given
-  DevBuf<float4> posf, sph;
-  DevBuf<int> pcf_idx, parent_sub, parent_bead, size_sub, size_bead, labels;
-  DevBuf<int2> cand;
-  DevBuf<unsigned int> cnt;
-  DevBuf<unsigned long long> gr, olig, so;  // [kFrameChunk] frames of outputs (labels too)
+  std::unique_ptr<AnLane> lane[2];
+  int lanes = 1, chunk = 1;          // lanes in use (the second from the first call with two frames), frames per chunk
+  int types_lane = 0;                // lane that holds the last types given
+  DevBuf<int> labels;
+  DevBuf<unsigned long long> gr, olig, so;  // [chunk] frames of outputs (labels too)
   unsigned int* cnt_host = nullptr;  // pinned copies of the counters, [kFrameChunk][C_COUNT]
   int cnt_last = 0;                  // the last enqueued frame's
   size_t contact_smem = 0;           // dynamic shared memory of k_an_contacts (two staged subunits per warp)
-  bool have_types = false;
+  bool have_types = false, no_second = false;
 };
 
 namespace {
@@ -594,25 +611,48 @@ souffle_status cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, #call);   \
   } while (0)
 
+cudaError_t alloc_lane(std::unique_ptr<AnLane>& lane, const AnParams& P) {
+  lane = std::make_unique<AnLane>();
+  AnLane& w = *lane;
+  const size_t N = (size_t)P.N, S = (size_t)P.S;
+  cudaError_t e = cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w.pcf_st, cudaStreamNonBlocking);
+  for (cudaEvent_t* v : {&w.copied, &w.prepared, &w.pcf_done, &w.done})
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = w.pos.alloc(3 * N);
+  if (e == cudaSuccess) e = w.types.alloc(N);
+  if (e == cudaSuccess) e = w.posf.alloc(N);
+  if (e == cudaSuccess) e = w.sph.alloc(S);
+  if (e == cudaSuccess) e = w.pcf_idx.alloc(N);
+  if (e == cudaSuccess) e = w.parent_sub.alloc(S);
+  if (e == cudaSuccess) e = w.parent_bead.alloc(N);
+  if (e == cudaSuccess) e = w.size_sub.alloc(S);
+  if (e == cudaSuccess) e = w.size_bead.alloc(N);
+  if (e == cudaSuccess) e = w.cand.alloc(P.cap);
+  if (e == cudaSuccess) e = w.cnt.alloc(C_COUNT);
+  return e;
+}
+
+// (every lane idle)
 souffle_status grow_candidates(souffle_analysis* h, long need) {
   const long cap = std::max<long>(2 * (long)h->P.cap, need + need / 4 + 1024);
   if (cap > (1L << 30)) return fail(SOUFFLE_ERR_NL_OVERFLOW, "analysis: more than 2^30 candidate subunit pairs");
-  AN_CHECK(h->cand.alloc(cap));
+  for (int k = 0; k < h->lanes; k++) AN_CHECK(h->lane[k]->cand.alloc(cap));
   h->P.cap = (int)cap;
   return SOUFFLE_OK;
 }
 
-souffle_status enqueue(souffle_analysis* h, const double* pos, const int* types, unsigned long long* gr,
+souffle_status enqueue(souffle_analysis* h, AnLane* w, const double* pos, const int* types, unsigned long long* gr,
                        unsigned long long* olig, unsigned long long* so, int* labels, int cnt_slot = 0) {
   const AnParams& P = h->P;
-  cudaStream_t st = h->st;
-  AN_CHECK(cudaMemsetAsync(h->cnt.p, 0, sizeof(unsigned int) * C_COUNT, st));
+  cudaStream_t st = w->st;
+  AN_CHECK(cudaMemsetAsync(w->cnt.p, 0, sizeof(unsigned int) * C_COUNT, st));
   const int nmax = std::max(P.N, P.S);
-  k_an_prep<<<(P.S + 7) / 8, 256, 0, st>>>(pos, types, P, h->posf.p, h->sph.p, h->parent_bead.p, h->size_bead.p,
-                                            h->parent_sub.p, h->size_sub.p, h->pcf_idx.p, gr, olig, so, h->cnt.p);
+  k_an_prep<<<(P.S + 7) / 8, 256, 0, st>>>(pos, types, P, w->posf.p, w->sph.p, w->parent_bead.p, w->size_bead.p,
+                                            w->parent_sub.p, w->size_sub.p, w->pcf_idx.p, gr, olig, so, w->cnt.p);
   // the pair correlation needs only the prepared frame, as the contacts do: the two run side by side
-  AN_CHECK(cudaEventRecord(h->prepared, st));
-  AN_CHECK(cudaStreamWaitEvent(h->pcf_st, h->prepared, 0));
+  AN_CHECK(cudaEventRecord(w->prepared, st));
+  AN_CHECK(cudaStreamWaitEvent(w->pcf_st, w->prepared, 0));
   const long Tp = (P.N + kPcfTile - 1) / kPcfTile;
   const int gpcf = (int)std::min<long>(Tp * (Tp + 1) / 2, 8L * h->sms);
   // the reference rule counts few pairs (those the long way round is short for), the minimum image
@@ -621,24 +661,24 @@ souffle_status enqueue(souffle_analysis* h, const double* pos, const int* types,
                               ? sizeof(unsigned short) * P.bins * kPcfTile
                               : sizeof(unsigned int) * (P.bins <= 512 ? kPcfTile / 32 : 1) * P.bins;
   if (P.image == SOUFFLE_IMAGE_REFERENCE)
-    k_an_pcf<SOUFFLE_IMAGE_REFERENCE><<<gpcf, kPcfTile, pcf_smem, h->pcf_st>>>(pos, h->posf.p, h->pcf_idx.p, P, gr, h->cnt.p);
+    k_an_pcf<SOUFFLE_IMAGE_REFERENCE><<<gpcf, kPcfTile, pcf_smem, w->pcf_st>>>(pos, w->posf.p, w->pcf_idx.p, P, gr, w->cnt.p);
   else
-    k_an_pcf<SOUFFLE_IMAGE_MINIMUM><<<gpcf, kPcfTile, pcf_smem, h->pcf_st>>>(pos, h->posf.p, h->pcf_idx.p, P, gr, h->cnt.p);
-  AN_CHECK(cudaEventRecord(h->pcf_done, h->pcf_st));
+    k_an_pcf<SOUFFLE_IMAGE_MINIMUM><<<gpcf, kPcfTile, pcf_smem, w->pcf_st>>>(pos, w->posf.p, w->pcf_idx.p, P, gr, w->cnt.p);
+  AN_CHECK(cudaEventRecord(w->pcf_done, w->pcf_st));
   const int cand_warps = (P.S + 1) / 2;
   const dim3 gcand((cand_warps + kCandWarps - 1) / kCandWarps, (P.S + kCandSeg - 1) / kCandSeg);
-  k_an_candidates<<<gcand, kCandWarps * 32, 0, st>>>(h->sph.p, P, h->cand.p, h->cnt.p);
+  k_an_candidates<<<gcand, kCandWarps * 32, 0, st>>>(w->sph.p, P, w->cand.p, w->cnt.p);
   const long items_max = (long)P.cap + P.S;
   const int gcon = (int)std::min<long>((items_max + kContactWarps - 1) / kContactWarps, 8L * h->sms);
-  k_an_contacts<<<gcon, kContactWarps * 32, h->contact_smem, st>>>(pos, h->posf.p, h->sph.p, h->cand.p, P,
-                                                                   h->parent_sub.p, h->parent_bead.p, h->cnt.p);
-  k_an_finish<<<(nmax + 255) / 256, 256, 0, st>>>(h->posf.p, P, h->parent_sub.p, h->parent_bead.p,
-                                                   h->size_sub.p, h->size_bead.p, labels);
-  k_an_hist<<<(nmax + 255) / 256, 256, 0, st>>>(h->posf.p, P, labels, h->size_sub.p, h->parent_bead.p,
-                                                 h->size_bead.p, olig, so, h->cnt.p);
+  k_an_contacts<<<gcon, kContactWarps * 32, h->contact_smem, st>>>(pos, w->posf.p, w->sph.p, w->cand.p, P,
+                                                                   w->parent_sub.p, w->parent_bead.p, w->cnt.p);
+  k_an_finish<<<(nmax + 255) / 256, 256, 0, st>>>(w->posf.p, P, w->parent_sub.p, w->parent_bead.p,
+                                                   w->size_sub.p, w->size_bead.p, labels);
+  k_an_hist<<<(nmax + 255) / 256, 256, 0, st>>>(w->posf.p, P, labels, w->size_sub.p, w->parent_bead.p,
+                                                 w->size_bead.p, olig, so, w->cnt.p);
   AN_CHECK(cudaGetLastError());
-  AN_CHECK(cudaStreamWaitEvent(st, h->pcf_done, 0));
-  AN_CHECK(cudaMemcpyAsync(h->cnt_host + cnt_slot * C_COUNT, h->cnt.p, sizeof(unsigned int) * C_COUNT, cudaMemcpyDeviceToHost, st));
+  AN_CHECK(cudaStreamWaitEvent(st, w->pcf_done, 0));
+  AN_CHECK(cudaMemcpyAsync(h->cnt_host + cnt_slot * C_COUNT, w->cnt.p, sizeof(unsigned int) * C_COUNT, cudaMemcpyDeviceToHost, st));
   h->cnt_last = cnt_slot;
   return SOUFFLE_OK;
 }
@@ -724,31 +764,15 @@ souffle_status souffle_analysis_create(int64_t n_beads, int32_t beads_per_subuni
   h->contact_smem = sizeof(float4) * 2 * kContactWarps * (size_t)P.np;
   cudaError_t e = cudaFuncSetAttribute(k_an_contacts, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)h->contact_smem);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
-  const size_t N = (size_t)P.N, S = (size_t)P.S;
+  const size_t S = (size_t)P.S;
+  const size_t frame_bytes = sizeof(unsigned long long) * (P.bins + 3 * S) + sizeof(int) * S;
+  h->chunk = (int)std::max<size_t>(1, std::min<size_t>(kFrameChunk, kChunkBytes / frame_bytes));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->copy_st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->pcf_st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->prepared, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->pcf_done, cudaEventDisableTiming);
-  for (int k = 0; k < 2; k++) {
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->copied[k], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->done[k], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = h->pos[k].alloc(3 * N);
-    if (e == cudaSuccess) e = h->types[k].alloc(N);
-  }
-  if (e == cudaSuccess) e = h->posf.alloc(N);
-  if (e == cudaSuccess) e = h->sph.alloc(S);
-  if (e == cudaSuccess) e = h->pcf_idx.alloc(N);
-  if (e == cudaSuccess) e = h->parent_sub.alloc(S);
-  if (e == cudaSuccess) e = h->parent_bead.alloc(N);
-  if (e == cudaSuccess) e = h->size_sub.alloc(S);
-  if (e == cudaSuccess) e = h->size_bead.alloc(N);
-  if (e == cudaSuccess) e = h->labels.alloc(kFrameChunk * S);
-  if (e == cudaSuccess) e = h->cand.alloc(P.cap);
-  if (e == cudaSuccess) e = h->cnt.alloc(C_COUNT);
-  if (e == cudaSuccess) e = h->gr.alloc(kFrameChunk * (size_t)P.bins);
-  if (e == cudaSuccess) e = h->olig.alloc(kFrameChunk * S);
-  if (e == cudaSuccess) e = h->so.alloc(kFrameChunk * 2 * S);
+  if (e == cudaSuccess) e = alloc_lane(h->lane[0], P);
+  if (e == cudaSuccess) e = h->labels.alloc(h->chunk * S);
+  if (e == cudaSuccess) e = h->gr.alloc(h->chunk * (size_t)P.bins);
+  if (e == cudaSuccess) e = h->olig.alloc(h->chunk * S);
+  if (e == cudaSuccess) e = h->so.alloc(h->chunk * 2 * S);
   if (e == cudaSuccess) e = cudaMallocHost(&h->cnt_host, sizeof(unsigned int) * C_COUNT * kFrameChunk);
   if (e != cudaSuccess) {
     souffle_analysis_destroy(h);
@@ -761,24 +785,15 @@ souffle_status souffle_analysis_create(int64_t n_beads, int32_t beads_per_subuni
 souffle_status souffle_analysis_destroy(souffle_analysis* h) {
   if (!h) return SOUFFLE_OK;
   cudaSetDevice(h->dev);
-  if (h->st) cudaStreamSynchronize(h->st);
   if (h->copy_st) cudaStreamSynchronize(h->copy_st);
-  if (h->pcf_st) cudaStreamSynchronize(h->pcf_st);
+  for (auto& w : h->lane) w.reset();
   if (h->cnt_host) cudaFreeHost(h->cnt_host);
-  for (int k = 0; k < 2; k++) {
-    if (h->copied[k]) cudaEventDestroy(h->copied[k]);
-    if (h->done[k]) cudaEventDestroy(h->done[k]);
-  }
-  if (h->prepared) cudaEventDestroy(h->prepared);
-  if (h->pcf_done) cudaEventDestroy(h->pcf_done);
-  if (h->pcf_st) cudaStreamDestroy(h->pcf_st);
   if (h->copy_st) cudaStreamDestroy(h->copy_st);
-  if (h->st) cudaStreamDestroy(h->st);
   delete h;
   return SOUFFLE_OK;
 }
 
-void* souffle_analysis_stream(souffle_analysis* h) { return h ? (void*)h->st : nullptr; }
+void* souffle_analysis_stream(souffle_analysis* h) { return h ? (void*)h->lane[0]->st : nullptr; }
 
 souffle_status souffle_analysis_enqueue(souffle_analysis* h, const double* pos_dev, const int32_t* types_dev,
                                         int64_t* pcf_dev, int64_t* oligomers_dev, int64_t* so_bins_dev,
@@ -786,7 +801,7 @@ souffle_status souffle_analysis_enqueue(souffle_analysis* h, const double* pos_d
   if (!h || !pos_dev || !types_dev || !pcf_dev || !oligomers_dev || !so_bins_dev)
     return fail(SOUFFLE_ERR_BAD_INPUT, "analysis_enqueue: NULL argument");
   AN_CHECK(cudaSetDevice(h->dev));
-  return enqueue(h, pos_dev, types_dev, reinterpret_cast<unsigned long long*>(pcf_dev),
+  return enqueue(h, h->lane[0].get(), pos_dev, types_dev, reinterpret_cast<unsigned long long*>(pcf_dev),
                  reinterpret_cast<unsigned long long*>(oligomers_dev),
                  reinterpret_cast<unsigned long long*>(so_bins_dev), labels_dev ? labels_dev : h->labels.p);
 }
@@ -794,7 +809,7 @@ souffle_status souffle_analysis_enqueue(souffle_analysis* h, const double* pos_d
 souffle_status souffle_analysis_synchronize(souffle_analysis* h) {
   if (!h) return fail(SOUFFLE_ERR_BAD_INPUT, "analysis_synchronize: NULL handle");
   AN_CHECK(cudaSetDevice(h->dev));
-  AN_CHECK(cudaStreamSynchronize(h->st));
+  AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
   const souffle_status s = frame_status(h, h->cnt_last);
   if (s == SOUFFLE_ERR_NL_OVERFLOW) {
     const souffle_status g = grow_candidates(h, h->cnt_host[h->cnt_last * C_COUNT + C_NCAND]);
@@ -812,71 +827,81 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
   AN_CHECK(cudaSetDevice(h->dev));
   const AnParams& P = h->P;
   const size_t N = (size_t)P.N, S = (size_t)P.S, bins = (size_t)P.bins;
-  // nothing enqueued earlier still reads the input slots
-  AN_CHECK(cudaStreamSynchronize(h->st));
-  // frame f's input into its slot, on the copy stream
-  auto copy_in = [&](int64_t f, int slot) -> souffle_status {
-    AN_CHECK(cudaMemcpyAsync(h->pos[slot].p, pos + 3 * N * f, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, h->copy_st));
-    if (types) {
-      AN_CHECK(cudaMemcpyAsync(h->types[slot].p, types + N * f, sizeof(int) * N, cudaMemcpyHostToDevice, h->copy_st));
-      h->have_types = true;
-      h->types_slot = slot;
+  // nothing enqueued earlier still reads the input or works in the lanes
+  AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
+  if (n_frames > 1 && h->chunk > 1 && h->lanes == 1 && !h->no_second) {
+    if (alloc_lane(h->lane[1], P) == cudaSuccess) {
+      h->lanes = 2;
+    } else {  // not enough memory: one lane
+      cudaGetLastError();
+      h->lane[1].reset();
+      h->no_second = true;
     }
-    AN_CHECK(cudaEventRecord(h->copied[slot], h->copy_st));
-    AN_CHECK(cudaStreamWaitEvent(h->st, h->copied[slot], 0));
+  }
+  // frame f's input into its lane, on the copy stream
+  auto copy_in = [&](int64_t f, int k) -> souffle_status {
+    AnLane& w = *h->lane[k];
+    AN_CHECK(cudaMemcpyAsync(w.pos.p, pos + 3 * N * f, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, h->copy_st));
+    if (types) {
+      AN_CHECK(cudaMemcpyAsync(w.types.p, types + N * f, sizeof(int) * N, cudaMemcpyHostToDevice, h->copy_st));
+      h->have_types = true;
+      h->types_lane = k;
+    }
+    AN_CHECK(cudaEventRecord(w.copied, h->copy_st));
+    AN_CHECK(cudaStreamWaitEvent(w.st, w.copied, 0));
     return SOUFFLE_OK;
   };
-  auto analyse = [&](int slot, int k) {
-    return enqueue(h, h->pos[slot].p, h->types[types ? slot : h->types_slot].p, h->gr.p + bins * k, h->olig.p + S * k,
-                   h->so.p + 2 * S * k, h->labels.p + S * k, k);
+  auto analyse = [&](int lane, int k) {
+    return enqueue(h, h->lane[lane].get(), h->lane[lane]->pos.p, h->lane[types ? lane : h->types_lane]->types.p, h->gr.p + bins * k,
+                   h->olig.p + S * k, h->so.p + 2 * S * k, h->labels.p + S * k, k);
   };
-  for (int64_t f0 = 0; f0 < n_frames; f0 += kFrameChunk) {
-    const int nf = (int)std::min<int64_t>(kFrameChunk, n_frames - f0);
+  auto drain = [&]() -> souffle_status {
+    for (int k = 0; k < h->lanes; k++) AN_CHECK(cudaStreamSynchronize(h->lane[k]->st));
+    return SOUFFLE_OK;
+  };
+  for (int64_t f0 = 0; f0 < n_frames; f0 += h->chunk) {
+    const int nf = (int)std::min<int64_t>(h->chunk, n_frames - f0);
     souffle_status s = SOUFFLE_OK;
     for (int k = 0; k < nf; k++) {
-      const int slot = k & 1;
-      // (the slot's last reader: two frames ago, or the chunk before, which has been waited for)
-      if (k >= 2) AN_CHECK(cudaStreamWaitEvent(h->copy_st, h->done[slot], 0));
-      if ((s = copy_in(f0 + k, slot)) != SOUFFLE_OK) return s;
-      if ((s = analyse(slot, k)) != SOUFFLE_OK) return s;
-      AN_CHECK(cudaEventRecord(h->done[slot], h->st));
+      const int lane = k % h->lanes;
+      // (the input's last reader: the lane's last frame, or the chunk before, which has been waited for)
+      if (k >= h->lanes) AN_CHECK(cudaStreamWaitEvent(h->copy_st, h->lane[lane]->done, 0));
+      if ((s = copy_in(f0 + k, lane)) != SOUFFLE_OK) return s;
+      if ((s = analyse(lane, k)) != SOUFFLE_OK) return s;
+      AN_CHECK(cudaEventRecord(h->lane[lane]->done, h->lane[lane]->st));
     }
-    AN_CHECK(cudaStreamSynchronize(h->st));
-    const int last_types = h->types_slot;
+    if ((s = drain()) != SOUFFLE_OK) return s;
     int good = 0;  // frames analysed without an error: their results are returned whatever follows
-    for (int k = 0; k < nf; k++) {
-      s = frame_status(h, k);
+    bool again = false;
+    for (; good < nf; good++) {
+      s = frame_status(h, good);
       // an overflowed candidate list is grown and its frame run again, by itself
       for (int attempt = 0; s == SOUFFLE_ERR_NL_OVERFLOW && attempt < 8; attempt++) {
-        if ((s = grow_candidates(h, h->cnt_host[k * C_COUNT + C_NCAND])) != SOUFFLE_OK) break;
-        // into the slot that does not hold the chunk's last types
-        if ((s = copy_in(f0 + k, k == nf - 1 ? last_types : 1 - last_types)) != SOUFFLE_OK) return s;
-        if ((s = analyse(k == nf - 1 ? last_types : 1 - last_types, k)) != SOUFFLE_OK) return s;
-        AN_CHECK(cudaStreamSynchronize(h->st));
-        s = frame_status(h, k);
+        if ((s = grow_candidates(h, h->cnt_host[good * C_COUNT + C_NCAND])) != SOUFFLE_OK) break;
+        again = true;
+        if ((s = copy_in(f0 + good, 0)) != SOUFFLE_OK) return s;
+        if ((s = analyse(0, good)) != SOUFFLE_OK) return s;
+        if ((s = drain()) != SOUFFLE_OK) return s;
+        s = frame_status(h, good);
       }
-      if (s != SOUFFLE_OK) {  // a call without types after this one sees the failed frame's
-        AN_CHECK(cudaStreamSynchronize(h->st));
-        const souffle_status c = copy_in(f0 + k, 0);
-        if (c != SOUFFLE_OK) return c;
-        h->cnt_last = k;
-        break;
-      }
-      good++;
+      if (s != SOUFFLE_OK) break;
     }
-    if (s == SOUFFLE_OK) {
-      h->types_slot = last_types;
-      h->cnt_last = nf - 1;
+    // a call without types after this one sees the last frame's, or the failed one's
+    h->cnt_last = std::min(good, nf - 1);
+    if (again || s != SOUFFLE_OK) {
+      const souffle_status c = copy_in(f0 + h->cnt_last, 0);
+      if (c != SOUFFLE_OK) return c;
     }
+    cudaStream_t st = h->lane[0]->st;
     if (pcf)
-      AN_CHECK(cudaMemcpyAsync(pcf + bins * f0, h->gr.p, sizeof(int64_t) * bins * good, cudaMemcpyDeviceToHost, h->st));
+      AN_CHECK(cudaMemcpyAsync(pcf + bins * f0, h->gr.p, sizeof(int64_t) * bins * good, cudaMemcpyDeviceToHost, st));
     if (oligomers)
-      AN_CHECK(cudaMemcpyAsync(oligomers + S * f0, h->olig.p, sizeof(int64_t) * S * good, cudaMemcpyDeviceToHost, h->st));
+      AN_CHECK(cudaMemcpyAsync(oligomers + S * f0, h->olig.p, sizeof(int64_t) * S * good, cudaMemcpyDeviceToHost, st));
     if (so_bins)
-      AN_CHECK(cudaMemcpyAsync(so_bins + 2 * S * f0, h->so.p, sizeof(int64_t) * 2 * S * good, cudaMemcpyDeviceToHost, h->st));
+      AN_CHECK(cudaMemcpyAsync(so_bins + 2 * S * f0, h->so.p, sizeof(int64_t) * 2 * S * good, cudaMemcpyDeviceToHost, st));
     if (labels)
-      AN_CHECK(cudaMemcpyAsync(labels + S * f0, h->labels.p, sizeof(int32_t) * S * good, cudaMemcpyDeviceToHost, h->st));
-    AN_CHECK(cudaStreamSynchronize(h->st));
+      AN_CHECK(cudaMemcpyAsync(labels + S * f0, h->labels.p, sizeof(int32_t) * S * good, cudaMemcpyDeviceToHost, st));
+    AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
     if (s != SOUFFLE_OK) return s;
   }
   return SOUFFLE_OK;
@@ -885,7 +910,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
 souffle_status souffle_analysis_last_counts(souffle_analysis* h, int64_t* candidate_pairs, int64_t* fp64_pairs) {
   if (!h) return fail(SOUFFLE_ERR_BAD_INPUT, "analysis_last_counts: NULL handle");
   AN_CHECK(cudaSetDevice(h->dev));
-  AN_CHECK(cudaStreamSynchronize(h->st));
+  AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
   if (candidate_pairs) *candidate_pairs = h->cnt_host[h->cnt_last * C_COUNT + C_NCAND];
   if (fp64_pairs) *fp64_pairs = h->cnt_host[h->cnt_last * C_COUNT + C_FP64];
   return SOUFFLE_OK;
