@@ -89,6 +89,31 @@ __device__ __forceinline__ double inv_sqrt(double r2, float r2f) {
 // a difference of fixed-point coordinates in FP32 from its high word (within L / 2^32)
 __device__ __forceinline__ float diff_f(long long d, float unit) { return (float)(int)(d >> 32) * unit; }
 
+// dx^2 + dy^2 + dz^2 of fixed-point differences, in their units: the 128-bit integer sum, rounded once to
+// FP64 by shifting its leading bits into place.  About 70 integer instructions, which this FP64-bound
+// code has to spare, for nine FP64 ones (three of them conversions).
+__device__ __forceinline__ double fixed_r2(const long long* d) {
+  unsigned long long hi = 0, lo = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const unsigned long long u = d[k] < 0 ? 0ull - (unsigned long long)d[k] : (unsigned long long)d[k];
+    const unsigned long long l = u * u;
+    lo += l;
+    hi += __umul64hi(u, u) + (lo < l ? 1 : 0);
+  }
+  int s = __clzll((long long)hi);
+  if (hi == 0) {
+    hi = lo;
+    lo = 0;
+    s = 64 + __clzll((long long)hi);
+    if (hi == 0) return 0.0;
+  }
+  const int n = s & 63;
+  const unsigned long long m = n ? hi << n | lo >> (64 - n) : hi;  // leading bit 63, worth 2^(127 - s)
+  const unsigned long long r = (m >> 11) + (m >> 10 & 1);          // 53 bits, the leading one at 52 (53 when rounding carries)
+  return __longlong_as_double((long long)(((unsigned long long)(1022 + 127 - s) << 52) + r));
+}
+
 // The screened Coulomb term e^(-kappa r) / r minus its value at the cut-off, 0 beyond the cut-off,
 // from exact fixed-point differences.  The cut-off is decided in FP32 except within a margin of it.
 struct PairCut {
@@ -109,10 +134,7 @@ struct PairCut {
     const float x = diff_f(d[0], unit), y = diff_f(d[1], unit), z = diff_f(d[2], unit);
     return x * x + y * y + z * z;
   }
-  __device__ __forceinline__ double r2(const long long* d) const {
-    const double x = (double)d[0], y = (double)d[1], z = (double)d[2];
-    return (x * x + y * y + z * z) * fx2;
-  }
+  __device__ __forceinline__ double r2(const long long* d) const { return fixed_r2(d) * fx2; }
   __device__ __forceinline__ double term_r(double r, double ir, float f, const double* tab) const {
     const double e = kappa_f * sqrtf(f) < kExpMaxArg ? exp_rc(r, c, tab) : 0.0;
     const double v = fma(e, ir, -shift);
@@ -133,7 +155,8 @@ struct PairCut {
 // are nearly all within the cut-off, so they are walked densely: rows p and np - 1 - p together
 // have np - 1 partners j > i, and two threads share such a pair of rows (even and odd partners),
 // which keeps every lane of the FP64 loop busy.  At 84,000 beads (2000 x 42)
-// 142 us, 83 % of the FP64 pipe while a CTA is resident; one thread per bead over every edge and quad
+// 115 us, 80 % of the FP64 pipe while a CTA is resident (142 with separations formed in FP64: fixed_r2);
+// one thread per bead over every edge and quad
 // that touches it took 203 us for the bonded terms alone, the former pair kernel 1786.
 __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
   extern __shared__ __align__(16) unsigned char esm[];
@@ -166,9 +189,8 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
     d[1] = fixed_diff(sy[i], sy[j], fx);
     d[2] = fixed_diff(sz[i], sz[j], fx);
   };
-  // |v| to within a rounding: r2 times the inverse root, then one correction by the residual
-  auto length = [](const double* v) {
-    const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+  // the root of r2 to within a rounding: r2 times the inverse root, then one correction by the residual
+  auto length = [](double r2) {
     const float r2f = (float)r2;
     if (!(r2f >= 0.01f && r2f < 1e30f)) return sqrt(r2);
     const double ir = inv_sqrt(r2, r2f), r = r2 * ir;
@@ -176,9 +198,9 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
   };
   for (int t = threadIdx.x; t < nsub * ne; t += blockDim.x) {
     const int s = t / ne, e = t - s * ne, pk = a.tpl_i[L.o_edge + e];
-    double d[3];
-    diff(s * np + (pk & 0xffff), s * np + (pk >> 16), d);
-    const double x = a.len0[e] - length(d);
+    const int i = s * np + (pk & 0xffff), j = s * np + (pk >> 16);
+    const long long d[3] = {sx[i] - sx[j], sy[i] - sy[j], sz[i] - sz[j]};
+    const double x = a.len0[e] - length(fixed_r2(d) * (fx * fx));
     s_edge[t] = 0.25 * P.ks_d * x * x;
   }
   for (int t = threadIdx.x; t < nsub * L.nf; t += blockDim.x) {  // area vectors 1/2 (b1 - b0) x (b2 - b1)
@@ -190,7 +212,7 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
     const double A[3] = {0.5 * (u[1] * v[2] - u[2] * v[1]), 0.5 * (u[2] * v[0] - u[0] * v[2]),
                          0.5 * (u[0] * v[1] - u[1] * v[0])};
     for (int k = 0; k < 3; k++) s_face[4 * t + k] = A[k];
-    s_face[4 * t + 3] = length(A);
+    s_face[4 * t + 3] = length(A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
   }
   __syncthreads();
   for (int t = threadIdx.x; t < nsub * nb; t += blockDim.x) {
@@ -330,7 +352,7 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
 // are listed row by row, and the FP64 terms run 128 listed pairs at a time, each row's terms then
 // summed with a fixed tree: deterministic.  Few pairs (147,000 at 84,000 beads) behind long
 // chains of loads and FP64 latency, the longest in subunits with several contacts: one warp per
-// subunit took 257 us there, four warps with a queue each 157, a CTA per subunit 68, two CTAs 63 (four: 75).
+// subunit took 257 us there, four warps with a queue each 157, a CTA per subunit 68, two CTAs 63 (four: 75); 60 with fixed_r2.
 constexpr int kEnergyCand = 1280;    // candidate subunits held per CTA
 constexpr int kEnergyScan = 16384;   // subunits up to which all are scanned
 constexpr int kScanBatch = 8;        // subunits per thread and round of the scan
