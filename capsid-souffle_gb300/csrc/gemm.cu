@@ -319,23 +319,6 @@ bool make_map(CUtensorMap* m, const void* p, int rows, int cols, int ld, int box
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A launch whose set-up (tensor memory, barriers, descriptors) may overlap the end of the kernel
-// before it; every kernel launched so calls pdl_wait before it touches global memory.
-template <class... P, class... A>
-cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
-}
-
 template <int BN, int ACT>
 cudaError_t launch(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const GemmEpi& e, cudaStream_t st) {
   using G = GemmTile<BN>;

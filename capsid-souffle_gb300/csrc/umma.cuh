@@ -3,6 +3,7 @@
 // TMEM), tcgen05.commit and tcgen05.ld.  Every wait is bounded: after kMaxPolls unsuccessful
 // try_wait calls it reports failure, and the caller raises an error flag instead of hanging.
 #pragma once
+#include "launch.cuh"
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -29,12 +30,6 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(ok));
   return ok != 0;
 }
-
-// Programmatic dependent launch: pdl_wait blocks until the kernels that this one depends on have
-// completed (at once without the launch attribute); pdl_launch lets the next one start its own
-// set-up.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
