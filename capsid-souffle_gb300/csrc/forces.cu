@@ -13,7 +13,7 @@
 // sums are combined in 64-bit fixed point (2^-32 units), so the total does not depend on summation
 // order.  In MD mode the kernel applies the second half-kick
 // (src/bead.h:113-117, src/md.cpp:450-455) in integer arithmetic, reduces kinetic energy and
-// momentum exactly (int64), and the last CTA of each system runs the Nose-Hoover chain
+// momentum exactly (int64), and the last CTA of each system (or k_step_end) runs the Nose-Hoover chain
 // (src/md.cpp:456-460, 401-406; src/functions.cpp:33-58) and the centre-of-mass velocity
 // (src/md.cpp:505-514).  No FP64 instruction runs per bead: GB300's FP64 rate is a small
 // fraction of its FP32 rate, so velocities, forces and positions are 64-bit fixed point and
@@ -583,18 +583,18 @@ __global__ void __launch_bounds__(1024) k_deal(DealArgs a) {
 // work items all fit the GPU at once (one CTA per item, cooperative launch).  The CTA keeps its
 // beads' positions, velocities and forces, the template tables and the system's thermostat state
 // in shared memory; only the high words of the positions pass through global memory.  A step is
-//   drift      own beads; publish the new high words; arrive at the grid barrier
-//   terms      own subunits' rows, quads and edges, then (the barrier having long completed) the
+//   drift      own beads; publish the new high words and count the arrival
+//   terms      own subunits' rows, quads and edges, then (the others having long arrived) the
 //              inter-subunit pairs
-//   finish     totals, second half kick, kinetic energy and momentum; arrive at the grid barrier
-//              with the sums; every CTA runs the thermostat chain itself, which costs the same
+//   finish     totals, second half kick, kinetic energy and momentum; send the sums and wait for
+//              the others'; every CTA runs the thermostat chain itself, which costs the same
 //              3 us once per SM instead of in one CTA, and saves handing its result around
 // The same operations as k_drift and k_forces, so the results are the same bits.  What it removes
 // is latency, which is all a small system's step consists of: two launches per step, the reload of
 // tables, state and tile (about 3 us), and the serial hand-over to the last CTA.  Per step, rebuilds
-// included: 19.6 -> 11.9 us at 200 beads, 23.3 -> 14.7 at 2,688, 24.8 -> 16.8 at 13,986, 36.2 ->
-// 27.2 at 84,000.  What is left there: the chain (2.7 us), the two barriers (1.5 us) and the wait
-// for the CTA with the most pairs.
+// included and no subunits in contact: 19.6 -> 10.2 us at 200 beads, 23.3 -> 11.9 at 2,688, 24.8 ->
+// 14.5 at 13,986, 36.2 -> 25.6 at 84,000.  What is left there: the chain (2.7 us), the two waits (1.2
+// us) and, with subunits in contact, the wait for the CTA with the most pairs.
 // A step has two waits, both among the CTAs of one system.  The first (positions published) counts
 // arrivals behind a fence.  The second needs none: the sums themselves count.  A sum's 64 bits are
 // added as two words of 32 with 1 << kSumCount on top, so whoever reads as many counts as the system
