@@ -1007,19 +1007,26 @@ __global__ void k_state_out(StateArgs a) {
 }  // namespace souffle
 
 namespace souffle {
-// The kernels of a step start while the one before them ends: the force kernel loads its tables, k_step_end
-// the state and the part of the chain that needs no sums (840,000 beads 7,369 -> 7,143 us per 40 steps, 64
-// replicas 5,586 -> 5,504 per 20).
+// Where CTAs draw items, the kernels of a step start while the one before them ends: the force kernel loads
+// its tables, k_step_end the state and the part of the chain that needs no sums (840,000 beads 7,369 ->
+// 7,143 us per 40 steps, 64 replicas 5,586 -> 5,504 per 20).  A step of one wave of CTAs is 2 % slower
+// that way (84,000 beads, L2 flushed before each step: 44.6 against 43.6 us).
 void launch_forces(const ForceArgs& a, int n_sys, int grid, int block, size_t smem, cudaStream_t s) {
   if (grid == a.n_items) {
-    launch_pdl(a.chain64 ? k_forces<true, false> : k_forces<false, false>, grid, block, smem, s, a);
+    if (a.chain64)
+      k_forces<true, false><<<grid, block, smem, s>>>(a);
+    else
+      k_forces<false, false><<<grid, block, smem, s>>>(a);
     return;
   }
   launch_pdl(a.chain64 ? k_forces<true, true> : k_forces<false, true>, grid, block, smem, s, a);
   if (a.mode != 0) launch_pdl(a.chain64 ? k_step_end<true> : k_step_end<false>, n_sys, 64, 0, s, a);
 }
-void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s) {
-  launch_pdl(k_drift, grid, block, 0, s, a);
+void launch_drift(const DriftArgs& a, bool overlap, int grid, int block, cudaStream_t s) {
+  if (overlap)
+    launch_pdl(k_drift, grid, block, 0, s, a);
+  else
+    k_drift<<<grid, block, 0, s>>>(a);
 }
 // shared memory of k_window: the force kernel's, then per-bead state, kick coefficients, system state
 size_t window_smem_bytes(size_t force_bytes, int subs, int np) {

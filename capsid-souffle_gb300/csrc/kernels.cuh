@@ -228,7 +228,8 @@ int pair_chunk(int np, int words);
 size_t pair_smem_bytes(int np, int words, int chunk);
 // grid: at most a wave of CTAs; with fewer than a.n_items a second kernel ends the step of n_sys systems
 void launch_forces(const ForceArgs& a, int n_sys, int grid, int block, size_t smem, cudaStream_t s);
-void launch_drift(const DriftArgs& a, int grid, int block, cudaStream_t s);
+// overlap: after a force kernel whose CTAs drew items (see launch_forces)
+void launch_drift(const DriftArgs& a, bool overlap, int grid, int block, cudaStream_t s);
 size_t window_smem_bytes(size_t force_bytes, int subs, int np);
 cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowArgs& q, int grid, int block, size_t smem,
                           cudaStream_t s);

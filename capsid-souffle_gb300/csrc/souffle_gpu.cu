@@ -499,7 +499,7 @@ DriftArgs drift_args(souffle_gpu_system* h) {
 void launch_drift_all(souffle_gpu_system* h) {
   const DriftArgs a = drift_args(h);
   const int threads = a.inter_ids ? h->threads : std::min(h->threads, (h->subs_per_cta * h->tpl.np + 31) / 32 * 32);
-  launch_drift(a, (int)h->work.size(), threads, h->stream);
+  launch_drift(a, h->force_grid < (int)h->work.size(), (int)h->work.size(), threads, h->stream);
 }
 
 // k_forces, preceded by the surrogate's far-field forces when it is on
