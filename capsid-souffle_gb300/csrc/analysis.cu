@@ -34,6 +34,7 @@
 #include <string>
 
 #include "devbuf.cuh"
+#include "launch.cuh"
 #include "souffle_analysis.h"
 
 namespace souffle {
@@ -762,8 +763,7 @@ souffle_status souffle_analysis_create(int64_t n_beads, int32_t beads_per_subuni
   P.sph_margin = (float)(8 * tol + 1e-4);
   P.cap = std::max(4096, 32 * P.S);
   h->contact_smem = sizeof(float4) * 2 * kContactWarps * (size_t)P.np;
-  cudaError_t e = cudaFuncSetAttribute(k_an_contacts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)h->contact_smem);
+  cudaError_t e = souffle::raise_smem_limit((const void*)k_an_contacts, h->contact_smem);
   const size_t S = (size_t)P.S;
   const size_t frame_bytes = sizeof(unsigned long long) * (P.bins + 3 * S) + sizeof(int) * S;
   h->chunk = (int)std::max<size_t>(1, std::min<size_t>(kFrameChunk, kChunkBytes / frame_bytes));

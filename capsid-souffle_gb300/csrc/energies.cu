@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace souffle {
 
@@ -829,8 +830,7 @@ size_t energy_sub_smem(const TplLayout& L, int spc) {
   return (size_t)spc * L.np * 24 + sizeof(double) * ((size_t)spc * (L.ne + L.nbend + 4 * L.nf + 2 * L.np) + L.np + 64);
 }
 cudaError_t set_energy_smem(const TplLayout& L) {
-  return cudaFuncSetAttribute(k_energy_sub, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)energy_sub_smem(L, energy_sub_per_cta(L.np)));
+  return raise_smem_limit((const void*)k_energy_sub, energy_sub_smem(L, energy_sub_per_cta(L.np)));
 }
 bool energy_needs_cells(int n_sub) { return n_sub > kEnergyScan; }
 void launch_energies(const EnergyArgs& a, int n, cudaStream_t s) {

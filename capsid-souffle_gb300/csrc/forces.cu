@@ -1043,7 +1043,7 @@ cudaError_t launch_window(const ForceArgs& a, const DriftArgs& d, const WindowAr
 cudaError_t window_wave_ctas(bool wide, int threads, size_t smem, int* ctas) {
   *ctas = 0;
   const void* fn = wide ? (const void*)k_window<true> : (const void*)k_window<false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit(fn, smem);
   if (e != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess) return e;
   int per_sm = 0, dev = 0, sms = 0;
@@ -1065,7 +1065,7 @@ namespace {
 // default may be smaller, which splits a one-wave grid into two waves).
 template <class Kernel>
 cudaError_t set_force_smem(Kernel* fn, size_t smem, int threads, int regs_sm, int smem_sm) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit((const void*)fn, smem);
   if (e != cudaSuccess) return e;
   cudaFuncAttributes fa{};
   if ((e = cudaFuncGetAttributes(&fa, fn)) != cudaSuccess) return e;

@@ -1,7 +1,10 @@
-// Programmatic dependent launch: a kernel that starts while the one before it in the stream ends.
+// Launch helpers: programmatic dependent launch (a kernel that starts while the one before it in the
+// stream ends) and the functions' shared-memory limits.
 #pragma once
 #include <cuda_runtime.h>
 
+#include <map>
+#include <mutex>
 #include <utility>
 
 namespace souffle {
@@ -26,6 +29,23 @@ cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem, cudaSt
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+// Lets kernel fn be launched with `bytes` of dynamic shared memory.  The limit belongs to the function
+// on its device, for every handle of the process, and a launch above it is refused: it is only ever
+// raised, so that a handle that needs less leaves the launches of the others as they are.
+inline cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
+  static std::mutex lock;
+  static std::map<std::pair<const void*, int>, size_t> limits;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> hold(lock);
+  size_t& limit = limits[{fn, dev}];
+  if (bytes <= limit) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit = bytes;
+  return e;
 }
 
 }  // namespace souffle

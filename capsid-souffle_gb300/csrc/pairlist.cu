@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace souffle {
 
@@ -505,8 +506,7 @@ void launch_pairs(const PairArgs& a, int n_sub, bool search, cudaStream_t s) {
   else k_pairs<false><<<n_sub, a.np * a.words <= 96 ? 64 : 128, smem, s>>>(a);
 }
 cudaError_t set_pairs_smem(size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute(k_pairs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_pairs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = raise_smem_limit((const void*)k_pairs<true>, smem);
+  return e != cudaSuccess ? e : raise_smem_limit((const void*)k_pairs<false>, smem);
 }
 }  // namespace souffle
