@@ -57,6 +57,7 @@ __device__ __noinline__ float3 bigbead_force(const ForceArgs& a, const SysParams
         continue;
       }
       k += __ffs(m) - 1;
+      if (k >= P.nbb) break;
     }
     const float3 d = dvec(__ldg(&a.bb_pos32[P.bb0 + k]), pi, unit);
     const float r2 = dot3(d, d);
@@ -273,7 +274,8 @@ __global__ void __launch_bounds__(256, kRun ? 4 : 5) k_forces(ForceArgs a) {
     if (w.sys != sys)
       for (int l = fetch; l < np; l += blockDim.x) m.w[l] = __ldg(&a.dh_w[w.sys * np + l]);
     const bool bb_filter = P.nbb > 0 && P.nbb <= 32 * kBBWords && w.nsub <= 16;
-    if (bb_filter && threadIdx.x < 16 * kBBWords) s_bbm[threadIdx.x] = 0u;
+    if (bb_filter)  // (CTAs of 64 threads and items of 16 subunits: more words than threads)
+      for (int t = threadIdx.x; t < w.nsub * kBBWords; t += blockDim.x) s_bbm[t] = 0u;
     __syncthreads();
     if (w.sys != sys) {
       if (kRun && sys >= 0 && a.mode != 0) flush();

@@ -108,3 +108,25 @@ def test_bad_big_beads_are_rejected():
         s.set_big_beads(g["big_pos"] + 10 * float(g["box"]), 6.0, -78.0, 3.5)
     with pytest.raises(gpu.SouffleError):
         s.set_big_beads(g["big_pos"], 6.0, -78.0, 3.5, system=5)
+
+
+@pytest.mark.parametrize("threads,subs", [(64, 16), (96, 13), (96, 16), (256, 16)])
+def test_big_beads_in_items_of_many_subunits(threads, subs):
+    """CTAs with fewer threads than words of big-bead flags: bitwise the forces and steps of the
+    default shape.  A batch of two systems, whose items hold subunits_per_cta subunits."""
+    from souffle_gb300 import geometry, gpu, workloads
+    w = workloads.make(geometry.patch_n3(), 50, seed=5)
+    big = workloads.place_big_beads(w, 40, radius=1.0)
+    p = gpu.system_params(w.opt, w.derived, 50, w.center_local)
+    out = []
+    for kw in ({}, {"threads_per_cta": threads, "subunits_per_cta": subs}):
+        s = gpu.GpuSystem(w.template, [p, p], **kw)
+        s.set_state(np.concatenate([w.state.pos, w.state.pos]), np.concatenate([w.state.vel, w.state.vel]))
+        s.set_big_beads(big, 2.0, -20.0, 1.0, system=0)
+        s.set_big_beads(big[::-1][:33], 2.0, 30.0, 1.5, system=1)
+        f = s.forces(rebuild=True)
+        s.md_begin()
+        s.md_steps(0, 12)
+        out.append([f, *s.get_state()])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
