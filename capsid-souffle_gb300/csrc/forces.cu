@@ -604,20 +604,21 @@ __global__ void __launch_bounds__(1024) k_deal(DealArgs a) {
 // behind them, two: 20 subunits 1,256 -> 1,196 us per 100 steps, 333 Brownian ones 1,242 -> 1,172 per
 // 50).  A CTA without inter-subunit pairs does not wait at the first; it cannot get further than the
 // second, so arrivals of two steps never mix.
-constexpr int kSumCount = 50;     // up to 2^14 CTAs, sums of up to 2^18 32-bit words
+constexpr int kSumCount = 50;     // fewer than 2^14 CTAs (kWindowMaxCtas), sums of up to 2^18 32-bit words
 constexpr int kWinWords = 16;     // a system's words per step: 8 of sums, 3 of random forces
 struct GridBarrier {
   unsigned int* count;    // arrivals, zero between launches
   unsigned int* err;
+  unsigned int polls;     // tries of a wait before it gives up
   unsigned int target;    // arrivals that complete the barrier in progress
   // thread 0 of the CTA, after a CTA barrier behind the writes to publish
   __device__ __forceinline__ void arrive() const {
     __threadfence();
     atomicAdd(count, 1u);
   }
-  // any thread; false when the wait ran out (kWindowPolls tries, some seconds)
+  // any thread; false when the wait ran out
   __device__ __forceinline__ bool wait(volatile int* abort_flag) const {
-    for (unsigned int i = 0; i < kWindowPolls; i++) {
+    for (unsigned int i = 0; i < polls; i++) {
       unsigned int v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
       if ((int)(v - target) >= 0) return true;
@@ -627,7 +628,6 @@ struct GridBarrier {
     atomicOr(err, kErrWindow);
     return false;
   }
-  static constexpr unsigned int kWindowPolls = 1u << 22;
 };
 
 // kWide: 512 threads and 64 registers (two CTAs per SM) instead of 256 and 48, for grids that fit.
@@ -663,18 +663,20 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
   __shared__ long long s_draw[3];       // sums of the random forces drawn ahead
   __shared__ int s_abort;
   __shared__ long long s_sum[7];  // kinetic energy, momentum; Brownian: mean random force
-  GridBarrier moved{q.count + 1 + w.sys, a.err, 0u};  // positions published
+  GridBarrier moved{q.count + 1 + w.sys, a.err, q.polls, 0u};  // positions published
   const int n_cta = a.sys_slots[w.sys].y;             // CTAs of the system
   const bool first_cta = w.sub_begin == P.sub0;       // of them, the one with the first subunit
   const float unit = P.unit32;
   const bool bd = P.brownian;
   if (threadIdx.x == 0) {
-    s_abort = 0;
+    // a window queued behind one that gave up leaves at once: the counters stand where that one left them
+    s_abort = (*(volatile unsigned int*)a.err & kErrWindow) != 0;
     s_queue = ForceQueue{0, 0, 0, 0};
   }
   for (int s = threadIdx.x; !kWide && s < w.nsub; s += blockDim.x)
     s_first[s] = ((q.deal ? q.deal[w.sub_begin + s] : w.sub_begin + s) - s) * np;
   __syncthreads();
+  if (s_abort) return;
   force_rows(a, m, bead, nbead, threadIdx.x, &s_queue);
   force_setup(a, m);
   for (int t = threadIdx.x; t < np; t += blockDim.x) m.w[t] = __ldg(&a.dh_w[w.sys * np + t]);
@@ -859,7 +861,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
       chain_pre = s_active;
       unsigned long long v = 0;
       bool done = false;
-      for (unsigned int i = 0; i < GridBarrier::kWindowPolls; i++) {
+      for (unsigned int i = 0; i < q.polls; i++) {
         if (lane < 8) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(acc + lane) : "memory");
         done = __all_sync(0xffffffffu, lane >= 8 || (v >> kSumCount) == (unsigned long long)n_cta);
         if (done || ((i & 255u) == 255u && *(volatile int*)&s_abort)) break;

@@ -131,9 +131,12 @@ struct DealArgs {
 void launch_deal(const DealArgs& a, cudaStream_t s);
 
 // The window kernel: steps per launch, its grid barrier and sums.
+constexpr unsigned int kWindowPolls = 1u << 22;  // tries of a wait before it gives up, some seconds
+constexpr int kWindowMaxCtas = (1 << 14) - 1;    // what its sums can count
 struct WindowArgs {
   int wide;              // the 512-thread form (as window_wave_ctas was asked about)
   int steps;
+  unsigned int polls;      // kWindowPolls (a test's wait may run out sooner)
   int forces_first;        // the first step's drift has run (and the pair lists were rebuilt after it)
   int n_sys;
   unsigned int* count;     // [1 + n_sys] CTAs that have left, then per system arrivals with new positions; zero between launches

@@ -306,10 +306,13 @@ souffle_status check_err(souffle_gpu_system* h) {
   const unsigned int e = *h->err_host;
   if (e) {
     CUDA_TRY(cudaMemsetAsync(h->err.p, 0, sizeof(unsigned int), h->stream));
-    if (e & kErrWindow) {  // the counters stand where the launch gave up
+    if (e & kErrWindow) {
+      // the counters stand where the launch gave up, and the state is between two steps: part of the
+      // positions have moved, velocities and thermostat are those before the window
+      h->began = h->have_state = false;
       CUDA_TRY(cudaMemsetAsync(h->win_count.p, 0, sizeof(unsigned int) * h->win_count.n, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->win_acc.p, 0, sizeof(unsigned long long) * h->win_acc.n, h->stream));
-      return fail(SOUFFLE_ERR_CUDA, "window kernel: a bounded wait ran out");
+      return fail(SOUFFLE_ERR_CUDA, "window kernel: a bounded wait ran out; set the state again");
     }
     if (e & kErrNonFinite) return fail(SOUFFLE_ERR_NONFINITE, "non-finite force or kinetic energy");
     if (e & kErrInterOverflow)
@@ -544,6 +547,7 @@ DealArgs deal_args(souffle_gpu_system* h) {
 cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_first) {
   WindowArgs q{};
   q.steps = len;
+  q.polls = h->window_polls;
   q.wide = h->window_wide ? 1 : 0;
   q.forces_first = forces_first ? 1 : 0;
   q.n_sys = h->n_sys;
@@ -632,7 +636,7 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
   h->force_smem = smem;
   // more items than one wave of CTAs: the form whose CTAs draw items
   h->force_grid = (int)h->work.size() <= std::max(wave, run_wave) ? (int)h->work.size() : run_wave;
-  h->window_ok = (int)h->work.size() <= win_wave;
+  h->window_ok = (int)h->work.size() <= std::min(win_wave, kWindowMaxCtas);
   h->window_wide = false;
   h->window_threads = threads;
   // Few enough items for CTAs of 64 registers (and no CTA shape asked for): the window kernel takes a warp
@@ -1568,6 +1572,16 @@ souffle_status souffle_gpu_autotune(souffle_gpu_system* h, int32_t trials, souff
     out->candidates = (int)cand.size();
   }
   return SOUFFLE_OK;
+}
+
+// Not in the public header, for tests: sets how often a wait of the window kernel tries before it gives
+// up, and returns the CTAs of the handle's windows (0: its steps do not take windows; -1: no handle).
+int32_t souffle_gpu_window_polls(souffle_gpu_system* h, uint32_t polls) {
+  if (!h || cudaSetDevice(h->opt.device) != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess) return -1;
+  h->window_polls = polls;
+  for (auto& g : h->graphs) cudaGraphExecDestroy(g.second);  // captured arguments changed
+  h->graphs.clear();
+  return window_usable(h) ? (int32_t)h->work.size() : 0;
 }
 
 souffle_status souffle_gpu_synchronize(souffle_gpu_system* h) {

@@ -57,6 +57,7 @@ struct souffle_gpu_system {
   bool window_wide = false;
   int window_threads = 256;
   size_t window_smem = 0;
+  unsigned int window_polls = kWindowPolls;
   DevBuf<unsigned int> win_count;
   DevBuf<unsigned int> force_ticket;  // force kernel: work items drawn
   DevBuf<unsigned long long> win_acc;

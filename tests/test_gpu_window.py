@@ -47,3 +47,29 @@ def test_windows_equal_single_steps(template, subs, over, kw):
         a += n
         for x, y in zip(result(one, len(ws)), result(win, len(ws))):
             assert np.array_equal(x, y), (a, np.abs(x - y).max())
+
+
+@pytest.mark.parametrize("template,S,over", [("patch_n3", 20, {}), ("bilayer_n5", 800, {}), ("bilayer_n5", 33, {"D": "b", "d": 100.0})])
+def test_a_wait_that_runs_out_is_reported_and_the_state_has_to_be_set_again(template, S, over):
+    w = workloads.make(geometry.template_by_name(template), S, seed=12, **over)
+    good = handle([w])
+    good.md_steps(0, 30)
+    want = result(good, 1)
+    s = handle([w])
+    polls = s.lib.souffle_gpu_window_polls
+    polls.argtypes, polls.restype = [gpu.C.c_void_p, gpu.C.c_uint32], gpu.C.c_int32
+    assert polls(s.h, 0) > 0  # every wait gives up at its first look
+    s.md_enqueue(0, 30)       # the windows behind the failing one leave at once
+    with pytest.raises(gpu.SouffleError) as e:
+        s.synchronize()
+    assert e.value.code == 2 and "wait ran out" in str(e.value)
+    for call in (lambda: s.md_steps(30, 10), s.md_begin, s.get_state, s.energies, lambda: s.forces(rebuild=False)):
+        with pytest.raises(gpu.SouffleError) as e:
+            call()
+        assert e.value.code == 6  # no state
+    polls(s.h, 1 << 22)
+    s.set_state(w.state.pos, w.state.vel)
+    s.md_begin()
+    s.md_steps(0, 30)
+    for x, y in zip(want, result(s, 1)):
+        assert np.array_equal(x, y)
