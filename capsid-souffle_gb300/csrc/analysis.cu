@@ -684,6 +684,26 @@ souffle_status enqueue(souffle_analysis* h, AnLane* w, const double* pos, const 
   return SOUFFLE_OK;
 }
 
+// Waits for the copy stream and both streams of every lane; the first error.
+cudaError_t drain(souffle_analysis* h) {
+  cudaError_t e = cudaStreamSynchronize(h->copy_st);
+  for (int k = 0; k < h->lanes; k++)
+    for (cudaStream_t st : {h->lane[k]->st, h->lane[k]->pcf_st}) {
+      const cudaError_t q = cudaStreamSynchronize(st);
+      if (e == cudaSuccess) e = q;
+    }
+  return e;
+}
+
+// A call that leaves early leaves nothing behind: no copy still reads the caller's frames, no kernel
+// still writes buffers that the next call uses.
+struct DrainOnExit {
+  souffle_analysis* h;
+  ~DrainOnExit() {
+    if (h) drain(h);
+  }
+};
+
 // Status of the frame enqueued with this counter slot (call after the stream has drained).
 souffle_status frame_status(souffle_analysis* h, int cnt_slot) {
   const unsigned flags = h->cnt_host[cnt_slot * C_COUNT + C_FLAGS];
@@ -801,9 +821,12 @@ souffle_status souffle_analysis_enqueue(souffle_analysis* h, const double* pos_d
   if (!h || !pos_dev || !types_dev || !pcf_dev || !oligomers_dev || !so_bins_dev)
     return fail(SOUFFLE_ERR_BAD_INPUT, "analysis_enqueue: NULL argument");
   AN_CHECK(cudaSetDevice(h->dev));
-  return enqueue(h, h->lane[0].get(), pos_dev, types_dev, reinterpret_cast<unsigned long long*>(pcf_dev),
+  DrainOnExit guard{h};
+  const souffle_status s = enqueue(h, h->lane[0].get(), pos_dev, types_dev, reinterpret_cast<unsigned long long*>(pcf_dev),
                  reinterpret_cast<unsigned long long*>(oligomers_dev),
                  reinterpret_cast<unsigned long long*>(so_bins_dev), labels_dev ? labels_dev : h->labels.p);
+  if (s == SOUFFLE_OK) guard.h = nullptr;  // enqueued, not waited for
+  return s;
 }
 
 souffle_status souffle_analysis_synchronize(souffle_analysis* h) {
@@ -828,7 +851,8 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
   const AnParams& P = h->P;
   const size_t N = (size_t)P.N, S = (size_t)P.S, bins = (size_t)P.bins;
   // nothing enqueued earlier still reads the input or works in the lanes
-  AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
+  AN_CHECK(drain(h));
+  DrainOnExit guard{h};
   if (n_frames > 1 && h->chunk > 1 && h->lanes == 1 && !h->no_second) {
     if (alloc_lane(h->lane[1], P) == cudaSuccess) {
       h->lanes = 2;
@@ -855,10 +879,6 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
     return enqueue(h, h->lane[lane].get(), h->lane[lane]->pos.p, h->lane[types ? lane : h->types_lane]->types.p, h->gr.p + bins * k,
                    h->olig.p + S * k, h->so.p + 2 * S * k, h->labels.p + S * k, k);
   };
-  auto drain = [&]() -> souffle_status {
-    for (int k = 0; k < h->lanes; k++) AN_CHECK(cudaStreamSynchronize(h->lane[k]->st));
-    return SOUFFLE_OK;
-  };
   for (int64_t f0 = 0; f0 < n_frames; f0 += h->chunk) {
     const int nf = (int)std::min<int64_t>(h->chunk, n_frames - f0);
     souffle_status s = SOUFFLE_OK;
@@ -870,7 +890,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
       if ((s = analyse(lane, k)) != SOUFFLE_OK) return s;
       AN_CHECK(cudaEventRecord(h->lane[lane]->done, h->lane[lane]->st));
     }
-    if ((s = drain()) != SOUFFLE_OK) return s;
+    AN_CHECK(drain(h));
     int good = 0;  // frames analysed without an error: their results are returned whatever follows
     bool again = false;
     for (; good < nf; good++) {
@@ -881,7 +901,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
         again = true;
         if ((s = copy_in(f0 + good, 0)) != SOUFFLE_OK) return s;
         if ((s = analyse(0, good)) != SOUFFLE_OK) return s;
-        if ((s = drain()) != SOUFFLE_OK) return s;
+        AN_CHECK(drain(h));
         s = frame_status(h, good);
       }
       if (s != SOUFFLE_OK) break;
@@ -904,6 +924,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
     AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
     if (s != SOUFFLE_OK) return s;
   }
+  guard.h = nullptr;  // every chunk has been waited for
   return SOUFFLE_OK;
 }
 
