@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <set>
+#include <string>
 #include <vector>
 
 #include "souffle_analysis.h"
