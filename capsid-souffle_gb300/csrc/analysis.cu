@@ -634,13 +634,36 @@ cudaError_t alloc_lane(std::unique_ptr<AnLane>& lane, const AnParams& P) {
   return e;
 }
 
-// (every lane idle)
+// (every lane idle)  Without memory for both lanes' lists the second lane goes; without any for the first
+// one's, its list is as long as before, or empty: a list that is too short is found out and grown.
 souffle_status grow_candidates(souffle_analysis* h, long need) {
   const long cap = std::max<long>(2 * (long)h->P.cap, need + need / 4 + 1024);
   if (cap > (1L << 30)) return fail(SOUFFLE_ERR_NL_OVERFLOW, "analysis: more than 2^30 candidate subunit pairs");
-  for (int k = 0; k < h->lanes; k++) AN_CHECK(h->lane[k]->cand.alloc(cap));
-  h->P.cap = (int)cap;
-  return SOUFFLE_OK;
+  cudaError_t e = h->lane[0]->cand.alloc(cap);
+  if (h->lanes == 2 && (e != cudaSuccess || h->lane[1]->cand.alloc(cap) != cudaSuccess)) {
+    cudaGetLastError();
+    if (h->types_lane == 1) {
+      AN_CHECK(cudaMemcpyAsync(h->lane[0]->types.p, h->lane[1]->types.p, sizeof(int) * (size_t)h->P.N, cudaMemcpyDeviceToDevice,
+                               h->copy_st));
+      AN_CHECK(cudaStreamSynchronize(h->copy_st));
+      h->types_lane = 0;
+    }
+    h->lane[1].reset();
+    h->lanes = 1;
+    h->no_second = true;
+    if (e != cudaSuccess) e = h->lane[0]->cand.alloc(cap);
+  }
+  if (e == cudaSuccess) {
+    h->P.cap = (int)cap;
+    return SOUFFLE_OK;
+  }
+  cudaGetLastError();
+  if (h->lane[0]->cand.alloc(h->P.cap) != cudaSuccess) {
+    cudaGetLastError();
+    h->lane[0]->cand.free();
+    h->P.cap = 0;
+  }
+  return cuda_fail(e, "analysis: candidate list");
 }
 
 souffle_status enqueue(souffle_analysis* h, AnLane* w, const double* pos, const int* types, unsigned long long* gr,

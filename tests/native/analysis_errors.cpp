@@ -3,6 +3,8 @@
 // it to the next wait for it.
 //   drains    for every runtime call of souffle_analysis_frames and _enqueue in turn, that call fails: the
 //             function reports it and leaves no stream busy
+//   grows     the candidate list overflows and allocations fail while it is grown: kernels get lists as
+//             long as they are told, one lane is enough for the call to succeed, and later calls work
 // Prints what went wrong and returns the number of failures.
 #include <cuda_runtime.h>
 
@@ -10,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <set>
 #include <string>
 #include <vector>
@@ -22,6 +25,14 @@ void record_error(const std::string&) {}
 
 namespace {
 int g_fail_at = -1, g_calls = 0;     // the call that fails, calls so far
+int g_allocs = 0, g_fail_alloc = -1, g_fail_allocs = 0;  // allocations so far; from which on and how many fail
+int g_overflows = 0;                 // frames still to be reported as overflowing
+int g_short_lists = 0;               // launches with a list shorter than its capacity
+std::map<void*, size_t> g_sizes;     // device memory
+std::map<const void*, std::string>& kernels() {  // (filled before main)
+  static std::map<const void*, std::string> m;
+  return m;
+}
 std::set<void*> g_busy;              // streams with work
 cudaStream_t g_launch = nullptr;     // stream of the launch being configured
 bool fails() { return g_calls++ == g_fail_at; }
@@ -42,10 +53,13 @@ const char* cudaGetErrorString(cudaError_t) { return "an error"; }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
   if (fails()) return cudaErrorMemoryAllocation;
+  const int k = g_allocs++ - g_fail_alloc;
+  if (g_fail_alloc >= 0 && k >= 0 && k < g_fail_allocs) return cudaErrorMemoryAllocation;
   *p = calloc(1, n);
+  g_sizes[*p] = n;
   return cudaSuccess;
 }
-cudaError_t cudaFree(void* p) { return free(p), cudaSuccess; }
+cudaError_t cudaFree(void* p) { return g_sizes.erase(p), free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) { return *p = calloc(1, n), cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { return *p = calloc(1, n), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return free(p), cudaSuccess; }
@@ -65,9 +79,14 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s) {
   if (e == cudaSuccess) memset(p, v, n);
   return e;
 }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t st) {
   const cudaError_t e = on(st);
   if (e == cudaSuccess) memcpy(d, s, n);
+  if (kind == cudaMemcpyDeviceToHost && n == 16 && g_overflows > 0) {  // a frame's counters
+    static_cast<unsigned*>(d)[1] = 100000;
+    static_cast<unsigned*>(d)[3] = 1;
+    g_overflows--;
+  }
   return e;
 }
 // what the compiler's launch code calls
@@ -83,13 +102,22 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* fn) {
   *k = reinterpret_cast<cudaKernel_t>(const_cast<void*>(fn));
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t s) {
+struct Params {  // AnParams of csrc/analysis.cu
+  double d[4];
+  float f[9];
+  int N, np, S, bins, pcf_type, so_type, image, cap;
+};
+cudaError_t cudaLaunchKernel(const void* fn, dim3, dim3, void** args, size_t, cudaStream_t s) {
   g_busy.insert(s);
+  if (kernels()[fn].find("k_an_candidates") != std::string::npos) {  // (spheres, parameters, list, counters)
+    const int cap = static_cast<Params*>(args[1])->cap;
+    void* list = *static_cast<void**>(args[2]);
+    if (cap > 0 && (!g_sizes.count(list) || g_sizes[list] < 8 * (size_t)cap)) g_short_lists++;
+  }
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t s) {
-  g_busy.insert(s);
-  return cudaSuccess;
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void** args, size_t n, cudaStream_t s) {
+  return cudaLaunchKernel(reinterpret_cast<const void*>(k), g, b, args, n, s);
 }
 void** __cudaRegisterFatBinary(void*) {
   static void* h = nullptr;
@@ -97,7 +125,9 @@ void** __cudaRegisterFatBinary(void*) {
 }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char*, char*, const char*, int, void*, void*, void*, void*, int*) {}
+void __cudaRegisterFunction(void**, const char* fn, char*, const char* name, int, void*, void*, void*, void*, int*) {
+  kernels()[fn] = name;
+}
 }
 
 namespace {
@@ -138,6 +168,33 @@ int drains() {
     }
   return bad;
 }
+
+int grows() {
+  int bad = 0;
+  for (int fail = 0; fail < 6; fail++)       // the first, second, ... allocation of the call
+    for (const int count : {1, 2, 100}) {    // and the ones after it
+      souffle_analysis* h = create();
+      if (frames(h) != SOUFFLE_OK) exit(102);
+      g_overflows = 2;
+      g_allocs = 0;
+      g_fail_alloc = fail;
+      g_fail_allocs = count;
+      const souffle_status s = frames(h);
+      const int failed = g_allocs - fail;
+      g_fail_alloc = -1;
+      g_overflows = 0;
+      if (failed > 0 && count == 1 && s != SOUFFLE_OK && ++bad) printf("grow: one failure (%d) fails the call\n", fail);
+      if (failed > 0 && count == 100 && fail == 0 && s == SOUFFLE_OK && ++bad) printf("grow: no memory, and no error\n");
+      // types of the last frame, as a program goes on
+      if (souffle_analysis_frames(h, kFrames, g_pos.data(), nullptr, g_pcf.data(), nullptr, nullptr, nullptr) != SOUFFLE_OK &&
+          ++bad)
+        printf("grow: the call after a failure (%d, %d) fails\n", fail, count);
+      souffle_analysis_destroy(h);
+    }
+  if (g_short_lists && ++bad) printf("grow: %d launches with a list shorter than its capacity\n", g_short_lists);
+  if (!g_sizes.empty() && ++bad) printf("grow: %zu allocations left\n", g_sizes.size());
+  return bad;
+}
 }  // namespace
 
-int main() { return drains(); }
+int main(int argc, char** argv) { return argc > 1 && !strcmp(argv[1], "grows") ? grows() : drains(); }

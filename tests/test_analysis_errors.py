@@ -24,6 +24,7 @@ def checker(tmp_path_factory):
     return exe
 
 
-def test_a_failing_call_leaves_no_work_behind(checker):
-    r = subprocess.run([checker], capture_output=True, text=True, timeout=120)
+@pytest.mark.parametrize("what", ["drains", "grows"])
+def test_failing_calls_and_allocations(checker, what):
+    r = subprocess.run([checker, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
