@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
   long long* sz = sy + a.spc * np;
   double* s_edge = reinterpret_cast<double*>(sz + a.spc * np);  // [spc * ne]
   double* s_quad = s_edge + a.spc * ne;                         // [spc * nb]
-  double* s_face = s_quad + a.spc * nb;                         // [spc * nf][4] area vector, magnitude
-  double* s_part = s_face + 4 * a.spc * L.nf;                   // [2][spc * np]
+  double* s_face = s_quad + a.spc * nb;                         // [spc * nf][4] area vector, magnitude (a.faces)
+  double* s_part = s_face + (a.faces ? 4 * a.spc * L.nf : 0);   // [2][spc * np]
   double* s_w = s_part + 2 * a.spc * np;                        // [np]
   double* s_tab = s_w + np;                                     // [64]
   const int g0 = a.n0 + s0 * np;
@@ -204,17 +204,17 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
     const double x = a.len0[e] - length(fixed_r2(d) * (fx * fx));
     s_edge[t] = 0.25 * P.ks_d * x * x;
   }
-  for (int t = threadIdx.x; t < nsub * L.nf; t += blockDim.x) {  // area vectors 1/2 (b1 - b0) x (b2 - b1)
-    const int s = t / L.nf, f = t - s * L.nf;
+  auto area = [&](int s, int f, double* A) {  // area vector 1/2 (b1 - b0) x (b2 - b1) and its magnitude
     const int* fb = a.tpl_i + L.o_face + 3 * f;
     double u[3], v[3];
     diff(s * np + fb[1], s * np + fb[0], u);
     diff(s * np + fb[2], s * np + fb[1], v);
-    const double A[3] = {0.5 * (u[1] * v[2] - u[2] * v[1]), 0.5 * (u[2] * v[0] - u[0] * v[2]),
-                         0.5 * (u[0] * v[1] - u[1] * v[0])};
-    for (int k = 0; k < 3; k++) s_face[4 * t + k] = A[k];
-    s_face[4 * t + 3] = length(A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
-  }
+    A[0] = 0.5 * (u[1] * v[2] - u[2] * v[1]);
+    A[1] = 0.5 * (u[2] * v[0] - u[0] * v[2]);
+    A[2] = 0.5 * (u[0] * v[1] - u[1] * v[0]);
+    A[3] = length(A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
+  };
+  for (int t = threadIdx.x; a.faces && t < nsub * L.nf; t += blockDim.x) area(t / L.nf, t % L.nf, s_face + 4 * t);
   __syncthreads();
   for (int t = threadIdx.x; t < nsub * nb; t += blockDim.x) {
     const int s = t / nb, k = t - s * nb, base = s * np;
@@ -233,9 +233,18 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
       e = P.kb_d * 0.25 * (1.0 - cos(beta - beta0));
     } else {
       const int* bf = a.tpl_i + L.o_bendf + 2 * k;
-      const double* A = s_face + 4 * (s * L.nf + bf[0]);
-      const double* B = s_face + 4 * (s * L.nf + bf[1]);
-      const double c = (A[0] * B[0] + A[1] * B[1] + A[2] * B[2]) / (A[3] * B[3]);
+      auto cosine = [](const double* A, const double* B) {
+        return (A[0] * B[0] + A[1] * B[1] + A[2] * B[2]) / (A[3] * B[3]);
+      };
+      double c;
+      if (a.faces) {
+        c = cosine(s_face + 4 * (s * L.nf + bf[0]), s_face + 4 * (s * L.nf + bf[1]));
+      } else {
+        double A[4], B[4];
+        area(s, bf[0], A);
+        area(s, bf[1], B);
+        c = cosine(A, B);
+      }
       e = P.kb_d * 0.25 * (1.0 - fabs(c));
     }
     s_quad[t] = e;
@@ -823,21 +832,30 @@ __global__ void __launch_bounds__(kTotalThreads) k_energy_totals(EnergyArgs a, i
 }  // namespace souffle
 
 namespace souffle {
-// Subunits per CTA of k_energy_sub (two threads per pair of rows, up to 128 threads) and its
-// dynamic shared memory.
-int energy_sub_per_cta(int np) { return std::max(1, 128 / (2 * ((np + 1) / 2))); }
-size_t energy_sub_smem(const TplLayout& L, int spc) {
-  return (size_t)spc * L.np * 24 + sizeof(double) * ((size_t)spc * (L.ne + L.nbend + 4 * L.nf + 2 * L.np) + L.np + 64);
+// Subunits per CTA of k_energy_sub (two threads per pair of rows, up to 128 threads), whether it keeps the
+// faces' area vectors in shared memory, and its dynamic shared memory.  Templates with edges or faces
+// by the thousand take fewer subunits, then form area vectors for each bending quad: a mesh without
+// bending edges may have more faces than shared memory holds.
+static size_t energy_sub_bytes(const TplLayout& L, int spc, bool faces) {
+  return (size_t)spc * L.np * 24 +
+         sizeof(double) * ((size_t)spc * (L.ne + L.nbend + (faces ? 4 * (size_t)L.nf : 0) + 2 * L.np) + L.np + 64);
+}
+EnergySubPlan energy_sub_plan(const TplLayout& L) {
+  EnergySubPlan p{std::max(1, 128 / (2 * ((L.np + 1) / 2))), true, 0};
+  while (p.spc > 1 && energy_sub_bytes(L, p.spc, true) > kMaxDynamicSmem) p.spc--;
+  p.faces = energy_sub_bytes(L, p.spc, true) <= kMaxDynamicSmem;
+  p.smem = energy_sub_bytes(L, p.spc, p.faces);
+  return p;
 }
 cudaError_t set_energy_smem(const TplLayout& L) {
-  return raise_smem_limit((const void*)k_energy_sub, energy_sub_smem(L, energy_sub_per_cta(L.np)));
+  return raise_smem_limit((const void*)k_energy_sub, energy_sub_plan(L).smem);
 }
 bool energy_needs_cells(int n_sub) { return n_sub > kEnergyScan; }
 void launch_energies(const EnergyArgs& a, int n, cudaStream_t s) {
   const int np = a.L.np, nsub = n / np;
   const int per = 2 * ((np + 1) / 2);
   const int threads = std::max(64, (a.spc * per + 31) / 32 * 32);
-  k_energy_sub<<<(nsub + a.spc - 1) / a.spc, threads, energy_sub_smem(a.L, a.spc), s>>>(a);
+  k_energy_sub<<<(nsub + a.spc - 1) / a.spc, threads, energy_sub_plan(a.L).smem, s>>>(a);
   if (a.ecut_el > 0) {
     k_energy_inter<<<dim3(nsub, std::min(2, (np + 15) / 16)), 128, energy_inter_bytes(np), s>>>(a);
   } else {  // no DH cut-off: every pair j > i

@@ -197,6 +197,7 @@ struct EnergyArgs {
   double exp_scale;        // -kappa 64 / ln2
   double inv_ecut3;        // 1 / ecut^3
   int spc;                 // subunits per CTA of k_energy_sub
+  bool faces;              // ... which keeps the faces' area vectors in shared memory
   int4* sph;               // [subunits] centre bead (high words) and bounding radius (float bits)
   int* rmax;               // largest bounding radius (float bits), zero between calls
   double* partials;        // [kTotalCtas][7]
@@ -212,8 +213,12 @@ struct EnergyArgs {
   double* ne_bb = nullptr; double* ce_bb = nullptr;
 };
 constexpr int kTotalThreads = 256, kTotalCtas = 304;  // k_energy_totals: two CTAs per SM
-int energy_sub_per_cta(int np);
-size_t energy_sub_smem(const TplLayout& L, int spc);
+struct EnergySubPlan {
+  int spc;
+  bool faces;
+  size_t smem;
+};
+EnergySubPlan energy_sub_plan(const TplLayout& L);
 cudaError_t set_energy_smem(const TplLayout& L);
 bool energy_needs_cells(int n_sub);
 

@@ -19,6 +19,7 @@
 
 namespace souffle {
 
+constexpr size_t kMaxDynamicSmem = 226 * 1024;  // of a CTA: 227 KB less room for static shared memory
 constexpr int kMaxNp = 256;        // beads per subunit
 constexpr int kMaxChain = 16;      // Nose-Hoover chain links
 constexpr int kMaxInterPerBead = 2047;  // inter-subunit pairs of one bead (force-kernel limb sums

@@ -1263,7 +1263,9 @@ souffle_status souffle_gpu_energies(souffle_gpu_system* h, int32_t system, souff
   a.el_shift = p.ecut_el > 0 ? std::exp(-p.kappa * p.ecut_el) / p.ecut_el : 0.0;
   a.exp_scale = -p.kappa * (64.0 / 0.69314718055994530942);
   a.inv_ecut3 = 1.0 / (p.ecut * p.ecut * p.ecut);
-  a.spc = energy_sub_per_cta(h->tpl.np);
+  const EnergySubPlan sub_plan = energy_sub_plan(h->L);
+  a.spc = sub_plan.spc;
+  a.faces = sub_plan.faces;
   a.sph = h->e_sph.p;
   a.rmax = h->e_scr.p;
   a.ticket = reinterpret_cast<unsigned int*>(h->e_scr.p + 1);
