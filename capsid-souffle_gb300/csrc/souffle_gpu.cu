@@ -539,6 +539,19 @@ size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
          sizeof(int) * force_rows_len(subs * np) + sizeof(float) * (np + L.n_float) + sizeof(int) * L.n_int;
 }
 
+// Bytes that decide whether a CTA shape is accepted: bonded tile, 72 bytes per bead, reductions and the
+// template's tables.  (The kernels' own scratch on top is not counted: plan_work finds room for it.)
+bool force_shape_ok(const souffle_gpu_system* h, int subs, int threads) {
+  const TplLayout& L = h->L;
+  const int np = h->tpl.np;
+  auto up4 = [](int n) { return (n + 3) & ~3; };
+  const size_t bytes = force_tile_bytes(subs, L.ne, L.nbend) + 32 * (size_t)(subs * np) + 32 * (size_t)(threads / 32) +
+                       sizeof(unsigned int) * force_slot_len(subs * np) + sizeof(int) * up4(subs * np + 1) +
+                       sizeof(float) * (np + up4(L.ne + 3 * np + L.nbend)) +
+                       sizeof(int) * up4(L.ne + 3 * L.nf + 6 * L.nbend + np * (L.maxdeg + L.maxrole + 2));
+  return bytes <= 200 * 1024;
+}
+
 DealArgs deal_args(souffle_gpu_system* h) {
   return DealArgs{h->inter_count.p, h->S, h->tpl.np, (int)h->work.size(), h->deal_key.p, h->deal_ticket.p, h->deal.p};
 }
@@ -561,7 +574,8 @@ cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_firs
 
 // Work items of up to `subs` subunits of one system each (one force-kernel CTA per item, in
 // system order), their partial-sum slots, the force kernel's shared memory, and `threads` threads
-// per CTA.  Cached graphs are dropped (their launch shapes change).
+// per CTA.  Cached graphs are dropped (their launch shapes change).  Items of more subunits than the
+// force kernel's shared memory holds are cut smaller (the results do not depend on the shape).
 //
 // A single system whose items leave part of one wave of CTAs empty is cut into exactly as many
 // items as the wave holds (or one per subunit), of floor or ceil(S / items) subunits with the
@@ -570,15 +584,16 @@ cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_firs
 // equal items of `subs` subunits would leave some SMs with one CTA more than others (2000
 // subunits in 3-subunit items: 667 CTAs on 152 SMs, 4 or 5 per SM).
 souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
+  if (!force_shape_ok(h, subs, threads)) return fail(SOUFFLE_ERR_BAD_INPUT, "template too large for shared memory");
+  while (subs > 1 && force_smem_for(h, subs, threads) > kMaxDynamicSmem) subs--;
   const size_t smem = force_smem_for(h, subs, threads);
-  if (smem > 200 * 1024) return fail(SOUFFLE_ERR_BAD_INPUT, "template too large for shared memory");
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   CUDA_TRY(set_kernel_smem(smem, threads, h->pair_smem));
   int wave = 0, run_wave = 0, win_wave = 0;
   CUDA_TRY(force_wave_ctas(false, threads, smem, &wave));
   CUDA_TRY(force_wave_ctas(true, threads, smem, &run_wave));
   size_t win_smem = window_smem_bytes(smem, subs, h->tpl.np);
-  if (win_smem <= 227 * 1024) CUDA_TRY(window_wave_ctas(false, threads, win_smem, &win_wave));
+  if (win_smem <= kMaxDynamicSmem) CUDA_TRY(window_wave_ctas(false, threads, win_smem, &win_wave));
   std::vector<WorkItem> work;
   std::vector<int2> slots;
   bool even_items = false;  // of floor or ceil(S / items) subunits, the longer ones first
@@ -653,7 +668,7 @@ souffle_status plan_work(souffle_gpu_system* h, int subs, int threads) {
     for (int wide = most; wide >= std::min(most, 256) && !h->window_wide; wide -= 32) {
       const size_t bytes = window_smem_bytes(force_smem_for(h, subs, wide), subs, np);
       int wide_wave = 0;
-      if (bytes <= 227 * 1024) CUDA_TRY(window_wave_ctas(true, wide, bytes, &wide_wave));
+      if (bytes <= kMaxDynamicSmem) CUDA_TRY(window_wave_ctas(true, wide, bytes, &wide_wave));
       if ((int)h->work.size() > wide_wave) continue;
       h->window_wide = true;
       h->window_threads = wide;
@@ -1520,7 +1535,7 @@ souffle_status souffle_gpu_autotune(souffle_gpu_system* h, int32_t trials, souff
   std::vector<std::pair<int, int>> cand;
   for (int subs : {1, 2, 3, 4, 6, 8})
     for (int thr : {96, 128, 192, 256}) {
-      if (force_smem_for(h, subs, thr) > 200 * 1024) continue;
+      if (!force_shape_ok(h, subs, thr)) continue;
       if (subs * np * 2 > 4 * thr) continue;  // more than two passes per thread pair
       if (subs * np * 2 < thr / 2) continue;   // most of the CTA idle
       cand.emplace_back(subs, thr);
