@@ -583,9 +583,11 @@ souffle_status souffle_mlp_forward(souffle_mlp* h, const float* x_dev, int32_t m
   if (!h || !x_dev || !y_dev || m < 1 || m > h->cap) return fail(SOUFFLE_ERR_BAD_INPUT, "bad argument");
   MLP_TRY(cudaSetDevice(h->device));
   const int L = kLayers - 1;
-  if (mlp_fused_supported(h->n_in, h->width, h->out_pad[L]) && h->n_out % 4 == 0 &&
-      (reinterpret_cast<uintptr_t>(y_dev) & 15) == 0) {
-    // one kernel from the caller's FP32 rows to the caller's FP32 rows (its stores want 16-byte rows)
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(x_dev), ya = reinterpret_cast<uintptr_t>(y_dev);
+  const bool apart = xa + sizeof(float) * (size_t)m * h->n_in <= ya || ya + sizeof(float) * (size_t)m * h->n_out <= xa;
+  if (mlp_fused_supported(h->n_in, h->width, h->out_pad[L]) && h->n_out % 4 == 0 && (ya & 15) == 0 && apart) {
+    // one kernel from the caller's FP32 rows to the caller's FP32 rows (its stores want 16-byte rows, and
+    // a tile's may go out before another tile's input has been read)
     const __nv_bfloat16* w[4] = {h->wb[0].p, h->wb[1].p, h->wb[2].p, h->wb[3].p};
     const int ldw[4] = {h->in[0], h->in[1], h->in[2], h->in[3]};
     const float* b[4] = {h->b[0].p, h->b[1].p, h->b[2].p, h->b[3].p};

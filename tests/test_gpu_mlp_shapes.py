@@ -43,3 +43,28 @@ def test_forward_shapes(n_in, width, n_out, m, off):
     ref = M.forward(p, x[rows], n_in, width, n_out, emulate=True)
     assert np.isfinite(got).all()
     assert np.abs(got[rows] - ref).max() <= 2e-2 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n_in,n_out,x_at,y_at", [
+    (32, 64, 0, 0),          # output rows longer than input rows, from the same place
+    (64, 32, 0, 0), (48, 48, 0, 0),
+    (32, 64, 5000 * 64 - 4, 0), (64, 32, 0, 5000 * 64 - 4),   # a few elements shared
+    (32, 64, 5000 * 64, 0), (64, 32, 0, 5000 * 64),           # neighbours, not overlapping
+])
+def test_forward_between_overlapping_buffers(n_in, n_out, x_at, y_at):
+    """Input and output rows that share memory: bitwise the result of separate buffers."""
+    torch = pytest.importorskip("torch")
+    from souffle_gb300 import gpu
+    m = 5000
+    torch.manual_seed(n_in + n_out)
+    x = torch.randn(m, n_in, device="cuda")
+    want = torch.empty(m, n_out, device="cuda")
+    net = gpu.Mlp(n_in, n_out, m, seed=3, width=128)
+    buf = torch.zeros(m * 128, device="cuda")
+    xs, ys = buf[x_at:x_at + m * n_in], buf[y_at:y_at + m * n_out]
+    xs.copy_(x.reshape(-1))
+    torch.cuda.synchronize()
+    net.forward(x.data_ptr(), m, want.data_ptr())
+    net.forward(xs.data_ptr(), m, ys.data_ptr())
+    torch.cuda.synchronize()
+    assert torch.equal(ys.reshape(m, n_out), want)
