@@ -572,6 +572,31 @@ cudaError_t launch_window_steps(souffle_gpu_system* h, int len, bool forces_firs
   return launch_window(force_args(h, 1, false), drift_args(h), q, (int)h->work.size(), h->window_threads, h->window_smem, h->stream);
 }
 
+// A graph of `len` steps: one window where the handle takes them, else the steps' kernels.  judge_mask: the
+// steps after which the surrogate is judged.
+cudaError_t capture_steps(souffle_gpu_system* h, int len, bool rebuild_first, unsigned long long judge_mask, cudaGraphExec_t* out) {
+  cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  cudaError_t launched = cudaSuccess;
+  if (len > 1 && window_usable(h)) {
+    if (rebuild_first) {
+      launch_drift_all(h);
+      launch_rebuild(h);
+      if (h->deal_ok) launch_deal(deal_args(h), h->stream);
+    }
+    launched = launch_window_steps(h, len, rebuild_first);
+  } else {
+    for (int k = 0; k < len; k++) launch_step(h, k == 0 && rebuild_first, (judge_mask >> k) & 1ull);
+  }
+  cudaGraph_t g = nullptr;
+  e = cudaStreamEndCapture(h->stream, &g);
+  if (launched != cudaSuccess) e = launched;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 // Work items of up to `subs` subunits of one system each (one force-kernel CTA per item, in
 // system order), their partial-sum slots, the force kernel's shared memory, and `threads` threads
 // per CTA.  Cached graphs are dropped (their launch shapes change).  Items of more subunits than the
@@ -1430,24 +1455,8 @@ souffle_status souffle_gpu_md_enqueue(souffle_gpu_system* h, int64_t first_step,
     const std::pair<int, unsigned long long> key(2 * len + (rebuild_first ? 1 : 0), judge_mask);
     auto it = h->graphs.find(key);
     if (it == h->graphs.end()) {
-      cudaGraph_t g;
-      CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t launched = cudaSuccess;
-      if (len > 1 && window_usable(h)) {
-        if (rebuild_first) {
-          launch_drift_all(h);
-          launch_rebuild(h);
-          if (h->deal_ok) launch_deal(deal_args(h), h->stream);
-        }
-        launched = launch_window_steps(h, len, rebuild_first);
-      } else {
-        for (int k = 0; k < len; k++) launch_step(h, k == 0 && rebuild_first, (judge_mask >> k) & 1ull);
-      }
-      CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
-      CUDA_TRY(launched);
-      cudaGraphExec_t ge;
-      CUDA_TRY(cudaGraphInstantiate(&ge, g, 0));
-      cudaGraphDestroy(g);
+      cudaGraphExec_t ge = nullptr;
+      CUDA_TRY(capture_steps(h, len, rebuild_first, judge_mask, &ge));
       it = h->graphs.emplace(key, ge).first;
     }
     CUDA_TRY(cudaGraphLaunch(it->second, h->stream));
