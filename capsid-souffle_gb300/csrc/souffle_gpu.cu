@@ -530,6 +530,8 @@ bool window_usable(const souffle_gpu_system* h) {
     if (P.nbb > 0) return false;
   return true;
 }
+// whole rebuild periods up to this length are one graph
+constexpr int kMaxPeriod = 64;
 
 size_t force_smem_for(const souffle_gpu_system* h, int subs, int threads) {
   const TplLayout& L = h->L;
@@ -1464,7 +1466,7 @@ souffle_status souffle_gpu_md_enqueue(souffle_gpu_system* h, int64_t first_step,
   };
   while (a < end) {
     souffle_status s;
-    if (a % B == 0 && end - a >= B && B <= 64) {
+    if (a % B == 0 && end - a >= B && B <= kMaxPeriod) {
       s = run_graph(B, true);
       a += B;
     } else {
@@ -1533,6 +1535,65 @@ souffle_status souffle_gpu_md_scalars(souffle_gpu_system* h, int32_t system, dou
   return SOUFFLE_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// Mean microseconds per step over at least n steps of graphs of one rebuild period, no rebuild in them.
+souffle_status time_steps(souffle_gpu_system* h, int n, cudaEvent_t e0, cudaEvent_t e1, double* us) {
+  const int len = h->prm[0].build_freq, runs = (n + len - 1) / len;
+  if (h->deal_ok) launch_deal(deal_args(h), h->stream);
+  cudaGraphExec_t g = nullptr;
+  CUDA_TRY(capture_steps(h, len, false, 0, &g));
+  cudaError_t e = cudaGraphLaunch(g, h->stream);  // warm-up
+  if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
+  for (int k = 0; k < runs && e == cudaSuccess; k++) e = cudaGraphLaunch(g, h->stream);
+  if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
+  if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+  cudaGraphExecDestroy(g);
+  CUDA_TRY(e);
+  float ms = 0;
+  CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+  *us = 1e3 * ms / ((double)runs * len);
+  return check_err(h);
+}
+
+// What timing at the current positions overwrites: the forces of the last step, which the next one starts
+// from, and, where steps are timed, velocities, kicks and thermostat, all zero so that nothing moves.
+struct SavedState {
+  DevBuf<long long> vel, force, kick;
+  DevBuf<SysState> state;
+  template <class T>
+  static cudaError_t copy(T* to, const T* from, size_t n, cudaStream_t st) {
+    return cudaMemcpyAsync(to, from, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
+  }
+  souffle_status save(souffle_gpu_system* h, bool rest) {
+    CUDA_TRY(vel.alloc(h->vel.n));
+    CUDA_TRY(force.alloc(h->force.n));
+    CUDA_TRY(kick.alloc(h->kick_c.n));
+    CUDA_TRY(state.alloc(h->d_state.n));
+    CUDA_TRY(copy(vel.p, h->vel.p, vel.n, h->stream));
+    CUDA_TRY(copy(force.p, h->force.p, force.n, h->stream));
+    CUDA_TRY(copy(kick.p, h->kick_c.p, kick.n, h->stream));
+    CUDA_TRY(copy(state.p, h->d_state.p, state.n, h->stream));
+    if (!rest) return SOUFFLE_OK;
+    CUDA_TRY(cudaMemsetAsync(h->vel.p, 0, sizeof(long long) * vel.n, h->stream));
+    CUDA_TRY(cudaMemsetAsync(h->kick_c.p, 0, sizeof(long long) * kick.n, h->stream));
+    CUDA_TRY(cudaMemsetAsync(h->d_state.p, 0, sizeof(SysState) * state.n, h->stream));
+    return SOUFFLE_OK;
+  }
+  souffle_status put_back(souffle_gpu_system* h) {
+    CUDA_TRY(copy(h->vel.p, vel.p, vel.n, h->stream));
+    CUDA_TRY(copy(h->force.p, force.p, force.n, h->stream));
+    CUDA_TRY(copy(h->kick_c.p, kick.p, kick.n, h->stream));
+    CUDA_TRY(copy(h->d_state.p, state.p, state.n, h->stream));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return SOUFFLE_OK;
+  }
+};
+}  // namespace
+
+extern "C" {
+
 souffle_status souffle_gpu_autotune(souffle_gpu_system* h, int32_t trials, souffle_tuning* out) {
   if (!h || trials < 1 || trials > 1000) return fail(SOUFFLE_ERR_BAD_INPUT, "bad argument");
   if (!h->have_state) return fail(SOUFFLE_ERR_STATE, "no state set");
@@ -1555,33 +1616,46 @@ souffle_status souffle_gpu_autotune(souffle_gpu_system* h, int32_t trials, souff
   launch_rebuild(h);
   souffle_status s = check_err(h);
   if (s != SOUFFLE_OK) return s;
+  // Where the default shape's steps run in windows, whole periods of steps are timed (a shape with too many
+  // items loses the window, by which 64 subunits take half the time), else the force kernel alone.
+  if ((s = plan_work(h, def_subs, def_threads)) != SOUFFLE_OK) return s;
+  const bool steps = window_usable(h) && h->prm[0].build_freq > 1 && h->prm[0].build_freq <= kMaxPeriod;
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
+  SavedState saved;
+  if ((s = saved.save(h, steps)) != SOUFFLE_OK) return s;
   double best = 1e30, def_us = 0;
   std::pair<int, int> best_shape = cand.front();
   for (auto& c : cand) {
     if ((s = plan_work(h, c.first, c.second)) != SOUFFLE_OK) break;
-    for (int k = 0; k < 3; k++) launch_forces_all(h, 0, false);
-    cudaEventRecord(e0, h->stream);
-    for (int k = 0; k < trials; k++) launch_forces_all(h, 0, false);
-    cudaEventRecord(e1, h->stream);
-    if (cudaEventSynchronize(e1) != cudaSuccess) {
-      s = fail(SOUFFLE_ERR_CUDA, "event synchronize failed");
-      break;
+    double us = 0;
+    if (steps) {
+      if ((s = time_steps(h, trials, e0, e1, &us)) != SOUFFLE_OK) break;
+    } else {
+      for (int k = 0; k < 3; k++) launch_forces_all(h, 0, false);
+      cudaEventRecord(e0, h->stream);
+      for (int k = 0; k < trials; k++) launch_forces_all(h, 0, false);
+      cudaEventRecord(e1, h->stream);
+      if (cudaEventSynchronize(e1) != cudaSuccess) {
+        s = fail(SOUFFLE_ERR_CUDA, "event synchronize failed");
+        break;
+      }
+      if ((s = check_err(h)) != SOUFFLE_OK) break;
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      us = 1e3 * ms / trials;
     }
-    if ((s = check_err(h)) != SOUFFLE_OK) break;
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    const double us = 1e3 * ms / trials;
     if (c.first == def_subs && c.second == def_threads) def_us = us;
     if (us < best) {
       best = us;
       best_shape = c;
     }
   }
-  // The default shape stays unless another is clearly faster: the search times forces-only
-  // launches, and differences of a few percent there are within run-to-run noise.
+  const souffle_status back = saved.put_back(h);
+  if (s == SOUFFLE_OK) s = back;
+  // The default shape stays unless another is clearly faster: differences of a few percent are within
+  // run-to-run noise.
   if (def_us > 0 && best > 0.97 * def_us) {
     best = def_us;
     best_shape = std::make_pair(def_subs, def_threads);

@@ -285,7 +285,7 @@ class GpuSystem:
         return (tf, sf, bf) if parts else tf
 
     def autotune(self, trials: int = 20) -> dict:
-        """Measure the force kernel at every candidate CTA shape and keep the fastest."""
+        """Measure the steps or the force kernel at every candidate CTA shape and keep the fastest."""
         t = Tuning_()
         _check(self.lib.souffle_gpu_autotune(self.h, trials, C.byref(t)))
         return {f: getattr(t, f) for f, _ in Tuning_._fields_}

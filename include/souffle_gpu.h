@@ -229,13 +229,15 @@ typedef struct souffle_kernel_times {
 souffle_status souffle_gpu_md_profile(souffle_gpu_system* h, int64_t first_step, int32_t n_steps,
                                       souffle_kernel_times* out);
 
-/* Autotuner (no reference counterpart): times the force kernel (forces only, no state change) at
- * every candidate CTA shape -- subunits per CTA and threads per CTA -- over the handle's current
- * state, keeps the fastest, and reports it.  trials = timed launches per shape.  The chosen shape
- * can be passed back through souffle_options to skip the search next time. */
+/* Autotuner (no reference counterpart): times every candidate CTA shape -- subunits per CTA and
+ * threads per CTA -- over the handle's current state, keeps the fastest, and reports it.  Where a
+ * rebuild period of the default shape's steps is one launch, steps at rest are timed (the state is put
+ * back), else the force kernel (forces only, no state change).  trials = timed steps or launches per
+ * shape, at least.  The chosen shape can be passed back through souffle_options to skip the search next
+ * time. */
 typedef struct souffle_tuning {
   int32_t subunits_per_cta, threads_per_cta;
-  double forces_us;          /* mean force-kernel time of the chosen shape */
+  double forces_us;          /* mean force-kernel (or step) time of the chosen shape */
   double default_forces_us;  /* the same for the default shape */
   int32_t candidates;        /* shapes measured */
 } souffle_tuning;

@@ -73,3 +73,34 @@ def test_a_wait_that_runs_out_is_reported_and_the_state_has_to_be_set_again(temp
     s.md_steps(0, 30)
     for x, y in zip(want, result(s, 1)):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("template,subs,over", [
+    ("patch_n3", [20], {}), ("bilayer_n5", [64], {}), ("bilayer_n5", [1700], {}), ("bilayer_n5", [5, 17, 2], {}),
+    ("bilayer_n5", [33], {"D": "b", "d": 100.0}), ("bilayer_n5", [3000], {})])
+@pytest.mark.parametrize("begun", [False, True])
+def test_autotune_keeps_the_windows_and_the_state(template, subs, over, begun):
+    """The shape is chosen by the steps that the handle takes: one that cannot take windows never wins over
+    one that can, and the steps timed leave no trace."""
+    ws = [workloads.make(geometry.template_by_name(template), S, seed=40 + S, **over) for S in subs]
+    a, b = handle(ws), handle(ws)
+    if begun:
+        a.md_steps(0, 10)
+        b.md_steps(0, 10)
+    else:
+        for s in (a, b):
+            s.set_state(np.concatenate([w.state.pos for w in ws]), np.concatenate([w.state.vel for w in ws]))
+    polls = b.lib.souffle_gpu_window_polls
+    polls.argtypes, polls.restype = [gpu.C.c_void_p, gpu.C.c_uint32], gpu.C.c_int32
+    had = polls(b.h, 1 << 22)
+    t = b.autotune(trials=20)
+    print(t, had, polls(b.h, 1 << 22))
+    assert t["candidates"] >= 3 and 0 < t["forces_us"] <= t["default_forces_us"]
+    assert (polls(b.h, 1 << 22) > 0) == (had > 0)
+    if not begun:
+        a.md_begin()
+        b.md_begin()
+    a.md_steps(10, 20)
+    b.md_steps(10, 20)
+    for x, y in zip(result(a, len(ws)), result(b, len(ws))):
+        assert np.array_equal(x, y)
