@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
       }
     }
-    if (!ok) {
+    if (!warp_agrees(ok)) {
       // MMAs issued before the timeout may still be writing tensor memory: wait (bounded) for
       // them before the CTA releases it
       if (elect_one()) {
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, it++) {
       const int b = it & 1;
       const int m0 = (t / n_tiles) * kBM, n0 = (t % n_tiles) * BN;
-      if (!mbar_wait(tfull0 + 8 * b, (uint32_t)(it >> 1) & 1u)) {
+      if (!warp_agrees(mbar_wait(tfull0 + 8 * b, (uint32_t)(it >> 1) & 1u))) {
         atomicOr(e.err, e.err_bit);
         break;
       }
@@ -483,13 +483,13 @@ __global__ void __launch_bounds__(kDwThreads, 1)
       }
       __syncwarp();
     }
-    if (!ok) {
+    if (!warp_agrees(ok)) {
       if (lane == 0) atomicOr(d.err, 1u);
       mbar_wait(done, 0);  // (bounded) MMAs issued so far may still be writing tensor memory
     }
   } else if (warp >= 4) {
     const int quarter = warp & 3;
-    if (mbar_wait(done, 0)) {
+    if (warp_agrees(mbar_wait(done, 0))) {
       tc_fence_after();
       const DwLayer& y = d.layer[l];
       const int row = m0 + quarter * 32 + lane;

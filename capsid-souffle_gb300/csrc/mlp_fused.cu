@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         epi_par ^= 1u;
       }
     }
-    if (!ok) {
+    if (!warp_agrees(ok)) {
       // MMAs issued before the failure may still be running: drain them (bounded) before the
       // tensor memory is released
       if (elect_one()) {
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
           const int i = nslots * p + s;
           if (i >= my_tiles) continue;
           if (((l + s) & 1) != grp) continue;
-          if (!fwait(accfull0 + 16 * s + 8 * (l & 1), (uint32_t)(l >> 1) & 1u, abort_flag)) {
+          if (!warp_agrees(fwait(accfull0 + 16 * s + 8 * (l & 1), (uint32_t)(l >> 1) & 1u, abort_flag))) {
             ok = false;
             break;
           }
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         }
       }
       // the slot's previous tile has finished its output layer (its MMAs read the buffer)
-      if (use > 0 && !fwait(xfree0 + 8 * s, (uint32_t)(use - 1) & 1u, abort_flag)) {
+      if (use > 0 && !warp_agrees(fwait(xfree0 + 8 * s, (uint32_t)(use - 1) & 1u, abort_flag))) {
         ok = false;
         break;
       }

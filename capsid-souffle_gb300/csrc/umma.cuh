@@ -17,6 +17,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// Bounded waits end lane by lane, so a warp whose wait ran out agrees on it before the next instruction that
+// needs all lanes (elect.sync, tcgen05.ld and the barriers): true when every lane's wait succeeded.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // One lane of a converged warp.  The tensor-core instructions are issued inside such a branch of
 // code that the whole warp runs: their operands then stay in uniform registers.  Issued from a
 // branch on lane == 0, whose operands the compiler keeps in per-lane registers, each
