@@ -1,10 +1,9 @@
 // Energy block of run_simulation (src/md.cpp:553-605), evaluated in FP64.
 //
-//   k_energy_bonded   BEAD::update_stretching_energy (src/bead.cpp:9-14),
-//                     EDGE::update_bending_energy (src/edge.cpp:51-67),
-//                     BEAD::update_kinetic_energy (src/bead.h:129-131)
-//   k_energy_sub      the bonded terms, kinetic energies and intra-subunit pairs of a few subunits
-//                     per CTA, and every subunit's bounding sphere
+//   k_energy_sub      the bonded terms (BEAD::update_stretching_energy, src/bead.cpp:9-14;
+//                     EDGE::update_bending_energy, src/edge.cpp:51-67), kinetic energies
+//                     (BEAD::update_kinetic_energy, src/bead.h:129-131) and intra-subunit pairs of a
+//                     few subunits per CTA, and every subunit's bounding sphere
 //   k_energy_inter    pairs j > i of beads in different subunits, CTA per subunit, over the
 //                     subunits whose spheres come within the reach of the pair terms
 //   k_energy_pairs    update_LJ_ES_energies_simplified (src/energies.cpp:24-93) without a DH
@@ -355,9 +354,11 @@ __global__ void __launch_bounds__(256) k_energy_sub(EnergyArgs a) {
 // Pairs of beads in different subunits, CTA (four warps) per half of the beads (rows) of subunit i
 // (all of them up to 16 beads): partners in subunits j > i
 // whose bounding spheres come within the reach of the pair terms.  Candidate subunits come from a
-// scan of all j > i (threads along j, 16 coalesced bytes each) up to kEnergyScan subunits -- 2000
-// subunits are two rounds of loads, less than the launches that build a grid -- and from the cells
-// of the subunit centres within reach beyond.  A candidate's beads are staged in shared memory;
+// scan of all j > i (threads along j, 16 coalesced bytes each) up to kEnergyScan subunits, and from the
+// cells of the subunit centres within reach beyond.  A call with the scan against one with the cells (four
+// launches to build them): 153 and 179 us at 1,000 subunits, 213 and 242 at 2,000, 341 and 362 at 4,000, 490
+// and 500 at 6,000, 638 and 617 at 8,000, 972 and 870 at 12,000, 1,353 and 1,121 at 16,000; so the lines
+// cross near 7,000, below where kEnergyScan has the change.  A candidate's beads are staged in shared memory;
 // every (row, 32 partners) item of the block passes an FP32 test with a margin at once, the hits
 // are listed row by row, and the FP64 terms run 128 listed pairs at a time, each row's terms then
 // summed with a fixed tree: deterministic.  Few pairs (147,000 at 84,000 beads) behind long

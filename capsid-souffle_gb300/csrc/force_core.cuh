@@ -188,8 +188,11 @@ struct DealtBeads {
 struct ForceQueue {
   int next, n_long, n_full, n_short;
 };
-constexpr int kPiece = 16;    // pairs of a piece
-constexpr int kLongRow = 48;  // lists above this length are one piece, for a whole warp
+constexpr int kPiece = 16;    // pairs of a piece: two for each of eight lanes
+// Lists above this length are one piece, for a whole warp (m.rows has room for three pieces).
+// From 32 or 16 pairs on instead: 64 subunits 1,390 -> 1,414 and 1,515 us per 100 steps, 2,000 of them
+// 3,190 -> 3,337 and 3,391, 64 replicas 5,485 -> 5,910 and 6,420 per 20 steps.
+constexpr int kLongRow = 48;
 
 // The beads' inter-subunit lists in pieces into m.rows: whole lists above kLongRow pairs (at 0 ..),
 // pieces of 9 to 16 pairs (at nbead ..) and of at most 8 (from 4 nbead down), each as

@@ -950,7 +950,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 256, kWide ? 2 : 5) k_window(For
 }
 
 // Host state in: double positions to 64-bit fixed point, the high-word copy, velocities to
-// 2^-32 fixed point.
+// 2^-40 fixed point.
 __global__ void k_state_in(StateArgs a) {
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.n) return;

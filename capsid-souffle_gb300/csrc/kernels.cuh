@@ -40,7 +40,7 @@ struct PairArgs {
   const SysParams* sys;
   const int* sub_sys;
   const float* q;       // [np] template charges (only q != 0 matters)
-  int np, words, n_beads_total;
+  int np, words;
   const int* cand;
   const int* cand_count;
   int cand_cap;
@@ -76,14 +76,13 @@ struct ForceArgs {
   const int* inter_count;
   int inter_cap;
   const float* dh_w;         // [n_sys * np] q * exp(kappa sigma/2)/(1 + kappa sigma/2) * sqrt(lb)
-  const PairTable* pt;
   const dfloat* inv_mass;    // [np] 1 / m as double-float (kick coefficients)
-  long long* kick_c;         // [n_sys * np] dt sqrt(expfac) / (2 m) * 2^62, written by the last CTA
+  long long* kick_c;         // [n_sys * np] dt sqrt(expfac) / (2 m) * 2^64, written at a step's end
   long long* fx; long long* fy; long long* fz;   // force, 2^-32 units
-  long long* vx; long long* vy; long long* vz;   // velocity, 2^-32 units
+  long long* vx; long long* vy; long long* vz;   // velocity, 2^-40 units
   float* sfx; float* sfy; float* sfz;   // optional stretching force out
   float* bfx; float* bfy; float* bfz;   // optional bending force out
-  long long* partial;        // [systems * 4] running KE and momentum sums (2^-32), zero between launches
+  long long* partial;        // [systems * 4] running KE (2^-32) and momentum (2^-40) sums, zero between launches
   unsigned int* err;
   int n_beads_total;
   int max_sub;               // subunits per CTA (shared-memory sizing)
@@ -173,7 +172,7 @@ struct EnergyArgs {
   const SysState* state;
   const long long* px; const long long* py; const long long* pz;
   const int4* pos32;
-  const long long* vx; const long long* vy; const long long* vz;   // 2^-32 units
+  const long long* vx; const long long* vy; const long long* vz;   // 2^-40 units
   const double* len0;      // [ne]
   const double* mass;      // [np]
   const double* q;         // [np]
@@ -226,7 +225,7 @@ void launch_cells_count(const CellArgs& a, int grid, int block, cudaStream_t s);
 void launch_cells_place(const CellArgs& a, cudaStream_t s);
 void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s);
 void launch_cells_sort(const CellArgs& a, cudaStream_t s);
-void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s);
+void launch_candidates(const CandArgs& a, cudaStream_t s);
 void launch_pairs(const PairArgs& a, int n_sub, bool search, cudaStream_t s);
 // k_pairs finds the candidates itself (no k_cells_* and k_candidates before it)
 bool pairs_search(int max_sub, int cand_cap);

@@ -189,8 +189,8 @@ __device__ __noinline__ bool pair_exact(const long long* px, const long long* py
 }
 
 // The pair lists of subunit i, one CTA of 128 threads (64 when the candidates are given and a block
-// has at most 96 items: many subunits, so throughput counts).  Candidates are taken in ascending j, so
-// each row's entries come out in ascending global id.
+// has at most 96 items: launch_pairs).  Candidates are taken in ascending j, so each row's entries come
+// out in ascending global id.
 //   search   (kSearch: systems of at most kSearchSubs subunits) the candidates by testing every
 //            subunit of the system, in order; otherwise they come from k_candidates
 //   stage    a chunk of candidates that stay in the pair list (far ones skipped by a warp ballot),
@@ -478,14 +478,12 @@ void launch_cells_scatter(const CellArgs& a, int grid, int block, cudaStream_t s
   k_cells_scatter<<<grid, block, 0, s>>>(a);
 }
 void launch_cells_sort(const CellArgs& a, cudaStream_t s) { k_cells_sort<<<(a.total_cells + 127) / 128, 128, 0, s>>>(a); }
-void launch_candidates(const CandArgs& a, int grid, int block, cudaStream_t s) {
-  (void)grid;
-  (void)block;
+void launch_candidates(const CandArgs& a, cudaStream_t s) {
   const int warps_per_block = 4;
   const int g = (a.c.n_sub_total + warps_per_block - 1) / warps_per_block;
   k_candidates<<<g, 32 * warps_per_block, sizeof(int) * warps_per_block * a.cap, s>>>(a);
 }
-// About 8 KB of staging per CTA (9 candidates of 42 beads), so that a one-wave grid of CTAs still
+// About 10 KB of staging per CTA (8 candidates of 42 beads), so that a one-wave grid of CTAs still
 // fits the shared memory of an SM.
 int pair_chunk(int np, int words) {
   const int per = np * (int)(sizeof(int4) + sizeof(unsigned int) * words + sizeof(int));
@@ -500,6 +498,12 @@ static size_t pair_smem_base(int np, int words, int chunk) {
 // beyond, and for the surrogate, which classifies the candidates first, they come from the cell grid.
 bool pairs_search(int max_sub, int cand_cap) { return max_sub <= kSearchSubs && cand_cap <= 4096; }
 size_t pair_smem_bytes(int np, int words, int chunk) { return pair_smem_base(np, words, chunk) + sizeof(int) * 4096; }
+// Candidates are given to systems of more than kSearchSubs subunits.  A block with few (row, word) items
+// leaves most of 128 threads idle in the search for pairs, and with many subunits the SMs are better
+// filled by more CTAs: a whole rebuild with 64 threads against 128, at 42 beads 136 and 147 us (20,000
+// subunits), at 10 beads 39 and 42 (3,000), 83 and 102 (20,000), 251 and 337 (80,000); 128 are ahead
+// below some 2,500 subunits (42 beads: 46 and 43 us at 2,000, 44 and 38 at 1,100).  With 60 to 100
+// beads (128 items and more) the two are alike.
 void launch_pairs(const PairArgs& a, int n_sub, bool search, cudaStream_t s) {
   const size_t smem = pair_smem_base(a.np, a.words, a.chunk);
   if (search) k_pairs<true><<<n_sub, 128, smem + sizeof(int) * a.cand_cap, s>>>(a);

@@ -41,7 +41,6 @@ struct TplLayout {
   int o_bendf;        // [nbend*2] face0, face1
   int o_bead_edges;   // [np*maxdeg] edge index (| 1 << 16 where the bead is the edge's second) or -1
   int o_bead_roles;   // [np*maxrole] bend*4+role or -1
-  int o_type;         // [np]
   int o_species;      // [np]
   int n_int;          // ints that the force kernels stage (o_bend, o_bendf, o_face, o_edge, o_bead_*, o_species)
   // float buffer offsets
@@ -155,7 +154,6 @@ struct WorkItem {
 struct PairTable {
   float sig6[kMaxSpecies * kMaxSpecies];   // sigma_i^6 (attractive) or shc^6 (WCA)
   float cut2[kMaxSpecies * kMaxSpecies];   // ecut^2 (attractive) or (1.12246205 shc)^2
-  float skip2[kMaxSpecies * kMaxSpecies];  // max(ecut^2, (1.12246205 shc)^2): beyond it no LJ
 };
 
 // Error flags raised by kernels and read by the host.
@@ -199,7 +197,7 @@ __device__ inline float hi_diff(int a, int b, float unit) {
 
 // ---- 64-bit fixed point without FP64 instructions -------------------------------------------
 // GB300 runs FP64 at a small fraction of its FP32 rate, so per-bead integration is done in
-// integers: velocities and forces are int64 in units of 2^-32, positions int64 in units of
+// integers: velocities are int64 in units of 2^-40, forces of 2^-32, positions of
 // L/2^64, and every product is an exact 64x64->128 multiply rounded to nearest.
 
 // round(a * b / 2^s) for 0 < s < 64, exact (128-bit product, ties away from zero is not needed:

@@ -212,8 +212,6 @@ souffle_status upload(souffle_gpu_system* h) {
   ti.insert(ti.end(), T.species.begin(), T.species.end());
   while (ti.size() % 4) ti.push_back(0);
   L.n_int = (int)ti.size();
-  L.o_type = (int)ti.size();
-  ti.insert(ti.end(), T.type.begin(), T.type.end());
   L.nspecies = T.nspecies;
   // directed attraction (src/forces.cpp:119-125) and the type-7 epsilon (src/forces.cpp:127)
   L.type7_bits = 0;
@@ -235,7 +233,6 @@ souffle_status upload(souffle_gpu_system* h) {
       const bool att = (L.lj_att_bits[a] >> b) & 1;
       pt.sig6[idx] = (float)(att ? std::pow(s1, 6) : std::pow(shc, 6));
       pt.cut2[idx] = (float)(att ? ecut * ecut : replj2 * shc * shc);
-      pt.skip2[idx] = (float)std::max(ecut * ecut, replj2 * shc * shc);
     }
   L.o_len0 = (int)tf.size();
   for (double v : T.len0) tf.push_back((float)v);
@@ -365,7 +362,6 @@ void launch_candidates_all(souffle_gpu_system* h) {
   cudaStream_t st = h->stream;
   CellArgs c = cell_args(h);
   launch_subunit_cells(h);
-  const int tb = 128, gb = (h->S + tb - 1) / tb;
   CandArgs ca{};
   ca.c = c;
   ca.pos32 = h->pos32.p;
@@ -373,7 +369,7 @@ void launch_candidates_all(souffle_gpu_system* h) {
   ca.cand = h->cand.p;
   ca.cand_count = h->cand_count.p;
   ca.err = h->err.p;
-  launch_candidates(ca, gb, tb, st);
+  launch_candidates(ca, st);
 }
 
 void launch_rebuild(souffle_gpu_system* h) {
@@ -392,7 +388,6 @@ void launch_rebuild(souffle_gpu_system* h) {
   pa.np = h->tpl.np;
   pa.words = h->L.words;
 
-  pa.n_beads_total = (int)h->N;
   pa.cand = h->cand.p;
   pa.cand_count = h->cand_count.p;
   pa.cand_cap = h->cand_cap;
@@ -426,7 +421,6 @@ ForceArgs force_args(souffle_gpu_system* h, int mode, bool want_parts) {
   a.inter_count = h->inter_count.p;
   a.inter_cap = h->inter_cap;
   a.dh_w = h->dh_w.p;
-  a.pt = h->pt.p;
   a.inv_mass = h->inv_mass.p;
   a.kick_c = h->kick_c.p;
   const int64_t N = h->N;

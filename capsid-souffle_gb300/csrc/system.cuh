@@ -81,7 +81,7 @@ struct souffle_gpu_system {
   DevBuf<int> d_sub_sys, d_bead_sys;
   DevBuf<long long> pos_fx;
   DevBuf<int4> pos32;
-  DevBuf<long long> vel, force, partial, kick_c;   // 2^-32 fixed point
+  DevBuf<long long> vel, force, partial, kick_c;   // fixed point: 2^-40, 2^-32, sums of both, 2^-64
   DevBuf<float> sbforce;
   DevBuf<double> staging;
   DevBuf<unsigned int> intra_mask;
@@ -89,7 +89,7 @@ struct souffle_gpu_system {
   DevBuf<int> cand, cand_count;
   DevBuf<int> cell_count, cell_start, sub_rank, sub_cell, cell_subs;
   DevBuf<float> dh_w;
-  DevBuf<PairTable> pt;
+  DevBuf<PairTable> pt;   // (the surrogate; the force kernels read their template tables)
   DevBuf<dfloat> inv_mass;
   DevBuf<double> mass_d, q_d, sigma_d, len0_d;
   DevBuf<int> type_d, lj_d;
