@@ -707,7 +707,15 @@ souffle_status enqueue(souffle_analysis* h, AnLane* w, const double* pos, const 
   return SOUFFLE_OK;
 }
 
-// Waits for the copy stream and both streams of every lane; the first error.
+// Waits for the frames in the lanes: a lane's stream ends behind its copies and its pair correlation.
+cudaError_t wait_lanes(souffle_analysis* h) {
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < h->lanes && e == cudaSuccess; k++) e = cudaStreamSynchronize(h->lane[k]->st);
+  return e;
+}
+
+// Waits for the copy stream and both streams of every lane, whatever part of a frame is in them; the
+// first error.
 cudaError_t drain(souffle_analysis* h) {
   cudaError_t e = cudaStreamSynchronize(h->copy_st);
   for (int k = 0; k < h->lanes; k++)
@@ -873,8 +881,9 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
   AN_CHECK(cudaSetDevice(h->dev));
   const AnParams& P = h->P;
   const size_t N = (size_t)P.N, S = (size_t)P.S, bins = (size_t)P.bins;
-  // nothing enqueued earlier still reads the input or works in the lanes
-  AN_CHECK(drain(h));
+  // nothing enqueued earlier still reads the input or works in the lanes (only lane 0 takes work that a
+  // call leaves behind)
+  AN_CHECK(cudaStreamSynchronize(h->lane[0]->st));
   DrainOnExit guard{h};
   if (n_frames > 1 && h->chunk > 1 && h->lanes == 1 && !h->no_second) {
     if (alloc_lane(h->lane[1], P) == cudaSuccess) {
@@ -913,7 +922,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
       if ((s = analyse(lane, k)) != SOUFFLE_OK) return s;
       AN_CHECK(cudaEventRecord(h->lane[lane]->done, h->lane[lane]->st));
     }
-    AN_CHECK(drain(h));
+    AN_CHECK(wait_lanes(h));
     int good = 0;  // frames analysed without an error: their results are returned whatever follows
     bool again = false;
     for (; good < nf; good++) {
@@ -924,7 +933,7 @@ souffle_status souffle_analysis_frames(souffle_analysis* h, int64_t n_frames, co
         again = true;
         if ((s = copy_in(f0 + good, 0)) != SOUFFLE_OK) return s;
         if ((s = analyse(0, good)) != SOUFFLE_OK) return s;
-        AN_CHECK(drain(h));
+        AN_CHECK(wait_lanes(h));
         s = frame_status(h, good);
       }
       if (s != SOUFFLE_OK) break;
