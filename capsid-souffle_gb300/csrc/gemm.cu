@@ -359,7 +359,7 @@ cudaError_t launch_act(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, 
 // All layers' weight gradients, the bias sums and the loss in one launch.  A layer is one to four
 // 128 x 128 tiles with K the whole batch (4096 rows), so one GEMM per layer kept one to six SMs busy for
 // 20 us, and the bias sums took another 7 us launch each.  Here a tile is 128 x 32, so that all layers
-// together are up to 58 CTAs, and the bias rows are CTAs beside them.  A narrower tile costs re-reads of
+// together are 18 CTAs (64-128-128-128-132) or 52 (256 wide), and the bias rows are CTAs beside them.  A narrower tile costs re-reads of
 // A from L2 and idle tensor columns, but what bounds a CTA is its K steps one after the other; splitting
 // the batch over CTAs as well was 3 us faster, but changes the order of the sums, and with it every
 // trained network.  A gradient call of 4096 rows: 307 us with a launch per layer and sum, 104 us now.

@@ -27,9 +27,10 @@
 //                   input buffer by ordinary stores
 //
 // What bounds it (118,016 rows, w = 128, clock64 marks): per 64-wide K stage the issuer needs about
-// 480 cycles where the MMAs compute for 256 -- their operands' 8 KB per K = 16 step are exactly
-// what shared memory delivers, and the epilogue's stores compete -- and the output layer's units
-// take 5,000 to 6,000 cycles.  65.7 us before: issue from a lane == 0 branch (230 cycles per MMA),
+// 480 cycles where the MMAs compute for 256, and the output layer's units take 5,000 to 6,000 cycles.
+// Counters name no saturated unit (tensor pipe 14 % of the elapsed cycles, LSU part of the l1tex data
+// pipe 42 %, issue 37 %, MUFU 16 %), but do not show the MMAs' operand reads: that these (8 KB per K =
+// 16 step, what shared memory delivers while it computes) and the epilogue's stores compete is inferred.  65.7 us before: issue from a lane == 0 branch (230 cycles per MMA),
 // two slots, one epilogue group, output rows stored one row per lane (7,000 to 9,000 cycles per
 // tile); 36.4 us now, w = 256 100.5 -> 69.0 us.  With FP32 rows in and out (souffle_mlp_forward)
 // a packing and an unpacking kernel, 41 and 47 us, went too: 168 -> 55.7 us per call.

@@ -179,7 +179,9 @@ souffle_status souffle_gpu_kinetic_energy(souffle_gpu_system* h, int32_t system,
 souffle_status souffle_gpu_md_begin(souffle_gpu_system* h);
 
 /* Run MD-loop iterations a = first_step .. first_step + n_steps - 1 for every
- * system (src/md.cpp:387-514).  Uses CUDA graphs for whole rebuild windows. */
+ * system (src/md.cpp:387-514).  Uses CUDA graphs for whole rebuild windows.  After
+ * SOUFFLE_ERR_CUDA because a bounded wait between the CTAs of a window ran out, the state is
+ * undefined: calls return SOUFFLE_ERR_STATE until souffle_gpu_set_state. */
 souffle_status souffle_gpu_md_steps(souffle_gpu_system* h, int64_t first_step, int32_t n_steps);
 
 /* souffle_gpu_md_steps without the wait: queues the same iterations on the handle's stream and

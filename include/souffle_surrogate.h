@@ -42,7 +42,8 @@ souffle_status souffle_mlp_set_params(souffle_mlp* h, const float* host_in, int6
 /* y_dev [m][n_out] = network(x_dev [m][n_in]); 1 <= m <= max_batch.  For n_in <= 64 and
  * n_out <= 256 the whole forward pass is one tensor-core kernel that keeps each 128-row tile's
  * activations on chip (SiLU through a hardware tanh approximation); other shapes run layer by
- * layer. */
+ * layer.  The two may overlap (the input is then packed first, as for output rows that are not
+ * 16-byte aligned). */
 souffle_status souffle_mlp_forward(souffle_mlp* h, const float* x_dev, int32_t m, float* y_dev);
 /* The same forward pass one GEMM per layer, activations through device memory (the path the
  * training steps use, with SiLU from an exponential and a division). */
