@@ -1553,31 +1553,33 @@ souffle_status time_steps(souffle_gpu_system* h, int n, cudaEvent_t e0, cudaEven
 
 // What timing at the current positions overwrites: the forces of the last step, which the next one starts
 // from, and, where steps are timed, velocities, kicks and thermostat, all zero so that nothing moves.
+// Velocities and forces go to the staging buffer.
 struct SavedState {
-  DevBuf<long long> vel, force, kick;
+  DevBuf<long long> kick;
   DevBuf<SysState> state;
   template <class T>
   static cudaError_t copy(T* to, const T* from, size_t n, cudaStream_t st) {
     return cudaMemcpyAsync(to, from, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
   }
+  static long long* vel(souffle_gpu_system* h) { return reinterpret_cast<long long*>(h->staging.p); }
+  static long long* force(souffle_gpu_system* h) { return vel(h) + h->vel.n; }
   souffle_status save(souffle_gpu_system* h, bool rest) {
-    CUDA_TRY(vel.alloc(h->vel.n));
-    CUDA_TRY(force.alloc(h->force.n));
+    static_assert(sizeof(long long) == sizeof(double), "staged as doubles");
     CUDA_TRY(kick.alloc(h->kick_c.n));
     CUDA_TRY(state.alloc(h->d_state.n));
-    CUDA_TRY(copy(vel.p, h->vel.p, vel.n, h->stream));
-    CUDA_TRY(copy(force.p, h->force.p, force.n, h->stream));
+    CUDA_TRY(copy(vel(h), h->vel.p, h->vel.n, h->stream));
+    CUDA_TRY(copy(force(h), h->force.p, h->force.n, h->stream));
     CUDA_TRY(copy(kick.p, h->kick_c.p, kick.n, h->stream));
     CUDA_TRY(copy(state.p, h->d_state.p, state.n, h->stream));
     if (!rest) return SOUFFLE_OK;
-    CUDA_TRY(cudaMemsetAsync(h->vel.p, 0, sizeof(long long) * vel.n, h->stream));
+    CUDA_TRY(cudaMemsetAsync(h->vel.p, 0, sizeof(long long) * h->vel.n, h->stream));
     CUDA_TRY(cudaMemsetAsync(h->kick_c.p, 0, sizeof(long long) * kick.n, h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_state.p, 0, sizeof(SysState) * state.n, h->stream));
     return SOUFFLE_OK;
   }
   souffle_status put_back(souffle_gpu_system* h) {
-    CUDA_TRY(copy(h->vel.p, vel.p, vel.n, h->stream));
-    CUDA_TRY(copy(h->force.p, force.p, force.n, h->stream));
+    CUDA_TRY(copy(h->vel.p, vel(h), h->vel.n, h->stream));
+    CUDA_TRY(copy(h->force.p, force(h), h->force.n, h->stream));
     CUDA_TRY(copy(h->kick_c.p, kick.p, kick.n, h->stream));
     CUDA_TRY(copy(h->d_state.p, state.p, state.n, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
