@@ -42,9 +42,10 @@ inline cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> hold(lock);
   size_t& limit = limits[{fn, dev}];
-  if (bytes <= limit) return cudaSuccess;
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) limit = bytes;
+  const size_t most = bytes > limit ? bytes : limit;
+  // (set again where it stands, too: a device that was reset has forgotten it)
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (e == cudaSuccess) limit = most;
   return e;
 }
 
